@@ -859,6 +859,39 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
     return out
 
 
+#: rows that one pass of ``gemm_split`` takes: bounds its scratch (six bytes a row and column of the input)
+GEMM_SPLIT_ROWS = 2048
+#: weights of at most this many rows (a router) stay with ``gemm_simt``, which has a kernel for them
+GEMM_SPLIT_MIN_OUT = 33
+
+
+def gemm_split_takes(w: torch.Tensor) -> bool:
+    """Whether ``gemm_split`` takes this weight (or part of one): bfloat16, rows on 16-byte borders for TMA."""
+    return (w.dtype == torch.bfloat16 and w.shape[0] >= GEMM_SPLIT_MIN_OUT and w.shape[1] % 8 == 0 and w.shape[1] > 0
+            and (w.shape[0] == 1 or w.stride(0) % 8 == 0) and w.data_ptr() % 16 == 0)
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``out[M, N] = a[M, K] @ w[N, K]^T`` with 32-bit ``a`` and ``out`` and a bfloat16 weight, on the tensor cores: every
+    number of ``a`` as the exact sum of three bfloat16 numbers, the sums taken in 32-bit (K a multiple of 8)."""
+    _check(a, "gemm input", torch.float32, 2)
+    ldw = _check_weight(w, "gemm weight", torch.bfloat16)
+    _check(out, "gemm output", torch.float32, 2)
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or tuple(out.shape) != (M, N):
+        raise KernelError(f"gemm: shapes do not fit: input {tuple(a.shape)}, weight {tuple(w.shape)}, output {tuple(out.shape)}")
+    if status is None:
+        status = status_word(a.device)
+    pieces = torch.empty((3, min(M, GEMM_SPLIT_ROWS), K), dtype=torch.bfloat16, device=a.device)
+    for first in range(0, M, GEMM_SPLIT_ROWS):
+        rows = min(GEMM_SPLIT_ROWS, M - first)
+        _call("gemm_split", "spy_gemm_split", _ptr(a[first:]), ctypes.c_longlong(K), _ptr(w), ctypes.c_longlong(ldw), _ptr(out[first:]), ctypes.c_longlong(N),
+              rows, N, K, _ptr(pieces), _ptr(status), _stream())
+        count_launches(1)                                     # the pieces, then the product
+    return out
+
+
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """``out[t, i] = silu(gate_up[t, i]) * gate_up[t, I + i]``; gate_up [T, 2I], out [T, I]."""
     _check(gate_up, "swiglu input", ndim=2)

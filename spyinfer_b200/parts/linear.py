@@ -1,8 +1,10 @@
 """``y = x @ W^T (+ b)`` for weights stored ``[out, in]``, as every projection of the model is.
 
 The kernel is chosen by storage types and shape: bfloat16 activations with bfloat16 weights
-go to the tcgen05 tensor-core kernel when it takes the shape, everything else (the float32
-path, 32-bit weights, odd shapes) to the 32-bit CUDA-core kernel.  The choice depends on the
+go to the tcgen05 tensor-core kernel when it takes the shape, 32-bit activations with bfloat16
+weights (the float32 path) to the tensor-core kernel that splits every activation into three exact
+bfloat16 pieces, everything else (32-bit weights, odd shapes, weights of a few rows) to the
+32-bit CUDA-core kernel.  The choice depends on the
 weight's shape only, never on the number of rows, so a token's result does not depend on the
 batch it is in.
 """
@@ -44,10 +46,11 @@ class Linear:
         self.out_features, self.in_features = weight.shape
         self.fast = (activation_dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
                      and kernels.tensor_core_gemm_takes(self.out_features, self.in_features))
+        self.split = not self.fast and activation_dtype == torch.float32 and kernels.gemm_split_takes(weight)
         self.prefetch_bytes = _prefetch_cap()
 
     def modules(self) -> List[str]:
-        return (["gemm_tcgen05"] if self.fast else ["gemm_simt"]) + (["swiglu"] if self.bias is not None else [])
+        return (["gemm_tcgen05"] if self.fast else (["gemm_split"] if self.split else []) + ["gemm_simt"]) + (["swiglu"] if self.bias is not None else [])
 
     def __call__(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None, epilogue: Optional[str] = None, defer: bool = False,
                  glu: Optional[tuple] = None) -> torch.Tensor:
@@ -71,7 +74,12 @@ class Linear:
         if epilogue is not None:
             raise ValueError("only the tensor-core product has fused epilogues")
         out = torch.empty((x.shape[0], self.out_features), dtype=out_dtype or x.dtype, device=x.device)
-        return kernels.gemm_simt(x, self.weight, out)
+        return self._plain(x, self.weight, out)
+
+    def _plain(self, x, w, out):
+        if self.split and x.dtype == torch.float32 and out.dtype == torch.float32:
+            return kernels.gemm_split(x, w, out)
+        return kernels.gemm_simt(x, w, out)
 
     def part(self, x: torch.Tensor, rows=None, cols=None, out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """The product with a part of the weight: ``rows = (first, end)`` of its output rows and/or ``cols = (first, end)`` of its
@@ -85,5 +93,7 @@ class Linear:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
         if self.fast and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0:
             return kernels.gemm_tcgen05(x, w, out=out)
-        return kernels.gemm_simt(x, w, out)
+        if self.split and not kernels.gemm_split_takes(w):
+            return kernels.gemm_simt(x, w, out)
+        return self._plain(x, w, out)
 
