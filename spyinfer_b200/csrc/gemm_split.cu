@@ -5,19 +5,25 @@
 //
 // The sums.  The tensor core adds into its accumulator by cutting, which leans toward zero a little at every step (measured:
 // 2.4e-8 of the result after 16 terms of K, 6.7e-8 after 64, 2.3e-7 after 256).  So the leading pieces' accumulator is taken
-// out of tensor memory every 32 terms of K and added to a sum in registers by an ordinary rounded addition; the other two pieces are 2^-8 and
-// 2^-16 of the size and are accumulated through.  Measured against 64 bits (random normals; relative 2-norm): see gemm_split's
-// test for the bound; at K = 4,096 2.0e-7 where the CUDA-core kernel, one chain over K, has 6.1e-7.
+// out of tensor memory every 32 terms of K and added to a sum in registers by an ordinary rounded addition; the other two
+// pieces are 2^-8 and 2^-16 of the size and are accumulated through.
+// Relative error (2-norm) against 64 bits at K = 96, 4,096 and 12,288: 0.7e-7, 1.6e-7 and 2.6e-7, where the CUDA-core kernel, one
+// chain over K, has 1.8e-7, 1.1e-6 and 2.0e-6.
 //
 // A row's result does not depend on M or on its neighbours: K is cut into slices by N and K alone (plan_slices), a slice's sum
 // runs over its chunks of 32 in order, and the slices are added in order.
 //
-// Bounds.  Few tokens: the weights' way through memory (2 bytes a weight; the CUDA-core kernel, 64 x 64 tiles with a
-// synchronous load a step, took 822 us a product at 4 tokens of the 8B layer sizes).  Many: the tensor cores (three passes).
+// Bounds.  Few tokens: the weights' way through memory (2 bytes a weight).  Many: the tensor cores (three passes).  Measured with
+// the pieces' kernel, from a graph, weights not in L2 (the CUDA-core kernel took 822 us a product on average at 4 tokens of these
+// sizes, 1,690 at 300):   N x K = 6,144 x 4,096: 15 us at 4 tokens, 81 at 300;   4,096 x 4,096: 13 and 68;   24,576 x 4,096: 39
+// (5.1 TB/s) and 221 (274 TFLOP/s of 32-bit product, three times that on the tensor cores);   4,096 x 12,288: 23 and 129;
+// 151,936 x 4,096: 202 (6.2 TB/s).
 // Tiles: up to 128 weight rows in the instruction's M slot and 16, 32 or 64 tokens in its N slot, each token three times (a
 // product with the leading pieces, N = BN, and one with the two others side by side, N = 2 BN), two blocks an SM up to 32
-// tokens so that enough weight bytes are under way; beyond 64 tokens 256 weight rows as two halves over 64 tokens, where
-// a stage's 56 KB feed 900 cycles of products and each half's sums are taken out while the other half multiplies.
+// tokens so that enough weight bytes are under way; beyond 64 tokens 256 weight rows as two halves over 64 tokens (56 KB a
+// stage for 24 products), where a half's sums are taken out while the other half multiplies.  A thread that waits, issues and
+// commits needs about 60 to 100 cycles for each, more than these small products take, so the leading and the other pieces of each
+// half are issued by a warp of their own (one warp for all: 27 us where this takes 20), and two chunks are handed over at a time where there is room.
 // The slices of a tile are the blocks of a cluster: their partial tiles meet through shared memory, no scratch, no second kernel.
 //
 // An element whose sum is no finite number is summed again from the operands term by term in 32-bit, so that infinities and
@@ -407,34 +413,45 @@ template <int BN, int HALVES> void configure(cudaLaunchConfig_t& cfg, cudaLaunch
     cfg.numAttrs = spy_pdl_enabled() ? 2 : 1;
 }
 
-// How many clusters of `slices` blocks of the few-token kernel the device holds at a time, asked once per device.
-int resident_clusters(int slices, int* count)
+// How many clusters of `slices` blocks the device holds at a time with `per_sm` blocks an SM, asked once per device.  The
+// occupancy query counts one block an SM for every kernel that uses tensor memory, although two share one (seen in their start
+// times), so the clusters of two blocks an SM are those of half as many blocks of one an SM.
+int resident_clusters(int slices, int per_sm, int* count)
 {
     static int known[SPY_MAX_DEVICES][MAX_SLICES + 1] = {};
-    int& c = known[spy_device()][slices];
+    const bool halve = per_sm == 2 && slices % 2 == 0;
+    const int ask = halve ? slices / 2 : slices;
+    int& c = known[spy_device()][ask];
     if (c == 0) {
         if (int rc = set_up<16, 1>()) return rc;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
-        configure<16, 1>(cfg, attr, dim3(1, 1, slices), slices, nullptr);
+        configure<16, 1>(cfg, attr, dim3(1, 1, ask), ask, nullptr);
         cfg.numAttrs = 1;
         int n = 0;
         SPY_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<16, 1>, &cfg));
-        if (n <= 0) SPY_FAIL("gemm_split: no cluster of %d blocks fits the device", slices);
+        if (n <= 0) SPY_FAIL("gemm_split: no cluster of %d blocks fits the device", ask);
         c = n;
     }
-    *count = c;
+    *count = per_sm == 2 && !halve ? 2 * c : c;
     return 0;
 }
 
-// Weight rows of a tile (a multiple of 8) for which `n_rows` take the fewest rounds of `clusters` tiles, and what that costs
-// in rows x K blocks of one block, a round's start and end counted as 350 of them.
-double plan_rows(int n_rows, int clusters, int k_blocks, int* rows_out)
+// Weight rows of a tile (a multiple of 8) for which `n_rows` weight rows in `slices` slices of `per` K blocks take the least
+// time, and that time in cycles: rounds of `clusters` tiles, a round's K blocks at the memory's rate (3,400 bytes a cycle once
+// five sixths of the places are taken) but no faster than a block's chain of waits and issues allows (720 cycles a K block
+// measured), and 5,500 cycles for its start and end.
+double plan_rows(int n_rows, int slices, int clusters, int per, int* rows_out)
 {
     double best = 0;
+    const auto round = [&](int tiles, int rows) {
+        const double blocks = (double)tiles * slices, places = (double)clusters * slices * 5.0 / 6.0;
+        const double memory = rows * 128.0 * (blocks > places ? blocks : places) / 3400.0;
+        return per * (memory > 720.0 ? memory : 720.0) + 5500.0;
+    };
     for (int rows = 128; rows >= 64; rows -= 8) {
-        const int tiles = (n_rows + rows - 1) / rows, rounds = (tiles + clusters - 1) / clusters;
-        const double cost = (double)rounds * ((double)rows * k_blocks + 350.0);
+        const int tiles = (n_rows + rows - 1) / rows, full = tiles / clusters, left = tiles - full * clusters;
+        const double cost = full * round(clusters, rows) + (left > 0 ? round(left, rows) : 0.0);
         if (rows == 128 || cost < best) {
             best = cost;
             *rows_out = rows;
@@ -452,8 +469,8 @@ int plan_slices(int n_rows, int k_blocks, int* slices_out)
         const int per = (k_blocks + z - 1) / z;
         if (z > 1 && (per < 4 || (k_blocks + per - 1) / per != z)) continue;
         int clusters = 0, rows = 0;
-        if (int rc = resident_clusters(z, &clusters)) return rc;
-        const double cost = plan_rows(n_rows, clusters, per, &rows) + 30.0 * (z - 1);
+        if (int rc = resident_clusters(z, 2, &clusters)) return rc;
+        const double cost = plan_rows(n_rows, z, clusters, per, &rows) + 250.0 * (z - 1);
         if (z == 1 || cost < best) {
             best = cost;
             *slices_out = z;
@@ -508,9 +525,8 @@ extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long
     int tile_rows = 256;
     if (M <= 64) {
         int clusters = 0;
-        if (int rc = resident_clusters(slices, &clusters)) return rc;
-        if (bn == 64) clusters = clusters > 1 ? clusters / 2 : 1;      // one block an SM
-        plan_rows(N, clusters, per, &tile_rows);
+        if (int rc = resident_clusters(slices, bn == 64 ? 1 : 2, &clusters)) return rc;
+        plan_rows(N, slices, clusters, per, &tile_rows);
     }
     CUtensorMap mw, ma;
     if (make_map(&mw, W, N, K, ldw, tile_rows) || make_map(&ma, pieces, 3LL * M, K, K, bn)) return 1;
@@ -521,4 +537,3 @@ extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long
     return SPY_SPLIT_LAUNCH(64, 1);
 #undef SPY_SPLIT_LAUNCH
 }
-extern "C" int spy_gemm_split_clusters(int slices, int* n) { return resident_clusters(slices, n); }
