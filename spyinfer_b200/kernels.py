@@ -384,10 +384,19 @@ def attention_generic(q: torch.Tensor, num_heads: int, head_dim: int, out: torch
         raise KernelError(f"attention: q {tuple(q.shape)} / out {tuple(out.shape)} do not fit {num_heads} heads of {head_dim}")
     if positions.shape[0] != T or seq_of_token.shape[0] != T:
         raise KernelError("attention: positions and seq_of_token must have one entry per token")
+    seqs = block_table.shape[0]
+    floats = 0
+    if block_table.shape[1] * page_size > 256:                # shorter rows are one block's work
+        need = build.load("attention_generic").spy_attention_generic_scratch
+        need.restype = ctypes.c_longlong
+        floats = int(need(T, seqs, num_heads, nkv, head_dim, block_table.shape[1], page_size))
+    scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
     _call("attention_generic", "spy_attention_generic", _ptr(q), ctypes.c_longlong(q.shape[1]), _ptr(out), _code(q, "attention queries"),
           _ptr(pages), _code(pages, "cache pages"), _ptr(block_table), block_table.shape[1], page_size, num_pages, num_heads, nkv, head_dim,
           _ptr(positions), _ptr(seq_of_token), T, int(window or 0), ctypes.c_float(scale), _ptr(status), _stream(), planes, int(keep_first),
-          int(bool(sink)), *_score_args(T, num_heads, softcap, slopes, sinks, out_scale))
+          int(bool(sink)), *_score_args(T, num_heads, softcap, slopes, sinks, out_scale), seqs, _ptr(scratch), ctypes.c_longlong(floats))
+    if floats:
+        count_launches(1)                                     # the chunks, then their sum
     return out
 
 

@@ -203,6 +203,43 @@ def test_attention_generic_mixed_batch(dtype, nh, nkv, hd, page_size, window):
                                                                          else dict(rtol=1e-4, atol=1e-5)))
 
 
+@pytest.mark.parametrize("nh,nkv,hd,page_size", [(8, 2, 32, 8), (5, 1, 128, 16), (34, 2, 64, 4), (8, 8, 20, 16)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (100, 0), (150, 130)])
+def test_attention_generic_rows_do_not_depend_on_their_company(nh, nkv, hd, page_size, window, keep):
+    """Prompt portions (several tokens a block) beside single tokens, at the edges of the chunks of 128 keys, against 64 bits and,
+    bit by bit, against each token alone (whose chunks go to blocks of their own).  A value row that is no finite number, seen by the
+    later tokens only, leaves the earlier ones as they were.  Bound: the probabilities and sums of up to 700 terms in 32-bit."""
+    from spyinfer_b200 import kernels
+    runs = [(0, 131), (127, 3), (255, 1), (700, 1), (383, 2)]                # (position of the first token, tokens)
+    width = -(-704 // page_size)
+    pages = torch.randn(len(runs) * width, 2, nkv, page_size, hd, device=DEV)
+    table = torch.randperm(len(runs) * width, device=DEV).view(len(runs), width).to(torch.int32)
+    pos = torch.tensor([p + i for p, n in runs for i in range(n)], dtype=torch.int32, device=DEV)
+    seq = torch.tensor([s for s, (_, n) in enumerate(runs) for _ in range(n)], dtype=torch.int32, device=DEV)
+    q = torch.randn(len(pos), nh * hd, device=DEV)
+
+    def attend(rows, pages):
+        out = torch.full((len(rows), nh * hd), float("nan"), device=DEV)
+        return kernels.attention_generic(q[rows].contiguous(), nh, hd, out, pages, table, pos[rows].contiguous(), seq[rows].contiguous(), hd ** -0.5,
+                                         window=window, keep_first=keep)
+
+    whole = attend(list(range(len(pos))), pages)
+    for t in range(len(pos)):
+        kv = pages[table[seq[t]].long()].double().permute(1, 2, 0, 3, 4).reshape(2, nkv, -1, hd)
+        j = torch.arange(kv.shape[2], device=DEV)
+        lo = max(0, int(pos[t]) - window + 1) if window else 0
+        seen = (j <= pos[t]) & ((j >= lo) | (j < keep))
+        k, v = (x.repeat_interleave(nh // nkv, 0)[:, seen] for x in kv)
+        ref = torch.einsum("hk,hkd->hd", torch.softmax(torch.einsum("hd,hkd->hk", q[t].double().view(nh, hd), k) * hd ** -0.5, -1), v)
+        torch.testing.assert_close(whole[t].double().view(nh, hd), ref, rtol=0, atol=700 * 2.0 ** -23)
+    for t in (0, 1, 126, 127, 128, 130, 131, 133, 134, 135, 136, 137):
+        assert torch.equal(attend([t], pages)[0], whole[t]), f"token {t}"
+    broken = pages.clone()
+    broken[table[0, 129 // page_size], 1, :, 129 % page_size] = float("inf")
+    out = attend(list(range(len(pos))), broken)
+    assert torch.equal(out[:129], whole[:129]) and out[129:131].isinf().any()
+
+
 def test_attention_generic_finds_one_far_key():
     """One key among hundreds is made to stand out (its score is far above the rest): the
     output must be that key's value row, wherever it lies: first slot of a page, last slot,
