@@ -73,7 +73,9 @@ constexpr int PREFIX_OFF = P_OFF + 2 * QP_BYTES;                 // int[MAX_SEQS
 constexpr int POS_OFF = PREFIX_OFF + (MAX_SEQS + 4) * 4;         // int[MAX_SEQS]: every sequence's position (-1: skipped)
 constexpr int RED_OFF = POS_OFF + MAX_SEQS * 4;                  // float[2][4][16] maxima, float[4][16] sums
 constexpr int BAR_OFF = RED_OFF + (2 * 4 * NCOLS + 4 * NCOLS) * 4;
+constexpr int MAX_ORDERED = 256;     // sequences that are put in order (a thread each finds one's place)
 constexpr int NUM_BARS = 4 * STAGES + 3 * 2 + 2 * QSLOTS + 2 + 1;
+constexpr int ORDER_OFF = POS_OFF + MAX_ORDERED * 4;             // uint8_t[MAX_ORDERED], where the positions of further sequences would lie
 constexpr int SMEM_TOTAL = BAR_OFF + NUM_BARS * 8 + 32 + 1024;   // then slack to align the base to 1024
 constexpr int TMEM_COLS = 64;                                    // S^T: 2 x 16 columns; O^T: 16 columns from 32
 
@@ -94,30 +96,34 @@ struct Params {
 };
 
 // A block's share of the batch's units: either the contiguous range [u0, u1) of the list of all
-// (sequence, kv head, tile) units, which cuts pairs wherever the range ends, or (whole) the pairs
-// first, first + stride, ... each with all its tiles.
+// (sequence, kv head, tile) units, which cuts pairs wherever the range ends, or (whole) pairs, each with all its tiles: one of
+// every `stride` pairs, the first-th, and with an order of the sequences (longest first) the first-th from the other end in every
+// second round, so that who got a long pair gets a short one next.
 struct Share {
     const int* prefix;   // [S + 1] tiles of the sequences before s
-    int S, nkv, u0, u1, first, stride;
+    int S, nkv, u0, u1, first, stride, step;   // step: from the first pair to the second; steps alternate and two make 2 * stride
     bool whole;
+    const uint8_t* order;   // null: the sequences as they are
 };
 
 // A run of tiles [t, t_end) of pair (s, kvh), whose keys span `tiles` tiles; `left` units (or, whole,
-// the next pair's index) remain for the block after this run.
+// the next pair's index) remain for the block after this run; `step` (whole) leads from that pair to the one behind it.
 struct Seg {
-    int s, kvh, t0, t, t_end, tiles, left;
+    int s, kvh, t0, t, t_end, tiles, left, step;
 };
 
 __device__ __forceinline__ bool seg_whole(Seg& g, const Share& sh, int pair)
 {
-    for (; pair < sh.S * sh.nkv; pair += sh.stride) {
-        g.s = pair / sh.nkv;
+    for (; pair < sh.S * sh.nkv; pair += g.step, g.step = 2 * sh.stride - g.step) {
+        const int at = pair / sh.nkv;
+        g.s = sh.order != nullptr ? sh.order[at] : at;
         g.tiles = sh.prefix[g.s + 1] - sh.prefix[g.s];
         if (g.tiles == 0) continue;
-        g.kvh = pair - g.s * sh.nkv;
+        g.kvh = pair - at * sh.nkv;
         g.t0 = g.t = 0;
         g.t_end = g.tiles;
-        g.left = pair + sh.stride;
+        g.left = pair + g.step;
+        g.step = 2 * sh.stride - g.step;
         return true;
     }
     return false;
@@ -125,6 +131,7 @@ __device__ __forceinline__ bool seg_whole(Seg& g, const Share& sh, int pair)
 
 __device__ __forceinline__ bool seg_first(Seg& g, const Share& sh)
 {
+    g.step = sh.step;
     if (sh.whole) return seg_whole(g, sh, sh.first);
     if (sh.u0 >= sh.u1) return false;
     int a = 0, b = sh.S;   // nkv * prefix[a] <= u0 < nkv * prefix[b]
@@ -194,6 +201,33 @@ __device__ __forceinline__ float result_scale(const Params& p, int tok, int head
     return p.scores.out_scale != nullptr ? __ldcg(p.scores.out_scale + (size_t)tok * p.nh + head) : 1.f;
 }
 
+// order: the sequences by their numbers of tiles (prefix[s + 1], not yet summed), most first; s_max_load: the tiles of the busiest
+// block when pairs are dealt out in that order, forwards and backwards in turns.  Called by the whole block.  Not inlined: the
+// kernel starts with a cold instruction cache in every layer, and these few hundred instructions in its way cost the steps that
+// do not need them 3 us a layer.
+__device__ __noinline__ void order_sequences(const int* prefix, int S, int nkv, uint8_t* order, int* s_max_load)
+{
+    const int tid = threadIdx.x, blocks = gridDim.x, pairs = S * nkv;
+    if (tid < S) {
+        const int mine = prefix[tid + 1];
+        int place = 0;
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) {
+            const int v = prefix[s + 1];
+            place += v > mine || (v == mine && s < tid) ? 1 : 0;
+        }
+        order[place] = (uint8_t)tid;
+    }
+    if (tid == 0) *s_max_load = 0;
+    __syncthreads();
+    for (int c = tid; c < blocks; c += NUM_THREADS) {
+        int load = 0;
+        for (int pair = c, step = 2 * blocks - 1 - 2 * c; pair < pairs; pair += step, step = 2 * blocks - step) load += prefix[order[pair / nkv] + 1];
+        atomicMax(s_max_load, load);
+    }
+    __syncthreads();                                            // the tiles are made sums next
+}
+
 // SCORES: a cap and/or a distance bias on the scores
 template <int HD, int GN, bool SCORES>
 __global__ void __maxnreg__(160)
@@ -219,6 +253,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_lred + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* s_max_tiles = reinterpret_cast<int*>(tmem_slot + 2);   // the most tiles any sequence has
+    int* s_max_load = s_max_tiles + 1;                          // the most tiles any block has when whole pairs are dealt out
+    uint8_t* order = smem + ORDER_OFF;                          // the sequences, most tiles first
 
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
@@ -261,7 +297,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
         pos_s[s] = pos;
         prefix[s + 1] = tiles_of(pos, spy_first_key(max(pos, 0), p.window));
     }
+    const int pairs = p.S * p.nkv, rounds = (pairs + (int)gridDim.x - 1) / (int)gridDim.x;
+    const bool in_order = p.S > 1 && p.S <= MAX_ORDERED && rounds > 1 && p.mode != 1;
+    static_assert(NUM_THREADS >= MAX_ORDERED, "a thread a sequence");
     __syncthreads();
+    if (in_order) order_sequences(prefix, p.S, p.nkv, order, s_max_load);
     if (warp == 0) {
         int carry = 0, most = 0;
         for (int base = 0; base < p.S; base += 32) {
@@ -290,13 +330,20 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     const int units = p.nkv * prefix[p.S];
     const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
     const int u0 = min(units, (int)blockIdx.x * per), u1 = min(units, u0 + per);
-    // Whole pairs, dealt round-robin, need no merge; they pay when the blocks then end about when an
-    // even split of the units would (short contexts, or many pairs per block).
-    const int pairs = p.S * p.nkv, rounds = (pairs + (int)gridDim.x - 1) / (int)gridDim.x;
-    // (measured at 1 to 200 requests of 640 to 8,192 keys: a tile costs about 1.05 us in the busiest block, the merges of an even
-    // split about four tiles' time, a little more with many pairs: whole pairs while rounds x longest <= 1.125 x share + 4)
-    const bool whole = p.mode == 2 || (p.mode == 0 && (long long)rounds * *s_max_tiles * 8 <= (long long)per * 9 + 32);
-    const Share share = {prefix, p.S, p.nkv, u0, u1, (int)blockIdx.x, (int)gridDim.x, whole};
+    // Whole pairs need no merge; they pay when the blocks then end about when an even split of the units would
+    // (short contexts, or many pairs per block).
+    // Measured at 1 to 256 requests of 100 to 8,192 keys: a tile costs about 1.05 us in the busiest block, the merges of an even
+    // split about four tiles' time, a little more with many pairs: whole pairs while the busiest block's tiles are at most
+    // 1.125 x share + 4.  Up to 256 requests the busiest block is that of pairs dealt out longest first, forwards and
+    // backwards in turns (64 requests of 152 to 1,216 keys, 32 heads over 8: 45.7 us split, 40.6 so; 256 of 87 to 700: 111 and
+    // 91; 47 of 272 to 2,176, 40 heads: 58.7 and 46.5).  Where every tile can have a block of its own the split is the shorter
+    // chain, from four tiles on (3 requests of 640 keys, 32 heads over 8: 8.3 us against 9.3; 8 of 256, two tiles: 8.1 against 6.1),
+    // and from two on with 16 heads a kv head, whose tiles take longer (8 requests of up to 400 keys: 10.0 against 13.0; 256: 9.2
+    // against 10.4).
+    const long long longest = in_order ? (long long)*s_max_load : (long long)rounds * *s_max_tiles;
+    const bool whole = p.mode == 2 || (p.mode == 0 && longest * 8 <= (long long)per * 9 + 32 && !(per == 1 && longest > (GN > 8 ? 1 : 3)));
+    const Share share = {prefix, p.S, p.nkv, u0, u1, (int)blockIdx.x, (int)gridDim.x,
+                         in_order ? 2 * (int)gridDim.x - 1 - 2 * (int)blockIdx.x : (int)gridDim.x, whole, in_order ? order : nullptr};
     const uint32_t k_s = smem_u32(smem + K_OFF), v_s = smem_u32(smem + V_OFF), q_s = smem_u32(smem + Q_OFF), p_s = smem_u32(smem + P_OFF);
 
     if (warp < 4) {
@@ -532,21 +579,23 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
                     moreq = seg_next(gq, share);
                 }
             };
-            if (moreq) issue_qk();
-            if (ok && moreq) issue_qk();
-            for (int ip = 0; morep && ok; ++ip) {
-                const int st = ip & 1, stage = ip % STAGES;
-                ok = mbar_wait(bar_p + st, (uint32_t)(ip >> 1) & 1, abort_flag) && mbar_wait(bar_vfull + stage, (uint32_t)(ip / STAGES) & 1, abort_flag);
-                if (!ok) break;
-                fence_after_sync();
-                const uint32_t vb = v_s + stage * STAGE_BYTES, pb = p_s + st * QP_BYTES;
+            // The first two turns only issue scores (one copy of that code: a kernel's first way through its instructions is a cold one)
+#pragma unroll 1
+            for (int ip = -2; morep && ok; ++ip) {
+                if (ip >= 0) {
+                    const int st = ip & 1, stage = ip % STAGES;
+                    ok = mbar_wait(bar_p + st, (uint32_t)(ip >> 1) & 1, abort_flag) && mbar_wait(bar_vfull + stage, (uint32_t)(ip / STAGES) & 1, abort_flag);
+                    if (!ok) break;
+                    fence_after_sync();
+                    const uint32_t vb = v_s + stage * STAGE_BYTES, pb = p_s + st * QP_BYTES;
 #pragma unroll
-                for (int s = 0; s < TILE / 16; ++s)   // 16 keys: 16 rows of V, 32 bytes along the rows of P^T
-                    umma(tmem_o, desc_mn_major(vb + s * 16 * 128, HALF_BYTES), desc_k_major(pb + (s >> 2) * (NCOLS * 128) + (s & 3) * 32), idesc_pv,
-                         (gp.t > gp.t0 || s > 0) ? 1u : 0u);
-                umma_commit(bar_o + st);
-                umma_commit(bar_vfree + stage);
-                if (++gp.t == gp.t_end) morep = seg_next(gp, share);
+                    for (int s = 0; s < TILE / 16; ++s)   // 16 keys: 16 rows of V, 32 bytes along the rows of P^T
+                        umma(tmem_o, desc_mn_major(vb + s * 16 * 128, HALF_BYTES), desc_k_major(pb + (s >> 2) * (NCOLS * 128) + (s & 3) * 32), idesc_pv,
+                             (gp.t > gp.t0 || s > 0) ? 1u : 0u);
+                    umma_commit(bar_o + st);
+                    umma_commit(bar_vfree + stage);
+                    if (++gp.t == gp.t_end) morep = seg_next(gp, share);
+                }
                 if (moreq) issue_qk();   // S^T's stage st is free: P^T of this tile was made from it
             }
         }

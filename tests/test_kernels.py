@@ -240,6 +240,28 @@ def test_attention_generic_rows_do_not_depend_on_their_company(nh, nkv, hd, page
     assert torch.equal(out[:129], whole[:129]) and out[129:131].isinf().any()
 
 
+@pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
+@pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
+@pytest.mark.parametrize("window", [None, 300])
+def test_attention_decode_of_ragged_batches(S, nh, nkv, window):
+    """Requests of very different lengths, whose pairs are dealt out longest first (up to 256 requests), split, or as the kernel
+    decides: each against the plain kernel.  Bound: two roundings of a probability and a result to bfloat16 (2^-8 each) on values of
+    a few units."""
+    from spyinfer_b200 import kernels
+    hd, page_size = 64, 16
+    ctx = [1 + (37 * i * i + 11 * i) % 900 for i in range(S)]
+    width = -(-max(ctx) // page_size)
+    pages = torch.randn(S * width, 2, nkv, page_size, hd, device=DEV).to(torch.bfloat16)
+    table = torch.randperm(S * width, device=DEV).view(S, width).to(torch.int32)
+    q = torch.randn(S, nh * hd, device=DEV).to(torch.bfloat16)
+    pos = torch.tensor([c - 1 for c in ctx], dtype=torch.int32, device=DEV)
+    starts = torch.arange(S + 1, dtype=torch.int32, device=DEV)
+    want = kernels.attention_generic(q, nh, hd, torch.empty_like(q), pages, table, pos, starts[:S], hd ** -0.5, window=window).float()
+    for share in ("auto", "split", "whole"):
+        out = kernels.attention_decode(q, nh, hd, torch.full_like(q, float("nan")), pages, table, pos, starts, S, hd ** -0.5, share=share, window=window)
+        torch.testing.assert_close(out.float(), want, rtol=1.6e-2, atol=2e-2)
+
+
 def test_attention_generic_finds_one_far_key():
     """One key among hundreds is made to stand out (its score is far above the rest): the
     output must be that key's value row, wherever it lies: first slot of a page, last slot,
