@@ -5,25 +5,26 @@
 //
 // The sums.  The tensor core adds into its accumulator by cutting, which leans toward zero a little at every step (measured:
 // 2.4e-8 of the result after 16 terms of K, 6.7e-8 after 64, 2.3e-7 after 256).  So the leading pieces' accumulator is taken
-// out of tensor memory every 32 terms of K and added to a sum in registers by an ordinary rounded addition; the other two
+// out of tensor memory every 64 terms of K (one K block) and added to a sum in registers by an ordinary rounded addition; the other two
 // pieces are 2^-8 and 2^-16 of the size and are accumulated through.
-// Relative error (2-norm) against 64 bits at K = 96, 4,096 and 12,288: 0.7e-7, 1.6e-7 and 2.6e-7, where the CUDA-core kernel, one
-// chain over K, has 1.8e-7, 1.1e-6 and 2.0e-6.
+// Relative error (2-norm) against 64 bits at K = 256, 4,096 and 12,288: 0.7e-7, 1.1e-7 and 1.4e-7, where the CUDA-core kernel, one
+// chain over K, has 2.9e-7, 1.1e-6 and 2.0e-6.  (Every 32 terms: 0.7e-7, 1.6e-7 and 2.6e-7, twice as many rounded additions.)
 //
 // A row's result does not depend on M or on its neighbours: K is cut into slices by N and K alone (plan_slices), a slice's sum
-// runs over its chunks of 32 in order, and the slices are added in order.
+// runs over its K blocks of 64 in order, and the slices are added in order.
 //
 // Bounds.  Few tokens: the weights' way through memory (2 bytes a weight).  Many: the tensor cores (three passes).  Measured with
 // the pieces' kernel, from a graph, weights not in L2 (the CUDA-core kernel took 822 us a product on average at 4 tokens of these
-// sizes, 1,690 at 300):   N x K = 6,144 x 4,096: 15 us at 4 tokens, 81 at 300;   4,096 x 4,096: 13 and 68;   24,576 x 4,096: 39
-// (5.1 TB/s) and 221 (274 TFLOP/s of 32-bit product, three times that on the tensor cores);   4,096 x 12,288: 23 and 129;
-// 151,936 x 4,096: 202 (6.2 TB/s).
+// sizes, 1,690 at 300):   N x K = 6,144 x 4,096: 15 us at 4 tokens, 72 at 300;   4,096 x 4,096: 12 and 62;   24,576 x 4,096: 41
+// (4.9 TB/s) and 191 (317 TFLOP/s of 32-bit product, three times that on the tensor cores);   4,096 x 12,288: 23 and 113;
+// 151,936 x 4,096: 200 (6.2 TB/s).
 // Tiles: up to 128 weight rows in the instruction's M slot and 16, 32 or 64 tokens in its N slot, each token three times (a
 // product with the leading pieces, N = BN, and one with the two others side by side, N = 2 BN), two blocks an SM up to 32
 // tokens so that enough weight bytes are under way; beyond 64 tokens 256 weight rows as two halves over 64 tokens (56 KB a
 // stage for 24 products), where a half's sums are taken out while the other half multiplies.  A thread that waits, issues and
 // commits needs about 60 to 100 cycles for each, more than these small products take, so the leading and the other pieces of each
-// half are issued by a warp of their own (one warp for all: 27 us where this takes 20), and two chunks are handed over at a time where there is room.
+// half are issued by a warp of their own (one warp for all: 27 us where this takes 20), and sums are handed over once a K block
+// (every 32 terms: 221 us where this takes 191).
 // The slices of a tile are the blocks of a cluster: their partial tiles meet through shared memory, no scratch, no second kernel.
 //
 // An element whose sum is no finite number is summed again from the operands term by term in 32-bit, so that infinities and
@@ -53,9 +54,7 @@ template <int BN, int HALVES> struct Shape {
     static constexpr int ROWS = 128 * HALVES;              // weight rows of a tile, at most
     static constexpr int Y_BYTES = BN * BK * 2;            // one piece of the tokens
     static constexpr int COLS = (HALVES == 1 ? 8 : 4) * BN;   // tensor-memory columns of a half: buffers of the leading pieces' sums, then the two other pieces'
-    static constexpr int BUFFERS = COLS / BN - 2;          // chunks whose sums may wait to be taken out
-    static constexpr int GROUP = BUFFERS > 2 ? 2 : 1;      // chunks handed over at a time: a wait or a commit costs the issuer as much as several small products
-    static constexpr int HANDS = BUFFERS / GROUP;
+    static constexpr int BUFFERS = COLS / BN - 2;          // blocks of K whose sums may wait to be taken out
     static constexpr int PER_SM = HALVES == 1 && BN <= 32 ? 2 : 1;
     static constexpr int AREA = (PER_SM == 2 ? 110 : 224) * 1024;
     static constexpr size_t SMEM = (size_t)AREA + 1024 /* alignment */ + 512 /* barriers */;
@@ -104,10 +103,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + S::AREA);
     uint64_t* empty_bar = full_bar + MAX_STAGES;
-    constexpr int NB = S::BUFFERS, NH = S::HANDS, G = S::GROUP;
-    uint64_t* sum_full = empty_bar + MAX_STAGES;           // [HALVES][NH] a group of chunks' sums of the leading pieces are complete
-    uint64_t* sum_empty = sum_full + NH * HALVES;          // [HALVES][NH] they have been taken out
-    uint64_t* done_bar = sum_empty + NH * HALVES;
+    constexpr int NB = S::BUFFERS;
+    uint64_t* sum_full = empty_bar + MAX_STAGES;           // [HALVES][NB] a K block's sums of the leading pieces are complete
+    uint64_t* sum_empty = sum_full + NB * HALVES;          // [HALVES][NB] they have been taken out
+    uint64_t* done_bar = sum_empty + NB * HALVES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -125,7 +124,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             mbar_init(full_bar + s, 1);
             mbar_init(empty_bar + s, S::ISSUERS);
         }
-        for (int i = 0; i < NH * HALVES; ++i) {
+        for (int i = 0; i < NB * HALVES; ++i) {
             mbar_init(sum_full + i, 1);
             mbar_init(sum_empty + i, 4);
         }
@@ -176,28 +175,23 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             uint32_t phase = 0;
             if (lead) {
                 const uint32_t idesc = instr_desc_bf16(128, BN, false, false);
-                uint64_t* full = sum_full + NH * half;
-                uint64_t* empty = sum_empty + NH * half;
+                uint64_t* full = sum_full + NB * half;
+                uint64_t* empty = sum_empty + NB * half;
                 int b = 0;
                 uint32_t taken = 1;                        // the parity of a buffer's release that its next use waits for
-                bool ok = true;
-                for (int i = 0; i < num_kb && ok; ++i) {
+                for (int i = 0; i < num_kb; ++i) {
                     if (!mbar_wait(full_bar + s, phase, abort_flag)) break;
                     const uint32_t xs = smem_u32(tiles + (size_t)s * stage_bytes);
                     const uint64_t dx = desc_k_major(xs + x_off), dy = desc_k_major(xs + x_bytes);
+                    if (i >= NB && !mbar_wait(empty + b, taken, abort_flag)) break;
+                    fence_after_sync();
 #pragma unroll
-                    for (int g = 0; g < 2 / G; ++g) {      // two chunks of 32 a block of K
-                        if (ok && i * (2 / G) + g >= NH) ok = mbar_wait(empty + b, taken, abort_flag);
-                        if (!ok) break;
-                        fence_after_sync();
-#pragma unroll
-                        for (int k = 2 * G * g; k < 2 * G * (g + 1); ++k)
-                            umma(acc + (uint32_t)((b * G + (k / 2) % G) * BN), dx + (uint64_t)(k * UMMA_K * 2 >> 4), dy + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (uint32_t)(k & 1));
-                        umma_commit(full + b);
-                        if (++b == NH) {
-                            b = 0;
-                            taken ^= 1;
-                        }
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        umma(acc + (uint32_t)(b * BN), dx + (uint64_t)(k * UMMA_K * 2 >> 4), dy + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, k > 0 ? 1u : 0u);
+                    umma_commit(full + b);
+                    if (++b == NB) {
+                        b = 0;
+                        taken ^= 1;
                     }
                     umma_commit(empty_bar + s);
                     if (++s == stages) {
@@ -233,21 +227,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         for (int c = 0; c < BN; ++c) sum[c] = 0.f;
         int b = 0;
         uint32_t phase = 0;
-        for (int n = 0; n < num_kb * (2 / G); ++n) {
-            if (!mbar_wait_warp(sum_full + NH * half + b, phase, abort_flag)) break;
+        for (int n = 0; n < num_kb; ++n) {
+            if (!mbar_wait_warp(sum_full + NB * half + b, phase, abort_flag)) break;
             fence_after_sync();
 #pragma unroll
-            for (int c = 0; c < G * BN; c += C) {
+            for (int c = 0; c < BN; c += C) {
                 uint32_t r[C];
-                tmem_load<C>(acc + (uint32_t)(b * G * BN + c), r);
+                tmem_load<C>(acc + (uint32_t)(b * BN + c), r);
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < C; ++e) sum[(c + e) % BN] += __uint_as_float(r[e]);
+                for (int e = 0; e < C; ++e) sum[c + e] += __uint_as_float(r[e]);
             }
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(sum_empty + NH * half + b);
-            if (++b == NH) {
+            if (lane == 0) mbar_arrive(sum_empty + NB * half + b);
+            if (++b == NB) {
                 b = 0;
                 phase ^= 1;
             }

@@ -107,7 +107,7 @@ def test_gemm_simt(dtypes, M, N, K):
 @pytest.mark.parametrize("N,K", [(33, 8), (100, 72), (384, 96), (264, 648), (4096, 1024)])
 def test_gemm_split(N, K):
     """The 32-bit product in three bfloat16 pieces against 64 bits, at the edges of its token tiles (16, 32, 64, then two halves
-    of 128 weight rows).  Bound of an element: the terms are exact; of every 32 of them the tensor core cuts two partial sums
+    of 128 weight rows).  Bound of an element: the terms are exact; of every 64 of them the tensor core cuts four partial sums
     (2^-23 each) and one rounded addition follows (2^-24), the slices and the two small pieces add at most 16 further roundings,
     all relative to the sum of the terms' sizes.  A row's result is the same in every company, and numbers that are not finite
     come out as in a plain sum."""
