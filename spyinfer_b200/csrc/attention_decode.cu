@@ -135,6 +135,7 @@ __device__ __forceinline__ bool seg_first(Seg& g, const Share& sh)
     if (sh.whole) return seg_whole(g, sh, sh.first);
     if (sh.u0 >= sh.u1) return false;
     int a = 0, b = sh.S;   // nkv * prefix[a] <= u0 < nkv * prefix[b]
+#pragma unroll 1
     while (b - a > 1) {
         const int mid = (a + b) >> 1;
         if (sh.nkv * sh.prefix[mid] <= sh.u0) a = mid; else b = mid;
@@ -283,10 +284,12 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     }
     if (warp == 4) tmem_alloc(tmem_slot, TMEM_COLS);
     // rows of Q^T beyond the G heads are never copied: keep them zero (their columns of S^T and O^T are not used)
+#pragma unroll 1
     for (int i = tid; i < QSLOTS * QP_BYTES / 16; i += NUM_THREADS) reinterpret_cast<uint4*>(smem + Q_OFF)[i] = make_uint4(0, 0, 0, 0);
     fence_async_proxy();
 
     // ---- the batch's units: tiles of every sequence, prefix sums, this block's share
+#pragma unroll 1
     for (int s = tid; s < p.S; s += NUM_THREADS) {
         const int tok = p.q_start[s];
         int pos = p.positions[tok];
@@ -304,6 +307,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     if (in_order) order_sequences(prefix, p.S, p.nkv, order, s_max_load);
     if (warp == 0) {
         int carry = 0, most = 0;
+#pragma unroll 1
         for (int base = 0; base < p.S; base += 32) {
             const int s = base + lane;
             int v = s < p.S ? prefix[s + 1] : 0;
@@ -638,6 +642,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
             key_range(p, pos_s, g.s, pos, lo);
             const int tile_first = lo / TILE;
             const int* bt = p.block_table + (size_t)g.s * p.table_width;
+#pragma unroll 1
             for (; g.t < g.t_end; ++g.t, ++i) {
                 const int stage = i % STAGES;
                 if (!waited && g.t == g.tiles - 1) {   // the pair's last tile holds the token the kernel ahead has just stored

@@ -139,6 +139,8 @@ __device__ __forceinline__ float relu_squared(float v) { const float p = fmaxf(v
 // EPI == 2: the result is relu(x)^2 of the product, element by element, in the plain layout; K is not split.
 // EPI == 1 (SwiGLU) and EPI == 3 (the same with the tanh form of gelu): the weight's rows alternate gate, up, gate, up, ...; the kernel stores
 // act(gate) * up, half as many output columns (ld counts those); one pass over K only.
+// The loops of this kernel are not unrolled where they wait or copy: in a step's chain of kernels every launch starts with a cold
+// instruction cache, and the shorter way through it is worth 0.5 % of a decode step (with the decode attention's, 1.1 % at 64 requests).
 template <int BN, typename TC, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, TC* __restrict__ out,
@@ -168,6 +170,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const int num_kb = kb1 - kb0;
 
     if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int s = 0; s < stages; ++s) {
             mbar_init(full_bar + s, 1);
             mbar_init(empty_bar + s, 1);
@@ -193,18 +196,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // tiles for the first stages are requested before the wait for the kernels ahead in
             // the stream, so weights already stream in while those are finishing.
             const int pre = min(num_kb, stages);
+#pragma unroll 1
             for (int i = 0; i < pre; ++i) {
                 uint8_t* xs = tiles + (size_t)i * stage_bytes;
                 mbar_expect_tx(full_bar + i, stage_tx);
                 tma_load_2d(smem_u32(xs), &map_x, (kb0 + i) * BK, x0, full_bar + i);
             }
             pdl_wait();
+#pragma unroll 1
             for (int i = 0; i < pre; ++i) {
                 uint8_t* xs = tiles + (size_t)i * stage_bytes;
                 tma_load_2d(smem_u32(xs + x_bytes), &map_y, (kb0 + i) * BK, y0, full_bar + i);
             }
             int s = 0;
             uint32_t phase = 1;   // of the round before: the first wait on a stage is for its first release
+#pragma unroll 1
             for (int i = pre; i < num_kb; ++i) {
                 if (!mbar_wait(empty_bar + s, phase ^ 1, abort_flag)) break;
                 uint8_t* xs = tiles + (size_t)s * stage_bytes;
@@ -227,6 +233,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 const long long share = ((next_bytes + blocks - 1) / blocks + 127) / 128 * 128;
                 long long at = me * share;
                 const long long end = at + share < next_bytes ? at + share : next_bytes;
+#pragma unroll 1
                 for (; at < end; at += 16384) {
                     const long long n = end - at < 16384 ? end - at : 16384;
                     l2_prefetch(next_weights + at, (uint32_t)(n & ~15LL));
@@ -238,6 +245,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             const uint32_t idesc = instr_desc_bf16(BM, BN, false, false);
             int s = 0;
             uint32_t phase = 0;
+#pragma unroll 1
             for (int i = 0; i < num_kb; ++i) {
                 if (!mbar_wait(full_bar + s, phase, abort_flag)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -315,6 +323,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 TC* gout = base + (size_t)y0 * ld + x0;
                 if ((outs & 3) == 0 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0) {
                     const int quads = outs >> 2;
+#pragma unroll 1
                     for (int i = e; i < rows * quads; i += 128) {
                         const int t = i / quads, q = i - t * quads;
                         const float4 v = *reinterpret_cast<const float4*>(staged + t * PLAIN_STAGE_LD + 4 * q);
@@ -330,6 +339,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                         }
                     }
                 } else {
+#pragma unroll 1
                     for (int i = e; i < rows * outs; i += 128) {
                         const int t = i / outs, q = i - t * outs;
                         store_elem(gout + (size_t)t * ld + q, staged[t * PLAIN_STAGE_LD + q]);
@@ -345,11 +355,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 TC* gout = base + (size_t)y0 * ld + x0 / 2;
                 if ((outs & 1) == 0 && (ld & 1) == 0 && (reinterpret_cast<uintptr_t>(gout) & 3) == 0) {
                     const int words = outs / 2;
+#pragma unroll 1
                     for (int i = e; i < rows * words; i += 128) {
                         const int t = i / words, q = i - t * words;
                         *reinterpret_cast<uint32_t*>(gout + (size_t)t * ld + 2 * q) = *reinterpret_cast<const uint32_t*>(staged + t * SWIGLU_STAGE_LD + 2 * q);
                     }
                 } else {
+#pragma unroll 1
                     for (int i = e; i < rows * outs; i += 128) {
                         const int t = i / outs, q = i - t * outs;
                         gout[(size_t)t * ld + q] = staged[t * SWIGLU_STAGE_LD + q];
@@ -358,6 +370,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             }
         } else if (num_kb <= 0) {
             // an empty K range contributes zeros (only possible for a trailing split)
+#pragma unroll 1
             for (int c = 0; c < BN; ++c) {
                 const int y = y0 + c;
                 if (x < x_rows && y < y_rows) {
