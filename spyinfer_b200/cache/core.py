@@ -13,7 +13,7 @@ from ..csrc import build
 
 c_int_p = ctypes.POINTER(ctypes.c_int)
 c_i32_p = ctypes.POINTER(ctypes.c_int32)
-c_i64_p = ctypes.POINTER(ctypes.c_int64)
+c_array = ctypes.c_void_p       # an array's address: plain numbers cost a call a third of what typed pointers do
 
 _lib: Optional[ctypes.CDLL] = None
 
@@ -51,7 +51,7 @@ def lib() -> ctypes.CDLL:
         for name in ("spy_cache_width", "spy_cache_min_free_pages", "spy_cache_num_free_slots", "spy_cache_num_live", "spy_cache_check"):
             getattr(L, name).argtypes = [ctypes.c_void_p]
         L.spy_cache_num_free_pages.argtypes = [ctypes.c_void_p, ctypes.c_int]
-        L.spy_cache_live.argtypes = [ctypes.c_void_p, c_i64_p]
+        L.spy_cache_live.argtypes = [ctypes.c_void_p, c_array]
         L.spy_cache_tables.argtypes = [ctypes.c_void_p, ctypes.c_int]
         L.spy_cache_tables.restype = c_i32_p
         L.spy_cache_has_request.argtypes = [ctypes.c_void_p, ctypes.c_int64]
@@ -62,11 +62,11 @@ def lib() -> ctypes.CDLL:
         L.spy_cache_reserve.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int]
         L.spy_cache_commit.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int]
         L.spy_cache_free_request.argtypes = [ctypes.c_void_p, ctypes.c_int64]
-        L.spy_cache_advance.argtypes = [ctypes.c_void_p, ctypes.c_int, c_i64_p, c_i32_p]
-        L.spy_cache_gather.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, c_i64_p, ctypes.c_int, c_i32_p, ctypes.c_int]
-        L.spy_cache_fill_batch.argtypes = [ctypes.c_void_p, ctypes.c_int, c_i64_p, c_i32_p, c_i32_p, c_i32_p, c_i32_p, ctypes.c_int] + [c_i32_p] * 7 + [c_int_p] * 3
-        L.spy_sched_step.argtypes = ([ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, c_i64_p, c_i32_p, c_i32_p, ctypes.c_int, c_i64_p, c_i32_p]
-                                     + [c_i64_p, c_i32_p, c_i32_p, c_i32_p, c_int_p, c_i64_p, c_int_p, c_int_p, c_i64_p])
+        L.spy_cache_advance.argtypes = [ctypes.c_void_p, ctypes.c_int, c_array, c_array]
+        L.spy_cache_gather.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, c_array, ctypes.c_int, c_array, ctypes.c_int]
+        L.spy_cache_fill_batch.argtypes = [ctypes.c_void_p, ctypes.c_int, c_array, c_array, c_array, c_array, c_array, ctypes.c_int] + [c_array] * 7 + [c_int_p] * 3
+        L.spy_sched_step.argtypes = ([ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, c_array, c_array, c_array, ctypes.c_int, c_array, c_array]
+                                     + [c_array, c_array, c_array, c_array, c_int_p, c_array, c_int_p, c_int_p, c_array])
         _lib = L
     return _lib
 
@@ -77,9 +77,11 @@ def check(code: int) -> None:
         raise _ERRORS.get(code, RuntimeError)(build.last_error("engine_core"))
 
 
-def i32(a):
-    return a.ctypes.data_as(c_i32_p)
+def i32(a) -> int:
+    """The address of an int32 array that the caller keeps until the call it is passed to has returned."""
+    return a.ctypes.data
 
 
-def i64(a):
-    return a.ctypes.data_as(c_i64_p)
+def i64(a) -> int:
+    """The same of an int64 array."""
+    return a.ctypes.data

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 from typing import Sequence
 
+import numpy as np
 import torch
 
 from .. import kernels
@@ -25,10 +26,11 @@ class Sampler:
         tokens = torch.empty(R, dtype=torch.int32, device=logits.device)
         if all(p.temperature == 0.0 for p in params):
             return kernels.sample(logits, tokens)
-        t = torch.tensor([p.temperature for p in params], dtype=torch.float32).to(logits.device, non_blocking=True)
-        s = torch.tensor([p.seed for p in params], dtype=torch.int64).to(logits.device, non_blocking=True)
-        d = torch.tensor(list(draws), dtype=torch.int64).to(logits.device, non_blocking=True)
-        k = None
-        if any(p.top_k > 0 and p.temperature > 0.0 for p in params):
-            k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(logits.device, non_blocking=True)
+        host = np.zeros((4, R), np.int64)                      # one transfer: seeds, draws, temperatures, top_k
+        host[0], host[1] = [p.seed for p in params], draws
+        host[2].view(np.float32)[:R] = [p.temperature for p in params]
+        host[3].view(np.int32)[:R] = [p.top_k for p in params]
+        dev = torch.from_numpy(host).to(logits.device, non_blocking=True)
+        s, d, t = dev[0], dev[1], dev[2].view(torch.float32)[:R]
+        k = dev[3].view(torch.int32)[:R] if any(p.top_k > 0 and p.temperature > 0.0 for p in params) else None
         return kernels.sample(logits, tokens, t, s, d, k)
