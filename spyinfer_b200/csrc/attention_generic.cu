@@ -272,13 +272,19 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
             kept_max = max(kept_max, kept_s[r]);
         }
         const int kept_chunks = (kept_max + CHUNK - 1) / CHUNK;
+        // A position beyond the table sees keys that have no page: the first such token is reported and its keys are left out, and no
+        // chunk beyond the table's is walked (there is no scratch for one).
+        if (pos_max / CHUNK >= A.max_chunks && tid == 0 && (!SPLIT || blockIdx.z == 0))
+            for (int r = 0; r < rows; r += nheads)
+                if (pos_s[r] / CHUNK >= A.max_chunks) report_status(A.status, SPY_STATUS_BAD_PAGE, t0 + r / nheads);
+        const int last_chunk = pos_max < 0 ? -1 : min(pos_max / CHUNK, A.max_chunks - 1);
         float m[R], l[R], acc[R];                                                // of the row, acc of this thread's dimension
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             m[r] = -INFINITY;
             l[r] = acc[r] = 0.f;
         }
-        for (int c = SPLIT ? blockIdx.z : 0; c <= pos_max / CHUNK && pos_max >= 0; c += SPLIT ? gridDim.z : 1) {
+        for (int c = SPLIT ? blockIdx.z : 0; c <= last_chunk; c += SPLIT ? gridDim.z : 1) {
             if (c >= kept_chunks && c < lo_min / CHUNK) continue;                // nothing to see between the kept keys and the windows
             const int j = c * CHUNK + tid;
             bool any = false;
@@ -396,9 +402,10 @@ __global__ void __launch_bounds__(CHUNK) attention_merge_kernel(TA* __restrict__
     const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, hd = A.hd;
     const int pos = A.positions[t], lo = spy_first_key(pos, A.window), kept_chunks = (min(A.keep_first, lo) + CHUNK - 1) / CHUNK;
     const float* part = A.partial + ((size_t)t * A.nh + h) * A.max_chunks * (hd + 2);
+    const int last_chunk = pos < 0 ? -1 : min(pos / CHUNK, A.max_chunks - 1);    // the chunks that attention_rows_kernel walks
     float m = -INFINITY, l = 0.f, acc = 0.f;
 #pragma unroll 4
-    for (int c = 0; c <= pos / CHUNK; ++c) {
+    for (int c = 0; c <= last_chunk; ++c) {
         if (c >= kept_chunks && c < lo / CHUNK) continue;
         const float* p = part + (size_t)c * (hd + 2);
         const float mc = p[hd], lc = p[hd + 1], v = tid < hd ? p[tid] : 0.f;

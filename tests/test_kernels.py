@@ -240,6 +240,51 @@ def test_attention_generic_rows_do_not_depend_on_their_company(nh, nkv, hd, page
     assert torch.equal(out[:129], whole[:129]) and out[129:131].isinf().any()
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(8, 2, 32), (6, 6, 128), (16, 1, 20)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (100, 0), (150, 130)])
+def test_attention_generic_of_positions_outside_the_table(nh, nkv, hd, window, keep):
+    """A position at and far beyond the end of the block table and a position of -1, where the chunks of a row go to blocks of their own
+    and where one block walks them: the keys without a page are left out and the token is reported, a row that sees no key is zero, the
+    rows beside it are what they are without it, and nothing outside a buffer is written (the guard zones)."""
+    from spyinfer_b200 import kernels
+    page_size, width = 16, 25                                  # 400 keys: the last chunk is not a whole one
+    pages = torch.randn(3 * width, 2, nkv, page_size, hd, device=DEV)
+    bt = torch.randperm(3 * width, device=DEV).view(3, width).to(torch.int32)
+
+    def attend(pos, seq, table):
+        q = q_all[:len(pos)].contiguous()
+        out, status = torch.full((len(pos), nh * hd), float("nan"), device=DEV), torch.zeros(2, dtype=torch.int32, device=DEV)
+        kernels.attention_generic(q, nh, hd, out, pages, table, torch.tensor(pos, dtype=torch.int32, device=DEV), torch.tensor(seq, dtype=torch.int32, device=DEV),
+                                  hd ** -0.5, window=window, keep_first=keep, status=status)
+        return q, out, status.tolist()
+
+    many = 1200 // nkv + 1                                     # so many rows of single sequences that no row is cut
+    q_all = torch.randn(3, nh * hd, device=DEV).repeat(many, 1)
+    for beyond in (400, 511, 512, 5000, 2 ** 31 - 1):
+        for at in range(3):                                    # the last row of all is where an overrun would leave the scratch
+            pos = [399, 130, 260]
+            pos[at] = beyond
+            q, out, status = attend(pos, [0, 1, 2], bt)
+            assert status == [3, at]
+            _, alone, ok = attend([399, 130, 260], [0, 1, 2], bt)
+            assert ok == [0, 0] and all(torch.equal(out[r], alone[r]) for r in range(3) if r != at)
+            j = torch.arange(400, device=DEV)
+            seen = (j >= (max(0, beyond - window + 1) if window else 0)) | ((j < keep) if window else False)
+            kv = pages[bt[at].long()].double().permute(1, 2, 0, 3, 4).reshape(2, nkv, 400, hd)
+            k, v = (x.repeat_interleave(nh // nkv, 0)[:, seen] for x in kv)
+            ref = torch.einsum("hk,hkd->hd", torch.softmax(torch.einsum("hd,hkd->hk", q[at].double().view(nh, hd), k) * hd ** -0.5, -1), v)
+            torch.testing.assert_close(out[at].double().view(nh, hd), ref, rtol=0, atol=700 * 2.0 ** -23)
+            _, walked, status = attend(pos * many, list(range(3 * many)), bt.repeat(many, 1))
+            assert status[0] == 3 and status[1] % 3 == at and torch.equal(walked[:3], out)
+    for at in range(3):
+        pos = [399, 130, 260]
+        pos[at] = -1
+        _, out, status = attend(pos, [0, 1, 2], bt)
+        assert status == [0, 0] and not out[at].any() and all(torch.equal(out[r], alone[r]) for r in range(3) if r != at)
+        _, walked, _ = attend(pos * many, list(range(3 * many)), bt.repeat(many, 1))
+        assert torch.equal(walked[:3], out)
+
+
 @pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
 @pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
 @pytest.mark.parametrize("window", [None, 300])
