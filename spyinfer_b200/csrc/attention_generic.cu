@@ -288,15 +288,17 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
             if (c >= kept_chunks && c < lo_min / CHUNK) continue;                // nothing to see between the kept keys and the windows
             const int j = c * CHUNK + tid;
             bool any = false;
-            for (int r = 0; r < rows; r += nheads) {
-                const bool sees = (j >= lo_s[r] || j < kept_s[r]) && j <= pos_s[r];
-                any |= sees;
-            }
+            int first_seer = 0;                                                  // the first row whose token sees the key
+            for (int r = rows - nheads; r >= 0; r -= nheads)
+                if ((j >= lo_s[r] || j < kept_s[r]) && j <= pos_s[r]) {
+                    any = true;
+                    first_seer = r;
+                }
             long long row = -1;
             if (any) {
                 const int lp = j / A.page_size;
                 const int page = lp < A.table_width ? bt[lp] : -1;
-                if (page < 0 || page >= A.num_pages) report_status(A.status, SPY_STATUS_BAD_PAGE, t0);
+                if (page < 0 || page >= A.num_pages) report_status(A.status, SPY_STATUS_BAD_PAGE, t0 + first_seer / nheads);
                 else row = ((((long long)page * A.planes) * A.nkv + kvh) * A.page_size + j % A.page_size) * hd;
             }
             row_s[tid] = row;

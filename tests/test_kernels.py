@@ -285,6 +285,21 @@ def test_attention_generic_of_positions_outside_the_table(nh, nkv, hd, window, k
         assert torch.equal(walked[:3], out)
 
 
+def test_attention_generic_names_the_token_that_sees_a_bad_page():
+    """Sixteen tokens of one sequence share a block: the token in the status word is one that sees the key without a page."""
+    from spyinfer_b200 import kernels
+    nh, hd, page_size = 2, 64, 8
+    pages, bt = torch.randn(6, 2, nh, page_size, hd, device=DEV), torch.arange(6, dtype=torch.int32, device=DEV).view(1, 6)
+    pos, seq = torch.arange(40, dtype=torch.int32, device=DEV), torch.zeros(40, dtype=torch.int32, device=DEV)
+    q, out = torch.randn(40, nh * hd, device=DEV), torch.empty(40, nh * hd, device=DEV)
+    for page in (1, 3):                                        # seen from tokens 8 and 24 on
+        bad, status = bt.clone(), torch.zeros(2, dtype=torch.int32, device=DEV)
+        bad[0, page] = 6
+        kernels.attention_generic(q, nh, hd, out, pages, bad, pos, seq, hd ** -0.5, status=status)
+        code, token = status.tolist()
+        assert code == 3 and 8 * page <= token < 40
+
+
 @pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
 @pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
 @pytest.mark.parametrize("window", [None, 300])
