@@ -182,14 +182,18 @@ struct AttnArgs {
 constexpr int KD = 64;                  // dimensions of the keys staged at a time
 constexpr int KLD = KD + 4;
 
-// The running softmax of a row takes a chunk's: returns the factors of what was there and of what comes.
-__device__ __forceinline__ void take_chunk(float& m, float& l, float mc, float lc, float& alpha, float& beta)
+// The running softmax of a row takes a chunk's: the factors of what was there and of what comes; false: there is no score above -inf so
+// far, nothing to add (as attention_generic_kernel leaves out chunks until one has such a score).  A chunk without one behind others is
+// added as it is: its probabilities are 0, or NaN where a score is NaN; a row with a NaN in its sum is stored as 0.
+__device__ __forceinline__ bool take_chunk(float& m, float& l, float mc, float lc, float& alpha, float& beta)
 {
     const float m_new = fmaxf(m, mc);
+    if (m_new == -INFINITY) return false;
     alpha = m == -INFINITY ? 0.f : expf(m - m_new);
-    beta = expf(mc - m_new);
+    beta = mc == -INFINITY ? 1.f : expf(mc - m_new);
     l = fmaf(l, alpha, lc * beta);
     m = m_new;
+    return true;
 }
 
 template <typename TA>
@@ -352,7 +356,7 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
             for (int r = 0; r < R; ++r) {
                 mc[r] = fmaxf(fmaxf(red[0][0][r], red[0][1][r]), fmaxf(red[0][2][r], red[0][3][r]));
                 const bool sees = row >= 0 && r < rows && (j >= lo_s[r] || j < kept_s[r]) && j <= pos_s[r];
-                const float p = sees && mc[r] != -INFINITY ? expf(s[r] - mc[r]) : 0.f;
+                const float p = !sees ? 0.f : mc[r] != -INFINITY ? expf(s[r] - mc[r]) : isnan(s[r]) ? s[r] : 0.f;
                 p_s[tid][r] = sees || r >= rows ? p : -1.f;
                 const float sum = warp_sum(p);
                 if (lane == 0) red[1][warp][r] = sum;
@@ -381,10 +385,9 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
                             part[hd + 1] = lc;
                         }
                     }
-                } else if (mc[r] != -INFINITY) {
+                } else {
                     float alpha, beta;
-                    take_chunk(m[r], l[r], mc[r], lc, alpha, beta);
-                    acc[r] = fmaf(acc[r], alpha, vs[r] * beta);
+                    if (take_chunk(m[r], l[r], mc[r], lc, alpha, beta)) acc[r] = fmaf(acc[r], alpha, vs[r] * beta);
                 }
             }
             __syncthreads();                                                     // the shared arrays are rewritten by the next chunk
@@ -411,10 +414,8 @@ __global__ void __launch_bounds__(CHUNK) attention_merge_kernel(TA* __restrict__
         if (c >= kept_chunks && c < lo / CHUNK) continue;
         const float* p = part + (size_t)c * (hd + 2);
         const float mc = p[hd], lc = p[hd + 1], v = tid < hd ? p[tid] : 0.f;
-        if (mc == -INFINITY) continue;
         float alpha, beta;
-        take_chunk(m, l, mc, lc, alpha, beta);
-        acc = fmaf(acc, alpha, v * beta);
+        if (take_chunk(m, l, mc, lc, alpha, beta)) acc = fmaf(acc, alpha, v * beta);
     }
     if (tid < hd) store_row(A, out, t, h, tid, acc, m, l);
 }

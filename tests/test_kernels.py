@@ -300,6 +300,42 @@ def test_attention_generic_names_the_token_that_sees_a_bad_page():
         assert code == 3 and 8 * page <= token < 40
 
 
+def test_attention_generic_of_scores_that_are_no_numbers():
+    """A NaN score makes its row 0 whether its key is alone in a chunk of 128 or beside others (one chunk a block, and all in one block);
+    scores of -inf weigh nothing, but a value of inf under one makes NaN; rows that do not see the key are as they were."""
+    from spyinfer_b200 import kernels
+    nh, nkv, hd, page_size, width = 4, 2, 32, 16, 32
+    q = torch.randn(1, nh * hd, device=DEV).abs().repeat(700, 1)                # positive: a key of -inf has a score of -inf
+    bt = torch.arange(width, dtype=torch.int32, device=DEV).view(1, width)
+
+    def attend(pos, k_rows=None, k_value=0.0, v_row=None):
+        pages = plain.clone()
+        for j in k_rows or ():
+            pages[j // page_size, 0, :, j % page_size] = k_value
+        if v_row is not None:
+            pages[v_row // page_size, 1, :, v_row % page_size] = float("inf")
+        outs = []
+        for n in (1, 700):                                     # 700 rows of single sequences: no row is cut
+            table = bt.repeat(n, 1)
+            outs.append(kernels.attention_generic(q[:n].contiguous(), nh, hd, torch.full((n, nh * hd), 7.0, device=DEV), pages, table,
+                                                  torch.full((n,), pos, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV), 0.1))
+        assert torch.equal(outs[0].nan_to_num(9.0), outs[1][:1].nan_to_num(9.0))
+        return outs[0]
+
+    plain = torch.randn(width, 2, nkv, page_size, hd, device=DEV)
+    nan, inf = float("nan"), float("inf")
+    for pos in (128, 140, 300, 511):                           # the own key: alone in its chunk, beside others, in a later chunk
+        good = attend(pos)
+        assert good.isfinite().all() and good.any(1).all()
+        assert not attend(pos, [pos], nan).any() and not attend(pos, [5], nan).any() and not attend(pos, range(pos + 1), nan).any()
+        if pos < 511:
+            assert torch.equal(attend(pos, [pos + 1], nan), good)
+    without = attend(128, [128], -inf)
+    assert without.isfinite().all() and not torch.equal(without, attend(128)) and torch.equal(without, attend(127))
+    assert attend(128, [128], -inf, v_row=128).isnan().all()
+    assert torch.equal(attend(300, range(128), -inf), attend(300, range(128), nan)) and attend(300, range(128), nan).any()
+
+
 @pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
 @pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
 @pytest.mark.parametrize("window", [None, 300])
