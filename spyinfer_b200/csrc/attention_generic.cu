@@ -162,6 +162,8 @@ attention_generic_kernel(const TA* __restrict__ q, long long q_row_stride, TA* _
 //
 // A chunk's maximum, sum and value sum are formed for themselves and added to the row's in the order of the chunks, whether one
 // block walks them or many, and a row's numbers do not depend on the rows beside it: results do not depend on the cut.
+// Value sums are formed with probabilities divided by CHUNK (a power of two: the same bits), so that a chunk's never exceed its largest value: relative to
+// the chunk's own maximum they could overflow where the chunk weighs next to nothing in its row.
 // A key that a row does not see is left out (p_s = -1), not multiplied by zero: what lies there may not be a finite number.
 struct AttnArgs {
     long long q_row_stride;
@@ -357,7 +359,7 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
                 mc[r] = fmaxf(fmaxf(red[0][0][r], red[0][1][r]), fmaxf(red[0][2][r], red[0][3][r]));
                 const bool sees = row >= 0 && r < rows && (j >= lo_s[r] || j < kept_s[r]) && j <= pos_s[r];
                 const float p = !sees ? 0.f : mc[r] != -INFINITY ? expf(s[r] - mc[r]) : isnan(s[r]) ? s[r] : 0.f;
-                p_s[tid][r] = sees || r >= rows ? p : -1.f;
+                p_s[tid][r] = sees || r >= rows ? p * (1.f / CHUNK) : -1.f;
                 const float sum = warp_sum(p);
                 if (lane == 0) red[1][warp][r] = sum;
             }
@@ -387,7 +389,7 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
                     }
                 } else {
                     float alpha, beta;
-                    if (take_chunk(m[r], l[r], mc[r], lc, alpha, beta)) acc[r] = fmaf(acc[r], alpha, vs[r] * beta);
+                    if (take_chunk(m[r], l[r], mc[r], lc, alpha, beta)) acc[r] = fmaf(acc[r], alpha, vs[r] * (CHUNK * beta));
                 }
             }
             __syncthreads();                                                     // the shared arrays are rewritten by the next chunk
@@ -415,7 +417,7 @@ __global__ void __launch_bounds__(CHUNK) attention_merge_kernel(TA* __restrict__
         const float* p = part + (size_t)c * (hd + 2);
         const float mc = p[hd], lc = p[hd + 1], v = tid < hd ? p[tid] : 0.f;
         float alpha, beta;
-        if (take_chunk(m, l, mc, lc, alpha, beta)) acc = fmaf(acc, alpha, v * beta);
+        if (take_chunk(m, l, mc, lc, alpha, beta)) acc = fmaf(acc, alpha, v * (CHUNK * beta));
     }
     if (tid < hd) store_row(A, out, t, h, tid, acc, m, l);
 }

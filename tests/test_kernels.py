@@ -336,6 +336,27 @@ def test_attention_generic_of_scores_that_are_no_numbers():
     assert torch.equal(attend(300, range(128), -inf), attend(300, range(128), nan)) and attend(300, range(128), nan).any()
 
 
+def test_attention_generic_of_the_largest_values():
+    """Values near the largest 32-bit number under keys of little weight, in a chunk of 128 keys behind one of full weight: no sum on the way
+    overflows.  Bound: the scores' rounding (2^-24 of their size of some 90, four times) and sums of 256 terms."""
+    from spyinfer_b200 import kernels
+    nh, hd, page_size, width = 2, 64, 16, 32
+    for low in (60.0, 80.0, 200.0):
+        pages = torch.randn(width, 2, nh, page_size, hd, device=DEV)
+        pages[:, 0] = 0.0
+        pages[8:, 0, :, :, 0] = -low                           # the keys from 128 on
+        pages[8:, 1] = 3e38 * torch.rand_like(pages[8:, 1])
+        q = torch.zeros(700, nh * hd, device=DEV)
+        q[:, ::hd] = 1.0
+        for n in (1, 700):                                     # one chunk a block, and all in one block
+            table = torch.arange(width, dtype=torch.int32, device=DEV).repeat(n, 1)
+            out = kernels.attention_generic(q[:n].contiguous(), nh, hd, torch.empty(n, nh * hd, device=DEV), pages, table,
+                                            torch.full((n,), 255, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV), 1.0)
+            kv = pages[:16].double().permute(1, 2, 0, 3, 4).reshape(2, nh, 256, hd)
+            ref = torch.einsum("hk,hkd->hd", torch.softmax(kv[0, :, :, 0], -1), kv[1])
+            torch.testing.assert_close(out[0].double().view(nh, hd), ref, rtol=4 * 90 * 2.0 ** -24 + 256 * 2.0 ** -24, atol=256 * 2.0 ** -24)
+
+
 @pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
 @pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
 @pytest.mark.parametrize("window", [None, 300])
