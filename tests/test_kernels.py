@@ -357,6 +357,35 @@ def test_attention_generic_of_the_largest_values():
             torch.testing.assert_close(out[0].double().view(nh, hd), ref, rtol=4 * 90 * 2.0 ** -24 + 256 * 2.0 ** -24, atol=256 * 2.0 ** -24)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,dtype", [(16, 1, 128, torch.float32), (20, 2, 64, torch.bfloat16)])
+def test_attention_generic_of_rows_longer_than_the_scratch_has_room_for(nh, nkv, hd, dtype):
+    """A prompt of 1,100 tokens behind none, and one behind 300 keys, over a table as wide as 40,960 keys: the scratch has room for the chunks of
+    the shorter rows, whose chunks go to blocks of their own, and one block walks those of the longer ones.  Bit by bit what each token gives alone."""
+    from spyinfer_b200 import kernels
+    from spyinfer_b200.csrc import build
+    import ctypes
+    page_size, runs = 16, [(0, 1100), (300, 40)]
+    need = build.load("attention_generic").spy_attention_generic_scratch
+    need.restype = ctypes.c_longlong
+    tokens = sum(n for _, n in runs)
+    slots = need(tokens, 2, nh, nkv, hd, 2560, page_size) // (tokens * nh * (hd + 2))
+    assert (slots == 0) == (nh == 20) and (slots == 0 or 3 <= slots < 9)       # nh = 20: so many blocks that no row is cut
+    pages = torch.randn(2 * 70, 2, nkv, page_size, hd, device=DEV).to(dtype)
+    table = torch.full((2, 2560), -1, dtype=torch.int32, device=DEV)
+    table[:, :70] = torch.randperm(2 * 70, device=DEV).view(2, 70).to(torch.int32)
+    pos = torch.tensor([p + i for p, n in runs for i in range(n)], dtype=torch.int32, device=DEV)
+    seq = torch.tensor([s for s, (_, n) in enumerate(runs) for _ in range(n)], dtype=torch.int32, device=DEV)
+    q = torch.randn(tokens, nh * hd, device=DEV).to(dtype)
+
+    def attend(rows):
+        out = torch.full((len(rows), nh * hd), float("nan"), device=DEV, dtype=dtype)
+        return kernels.attention_generic(q[rows].contiguous(), nh, hd, out, pages, table, pos[rows].contiguous(), seq[rows].contiguous(), hd ** -0.5)
+
+    whole = attend(list(range(tokens)))
+    for t in [0, 1, 127, 128] + [slots * 128 + d for d in (-2, -1, 0, 1, 15, 16) if slots] + [1023, 1024, 1099, 1100, 1139]:
+        assert torch.equal(attend([t])[0], whole[t]), f"token {t}"
+
+
 @pytest.mark.parametrize("S", [2, 37, 150, 256, 257])
 @pytest.mark.parametrize("nh,nkv", [(8, 2), (16, 1)])
 @pytest.mark.parametrize("window", [None, 300])
