@@ -76,6 +76,9 @@ constexpr int BAR_OFF = RED_OFF + (2 * 4 * NCOLS + 4 * NCOLS) * 4;
 constexpr int MAX_ORDERED = 256;     // sequences that are put in order (a thread each finds one's place)
 constexpr int NUM_BARS = 4 * STAGES + 3 * 2 + 2 * QSLOTS + 2 + 1;
 constexpr int ORDER_OFF = POS_OFF + MAX_ORDERED * 4;             // uint8_t[MAX_ORDERED], where the positions of further sequences would lie
+constexpr int KEYS_OFF = ORDER_OFF + MAX_ORDERED;                // uint32_t[MAX_ORDERED]
+constexpr int SORTED_OFF = KEYS_OFF + MAX_ORDERED * 4;           // int[MAX_ORDERED]
+static_assert(SORTED_OFF + MAX_ORDERED * 4 <= RED_OFF && KEYS_OFF % 16 == 0, "the order lies behind the positions of as many sequences");
 constexpr int SMEM_TOTAL = BAR_OFF + NUM_BARS * 8 + 32 + 1024;   // then slack to align the base to 1024
 constexpr int TMEM_COLS = 64;                                    // S^T: 2 x 16 columns; O^T: 16 columns from 32
 
@@ -202,31 +205,39 @@ __device__ __forceinline__ float result_scale(const Params& p, int tok, int head
     return p.scores.out_scale != nullptr ? __ldcg(p.scores.out_scale + (size_t)tok * p.nh + head) : 1.f;
 }
 
-// order: the sequences by their numbers of tiles (prefix[s + 1], not yet summed), most first; s_max_load: the tiles of the busiest
+// order: the sequences by their numbers of tiles (prefix[s + 1] - prefix[s]), most first; s_max_load: the tiles of the busiest
 // block when pairs are dealt out in that order, forwards and backwards in turns.  Called by the whole block.  Not inlined: the
 // kernel starts with a cold instruction cache in every layer, and these few hundred instructions in its way cost the steps that
 // do not need them 3 us a layer.
-__device__ __noinline__ void order_sequences(const int* prefix, int S, int nkv, uint8_t* order, int* s_max_load)
+__device__ __noinline__ void order_sequences(const int* prefix, int S, int nkv, uint8_t* order, uint32_t* keys, int* sorted, int* s_max_load)
 {
     const int tid = threadIdx.x, blocks = gridDim.x, pairs = S * nkv;
+    const int mine = tid < S ? prefix[tid + 1] - prefix[tid] : 0;
+    const uint32_t key = (uint32_t)mine << 8 | (uint32_t)(MAX_ORDERED - 1 - tid);        // tiles: 24 bits hold any 32-bit position's
+    if (tid < MAX_ORDERED) keys[tid] = tid < S ? key : 0;
+    if (tid == 0) *s_max_load = 0;
+    __syncthreads();
     if (tid < S) {
-        const int mine = prefix[tid + 1];
         int place = 0;
 #pragma unroll 4
-        for (int s = 0; s < S; ++s) {
-            const int v = prefix[s + 1];
-            place += v > mine || (v == mine && s < tid) ? 1 : 0;
+        for (int s = 0; s < S; s += 4) {
+            const uint4 k = *reinterpret_cast<const uint4*>(keys + s);
+            place += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
         }
         order[place] = (uint8_t)tid;
+        sorted[place] = mine;
     }
-    if (tid == 0) *s_max_load = 0;
     __syncthreads();
     for (int c = tid; c < blocks; c += NUM_THREADS) {
         int load = 0;
-        for (int pair = c, step = 2 * blocks - 1 - 2 * c; pair < pairs; pair += step, step = 2 * blocks - step) load += prefix[order[pair / nkv] + 1];
+#pragma unroll 4
+        for (int first = 0; first < pairs; first += 2 * blocks) {
+            const int there = first + c, back = first + 2 * blocks - 1 - c;
+            load += (there < pairs ? sorted[there / nkv] : 0) + (back < pairs ? sorted[back / nkv] : 0);
+        }
         atomicMax(s_max_load, load);
     }
-    __syncthreads();                                            // the tiles are made sums next
+    __syncthreads();
 }
 
 // SCORES: a cap and/or a distance bias on the scores
@@ -254,7 +265,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_lred + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* s_max_tiles = reinterpret_cast<int*>(tmem_slot + 2);   // the most tiles any sequence has
-    int* s_max_load = s_max_tiles + 1;                          // the most tiles any block has when whole pairs are dealt out
+    int* s_max_load = s_max_tiles + 1;                          // the most tiles any block has when whole pairs are dealt out longest first
     uint8_t* order = smem + ORDER_OFF;                          // the sequences, most tiles first
 
     pdl_launch_dependents();
@@ -300,11 +311,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
         pos_s[s] = pos;
         prefix[s + 1] = tiles_of(pos, spy_first_key(max(pos, 0), p.window));
     }
-    const int pairs = p.S * p.nkv, rounds = (pairs + (int)gridDim.x - 1) / (int)gridDim.x;
-    const bool in_order = p.S > 1 && p.S <= MAX_ORDERED && rounds > 1 && p.mode != 1;
-    static_assert(NUM_THREADS >= MAX_ORDERED, "a thread a sequence");
     __syncthreads();
-    if (in_order) order_sequences(prefix, p.S, p.nkv, order, s_max_load);
     if (warp == 0) {
         int carry = 0, most = 0;
 #pragma unroll 1
@@ -338,14 +345,34 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
     // (short contexts, or many pairs per block).
     // Measured at 1 to 256 requests of 100 to 8,192 keys: a tile costs about 1.05 us in the busiest block, the merges of an even
     // split about four tiles' time, a little more with many pairs: whole pairs while the busiest block's tiles are at most
-    // 1.125 x share + 4.  Up to 256 requests the busiest block is that of pairs dealt out longest first, forwards and
-    // backwards in turns (64 requests of 152 to 1,216 keys, 32 heads over 8: 45.7 us split, 40.6 so; 256 of 87 to 700: 111 and
-    // 91; 47 of 272 to 2,176, 40 heads: 58.7 and 46.5).  Where every tile can have a block of its own the split is the shorter
+    // 1.125 x share + 4.  Where pairs dealt out as they come do not keep to that, batches of up to 256 requests of different lengths are put in
+    // order first and dealt out longest first, forwards and backwards in turns (64 requests of 152 to 1,216 keys, 32 heads over 8: 45.7 us split,
+    // 40.6 so; 256 of 87 to 700: 111 and 91; 47 of 272 to 2,176, 40 heads: 58.7 and 46.5).  The ordering itself takes 1.6 to 3 us:
+    // where the pairs as they come end in time it is left out (32 requests of one length, 32 heads over 8: 300 keys 15.3 us with it, 13.4 without; 1,216 keys
+    // 34.1 and 31.1), and where it cannot bring the busiest block down.
+    // Where every tile can have a block of its own the split is the shorter
     // chain, from four tiles on (3 requests of 640 keys, 32 heads over 8: 8.3 us against 9.3; 8 of 256, two tiles: 8.1 against 6.1),
-    // and from two on with 16 heads a kv head, whose tiles take longer (8 requests of up to 400 keys: 10.0 against 13.0; 256: 9.2
-    // against 10.4).
-    const long long longest = in_order ? (long long)*s_max_load : (long long)rounds * *s_max_tiles;
-    const bool whole = p.mode == 2 || (p.mode == 0 && longest * 8 <= (long long)per * 9 + 32 && !(per == 1 && longest > (GN > 8 ? 1 : 3)));
+    // and from two on with 9 to 16 heads a kv head, whose tiles take longer (2, 8, 16 and 32 requests of 200 keys, 16 heads: 9.1, 9.9, 10.1 and 10.1 against
+    // 10.0, 10.4, 10.8 and 10.9; of 400 keys 10.5, 11.6, 11.7 and 12.1 against 13.0, 13.3, 13.5 and 13.8; the same way with 9 and with 12 heads).
+    const int pairs = p.S * p.nkv, rounds = (pairs + (int)gridDim.x - 1) / (int)gridDim.x;
+    const auto in_time = [&](long long tiles) { return tiles * 8 <= (long long)per * 9 + 32; };
+    long long longest = (long long)rounds * *s_max_tiles;
+    static_assert(NUM_THREADS >= MAX_ORDERED, "a thread a sequence");
+    bool in_order = false;
+    if (p.S > 1 && p.S <= MAX_ORDERED && rounds > 1 && p.mode != 1 && !in_time(longest)) {
+        // What the order leads to if lengths fall evenly from the longest around the mean: with every two rounds a block gets the same sum, u less
+        // than twice the longest in the first; r rounds, and those who get one fewer (never below the longest).  The ordering counts as two tiles,
+        // or as none where it brings the busiest block down by a third.
+        const float most = (float)*s_max_tiles, u = 2.f * (most - (float)units / (float)pairs) * (float)gridDim.x / (float)pairs;
+        const auto after = [&](int r) { return r * most - 0.5f * u * (float)(r * r - (r & 1)); };
+        const int best = (int)ceilf(fmaxf(most, fmaxf(after(rounds), after(rounds - 1))));
+        in_order = in_time(best + 2) || (in_time(best) && 3 * best <= 2 * longest);
+    }
+    if (in_order) {
+        order_sequences(prefix, p.S, p.nkv, order, reinterpret_cast<uint32_t*>(smem + KEYS_OFF), reinterpret_cast<int*>(smem + SORTED_OFF), s_max_load);
+        longest = *s_max_load;
+    }
+    const bool whole = p.mode == 2 || (p.mode == 0 && in_time(longest) && !(per == 1 && longest > (GN > 8 ? 1 : 3)));
     const Share share = {prefix, p.S, p.nkv, u0, u1, (int)blockIdx.x, (int)gridDim.x,
                          in_order ? 2 * (int)gridDim.x - 1 - 2 * (int)blockIdx.x : (int)gridDim.x, whole, in_order ? order : nullptr};
     const uint32_t k_s = smem_u32(smem + K_OFF), v_s = smem_u32(smem + V_OFF), q_s = smem_u32(smem + Q_OFF), p_s = smem_u32(smem + P_OFF);
@@ -583,10 +610,17 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap page_map, const __gr
                     moreq = seg_next(gq, share);
                 }
             };
-            // The first two turns only issue scores (one copy of that code: a kernel's first way through its instructions is a cold one)
+            // Head size 128: the first two turns only issue scores (one copy of that code: a kernel's first way through its instructions is a cold one).
+            // Up to 64 a tile takes half as long and this warp sets the pace: a loop of its own for the turns behind the first two (20 requests of
+            // 8,192 keys, 16 heads of 64 over 16: 143 us in one loop, 137 so).
+            constexpr bool AHEAD = HD == 64;
+            if constexpr (AHEAD) {
+                if (moreq) issue_qk();
+                if (ok && moreq) issue_qk();
+            }
 #pragma unroll 1
-            for (int ip = -2; morep && ok; ++ip) {
-                if (ip >= 0) {
+            for (int ip = AHEAD ? 0 : -2; morep && ok; ++ip) {
+                if (AHEAD || ip >= 0) {
                     const int st = ip & 1, stage = ip % STAGES;
                     ok = mbar_wait(bar_p + st, (uint32_t)(ip >> 1) & 1, abort_flag) && mbar_wait(bar_vfull + stage, (uint32_t)(ip / STAGES) & 1, abort_flag);
                     if (!ok) break;

@@ -408,6 +408,27 @@ def test_attention_decode_of_ragged_batches(S, nh, nkv, window):
         torch.testing.assert_close(out.float(), want, rtol=1.6e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("S,nkv", [(20, 8), (32, 8), (256, 1), (300, 1)])
+@pytest.mark.parametrize("ctx", [128, 300])
+def test_attention_decode_of_batches_of_one_length(S, nkv, ctx):
+    """More pairs than blocks, all of one length (dealt out as they come) and with one that is longer by a tile (in order or not): each against
+    the plain kernel.  Bound as above."""
+    from spyinfer_b200 import kernels
+    nh, hd, page_size = 2 * nkv, 64, 16
+    for longer in (0, 128):
+        lens = [ctx] * (S - 1) + [ctx + longer]
+        width = -(-max(lens) // page_size)
+        pages = torch.randn(S * width, 2, nkv, page_size, hd, device=DEV).to(torch.bfloat16)
+        table = torch.randperm(S * width, device=DEV).view(S, width).to(torch.int32)
+        q = torch.randn(S, nh * hd, device=DEV).to(torch.bfloat16)
+        pos = torch.tensor([c - 1 for c in lens], dtype=torch.int32, device=DEV)
+        starts = torch.arange(S + 1, dtype=torch.int32, device=DEV)
+        want = kernels.attention_generic(q, nh, hd, torch.empty_like(q), pages, table, pos, starts[:S], hd ** -0.5).float()
+        for share in ("auto", "split", "whole"):
+            out = kernels.attention_decode(q, nh, hd, torch.full_like(q, float("nan")), pages, table, pos, starts, S, hd ** -0.5, share=share)
+            torch.testing.assert_close(out.float(), want, rtol=1.6e-2, atol=2e-2)
+
+
 def test_attention_generic_finds_one_far_key():
     """One key among hundreds is made to stand out (its score is far above the rest): the
     output must be that key's value row, wherever it lies: first slot of a page, last slot,
