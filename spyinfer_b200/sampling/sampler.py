@@ -26,11 +26,20 @@ class Sampler:
         tokens = torch.empty(R, dtype=torch.int32, device=logits.device)
         if all(p.temperature == 0.0 for p in params):
             return kernels.sample(logits, tokens)
+        draws = list(draws)
+        if not len(params) == len(draws) == R:                 # a single number would be spread over all rows
+            raise kernels.KernelError("sample: temperature, seed and draw need one entry per row")
+        use_k = any(p.top_k > 0 and p.temperature > 0.0 for p in params)
+        if use_k and max(p.top_k for p in params) > np.iinfo(np.int32).max:     # where no row uses it its size does not matter
+            raise kernels.KernelError("sample: top_k does not fit 32 bits")
         host = np.zeros((4, R), np.int64)                      # one transfer: seeds, draws, temperatures, top_k
-        host[0], host[1] = [p.seed for p in params], draws
+        try:
+            host[0], host[1] = [p.seed for p in params], draws
+        except OverflowError:
+            raise ValueError("sample: seeds and draws must fit 64 bits") from None
         host[2].view(np.float32)[:R] = [p.temperature for p in params]
-        host[3].view(np.int32)[:R] = [p.top_k for p in params]
+        if use_k:
+            host[3].view(np.int32)[:R] = [p.top_k for p in params]
         dev = torch.from_numpy(host).to(logits.device, non_blocking=True)
         s, d, t = dev[0], dev[1], dev[2].view(torch.float32)[:R]
-        k = dev[3].view(torch.int32)[:R] if any(p.top_k > 0 and p.temperature > 0.0 for p in params) else None
-        return kernels.sample(logits, tokens, t, s, d, k)
+        return kernels.sample(logits, tokens, t, s, d, dev[3].view(torch.int32)[:R] if use_k else None)
