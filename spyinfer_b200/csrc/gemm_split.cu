@@ -1,7 +1,7 @@
 // The float32 path's matrix product on the 5th-generation tensor cores:  C[M, N] = A[M, K] . W[N, K]^T with 32-bit A and C and
-// bfloat16 W.  A 32-bit number is exactly the sum of three bfloat16 numbers (24 bits of mantissa in runs of eight, cut, not
-// rounded), so three tensor-core products with the same weight tile give every term of the 32-bit product exactly; what is
-// left is how the terms are summed.
+// bfloat16 W.  A finite 32-bit number is exactly the sum of three bfloat16 numbers (24 bits of mantissa in runs of eight, cut, not
+// rounded), the second and third scaled by powers of two where they are stored, so three tensor-core products with the same weight tile give every term
+// of the 32-bit product exactly; what is left is how the terms are summed.
 //
 // The sums.  The tensor core adds into its accumulator by cutting, which leans toward zero a little at every step (measured:
 // 2.4e-8 of the result after 16 terms of K, 6.7e-8 after 64, 2.3e-7 after 256).  So the leading pieces' accumulator is taken
@@ -46,6 +46,7 @@ constexpr int BK = 64;            // 64 bfloat16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int MAX_STAGES = 8;
 constexpr int MAX_SLICES = 8;     // blocks of a cluster
+constexpr float PIECE_SCALE = 256.f;   // of the second piece; of the third its square (split3)
 
 template <int BN, int HALVES> struct Shape {
     static constexpr int ISSUERS = 2 * HALVES;             // warps that issue products: a half's leading pieces, a half's two others
@@ -256,7 +257,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             tmem_load<C>(acc + (uint32_t)((NB + 1) * BN + c), r2);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < C; ++e) staged[(size_t)(c + e) * S::LD] = sum[c + e] + (__uint_as_float(r1[e]) + __uint_as_float(r2[e]));
+            for (int e = 0; e < C; ++e) staged[(size_t)(c + e) * S::LD] =
+                fmaf(fmaf(__uint_as_float(r2[e]), 1.f / PIECE_SCALE, __uint_as_float(r1[e])), 1.f / PIECE_SCALE, sum[c + e]);   // the scales are powers of two: two rounded additions
         }
         fence_before_sync();
     }
@@ -323,6 +325,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 }
 
 // The three pieces of 32-bit rows: pieces[p][m][k], eight numbers a thread.  Numbers that are not finite go into the first piece alone.
+// The second piece is stored 2^PIECE_SHIFT times as large, the third 2^(2 PIECE_SHIFT): as they are, their last bits would lie below the smallest
+// bfloat16 number (2^-133) for numbers under 2^-110.
 __device__ __forceinline__ void split3(float a, uint32_t& p0, uint32_t& p1, uint32_t& p2)
 {
     const uint32_t u = __float_as_uint(a);
@@ -332,10 +336,10 @@ __device__ __forceinline__ void split3(float a, uint32_t& p0, uint32_t& p1, uint
         return;
     }
     p0 = u >> 16;
-    const float r = a - __uint_as_float(u & 0xffff0000u);          // exact: the low 16 bits of the mantissa
+    const float r = (a - __uint_as_float(u & 0xffff0000u)) * PIECE_SCALE;        // exact: the low 16 bits of the mantissa, below 2^-7 of the number
     const uint32_t ur = __float_as_uint(r);
     p1 = ur >> 16;
-    p2 = __float_as_uint(r - __uint_as_float(ur & 0xffff0000u)) >> 16;   // what is left has at most eight bits
+    p2 = __float_as_uint((r - __uint_as_float(ur & 0xffff0000u)) * PIECE_SCALE) >> 16;   // what is left has at most eight bits
 }
 
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, long long lda, bf16* __restrict__ pieces, int m_rows, int K, int vec)

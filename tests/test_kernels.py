@@ -132,6 +132,20 @@ def test_gemm_split(N, K):
     assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out[out.isinf()], plain[plain.isinf()]) and torch.equal(out.isinf(), plain.isinf())
 
 
+@pytest.mark.parametrize("low", [-100, -110, -116, -120, -126, -132])
+def test_gemm_split_of_the_smallest_numbers(low):
+    """Activations down to the smallest numbers of 32 bits: every bit of them takes part (error no larger than the CUDA-core product's against
+    64 bits, whose own grows where results are no longer normal numbers; 2^-149 is half a unit of those)."""
+    from spyinfer_b200 import kernels
+    a = torch.randn(33, 512, device=DEV) * 2.0 ** (low / 2) * 2.0 ** (low - low / 2)
+    w = (torch.randn(100, 512, device=DEV) * 4).to(torch.bfloat16)
+    ref = a.double() @ w.double().t()
+    split, plain = kernels.gemm_split(a, w, torch.empty(33, 100, device=DEV)), kernels.gemm_simt(a, w, torch.empty(33, 100, device=DEV))
+    assert (split.double() - ref).norm() <= (plain.double() - ref).norm() + ref.numel() ** 0.5 * 2.0 ** -149
+    exact = kernels.gemm_split(a, torch.eye(100, 512, device=DEV).to(torch.bfloat16), torch.empty(33, 100, device=DEV))
+    assert torch.equal(exact, a[:, :100])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,I", [(1, 8), (7, 224), (33, 1000)])
 def test_swiglu(dtype, T, I):
