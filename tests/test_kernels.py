@@ -146,6 +146,21 @@ def test_gemm_split_of_the_smallest_numbers(low):
     assert torch.equal(exact, a[:, :100])
 
 
+@pytest.mark.parametrize("N,K", [(264, 8), (100, 72), (384, 648)])
+def test_gemm_split_of_numbers_that_are_not_finite(N, K):
+    """An infinity or a NaN at the first place, at every border of the terms taken together and at the last one, in the activations and in the
+    weights, and whole rows of them: what a plain sum in order gives (the CUDA-core product's)."""
+    from spyinfer_b200 import kernels
+    places = sorted({0, 7, 8 % K, 15 % K, 16 % K, K - 9 if K > 8 else 0, K - 8, K - 1})
+    a, w = torch.randn(2 * len(places) + 3, K, device=DEV), (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+    for i, k in enumerate(places):
+        a[2 * i, k], a[2 * i + 1, k] = float("inf"), float("nan")
+        w[3 * i + 1, k], w[3 * i + 2, k] = -float("inf"), float("nan")
+    a[-3], a[-2], a[-1] = float("nan"), float("inf"), -float("inf")
+    out, plain = kernels.gemm_split(a, w, torch.empty(len(a), N, device=DEV)), kernels.gemm_simt(a, w, torch.empty(len(a), N, device=DEV))
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out[out.isinf()], plain[plain.isinf()]) and torch.equal(out.isinf(), plain.isinf())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,I", [(1, 8), (7, 224), (33, 1000)])
 def test_swiglu(dtype, T, I):
