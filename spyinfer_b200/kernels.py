@@ -881,6 +881,18 @@ def gemm_split_takes(w: torch.Tensor) -> bool:
             and (w.shape[0] == 1 or w.stride(0) % 8 == 0) and w.data_ptr() % 16 == 0)
 
 
+#: shorter rows stay with ``gemm_simt`` too, whose order of sums is the more exact one there for numbers of very different sizes (8 terms:
+#: error 3.7e-8 against 5.3e-8).  From 64 terms on ``gemm_split`` has half its error or less (64 terms 0.7e-7 against 1.4e-7, 4,096 1.1e-7 against 1.1e-6)
+#: and from 128 on it is the faster one at every size measured (1 to 2,048 rows, 33 to 24,576 outputs); between them it is up to 16 rows (256 outputs, 64 terms, 4 rows: 3.5 us
+#: against 4.5; 300 rows: 9.5 against 5.3)
+GEMM_SPLIT_MIN_IN = 64
+
+
+def gemm_split_pays(w: torch.Tensor) -> bool:
+    """Whether a product with this weight (or part of one) goes to ``gemm_split``: by the weight alone, never by the rows."""
+    return w.shape[1] >= GEMM_SPLIT_MIN_IN and gemm_split_takes(w)
+
+
 def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[M, N] = a[M, K] @ w[N, K]^T`` with 32-bit ``a`` and ``out`` and a bfloat16 weight, on the tensor cores: every
     number of ``a`` as the exact sum of three bfloat16 numbers, the sums taken in 32-bit (K a multiple of 8)."""

@@ -3,7 +3,7 @@
 The kernel is chosen by storage types and shape: bfloat16 activations with bfloat16 weights
 go to the tcgen05 tensor-core kernel when it takes the shape, 32-bit activations with bfloat16
 weights (the float32 path) to the tensor-core kernel that splits every activation into three exact
-bfloat16 pieces, everything else (32-bit weights, odd shapes, weights of a few rows) to the
+bfloat16 pieces, everything else (32-bit weights, odd shapes, weights of a few or of short rows) to the
 32-bit CUDA-core kernel.  The choice depends on the
 weight's shape only, never on the number of rows, so a token's result does not depend on the
 batch it is in.
@@ -46,7 +46,7 @@ class Linear:
         self.out_features, self.in_features = weight.shape
         self.fast = (activation_dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
                      and kernels.tensor_core_gemm_takes(self.out_features, self.in_features))
-        self.split = not self.fast and activation_dtype == torch.float32 and kernels.gemm_split_takes(weight)
+        self.split = not self.fast and activation_dtype == torch.float32 and kernels.gemm_split_pays(weight)
         self.prefetch_bytes = _prefetch_cap()
 
     def modules(self) -> List[str]:
@@ -93,7 +93,7 @@ class Linear:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
         if self.fast and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0:
             return kernels.gemm_tcgen05(x, w, out=out)
-        if self.split and not kernels.gemm_split_takes(w):
+        if self.split and not kernels.gemm_split_pays(w):
             return kernels.gemm_simt(x, w, out)
         return self._plain(x, w, out)
 
