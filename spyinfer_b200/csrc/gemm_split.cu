@@ -10,7 +10,7 @@
 // Relative error (2-norm) against 64 bits at K = 256, 4,096 and 12,288: 0.7e-7, 1.1e-7 and 1.4e-7, where the CUDA-core kernel, one
 // chain over K, has 2.9e-7, 1.1e-6 and 2.0e-6.  (Every 32 terms: 0.7e-7, 1.6e-7 and 2.6e-7, twice as many rounded additions.)
 //
-// A row's result does not depend on M or on its neighbours: K is cut into slices by N and K alone (plan_slices), a slice's sum
+// A row's result does not depend on M or on its neighbours: K is cut into slices by N, K and the device (plan_slices), a slice's sum
 // runs over its K blocks of 64 in order, and the slices are added in order.
 //
 // Bounds.  Few tokens: the weights' way through memory (2 bytes a weight).  Many: the tensor cores (three passes).  Measured with
@@ -471,7 +471,7 @@ double plan_rows(int n_rows, int slices, int clusters, int per, int* rows_out)
     return best;
 }
 
-// Into how many slices K is cut: by N and K alone, for a step of few tokens (whose blocks should fill the device and whose
+// Into how many slices K is cut: by N, K and what the device holds, for a step of few tokens (whose blocks should fill the device and whose
 // weights should arrive evenly); steps of many tokens use the same slices, so that a row's sums never depend on its company.
 int plan_slices(int n_rows, int k_blocks, int* slices_out)
 {

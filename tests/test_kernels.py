@@ -161,6 +161,36 @@ def test_gemm_split_of_numbers_that_are_not_finite(N, K):
     assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out[out.isinf()], plain[plain.isinf()]) and torch.equal(out.isinf(), plain.isinf())
 
 
+@pytest.mark.parametrize("N,K", [(264, 12288), (1000, 4104)])
+def test_gemm_split_of_long_rows(N, K):
+    """K cut into slices that are added in order, its last block of 64 not a whole one: against 64 bits, no further off than the CUDA-core
+    product, and each row as it is alone."""
+    import ctypes
+    from spyinfer_b200 import kernels
+    from spyinfer_b200.csrc import build
+    slices = ctypes.c_int(0)
+    assert build.load("gemm_split").spy_gemm_split_slices(N, K, ctypes.byref(slices)) == 0 and slices.value > 1
+    a = torch.randn(70, K, device=DEV) * torch.exp(2 * torch.randn(70, K, device=DEV))
+    w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+    ref = a.double() @ w.double().t()
+    whole, plain = kernels.gemm_split(a, w, torch.full((70, N), float("nan"), device=DEV)), kernels.gemm_simt(a, w, torch.empty(70, N, device=DEV))
+    assert (whole.double() - ref).norm() <= (plain.double() - ref).norm()
+    for rows in ([0], [69], list(range(20)), list(range(6, 70))):
+        assert torch.equal(kernels.gemm_split(a[rows].contiguous(), w, torch.empty(len(rows), N, device=DEV)), whole[rows])
+
+
+def test_gemm_split_takes_many_rows_in_passes():
+    """More rows than one pass takes, by one and by a whole tile and one: every row as it is alone."""
+    from spyinfer_b200 import kernels
+    w = (torch.randn(100, 72, device=DEV) / 8).to(torch.bfloat16)
+    for M in (kernels.GEMM_SPLIT_ROWS + 1, 2 * kernels.GEMM_SPLIT_ROWS + 65):
+        a = torch.randn(M, 72, device=DEV)
+        whole = kernels.gemm_split(a, w, torch.full((M, 100), float("nan"), device=DEV))
+        for first in range(0, M, 512):
+            part = a[first:first + 512].contiguous()
+            assert torch.equal(kernels.gemm_split(part, w, torch.empty(len(part), 100, device=DEV)), whole[first:first + 512])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,I", [(1, 8), (7, 224), (33, 1000)])
 def test_swiglu(dtype, T, I):
