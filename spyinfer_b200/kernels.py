@@ -871,13 +871,15 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
 
 #: rows that one pass of ``gemm_split`` takes: bounds its scratch (six bytes a row and column of the input)
 GEMM_SPLIT_ROWS = 2048
-#: weights of at most this many rows (a router) stay with ``gemm_simt``, which has a kernel for them
+#: weights of fewer rows (a router) stay with ``gemm_simt``, which has a kernel for them
 GEMM_SPLIT_MIN_OUT = 33
+#: most rows of a weight: its tiles of at least 64 rows are one dimension of the grid
+GEMM_SPLIT_MAX_OUT = 65535 * 64
 
 
 def gemm_split_takes(w: torch.Tensor) -> bool:
     """Whether ``gemm_split`` takes this weight (or part of one): bfloat16, rows on 16-byte borders for TMA."""
-    return (w.dtype == torch.bfloat16 and w.shape[0] >= GEMM_SPLIT_MIN_OUT and w.shape[1] % 8 == 0 and w.shape[1] > 0
+    return (w.dtype == torch.bfloat16 and GEMM_SPLIT_MIN_OUT <= w.shape[0] <= GEMM_SPLIT_MAX_OUT and w.shape[1] % 8 == 0 and w.shape[1] > 0
             and (w.shape[0] == 1 or w.stride(0) % 8 == 0) and w.data_ptr() % 16 == 0)
 
 

@@ -22,3 +22,9 @@ def test_products_of_the_float32_path(N, K, split, monkeypatch):
         went.clear()
         whole.part(torch.zeros(2, K), rows=rows, cols=cols)
         assert went == [("split" if split else "simt", (N, K))]
+
+
+def test_a_weight_of_more_rows_than_the_split_products_grid_takes():
+    """Such a weight (made without memory) stays with the CUDA-core product, which takes any number of rows."""
+    for rows, split in ((65535 * 64, True), (65535 * 64 + 1, False)):
+        assert Linear(torch.empty(rows, 64, dtype=torch.bfloat16, device="meta"), torch.float32).split == split
