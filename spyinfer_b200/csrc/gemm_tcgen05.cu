@@ -12,7 +12,7 @@
 //     fixed order; the number of splits depends only on the shape class, so a token's result
 //     does not depend on the batch beyond rounding;
 //   more tokens (gemm_tcgen05_persistent_kernel): 128 tokens x 256 outputs a tile, one block an SM;
-//   512 tokens and more (gemm_tcgen05_pair_kernel): 256 x 256 tiles on pairs of blocks.
+//   most products of more than 128 tokens (gemm_tcgen05_pair_kernel): 256 weight rows x up to 256 tokens on pairs of blocks.
 // Tails: rows beyond M or N and the end of K are zero-filled by TMA; stores are predicated.
 // K must be a multiple of 8 (16-byte rows for TMA).  No cluster multicast is used.
 //
@@ -750,11 +750,19 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
 }
 
 // The product for many tokens on PAIRS of blocks (cta_group::2): a cluster of two blocks on
-// neighbouring SMs computes one 256 x 256 tile.  Each block loads its 128 rows of X and its 128 of
-// the tile's 256 rows of Y (a third less shared-memory fill per flop than 128 x 256 tiles of
-// single blocks), the leader (rank 0) issues tcgen05.mma.cta_group::2 instructions of 256 x 256 x 16
-// that read both blocks' shared memory and accumulate each block's 128 rows in its own tensor
-// memory; both blocks' four epilogue warps read their halves back.  Barriers: the TMA loads of
+// neighbouring SMs computes one tile of 256 weight rows (X, in the instruction's M slot) and up to 256
+// tokens (Y, in its N slot).  Each block loads its 128 rows of X and its half of the tile's rows of Y (a
+// third less shared-memory fill per flop than 128 x 256 tiles of single blocks), the leader (rank 0)
+// issues tcgen05.mma.cta_group::2 instructions of 256 x tokens x 16 that read both blocks' shared memory
+// and accumulate each block's 128 rows in its own tensor memory; both blocks' four epilogue warps read
+// their halves back and turn them in shared memory on the way out.
+// The weights sit in the M slot because the N slot can be any multiple of 32: the tokens are cut into tiles of
+// nearly equal height (TokenTiles), where whole tiles of 256 tokens in the M slot multiplied up to 255 rows
+// of nothing and fetched the weights once more for them.  What bounds the loop is the tiles' way from L2 to the
+// SMs (11 to 11.7 TB/s whatever the height), so the gain is what the lower tiles need not fetch.  Four products of a layer (us; 256-token
+// tiles in the M slot, then these): 8B sizes, 129 tokens 111 -> 93, 192 113 -> 98, 257 151 -> 142, 513 227 -> 213, 576 229 -> 217, 769 276 ->
+// 260, 1,025 343 -> 326, 2,048 538 -> 539; 14B sizes, 576 366 -> 331, 800 475 -> 436, 1,300 672 -> 638, 1,548 776 -> 742.
+// Barriers: the TMA loads of
 // both blocks complete on the LEADER's full barrier (no multicast of data; the barrier operand is
 // the leader's, which cta_group::2 loads allow); a commit with cluster multicast frees a stage,
 // and publishes an accumulator, in both blocks; the peer's epilogue threads arrive on the
@@ -833,27 +841,119 @@ struct PairWalk {
 constexpr int PAIR_TAIL_MAX_TILES = 512;
 __device__ int g_pair_tail_count[2 * PAIR_TAIL_MAX_TILES];   // [tail tile][block of the pair]: segments of the tile that have arrived
 
-constexpr int PAIR_STAGES = 6;
-constexpr int PAIR_X_BYTES = BM * BK * 2;                    // 128 rows of X
-constexpr int PAIR_STAGE_BYTES = 2 * PAIR_X_BYTES;           // and 128 rows of Y
-constexpr size_t PAIR_SMEM = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+constexpr int PAIR_MAX_STAGES = 10;
+constexpr int PAIR_X_BYTES = BM * BK * 2;                    // 128 rows of weights
+constexpr int PAIR_AREA = 6 * 2 * PAIR_X_BYTES;              // the ring: six stages at 256 tokens a tile, more at fewer
+constexpr int PAIR_STAGED_LD = 36;                           // floats between the tokens of a warp's staged chunk (32 outputs and a pad, rows 16 bytes aligned)
+constexpr int PAIR_STAGED_BYTES = 32 * PAIR_STAGED_LD * 4;   // a warp's 32 tokens
+constexpr size_t PAIR_SMEM = (size_t)PAIR_AREA + 4 * PAIR_STAGED_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+__host__ __device__ constexpr int pair_stage_bytes(int token_rows) { return PAIR_X_BYTES + token_rows / 2 * BK * 2; }
+__host__ __device__ constexpr int pair_stages(int token_rows)
+{
+    const int n = PAIR_AREA / pair_stage_bytes(token_rows);
+    return n < PAIR_MAX_STAGES ? n : PAIR_MAX_STAGES;
+}
+
+// The tokens of a product in `count` tiles whose heights are multiples of 32 and differ by 32 at most: the first `tall` tiles have
+// `rows` tokens, the others 32 fewer, so what the tensor cores multiply beside the tokens themselves is less than 32 rows in all.
+struct TokenTiles {
+    int count, rows, tall;
+    __host__ __device__ int first(int t) const { return t * rows - (t > tall ? (t - tall) * 32 : 0); }
+    __host__ __device__ int height(int t) const { return t < tall ? rows : rows - 32; }
+};
+static inline TokenTiles token_tiles(int M)
+{
+    TokenTiles t;
+    t.count = (M + 255) / 256;
+    const int runs = (M + 31) / 32, each = runs / t.count, more = runs % t.count;
+    t.rows = 32 * (more > 0 ? each + 1 : each);
+    t.tall = more > 0 ? more : t.count;
+    return t;
+}
+
+// Stores one chunk of a tile that has the weights in its rows: this lane holds output x0 + lane of the 32 tokens from y on, `staged`
+// is the warp's own place in shared memory, where the chunk is turned so that it leaves in rows of 16 bytes a lane.  For the gated
+// epilogues lanes 2i and 2i + 1 hold gate row and up row of output x0 / 2 + i: of two tokens at a time the even lane sends the
+// second's gate and finishes the first, the odd lane sends the first's up and finishes the second.
+template <typename TC, int EPI>
+__device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int lane, int x0, int y, int x_rows, int y_rows, const uint32_t (&r)[32],
+                                                   float* staged, float row_bias, const GluArgs& glu)
+{
+    const int count = min(32, y_rows - y);
+    if (x0 >= x_rows || count <= 0) return;    // the same for the whole warp
+    if constexpr (gated_epilogue(EPI)) {
+        constexpr int LD = 24;                 // bfloat16 elements between the tokens: 16 outputs and a pad, rows 16 bytes aligned
+        bf16* turned = reinterpret_cast<bf16*>(staged);
+        const bool odd = (lane & 1) != 0;
+        const int outs = min(16, (x_rows - x0) / 2);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            const float a = __uint_as_float(r[j]) + row_bias, b = __uint_as_float(r[j + 1]) + row_bias;
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            turned[(j + (odd ? 1 : 0)) * LD + (lane >> 1)] = __float2bfloat16_rn(gated_mul<EPI>(odd ? got : a, odd ? b : got, glu));
+        }
+        __syncwarp();
+        TC* dst = base + (size_t)y * ld + x0 / 2;
+        if (outs == 16 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = i * 16 + (lane >> 1), part = lane & 1;
+                if (t < count) *reinterpret_cast<uint4*>(dst + (size_t)t * ld + part * 8) = *reinterpret_cast<const uint4*>(turned + t * LD + part * 8);
+            }
+        } else {
+            for (int i = lane; i < 32 * 16; i += 32) {
+                const int t = i >> 4, o = i & 15;
+                if (t < count && o < outs) dst[(size_t)t * ld + o] = from_f32<TC>(__bfloat162float(turned[t * LD + o]));
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) staged[j * PAIR_STAGED_LD + lane] = EPI == 2 ? relu_squared(__uint_as_float(r[j])) : __uint_as_float(r[j]);
+        __syncwarp();
+        const int outs = min(32, x_rows - x0);
+        TC* dst = base + (size_t)y * ld + x0;
+        if (outs == 32 && (ld & (16 / (int)sizeof(TC) - 1)) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            if constexpr (sizeof(TC) == 4) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int t = i * 4 + (lane >> 3), part = lane & 7;
+                    if (t < count) *reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4) = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int t = i * 8 + (lane >> 2), part = lane & 3;
+                    const float4 v = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 8);
+                    const float4 w = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 8 + 4);
+                    if (t < count)
+                        *reinterpret_cast<uint4*>(dst + (size_t)t * ld + part * 8) =
+                            make_uint4(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w), pack_bf16(w.x, w.y), pack_bf16(w.z, w.w));
+                }
+            }
+        } else if (lane < outs) {
+            for (int t = 0; t < count; ++t) store_elem(dst + (size_t)t * ld + lane, staged[t * PAIR_STAGED_LD + lane]);
+        }
+    }
+    __syncwarp();   // the next chunk's numbers may come
+}
 
 template <typename TC, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, TC* __restrict__ out,
-                         long long ld, int x_rows, int y_rows, int k_blocks, int x_tiles, int num_tiles, int splits, int kb_per_split,
+                         long long ld, int x_rows, int y_rows, int k_blocks, TokenTiles tokens, int num_tiles, int splits, int kb_per_split,
                          long long split_stride, int tail_tiles, int tail_p, int tail_x, float* __restrict__ workspace, int* status, GluArgs glu)
 {
     // splits > 1 (few tiles, 512 tokens or so): a work unit is one tile over one range of kb_per_split K blocks; unit u is
     // tile u % num_tiles of range u / num_tiles, and its 32-bit partial tile goes to out + range * split_stride (the
     // caller sums the ranges in order).  With one range a unit is a whole tile.
-    constexpr int BN = 256;
+    constexpr int BN = 256;                          // tensor-memory columns of an accumulator: as many as the tile has tokens are used
+    const int stages = pair_stages(tokens.rows), stage_bytes = pair_stage_bytes(tokens.rows);   // a lower tile's copies bring spare rows behind its own
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* tiles = smem;
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES);   // the leader's are used
-    uint64_t* empty_bar = full_bar + PAIR_STAGES;   // every block's own
-    uint64_t* acc_full = empty_bar + PAIR_STAGES;   // [2] every block's own
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + PAIR_AREA + 4 * PAIR_STAGED_BYTES);   // the leader's are used
+    uint64_t* empty_bar = full_bar + PAIR_MAX_STAGES;   // every block's own
+    uint64_t* acc_full = empty_bar + PAIR_MAX_STAGES;   // [2] every block's own
     uint64_t* acc_empty = acc_full + 2;             // [2] the leader's are used: 256 arrivals
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -863,7 +963,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     const uint32_t rank = cluster_ctarank();
     const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < PAIR_STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(full_bar + s, 1);
             mbar_init(empty_bar + s, 1);
         }
@@ -884,64 +984,68 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     pdl_launch_dependents();
     if (warp == 0) {
         if (lane == 0) {
-            long long g = 0;
+            int s = 0;
+            uint32_t phase = 0;   // of the ring's round; the first round's waits end at once
             bool ok = true, first = true;
             PairWalk walk(cluster, clusters, num_tiles, splits, kb_per_split, k_blocks, tail_tiles, tail_p, tail_x);
             PairUnit u;
             while (ok && walk.next(u)) {
                 const int tile = u.tile, kb0 = u.kb0, nkb = u.nkb;
-                const int x0 = (tile % x_tiles) * (2 * BM) + (int)rank * BM, y0 = (tile / x_tiles) * BN + (int)rank * (BN / 2);
+                const int ty = tile % tokens.count;
+                const int x0 = (tile / tokens.count) * (2 * BM) + (int)rank * BM, y0 = tokens.first(ty) + (int)rank * (tokens.height(ty) / 2);
                 int kb = 0;
                 if (first) {
-                    // the weights (Y) of the first stages are requested before the wait for the kernels ahead in the stream
-                    const int pre = min(nkb, PAIR_STAGES);
+                    // the weights of the first stages are requested before the wait for the kernels ahead in the stream
+                    const int pre = min(nkb, stages);
                     for (int i = 0; i < pre; ++i) {
-                        if (rank == 0) mbar_expect_tx(full_bar + i, 2 * PAIR_STAGE_BYTES);
-                        tma_load_2d_pair(smem_u32(tiles + (size_t)i * PAIR_STAGE_BYTES + PAIR_X_BYTES), &map_y, (kb0 + i) * BK, y0, map_to_rank(smem_u32(full_bar + i), 0));
+                        if (rank == 0) mbar_expect_tx(full_bar + i, 2u * stage_bytes);
+                        tma_load_2d_pair(smem_u32(tiles + (size_t)i * stage_bytes), &map_x, (kb0 + i) * BK, x0, map_to_rank(smem_u32(full_bar + i), 0));
                     }
                     pdl_wait();
                     for (int i = 0; i < pre; ++i)
-                        tma_load_2d_pair(smem_u32(tiles + (size_t)i * PAIR_STAGE_BYTES), &map_x, (kb0 + i) * BK, x0, map_to_rank(smem_u32(full_bar + i), 0));
+                        tma_load_2d_pair(smem_u32(tiles + (size_t)i * stage_bytes + PAIR_X_BYTES), &map_y, (kb0 + i) * BK, y0, map_to_rank(smem_u32(full_bar + i), 0));
                     kb = pre;
-                    g = pre;
+                    if (pre == stages) phase = 1;
+                    else s = pre;
                     first = false;
                 }
-                for (; kb < nkb; ++kb, ++g) {
-                    const int s = (int)(g % PAIR_STAGES);
-                    const uint32_t phase = (uint32_t)(g / PAIR_STAGES) & 1;
-                    if (g >= PAIR_STAGES && !mbar_wait(empty_bar + s, phase ^ 1, abort_flag)) { ok = false; break; }
-                    uint8_t* xs = tiles + (size_t)s * PAIR_STAGE_BYTES;
-                    if (rank == 0) mbar_expect_tx(full_bar + s, 2 * PAIR_STAGE_BYTES);   // both blocks' bytes
+                for (; kb < nkb; ++kb) {
+                    if (!mbar_wait(empty_bar + s, phase ^ 1, abort_flag)) { ok = false; break; }
+                    uint8_t* xs = tiles + (size_t)s * stage_bytes;
+                    if (rank == 0) mbar_expect_tx(full_bar + s, 2u * stage_bytes);   // both blocks' bytes
                     const uint32_t leader_full = map_to_rank(smem_u32(full_bar + s), 0);
                     tma_load_2d_pair(smem_u32(xs), &map_x, (kb0 + kb) * BK, x0, leader_full);
                     tma_load_2d_pair(smem_u32(xs + PAIR_X_BYTES), &map_y, (kb0 + kb) * BK, y0, leader_full);
+                    if (++s == stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
                 }
             }
             if (first) pdl_wait();
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = instr_desc_bf16(2 * BM, BN, false, false);
-            long long g = 0;
+            int s = 0;
+            uint32_t phase = 0;
             int i = 0;
             bool ok = true;
             PairWalk walk(cluster, clusters, num_tiles, splits, kb_per_split, k_blocks, tail_tiles, tail_p, tail_x);
             PairUnit u;
             for (; ok && walk.next(u); ++i) {
                 const int nkb = u.nkb;
+                const uint32_t idesc = instr_desc_bf16(2 * BM, tokens.height(u.tile % tokens.count), false, false);
                 const int buf = i & 1;
                 const uint32_t aph = (uint32_t)(i >> 1) & 1;
                 if (i >= 2) ok = mbar_wait(acc_empty + buf, aph ^ 1, abort_flag);   // both blocks' epilogues have read this buffer's last tile
                 if (!ok) break;
                 fence_after_sync();
                 const uint32_t acc = tmem_base + (uint32_t)buf * BN;
-                for (int kb = 0; kb < nkb; ++kb, ++g) {
-                    const int s = (int)(g % PAIR_STAGES);
-                    const uint32_t phase = (uint32_t)(g / PAIR_STAGES) & 1;
+                for (int kb = 0; kb < nkb; ++kb) {
                     ok = mbar_wait(full_bar + s, phase, abort_flag);
                     if (!ok) break;
                     fence_after_sync();
-                    const uint8_t* xs = tiles + (size_t)s * PAIR_STAGE_BYTES;
+                    const uint8_t* xs = tiles + (size_t)s * stage_bytes;
                     const uint64_t dx = desc_k_major(smem_u32(xs)), dy = desc_k_major(smem_u32(xs + PAIR_X_BYTES));
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -949,12 +1053,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         umma_pair(acc, dx + adv, dy + adv, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     }
                     umma_commit_pair(empty_bar + s);
+                    if (++s == stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
                 }
                 if (ok) umma_commit_pair(acc_full + buf);
             }
         }
     } else {
         const int quarter = warp & 3;
+        float* staged = reinterpret_cast<float*>(smem + PAIR_AREA + quarter * PAIR_STAGED_BYTES);
         pdl_wait();   // the output buffer may still be in use by a kernel ahead in the stream
         int i = 0;
         bool ok = true;
@@ -966,19 +1075,20 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             TC* unit_out = out + (size_t)u.range * split_stride;
             const int buf = i & 1;
             const uint32_t aph = (uint32_t)(i >> 1) & 1;
-            const int x0 = (tile % x_tiles) * (2 * BM) + (int)rank * BM, y0 = (tile / x_tiles) * BN;
+            const int x0 = (tile / tokens.count) * (2 * BM) + (int)rank * BM + quarter * 32, ty = tile % tokens.count;   // the warp's first output
+            const int y0 = tokens.first(ty), height = tokens.height(ty), y_end = min(y_rows, y0 + height);
+            const float row_bias = (EPI == 4 && glu.bias != nullptr && x0 + lane < x_rows) ? glu.bias[x0 + lane] : 0.f;
             ok = mbar_wait(acc_full + buf, aph, abort_flag);
             if (!ok) break;
             fence_after_sync();
             const int row = quarter * 32 + lane;
-            const int x = x0 + row;
             if (!u.partial) {
 #pragma unroll 1
-                for (int c = 0; c < BN; c += 32) {
+                for (int c = 0; c < height; c += 32) {
                     uint32_t r[32];
                     tmem_load<32>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c), r);
                     tmem_wait_ld();
-                    store_chunk_normal<TC, EPI>(unit_out, ld, x, y0 + c, x_rows, y_rows, r, glu);
+                    store_chunk_turned<TC, EPI>(unit_out, ld, lane, x0, y0 + c, x_rows, y_end, r, staged, row_bias, glu);
                 }
                 fence_before_sync();
                 if (rank == 0) mbar_arrive(acc_empty + buf);
@@ -990,7 +1100,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             const int segments = tail_p + (tail_x < k_blocks ? 1 : 0);   // of every tail tile, in the order of their K ranges
             float* mine = workspace + (((size_t)tile_rel * (tail_p + 1) + u.seg) * 2 + rank) * STREAM_TILE_FLOATS;
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
+            for (int c = 0; c < height; c += 32) {
                 uint32_t r[32];
                 tmem_load<32>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c), r);
                 tmem_wait_ld();
@@ -1014,7 +1124,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             if (!last) continue;
             __threadfence();
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
+            for (int c = 0; c < height; c += 32) {
                 float4 sum[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1049,7 +1159,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                     r[4 * j + 2] = __float_as_uint(sum[j].z);
                     r[4 * j + 3] = __float_as_uint(sum[j].w);
                 }
-                store_chunk_normal<TC, EPI>(unit_out, ld, x, y0 + c, x_rows, y_rows, r, glu);
+                store_chunk_turned<TC, EPI>(unit_out, ld, lane, x0, y0 + c, x_rows, y_end, r, staged, row_bias, glu);
             }
             if (row == 0) g_pair_tail_count[tile_rel * 2 + (int)rank] = 0;   // for the next product: nobody else touches it in this one
         }
@@ -1340,7 +1450,7 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
     CUtensorMap mx, my;
     if (swap) {
         if (make_map(&mx, W, N, K, ldw, plan.tile_rows) || make_map(&my, A, M, K, lda, bn)) return 1;
-    } else {
+    } else if (plan.kind == SINGLE) {
         if (make_map(&mx, A, M, K, lda, BM) || make_map(&my, W, N, K, ldw, bn)) return 1;
     }
     const int x_rows = swap ? N : M, y_rows = swap ? M : N;
@@ -1352,10 +1462,9 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
     // blocks, which share the K blocks of their 128 x 256 tiles out over all SMs
     if (plan.kind == PAIRS) {
         // many tokens, one pass over K, at least two 256-row tiles: pairs of blocks on 256 x 256 tiles
-        CUtensorMap my_half;
-        if (make_map(&my_half, W, N, K, ldw, BM)) return 1;
-        const int x_tiles = (M + 2 * BM - 1) / (2 * BM), y_tiles = (N + 255) / 256;
-        const long long num_tiles = (long long)x_tiles * y_tiles;
+        const TokenTiles tokens = token_tiles(M);
+        if (make_map(&mx, W, N, K, ldw, BM) || make_map(&my, A, M, K, lda, tokens.rows / 2)) return 1;
+        const long long num_tiles = (long long)((N + 2 * BM - 1) / (2 * BM)) * tokens.count;
         if (num_tiles > 0x7fffffffLL) SPY_FAIL("gemm_tcgen05: %lld tiles exceed the kernel's range", num_tiles);
         static int clusters_of_device[SPY_MAX_DEVICES] = {};
         int& clusters_max = clusters_of_device[spy_device()];
@@ -1388,8 +1497,8 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
         const int kb_per_split = (k_blocks + splits - 1) / splits;
         if (splits > 1) {
             // ranges of K: 32-bit partial tiles into the scratch, [range][M][N]
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (float*)scratch,
-                               (long long)N, M, N, k_blocks, x_tiles, (int)num_tiles, splits, kb_per_split, split_stride, 0, 1, 0, (float*)nullptr, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (float*)scratch,
+                               (long long)N, N, M, k_blocks, tokens, (int)num_tiles, splits, kb_per_split, split_stride, 0, 1, 0, (float*)nullptr, status, glu);
             SPY_CHECK_LAUNCH("gemm_tcgen05 (pairs, K ranges)");
             if (!defer_reduce) {
                 if (int rc = reduce_splits(scratch, C, c_dtype, ldc, M, N, splits, stream)) return rc;
@@ -1413,23 +1522,23 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
             }
         }
         if (epilogue == 2)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 2>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (bf16*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 2>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (epilogue == 1)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 1>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (bf16*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 1>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (epilogue == 3)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 3>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (bf16*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 3>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (epilogue == 4)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 4>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (bf16*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 4>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (c_dtype == SPY_F32)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (float*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (float*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my_half, (bf16*)C, ldc,
-                               M, N, k_blocks, x_tiles, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
+            spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
+                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         SPY_CHECK_LAUNCH("gemm_tcgen05 (pairs)");
         return 0;
     }

@@ -860,6 +860,31 @@ def test_gemm_tcgen05_shares_the_last_round_of_tiles(M, N, K, epilogue, out_dtyp
         assert (outs[0].float() - outs[2].float()).abs().max().item() <= 2.0 ** -6 * max(1.0, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("epilogue,out_dtype", [(None, torch.bfloat16), (None, torch.float32), ("swiglu", torch.bfloat16), ("relu2", torch.bfloat16)])
+@pytest.mark.parametrize("M", [129, 160, 161, 257, 320, 513, 545, 800, 1025])
+def test_gemm_tcgen05_cuts_many_tokens_into_tiles_of_several_heights(M, epilogue, out_dtype):
+    """Pairs of blocks at token counts around the edges of their token tiles (heights of 160 to 256, the last ones of a product 32
+    lower): every token once, with each epilogue; an N that ends inside a warp's 32 outputs and rows that are no multiple of 16 bytes."""
+    from spyinfer_b200 import kernels
+    torch.manual_seed(M)
+    N, K = 9612, 136
+    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+    ref = a.float() @ w.float().t()
+    if epilogue == "swiglu":
+        ref = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
+    elif epilogue == "relu2":
+        ref = ref.clamp(min=0) ** 2
+    out = torch.full((M + 1, ref.shape[1]), 77.0, device=DEV, dtype=out_dtype)       # the row behind the last stays what it is
+    kernels.gemm_tcgen05(a, w, out[:M], epilogue=epilogue)
+    torch.cuda.synchronize()
+    assert bool((out[M] == 77.0).all())
+    if out_dtype == torch.float32:
+        torch.testing.assert_close(out[:M], ref, rtol=1e-4, atol=2e-4)
+    else:
+        torch.testing.assert_close(out[:M].float(), ref.to(torch.bfloat16).float(), rtol=1.6e-2, atol=4e-3)
+
+
 @pytest.mark.parametrize("M,I,K", [(3, 100, 64), (16, 328, 200), (40, 1000, 136), (64, 6144, 512), (70, 520, 264), (128, 12288, 1024), (130, 520, 264), (300, 12288, 1024),
                                    (520, 1000, 136), (1100, 2304, 512)])   # 512 rows and more: pairs of blocks on 256 x 256 tiles
 def test_gemm_tcgen05_swiglu_epilogue(M, I, K):
