@@ -52,7 +52,25 @@ struct ScanArgs {
     int H, dk, dv;
     float q_scale, cap;     // cap: mLSTM: the gates' cap;   gated linear attention: 1 / tau
     int* status;
+    const int* flags;       // null, or what the chunks' kernels left (see "runs of tokens as products"): the requests that those took are not walked here
 };
+
+// Which form a request takes where both run: see "runs of tokens as products" below.
+constexpr int CHUNK_MIN = 48;
+template <int MODE> struct ChunkOf { static constexpr int C = MODE == 1 ? 32 : 64; };   // tokens of a chunk
+// A chunk's place in the scratch: chunk j of sequence s at q_start[s] / C + s + j, which no two chunks share.
+__device__ __forceinline__ int chunk_slot(int t_begin, int seq, int C) { return t_begin / C + seq; }
+// Whether head h of a request takes the products: every block that asks gets the same answer.
+template <int MODE>
+__device__ __forceinline__ bool takes_chunks(const ScanArgs& A, int seq, int h, int t_begin, int t_end)
+{
+    constexpr int C = ChunkOf<MODE>::C;
+    if (A.flags == nullptr || t_end - t_begin < CHUNK_MIN) return false;
+    const int first = chunk_slot(t_begin, seq, C), n = (t_end - t_begin + C - 1) / C;
+    int bad = 0;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) bad |= A.flags[(size_t)(first + j) * A.H + h];
+    return __syncthreads_or(bad) == 0;
+}
 
 constexpr int THREADS = 256;      // 8 warps; warp w owns the columns 4w .. 4w + 3 of the tile, lane = 4 * (row group) + (column of the four)
 
@@ -93,7 +111,7 @@ __global__ void __launch_bounds__(THREADS, NR <= 8 ? 2 : 1) scan_kernel(ScanArgs
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col = warp * CW + lane % CW, rg = lane / CW, r0 = rg * NR;
     const int t_begin = A.q_start[seq], t_end = A.q_start[seq + 1];
-    if (t_begin >= t_end) return;
+    if (t_begin >= t_end || takes_chunks<MODE>(A, seq, h, t_begin, t_end)) return;
     const int slot = A.state_slot[seq];
     if (slot < 0 || slot >= A.num_slots) {
         if (tid == 0) report_status(A.status, SPY_STATUS_BAD_PAGE, t_begin);
@@ -531,6 +549,772 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
     }
 }
 
+// ---- runs of tokens as products --------------------------------------------------------------------------------------------
+//
+// A request that brings CHUNK_MIN tokens or more is walked in chunks of C tokens instead of token by token.  Written out over a
+// chunk, each recurrence gives the chunk's outputs and the state behind it as products with the state S ahead of it and the
+// chunk's values V, whose other factors do not depend on S:
+//   matrix memory:  o_t = (alpha_t (P V)_t + beta_t S^T q_t) / ...,   S' = g S + K^T diag(kappa) V,   P_ts = exp(F_t - F_s + i_s - l_t) q_t . k_s
+//                   (F: the forget gates' sums from the chunk's start, l: the running maximum as if the chunk were the first; the true
+//                   maximum is max(F_t + m, l_t), alpha and beta are what is left of l and of F + m under it: every exponent is at most 0);
+//   linear attention:  o_t = (P V)_t + S^T (q_t a_1..a_t),   S' = diag(a_1..a_C) S + (k_s a_s+1..a_C)^T V,   P_ts = sum over channels of q_t k_s a_s+1..a_t;
+//   delta rule:     with A_t = w_1..w_t, p_t = u_t A_t-1, b_s = r_s u_s / A_s, c_s = k_s / A_s, g_t = q_t A_t (w is above exp(-exp(-1/2)) = 0.545, so A_32
+//                   above 3.7e-9) and (I + L) [P' | M'] = [p | M], L = p b^T and M = p c^T below the diagonal:
+//                   [o; S'] = W [S; V] with the rows g - X P' and Y - X M' (X = g b^T, Y = g c^T up to the diagonal) for the outputs and
+//                   A_C (I - b^T P') and A_C (c^T - b^T M') for the state.
+// (The delta rule's form inverts a unit triangular matrix, as the published chunked forms of delta rules do, after Yang et al., 2024; the
+// decays of linear attention are taken relative to sub-blocks of 16 tokens, so that no factor exceeds 1.)
+//
+// Two kernels: chunk_*_kernel makes these factors, a block a (chunk, head), all chunks side by side; walk_*_kernel carries S through a
+// request's chunks, a block 16 value columns of a (request, head).  What bounds the walk is the CUDA cores' additions (a chunk of 64
+// tokens at 128 x 16 needs 330 K of them) and the shared-memory reads beside them; the token-by-token kernel above spends 270
+// to 300 ns a token, nearly all of it waiting.
+// MEASURED_PLACEHOLDER
+//
+// Which form a request takes is decided on the device by one rule (takes_chunks) in both kernels: runs of fewer than CHUNK_MIN tokens and
+// requests with a number among their q, k, v, decays or gates that is not below HUGE_INPUT in magnitude (or is no number) are walked token
+// by token as before: in the products an infinity of a later token would meet the zeros of an earlier one.
+constexpr float HUGE_INPUT = 1e10f;
+constexpr int WALK_COLS = 16;          // value columns a block of the walk owns
+constexpr int WALK_LD = WALK_COLS + 4; // floats between the rows of a tile of them in shared memory
+
+struct ChunkArgs {
+    ScanArgs s;
+    float* work;       // [slots][H][chunk_floats(mode, dk)]
+    int* flags;        // [slots][H]: the chunk holds a number that keeps its request off the products
+    int num_seqs;
+};
+
+// what a chunk of one head takes of the scratch, in floats
+__host__ __device__ constexpr int chunk_floats(int mode, int dk)
+{
+    return mode == 0 ? 64 * 64 + 4 * 64 + dk : (mode == 2 ? 64 * 64 + 2 * 64 * dk + dk : (dk + 32) * (dk + 32));
+}
+
+// The (sequence, chunk) of a place in the scratch; false where there is none.
+template <int C>
+__device__ __forceinline__ bool chunk_of_slot(const ChunkArgs& A, int slot, int& seq, int& t0, int& n_tok)
+{
+    int lo = 0, hi = A.num_seqs;           // the last sequence whose first place is at most `slot`
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (chunk_slot(A.s.q_start[mid], mid, C) <= slot) lo = mid;
+        else hi = mid;
+    }
+    seq = lo;
+    const int t_begin = A.s.q_start[lo], t_end = A.s.q_start[lo + 1];
+    t0 = t_begin + (slot - chunk_slot(t_begin, lo, C)) * C;
+    n_tok = min(C, t_end - t0);
+    return slot >= chunk_slot(t_begin, lo, C) && t0 < t_end && t_end - t_begin >= CHUNK_MIN;
+}
+
+__device__ __forceinline__ bool huge(float x) { return !(fabsf(x) < HUGE_INPUT); }
+__device__ __forceinline__ bool huge4(float4 v) { return huge(v.x) | huge(v.y) | huge(v.z) | huge(v.w); }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s)))); }
+
+// Brings rows [0, n_tok) of DK columns into shared memory (rows of LD floats), zeros up to C rows; true if a number is huge.
+template <int C, int DK, int LD>
+__device__ __forceinline__ bool load_rows(float* dst, const float* src, long long ld, int n_tok)
+{
+    bool bad = false;
+    for (int idx = threadIdx.x; idx < C * (DK / 4); idx += THREADS) {
+        const int t = idx / (DK / 4), c = 4 * (idx - t * (DK / 4));
+        const float4 v = t < n_tok ? ld4(src + (size_t)t * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        bad |= huge4(v);
+        st4(dst + t * LD + c, v);
+    }
+    return bad;
+}
+__device__ __forceinline__ bool huge_values(const ScanArgs& A, int h, int t0, int n_tok)
+{
+    bool bad = false;
+    const int quads = A.dv >> 2;
+    for (int idx = threadIdx.x; idx < n_tok * quads; idx += THREADS) {
+        const int t = idx / quads, c = 4 * (idx - t * quads);
+        bad |= huge4(ld4(A.proj + (size_t)(t0 + t) * A.ld + A.off_v + (size_t)h * A.dv + c));
+    }
+    return bad;
+}
+
+template <int DK>
+__global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
+{
+    constexpr int C = 64, LD = DK + 4;
+    extern __shared__ __align__(16) float sm[];
+    float *q_s = sm, *k_s = sm + C * LD;
+    __shared__ double from_s[C], to_s[C];          // i_s - F_s and F_t - l_t
+    __shared__ float kappa_s[C];
+    pdl_enter();
+    int seq, t0, n_tok;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    const ScanArgs& a = A.s;
+    float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(0, DK);
+    float *P = mine, *F = mine + C * C, *loc = F + C, *kap = loc + C, *psum = kap + C, *ksum = psum + C;
+    const float* rows = a.proj + (size_t)t0 * a.ld;
+    bool bad = load_rows<C, DK, LD>(q_s, rows + a.off_q + h * DK, a.ld, n_tok);
+    bad |= load_rows<C, DK, LD>(k_s, rows + a.off_k + h * DK, a.ld, n_tok);
+    bad |= huge_values(a, h, t0, n_tok);
+    if (warp == 0) {
+        // the gates' sums and the running maximum in 64-bit (differences of sums are taken below); a lane owns tokens 2 lane and 2 lane + 1
+        double f[2], e[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = 2 * lane + j;
+            float ig = -INFINITY, fg = 0.f;
+            if (t < n_tok) {
+                const float x1 = rows[(size_t)t * a.ld + a.off_x1 + h] + a.bias1[h], x2 = rows[(size_t)t * a.ld + a.off_x2 + h] + a.bias2[h];
+                bad |= isnan(x1) || isnan(x2);
+                ig = a.cap * tanhf(x1 / a.cap);
+                fg = log_sigmoidf_(a.cap * tanhf(x2 / a.cap));
+            }
+            f[j] = fg;
+            e[j] = ig;
+        }
+        double sum = f[0] + f[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
+        }
+        const double F0 = sum - f[1], F1 = sum;
+        e[0] -= F0;
+        e[1] -= F1;
+        double most = fmax(e[0], e[1]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, most, o);
+            if (lane >= o) most = fmax(most, up);
+        }
+        double before = __shfl_up_sync(0xffffffffu, most, 1);
+        if (lane == 0) before = -INFINITY;
+        const double l0 = F0 + fmax(before, e[0]), l1 = F1 + most;
+        const double F_end = __shfl_sync(0xffffffffu, F1, 31), l_end = __shfl_sync(0xffffffffu, l1, 31);     // padding tokens change neither
+        from_s[2 * lane] = e[0];
+        from_s[2 * lane + 1] = e[1];
+        to_s[2 * lane] = F0 - l0;
+        to_s[2 * lane + 1] = F1 - l1;
+        const float k0 = expf((float)(F_end - l_end + e[0])), k1 = expf((float)(F_end - l_end + e[1]));
+        kappa_s[2 * lane] = k0;
+        kappa_s[2 * lane + 1] = k1;
+        *reinterpret_cast<float2*>(F + 2 * lane) = make_float2((float)F0, (float)F1);
+        *reinterpret_cast<float2*>(loc + 2 * lane) = make_float2((float)l0, (float)l1);
+        *reinterpret_cast<float2*>(kap + 2 * lane) = make_float2(k0, k1);
+    }
+    const int any = __syncthreads_or(bad);
+    if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
+    // P: a thread has 4 x 4 of the 64 x 64, rows 4 ty + i, columns tx + 16 j
+    const int tx = tid & 15, ty = tid >> 4;
+    float acc[4][4] = {};
+    for (int c = 0; c < DK; c += 4) {
+        float4 kk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kk[j] = ld4(k_s + (tx + 16 * j) * LD + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 qq = ld4(q_s + (4 * ty + i) * LD + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = dot4(qq, kk[j], acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i;
+        float row = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int s = tx + 16 * j;
+            const float p = s <= t ? expf((float)(to_s[t] + from_s[s])) * (acc[i][j] * a.q_scale) : 0.f;
+            P[t * C + s] = p;
+            row += p;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) row += __shfl_xor_sync(0xffffffffu, row, o);
+        if (tx == 0) psum[t] = row;
+    }
+    for (int c = tid; c < DK; c += THREADS) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < C; ++t) s = fmaf(kappa_s[t], k_s[t * LD + c], s);
+        ksum[c] = s;
+    }
+}
+
+template <int DK>
+__global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
+{
+    constexpr int C = 64, LD = DK + 4, B = 16;     // sub-blocks of 16 tokens
+    extern __shared__ __align__(16) float sm[];
+    float *q_s = sm, *k_s = q_s + C * LD, *a_s = k_s + C * LD;
+    pdl_enter();
+    int seq, t0, n_tok;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    const ScanArgs& a = A.s;
+    float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(2, DK);
+    float *P = mine, *Q = mine + C * C, *K = Q + C * DK, *dec = K + C * DK;
+    const float* rows = a.proj + (size_t)t0 * a.ld;
+    bool bad = load_rows<C, DK, LD>(q_s, rows + a.off_q + h * DK, a.ld, n_tok);
+    bad |= load_rows<C, DK, LD>(k_s, rows + a.off_k + h * DK, a.ld, n_tok);
+    bad |= huge_values(a, h, t0, n_tok);
+    for (int idx = tid; idx < C * DK; idx += THREADS) {
+        const int t = idx / DK, c = idx - t * DK;
+        float d = 1.f;
+        if (t < n_tok) {
+            const float z = a.extra[(size_t)(t0 + t) * a.H * DK + h * DK + c] + a.bias2[h * DK + c];
+            bad |= isnan(z);
+            d = expf(log_sigmoidf_(z) * a.cap);
+        }
+        a_s[t * LD + c] = d;
+    }
+    const int any = __syncthreads_or(bad);
+    if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
+    // inside a sub-block: k_s carried from its token on, a decay at a time; a warp takes every eighth token, a lane DK / 32 channels
+    for (int s = warp; s < C; s += THREADS / 32) {
+        const int end = (s / B + 1) * B;
+        constexpr int E = DK / 32;
+        float w[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) w[e] = k_s[s * LD + lane + 32 * e];
+        float keep = 0.f;                          // lane t - s keeps P_ts
+        for (int t = s; t < end; ++t) {
+            float d = 0.f;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (t > s) w[e] *= a_s[t * LD + lane + 32 * e];
+                d = fmaf(w[e], q_s[t * LD + lane + 32 * e], d);
+            }
+            d = warp_sum(d);
+            if (lane == t - s) keep = d;
+        }
+        if (s + lane < end) P[(s + lane) * C + s] = keep * a.q_scale;
+    }
+    for (int idx = tid; idx < C * C; idx += THREADS)
+        if ((idx & (C - 1)) > idx / C) P[idx] = 0.f;
+    __syncthreads();
+    // q from its sub-block's start, k to its sub-block's end; a_s's last row of a sub-block then holds the sub-block's product
+    for (int idx = tid; idx < DK * (C / B); idx += THREADS) {
+        const int c = idx % DK, b0 = idx / DK * B;
+        float run = 1.f;
+        for (int t = b0; t < b0 + B; ++t) {
+            run *= a_s[t * LD + c];
+            q_s[t * LD + c] *= run * a.q_scale;
+        }
+        float back = 1.f;
+        for (int t = b0 + B - 1; t >= b0; --t) {
+            k_s[t * LD + c] *= back;
+            back *= a_s[t * LD + c];
+        }
+        a_s[(b0 + B - 1) * LD + c] = run;
+    }
+    __syncthreads();
+    // across sub-blocks, one after the other: the keys so far reach the end of the sub-block ahead.  A thread has row t = b B + tid / 16
+    // and the columns tid % 16 + 16 j.
+    for (int b = 1; b < C / B; ++b) {
+        const int t = b * B + (tid >> 4), s0 = tid & 15;
+        float acc[C / B - 1] = {};
+        for (int c = 0; c < DK; c += 4) {
+            const float4 qq = ld4(q_s + t * LD + c);
+#pragma unroll
+            for (int j = 0; j < C / B - 1; ++j)
+                if (j < b) acc[j] = dot4(qq, ld4(k_s + (s0 + 16 * j) * LD + c), acc[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < C / B - 1; ++j)
+            if (j < b) P[t * C + s0 + 16 * j] = acc[j];
+        __syncthreads();
+        for (int idx = tid; idx < b * B * DK; idx += THREADS) {
+            const int s = idx / DK, c = idx - s * DK;
+            k_s[s * LD + c] *= a_s[(b * B + B - 1) * LD + c];
+        }
+        __syncthreads();
+    }
+    for (int idx = tid; idx < C * DK; idx += THREADS) {
+        const int t = idx / DK, c = idx - t * DK;
+        float q = q_s[t * LD + c];
+        for (int b = 0; b < t / B; ++b) q *= a_s[(b * B + B - 1) * LD + c];
+        Q[idx] = q;
+        K[idx] = k_s[t * LD + c];
+        if (t == 0) {
+            float d = 1.f;
+#pragma unroll
+            for (int b = 0; b < C / B; ++b) d *= a_s[(b * B + B - 1) * LD + c];
+            dec[c] = d;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
+{
+    constexpr int C = 32, D = 64, LD = D + 4, R = D + C, LDM = R + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* pg = sm;                    // [2 C][LD]: p, then g (first: q)
+    float* bc = pg + 2 * C * LD;       // [2 C][LD]: b, then c (first: the rates, k)
+    float* PM = bc + 2 * C * LD;       // [C][LDM]: P' | M' (first: the decays)
+    float* XB = PM + C * LDM;          // [C][LDM]: token s: X_ts of the outputs t, then b_s of the state's rows
+    float* L = XB + C * LDM;           // [C][C + 1]
+    float* Y = L + C * (C + 1);        // [C][C + 1]
+    __shared__ float inv_s[C], last_s[D];
+    pdl_enter();
+    int seq, t0, n_tok;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    const ScanArgs& a = A.s;
+    float* W = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(1, D);
+    const float* rows = a.proj + (size_t)t0 * a.ld;
+    bool bad = load_rows<C, D, LD>(pg + C * LD, rows + a.off_q + h * D, a.ld, n_tok);
+    bad |= load_rows<C, D, LD>(bc + C * LD, rows + a.off_k + h * D, a.ld, n_tok);
+    bad |= huge_values(a, h, t0, n_tok);
+    for (int idx = tid; idx < C * D; idx += THREADS) {
+        const int t = idx / D, c = idx - t * D;
+        float rate = 0.f, w = 1.f;
+        if (t < n_tok) {
+            const float x1 = rows[(size_t)t * a.ld + a.off_x1 + h * D + c] + a.bias1[h * D + c];
+            const float x2 = a.extra[(size_t)(t0 + t) * a.H * D + h * D + c] + a.bias2[h * D + c];
+            bad |= isnan(x1) || isnan(x2);
+            rate = sigmoidf_(x1);
+            w = expf(-0.60653065971263342f * sigmoidf_(x2));     // exp(-1/2) = 0.6065...
+        }
+        bc[t * LD + c] = rate;
+        PM[t * LDM + c] = w;
+    }
+    const int any = __syncthreads_or(bad);
+    if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
+    for (int t = warp; t < C; t += THREADS / 32) {
+        const float k0 = bc[(C + t) * LD + lane], k1 = bc[(C + t) * LD + lane + 32];
+        const float sq = warp_sum(k0 * k0 + k1 * k1);
+        if (lane == 0) inv_s[t] = 1.0f / sqrtf(sq + 1e-6f);
+    }
+    __syncthreads();
+    if (tid < D) {
+        float run = 1.f;
+        for (int t = 0; t < C; ++t) {
+            const float k = bc[(C + t) * LD + tid], u = k * inv_s[t], rate = bc[t * LD + tid];
+            pg[t * LD + tid] = u * run;
+            run *= PM[t * LDM + tid];
+            const float back = 1.0f / run;
+            pg[(C + t) * LD + tid] *= run;
+            const float b = rate * u * back;
+            bc[t * LD + tid] = b;
+            bc[(C + t) * LD + tid] = k * back;
+            XB[t * LDM + C + tid] = b;
+        }
+        last_s[tid] = run;
+    }
+    __syncthreads();
+    {
+        // [p; g] [b; c]^T, 64 x 64: rows 4 ty + i, columns tx + 16 j
+        const int tx = tid & 15, ty = tid >> 4;
+        float acc[4][4] = {};
+        for (int c = 0; c < D; c += 4) {
+            float4 kk[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) kk[j] = ld4(bc + (tx + 16 * j) * LD + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 qq = ld4(pg + (4 * ty + i) * LD + c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = dot4(qq, kk[j], acc[i][j]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int row = 4 * ty + i, s = (tx + 16 * j) & (C - 1), t = row & (C - 1);
+                const float v = acc[i][j];
+                if (row < C) {
+                    if (j < 2) L[t * (C + 1) + s] = s < t ? v : 0.f;
+                    else PM[t * LDM + D + s] = s < t ? v : 0.f;
+                } else {
+                    if (j < 2) XB[s * LDM + t] = s <= t ? v : 0.f;
+                    else Y[t * (C + 1) + s] = s <= t ? v : 0.f;
+                }
+            }
+    }
+    for (int idx = tid; idx < C * D; idx += THREADS) PM[idx / D * LDM + idx % D] = pg[idx / D * LD + idx % D];     // the decays have been used
+    __syncthreads();
+    if (tid < R) {
+        float x[C];
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+            float v = PM[t * LDM + tid];
+#pragma unroll
+            for (int s = 0; s < t; ++s) v = fmaf(-L[t * (C + 1) + s], x[s], v);
+            x[t] = v;
+            PM[t * LDM + tid] = v;
+        }
+    }
+    __syncthreads();
+    {
+        // [X; b^T] [P' | M'], 96 x 96: rows ty + 16 i (outputs, then the state's rows), columns tx + 16 j
+        const int tx = tid & 15, ty = tid >> 4;
+        float acc[6][6] = {};
+#pragma unroll 4
+        for (int s = 0; s < C; ++s) {
+            float x[6], m[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                x[i] = XB[s * LDM + ty + 16 * i];
+                m[i] = PM[s * LDM + tx + 16 * i];
+            }
+#pragma unroll
+            for (int i = 0; i < 6; ++i)
+#pragma unroll
+                for (int j = 0; j < 6; ++j) acc[i][j] = fmaf(x[i], m[j], acc[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const int row = ty + 16 * i, col = tx + 16 * j;
+                float v;
+                if (i < 2) v = (j < 4 ? pg[(C + row) * LD + col] : Y[row * (C + 1) + col - D]) - acc[i][j];
+                else v = last_s[row - C] * ((j < 4 ? (row - C == col ? 1.f : 0.f) : bc[(C + col - D) * LD + row - C]) - acc[i][j]);
+                W[row * R + col] = v;
+            }
+    }
+}
+
+// Sums the eight warps' parts of a tile of ROWS x 16 that a thread's accumulators hold (rows g + 8 j, columns 4 cg ..): through shared memory.
+template <int NJ>
+__device__ __forceinline__ void put_parts(float* red, int warp, int g, int cg, const float (&acc)[NJ][4])
+{
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) st4(red + ((size_t)warp * 8 * NJ + g + 8 * j) * WALK_COLS + 4 * cg, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+}
+template <int ROWS>
+__device__ __forceinline__ float4 sum_parts(const float* red, int row, int cg)
+{
+    float4 v = ld4(red + (size_t)row * WALK_COLS + 4 * cg);
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+        const float4 p = ld4(red + ((size_t)w * ROWS + row) * WALK_COLS + 4 * cg);
+        v.x += p.x;
+        v.y += p.y;
+        v.z += p.z;
+        v.w += p.w;
+    }
+    return v;
+}
+// acc[j][c] += sum over four k of x[row g + 8 j][k ..] * y[k ..][4 cg + c]; x rows LDX floats apart, y rows WALK_LD
+template <int NJ, int LDX>
+__device__ __forceinline__ void tile_fma(float (&acc)[NJ][4], const float* x, const float* y)
+{
+    float yy[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) *reinterpret_cast<float4*>(yy[k]) = ld4(y + k * WALK_LD);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        float xx[4];
+        *reinterpret_cast<float4*>(xx) = ld4(x + (size_t)8 * j * LDX);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(xx[k], yy[k][c], acc[j][c]);
+    }
+}
+
+// Matrix memory and linear attention: a warp owns DK / 8 rows of the block's 16 columns of S.
+template <int MODE, int DK> struct WalkSmem {
+    static constexpr int C = 64, LDK = DK + 4, LDP = C + 4;
+    static constexpr int Q = 0, P = Q + C * LDK, K = P + C * LDP, V = K + C * LDK, X = V + C * WALK_LD;     // floats; X: F, l, kappa, psum, ksum | the decays
+    static constexpr int STAGE = X + (MODE == 0 ? 4 * C + DK : DK);
+    static constexpr int S = 2 * STAGE, N = S + DK * WALK_LD, TOTAL = N + DK + 3 * C;      // N: n; then alpha, beta, n . q
+    static constexpr size_t BYTES = TOTAL * sizeof(float);
+    static_assert(8 * C * WALK_COLS <= K, "the parts of the outputs fit the place of q and P");
+};
+
+template <int MODE, int DK>
+__global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
+{
+    using L = WalkSmem<MODE, DK>;
+    constexpr int C = L::C, LDK = L::LDK, LDP = L::LDP, KW = DK / 8;       // KW: rows of S a warp owns
+    extern __shared__ __align__(16) float sm[];
+    float *S_s = sm + L::S, *n_s = sm + L::N, *alpha_s = n_s + DK, *beta_s = alpha_s + C, *nq_s = beta_s + C;
+    pdl_enter();
+    const ScanArgs& a = A.s;
+    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS, dv = a.dv;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
+    const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
+    if (t_begin >= t_end || !takes_chunks<MODE>(a, seq, h, t_begin, t_end)) return;
+    const int slot = a.state_slot[seq];
+    if (slot < 0 || slot >= a.num_slots) {
+        if (tid == 0) report_status(a.status, SPY_STATUS_BAD_PAGE, t_begin);
+        return;
+    }
+    float* st = a.state + ((size_t)slot * a.H + h) * a.record;
+    float* st_nm = st + (size_t)DK * dv + (size_t)(c0 / 8) * (DK + 1);      // two copies of n and m: one for every 8 columns
+    for (int idx = tid; idx < DK * 4; idx += THREADS) st4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3), ld4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3)));
+    float m = 0.f;
+    if (MODE == 0) {
+        for (int r = tid; r < DK; r += THREADS) n_s[r] = st_nm[r];
+        m = st_nm[DK];
+    }
+    const int first_slot = chunk_slot(t_begin, seq, C);
+    auto request = [&](int t0, int stage) {
+        const int n_tok = min(C, t_end - t0);
+        float* base = sm + stage * L::STAGE;
+        const float* mine = A.work + ((size_t)(first_slot + (t0 - t_begin) / C) * a.H + h) * chunk_floats(MODE, DK);
+        const float* rows = a.proj + (size_t)t0 * a.ld;
+        for (int idx = tid; idx < C * (DK / 4); idx += THREADS) {
+            const int t = idx / (DK / 4), c = 4 * (idx - t * (DK / 4));
+            if (MODE == 2) {
+                cp_async16(base + L::Q + t * LDK + c, mine + C * C + t * DK + c);
+                cp_async16(base + L::K + t * LDK + c, mine + C * C + C * DK + t * DK + c);
+            } else if (t < n_tok) {
+                cp_async16(base + L::Q + t * LDK + c, rows + (size_t)t * a.ld + a.off_q + h * DK + c);
+                cp_async16(base + L::K + t * LDK + c, rows + (size_t)t * a.ld + a.off_k + h * DK + c);
+            } else {
+                st4(base + L::Q + t * LDK + c, make_float4(0.f, 0.f, 0.f, 0.f));
+                st4(base + L::K + t * LDK + c, make_float4(0.f, 0.f, 0.f, 0.f));
+            }
+        }
+        for (int idx = tid; idx < C * C / 4; idx += THREADS) cp_async16(base + L::P + (idx >> 4) * LDP + 4 * (idx & 15), mine + 4 * idx);
+        for (int idx = tid; idx < C * 4; idx += THREADS) {
+            const int t = idx >> 2, c = 4 * (idx & 3);
+            if (t < n_tok) cp_async16(base + L::V + t * WALK_LD + c, rows + (size_t)t * a.ld + a.off_v + h * dv + c0 + c);
+            else st4(base + L::V + t * WALK_LD + c, make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+        const float* extra = mine + C * C + (MODE == 2 ? 2 * C * DK : 0);
+        for (int idx = tid; idx < (MODE == 0 ? 4 * C + DK : DK) / 4; idx += THREADS) cp_async16(base + L::X + 4 * idx, extra + 4 * idx);
+    };
+    request(t_begin, 0);
+    int stage = 0;
+    for (int t0 = t_begin; t0 < t_end; t0 += C, stage ^= 1) {
+        const int n_tok = min(C, t_end - t0);
+        float* base = sm + stage * L::STAGE;
+        float *Q = base + L::Q, *K = base + L::K, *P = base + L::P, *V = base + L::V, *X = base + L::X;
+        cp_async_wait_all();
+        __syncthreads();                           // this chunk has landed, the chunk before is done with
+        if (t0 + C < t_end) request(t0 + C, stage ^ 1);
+        float keep = 1.f, add = 1.f;               // of the old state and of the chunk's sum
+        if (MODE == 0) {
+            if (tid < C) {
+                const float l = X[C + tid], f = X[tid] + m, top = fmaxf(f, l);
+                alpha_s[tid] = expf(l - top);
+                beta_s[tid] = expf(f - top);
+            }
+            const float l = X[C + C - 1], f = X[C - 1] + m, top = fmaxf(f, l);     // behind the chunk (padding tokens change nothing)
+            keep = expf(f - top);
+            add = expf(l - top);
+            // n . q: four threads a token
+            const int t = tid >> 2, part = tid & 3;
+            float s = 0.f;
+#pragma unroll
+            for (int c = 0; c < DK / 4; c += 4) s = dot4(ld4(Q + t * LDK + 4 * c + 4 * part), ld4(n_s + 4 * c + 4 * part), s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (part == 0) nq_s[t] = s;
+        }
+        // what the state ahead of the chunk gives: this warp's rows of it
+        float acc[8][4] = {};
+#pragma unroll
+        for (int k = 0; k < KW; k += 4) tile_fma<8, LDK>(acc, Q + g * LDK + warp * KW + k, S_s + (warp * KW + k) * WALK_LD + 4 * cg);
+        if (MODE == 0) {
+            __syncthreads();                       // alpha, beta and n . q are there; n has been read
+            float own[8][4] = {};
+#pragma unroll
+            for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(own, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float al = alpha_s[g + 8 * j], be = beta_s[g + 8 * j] * a.q_scale;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(be, acc[j][c], al * own[j][c]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(acc, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
+        }
+        __syncthreads();                           // q, P and the values as they came have been read
+        float* red = Q;
+        put_parts<8>(red, warp, g, cg, acc);
+        if (MODE == 0) {
+            if (tid < C * 4) {                     // the values as the state takes them
+                float* v = V + (tid >> 2) * WALK_LD + 4 * (tid & 3);
+                const float s = X[2 * C + (tid >> 2)] * add;
+                float4 x = ld4(v);
+                st4(v, make_float4(x.x * s, x.y * s, x.z * s, x.w * s));
+            }
+            for (int r = tid; r < DK; r += THREADS) n_s[r] = fmaf(keep, n_s[r], add * X[4 * C + r]);
+        }
+        __syncthreads();
+        {
+            const int t = tid >> 2, part = tid & 3;
+            float4 o = sum_parts<C>(red, t, part);
+            if (MODE == 0) {
+                const float l = X[C + t], f = X[t] + m;
+                const float nq = fmaf(beta_s[t] * a.q_scale, nq_s[t], alpha_s[t] * X[3 * C + t]);
+                const float d = fmaxf(fabsf(nq), expf(-fmaxf(f, l))) + 1e-6f;
+                o = make_float4(o.x / d, o.y / d, o.z / d, o.w / d);
+            }
+            if (t < n_tok) st4(a.out + (size_t)(t0 + t) * a.H * dv + h * dv + c0 + 4 * part, o);
+        }
+        // The state behind the chunk.  A warp's rows: a lane has half of them and four columns, over every fourth token; the four sums meet
+        // by shuffles, each lane keeping a quarter.
+        {
+            constexpr int RL = KW / 2;             // rows of a lane
+            const int rg = lane >> 4, sg = lane >> 2 & 3, r0 = warp * KW + rg * RL;
+            float u[RL][4] = {};
+#pragma unroll 4
+            for (int s = sg; s < C; s += 4) {
+                float kk[RL], vv[4];
+#pragma unroll
+                for (int r = 0; r < RL; r += 4) *reinterpret_cast<float4*>(kk + r) = ld4(K + s * LDK + r0 + r);
+                *reinterpret_cast<float4*>(vv) = ld4(V + s * WALK_LD + 4 * cg);
+#pragma unroll
+                for (int r = 0; r < RL; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) u[r][c] = fmaf(kk[r], vv[c], u[r][c]);
+            }
+            // lanes sg and sg ^ 2 halve the rows, then sg and sg ^ 1: a lane ends with RL / 4 rows
+            constexpr int H2 = RL / 2, H4 = RL / 4;
+            const bool up2 = (sg & 2) != 0, up1 = (sg & 1) != 0;
+            float half[H2][4], mine[H4][4];
+#pragma unroll
+            for (int r = 0; r < H2; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float give = up2 ? u[r][c] : u[r + H2][c], own = up2 ? u[r + H2][c] : u[r][c];
+                    half[r][c] = own + __shfl_xor_sync(0xffffffffu, give, 8);
+                }
+#pragma unroll
+            for (int r = 0; r < H4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float give = up1 ? half[r][c] : half[r + H4][c], own = up1 ? half[r + H4][c] : half[r][c];
+                    mine[r][c] = own + __shfl_xor_sync(0xffffffffu, give, 4);
+                }
+#pragma unroll
+            for (int r = 0; r < H4; ++r) {
+                const int row = r0 + (up2 ? H2 : 0) + (up1 ? H4 : 0) + r;
+                float* s = S_s + row * WALK_LD + 4 * cg;
+                const float d = MODE == 0 ? keep : X[row];
+                float4 o = ld4(s);
+                st4(s, make_float4(fmaf(d, o.x, mine[r][0]), fmaf(d, o.y, mine[r][1]), fmaf(d, o.z, mine[r][2]), fmaf(d, o.w, mine[r][3])));
+            }
+        }
+        if (MODE == 0) m = fmaxf(X[C - 1] + m, X[C + C - 1]);
+    }
+    __syncthreads();
+    for (int idx = tid; idx < DK * 4; idx += THREADS) st4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3), ld4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3)));
+    if (MODE == 0) {
+        for (int cp = 0; cp < 2; ++cp) {
+            for (int r = tid; r < DK; r += THREADS) st_nm[(size_t)cp * (DK + 1) + r] = n_s[r];
+            if (tid == 0) st_nm[(size_t)cp * (DK + 1) + DK] = m;
+        }
+    }
+}
+
+// Delta rule: [outputs of 32 tokens; the state's 64 rows] = W [the state; the values], a warp 12 of the 96 columns of W.
+struct DeltaSmem {
+    static constexpr int C = 32, D = 64, R = C + D, LDW = R + 4;
+    static constexpr int W = 0, V = W + R * LDW, STAGE = V + C * WALK_LD;
+    static constexpr int S = 2 * STAGE, RED = S + D * WALK_LD, TOTAL = RED + 8 * R * WALK_COLS;
+    static constexpr size_t BYTES = TOTAL * sizeof(float);
+};
+
+__global__ void __launch_bounds__(THREADS, 1) walk_delta_kernel(ChunkArgs A)
+{
+    using L = DeltaSmem;
+    constexpr int C = L::C, D = L::D, R = L::R, LDW = L::LDW, KW = R / 8;
+    extern __shared__ __align__(16) float sm[];
+    float *S_s = sm + L::S, *red = sm + L::RED;
+    pdl_enter();
+    const ScanArgs& a = A.s;
+    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
+    const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
+    if (t_begin >= t_end || !takes_chunks<1>(a, seq, h, t_begin, t_end)) return;
+    const int slot = a.state_slot[seq];
+    if (slot < 0 || slot >= a.num_slots) {
+        if (tid == 0) report_status(a.status, SPY_STATUS_BAD_PAGE, t_begin);
+        return;
+    }
+    float* st = a.state + ((size_t)slot * a.H + h) * a.record;
+    st4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3), ld4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3)));      // 64 rows of four quads: one a thread
+    const int first_slot = chunk_slot(t_begin, seq, C);
+    auto request = [&](int t0, int stage) {
+        const int n_tok = min(C, t_end - t0);
+        float* base = sm + stage * L::STAGE;
+        const float* W = A.work + ((size_t)(first_slot + (t0 - t_begin) / C) * a.H + h) * chunk_floats(1, D);
+        for (int idx = tid; idx < R * R / 4; idx += THREADS) cp_async16(base + L::W + idx / (R / 4) * LDW + 4 * (idx % (R / 4)), W + 4 * idx);
+        if (tid < C * 4) {
+            const int t = tid >> 2, c = 4 * (tid & 3);
+            if (t < n_tok) cp_async16(base + L::V + t * WALK_LD + c, a.proj + (size_t)(t0 + t) * a.ld + a.off_v + h * D + c0 + c);
+            else st4(base + L::V + t * WALK_LD + c, make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+    };
+    request(t_begin, 0);
+    int stage = 0;
+    for (int t0 = t_begin; t0 < t_end; t0 += C, stage ^= 1) {
+        const int n_tok = min(C, t_end - t0);
+        const float *W = sm + stage * L::STAGE + L::W, *V = sm + stage * L::STAGE + L::V;
+        cp_async_wait_all();
+        __syncthreads();                           // this chunk has landed, the state of the chunk before is written
+        if (t0 + C < t_end) request(t0 + C, stage ^ 1);
+        float acc[R / 8][4] = {};
+#pragma unroll
+        for (int i = 0; i < KW; i += 4) {
+            const int k = warp * KW + i;           // 4 consecutive columns of W: all of the state or all of the values
+            tile_fma<R / 8, LDW>(acc, W + g * LDW + k, (k < D ? S_s + k * WALK_LD : V + (k - D) * WALK_LD) + 4 * cg);
+        }
+        put_parts<R / 8>(red, warp, g, cg, acc);
+        __syncthreads();
+        for (int idx = tid; idx < R * 4; idx += THREADS) {
+            const int row = idx >> 2, part = idx & 3;
+            const float4 o = sum_parts<R>(red, row, part);
+            if (row >= C) st4(S_s + (row - C) * WALK_LD + 4 * part, o);
+            else if (row < n_tok) st4(a.out + (size_t)(t0 + row) * a.H * D + h * D + c0 + 4 * part, o);
+        }
+    }
+    __syncthreads();
+    st4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3), ld4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3)));
+}
+
+template <typename Args> static int launch_chunk_kernel(void (*kernel)(Args), dim3 grid, size_t smem, cudaStream_t stream, const Args& A)
+{
+    SPY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    spy_launch(kernel, grid, dim3(THREADS), smem, stream, A);
+    return 0;
+}
+
+// Which sizes take chunks: keys of 64 or 128 channels (the delta rule's states of 64 x 64), value columns in sixteens, steps of
+// CHUNK_MIN tokens or more whose factors fit 512 MB (200 K tokens of 8 heads of the matrix memory, 14 K of 32 heads of the delta rule).
+static long long chunk_work_floats(int mode, int tokens, int num_seqs, int H, int dk, int dv)
+{
+    if (tokens < CHUNK_MIN || dv % WALK_COLS != 0 || !(mode == 1 ? dk == 64 && dv == 64 : dk == 64 || dk == 128)) return 0;
+    const long long slots = tokens / (mode == 1 ? 32 : 64) + (long long)num_seqs + 1;
+    const long long floats = slots * H * (chunk_floats(mode, dk) + 4LL);
+    return floats <= (128LL << 20) && slots <= 0x7fffffff ? floats : 0;
+}
+
+template <int MODE> static int launch_chunks(ScanArgs& S, int tokens, int num_seqs, float* work, cudaStream_t stream)
+{
+    const int slots = tokens / ChunkOf<MODE>::C + num_seqs + 1;
+    ChunkArgs A = {S, work, nullptr, num_seqs};
+    A.flags = reinterpret_cast<int*>(work + (size_t)slots * S.H * chunk_floats(MODE, S.dk));
+    A.s.flags = S.flags = A.flags;
+    const dim3 chunks(slots, S.H), walk(num_seqs, S.H, S.dv / WALK_COLS);
+    int rc;
+    if constexpr (MODE == 1) {
+        constexpr int C = 32, D = 64, R = C + D;
+        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, (4 * C * (D + 4) + 2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
+        if (!rc) rc = launch_chunk_kernel(walk_delta_kernel, walk, DeltaSmem::BYTES, stream, A);
+    } else {
+        const size_t rows = (MODE == 0 ? 2 : 3) * 64 * (size_t)(S.dk + 4) * sizeof(float);
+        auto chunk = MODE == 0 ? (S.dk == 64 ? chunk_memory_kernel<64> : chunk_memory_kernel<128>) : (S.dk == 64 ? chunk_linear_kernel<64> : chunk_linear_kernel<128>);
+        rc = launch_chunk_kernel(chunk, chunks, rows, stream, A);
+        if (!rc) rc = S.dk == 64 ? launch_chunk_kernel(walk_kernel<MODE, 64>, walk, WalkSmem<MODE, 64>::BYTES, stream, A)
+                                 : launch_chunk_kernel(walk_kernel<MODE, 128>, walk, WalkSmem<MODE, 128>::BYTES, stream, A);
+    }
+    if (rc) return rc;
+    SPY_CHECK_LAUNCH("recurrence (chunks)");
+    return 0;
+}
+
 template <int MODE, int RG> static int launch_scan_rg(ScanArgs& A, int num_seqs, int longest, cudaStream_t stream)
 {
     constexpr int CTB = 8 * (32 / RG);
@@ -603,48 +1387,65 @@ template <int MODE> static int launch_scan_mode(ScanArgs& A, int num_seqs, int l
     return launch_scan_rg<MODE, 32>(A, num_seqs, longest, stream);
 }
 
-static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, cudaStream_t stream)
+// work: null, or scratch of spy_scan_chunk_floats floats for `tokens` tokens, 16-byte aligned.
+static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, int tokens, float* work, long long work_floats, cudaStream_t stream)
 {
     if (num_seqs <= 0) return 0;
     if (A.H <= 0 || A.dk <= 0 || A.dv <= 0) SPY_FAIL("recurrence: heads %d, key size %d and value size %d must be positive", A.H, A.dk, A.dv);
     if (A.H > 65535) SPY_FAIL("recurrence: %d heads exceed the grid limit", A.H);
     if ((A.dv + CT - 1) / CT > 65535) SPY_FAIL("recurrence: a value size of %d exceeds the grid limit", A.dv);
+    // chunks want whole 16-byte pieces of every row, state and output
+    const bool aligned = ((A.ld | A.off_q | A.off_k | A.off_v | (mode == 1 ? A.off_x1 : 0)) & 3) == 0 && A.record % 4 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(A.proj) | reinterpret_cast<uintptr_t>(A.state) | reinterpret_cast<uintptr_t>(A.out) |
+                           reinterpret_cast<uintptr_t>(work)) & 15) == 0;
+    if (work != nullptr && longest >= CHUNK_MIN && aligned) {
+        const long long need = chunk_work_floats(mode, tokens, num_seqs, A.H, A.dk, A.dv);
+        if (need > work_floats) SPY_FAIL("recurrence: %lld floats of scratch for %d tokens, %lld are needed", work_floats, tokens, need);
+        if (need > 0) {
+            const int rc = mode == 0 ? launch_chunks<0>(A, tokens, num_seqs, work, stream)
+                           : mode == 1 ? launch_chunks<1>(A, tokens, num_seqs, work, stream) : launch_chunks<2>(A, tokens, num_seqs, work, stream);
+            if (rc) return rc;
+        }
+    }
     if (mode == 2) return launch_scan_mode<2>(A, num_seqs, longest, stream);
     return mode == 0 ? launch_scan_mode<0>(A, num_seqs, longest, stream) : launch_scan_mode<1>(A, num_seqs, longest, stream);
 }
+
+// Floats of scratch with which a step's longer requests are walked in chunks; 0: these sizes are walked token by token.
+extern "C" long long spy_scan_chunk_floats(int mode, int tokens, int num_seqs, int H, int dk, int dv) { return chunk_work_floats(mode, tokens, num_seqs, H, dk, dv); }
 
 // State record of one head, in floats.
 extern "C" long long spy_mlstm_record(int dk, int dv) { return ((long long)dk * dv + (long long)((dv + 7) / 8) * (dk + 1) + 3) / 4 * 4; }
 
 extern "C" int spy_mlstm_scan(const float* proj, long long ld, int off_q, int off_k, int off_v, int off_i, int off_f, const float* bias_i, const float* bias_f,
                               float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest, float* out, int H, int dk,
-                              int dv, float q_scale, float cap, int* status, cudaStream_t stream)
+                              int dv, float q_scale, float cap, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
 {
     if (!(cap > 0.f)) SPY_FAIL("mlstm: the gates' cap must be positive");
     ScanArgs A = {proj, ld, off_q, off_k, off_v, off_i, off_f, nullptr, bias_i, bias_f, state, spy_mlstm_record(dk, dv), num_slots, q_start, state_slot, out,
-                  H, dk, dv, q_scale, cap, status};
-    return launch_scan(0, A, num_seqs, longest, stream);
+                  H, dk, dv, q_scale, cap, status, nullptr};
+    return launch_scan(0, A, num_seqs, longest, tokens, work, work_floats, stream);
 }
 
 extern "C" int spy_delta_scan(const float* proj, long long ld, int off_r, int off_k, int off_v, int off_a, const float* decay_pre, const float* bias_a,
                               const float* decay_offset, float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest,
-                              float* out, int H, int dk, int* status, cudaStream_t stream)
+                              float* out, int H, int dk, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
 {
     ScanArgs A = {proj, ld, off_r, off_k, off_v, off_a, 0, decay_pre, bias_a, decay_offset, state, (long long)dk * dk, num_slots, q_start, state_slot, out,
-                  H, dk, dk, 1.0f, 1.0f, status};
-    return launch_scan(1, A, num_seqs, longest, stream);
+                  H, dk, dk, 1.0f, 1.0f, status, nullptr};
+    return launch_scan(1, A, num_seqs, longest, tokens, work, work_floats, stream);
 }
 
 // Gated linear attention with a decay per key channel: proj holds q, k, v at `off_*`; decay_pre [T, H * dk] the decay's
 // pre-activation z, to which decay_bias [H * dk] is added: a = exp(logsigmoid(z + bias) / tau).  q is scaled by q_scale.
 extern "C" int spy_gla_scan(const float* proj, long long ld, int off_q, int off_k, int off_v, const float* decay_pre, const float* decay_bias, float inv_tau,
                             float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest, float* out, int H, int dk, int dv,
-                            float q_scale, int* status, cudaStream_t stream)
+                            float q_scale, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
 {
     if (!(inv_tau > 0.f)) SPY_FAIL("gated linear attention: tau must be positive");
     ScanArgs A = {proj, ld, off_q, off_k, off_v, 0, 0, decay_pre, nullptr, decay_bias, state, (long long)dk * dv, num_slots, q_start, state_slot, out,
-                  H, dk, dv, q_scale, inv_tau, status};
-    return launch_scan(2, A, num_seqs, longest, stream);
+                  H, dk, dv, q_scale, inv_tau, status, nullptr};
+    return launch_scan(2, A, num_seqs, longest, tokens, work, work_floats, stream);
 }
 
 // out[t, j] = act(proj[t, off + j]) for j < n: the inner activation of a two-step (low-rank) projection; act 0: tanh, 1: none.

@@ -495,6 +495,16 @@ def _scan_common(proj, state, q_start, state_slot, out, heads, dv):
         raise KernelError(f"recurrence output: expected {(proj.shape[0], heads * dv)}, found {tuple(out.shape)}")
 
 
+def _scan_chunk_work(mode: int, proj: torch.Tensor, num_seqs: int, longest: Optional[int], heads: int, dk: int, dv: int):
+    """Scratch for a step whose longer requests are walked in chunks (csrc/recurrence.cu), and its floats; None and 0 where none are."""
+    if longest is not None and longest <= 1:
+        return None, 0
+    f = build.load("recurrence").spy_scan_chunk_floats
+    f.restype = ctypes.c_longlong
+    floats = int(f(mode, proj.shape[0], int(num_seqs), heads, dk, dv))
+    return (torch.empty(floats, dtype=torch.float32, device=proj.device), floats) if floats else (None, 0)
+
+
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i: torch.Tensor, bias_f: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
                state_slot: torch.Tensor, num_seqs: int, out: torch.Tensor, heads: int, dk: int, dv: int, q_scale: float, cap: float,
                status: Optional[torch.Tensor] = None, longest: Optional[int] = None) -> torch.Tensor:
@@ -510,9 +520,10 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i: torch.Tensor, bias_f: torch.
     oq, ok, ov, oi, of = (int(o) for o in offsets)
     if max(oq + heads * dk, ok + heads * dk, ov + heads * dv, oi + heads, of + heads) > proj.shape[1] or bias_i.shape[0] != heads or bias_f.shape[0] != heads:
         raise KernelError("mlstm: the column offsets or the biases do not fit the projection")
+    work, floats = _scan_chunk_work(0, proj, num_seqs, longest, heads, dk, dv)
     _call("recurrence", "spy_mlstm_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), oq, ok, ov, oi, of, _ptr(bias_i), _ptr(bias_f), _ptr(state),
           state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk, dv,
-          ctypes.c_float(q_scale), ctypes.c_float(cap), _ptr(status), _stream())
+          ctypes.c_float(q_scale), ctypes.c_float(cap), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
     return out
 
 
@@ -532,9 +543,10 @@ def delta_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, bias_a: tor
     n = heads * dk
     if max(o_r, ok, ov, oa) + n > proj.shape[1] or tuple(decay_pre.shape) != (proj.shape[0], n) or bias_a.shape[0] != n or decay_offset.shape[0] != n:
         raise KernelError("delta rule: the column offsets, the decay or the biases do not fit the projection")
+    work, floats = _scan_chunk_work(1, proj, num_seqs, longest, heads, dk, dk)
     _call("recurrence", "spy_delta_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), o_r, ok, ov, oa, _ptr(decay_pre), _ptr(bias_a), _ptr(decay_offset),
           _ptr(state), state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk,
-          _ptr(status), _stream())
+          _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
     return out
 
 
@@ -553,9 +565,10 @@ def gla_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, decay_bias: t
     n = heads * dk
     if max(oq + n, ok + n, ov + heads * dv) > proj.shape[1] or tuple(decay_pre.shape) != (proj.shape[0], n) or decay_bias.shape[0] != n or not tau > 0:
         raise KernelError("gated linear attention: the column offsets, the decay or its bias do not fit the projection, or tau is not positive")
+    work, floats = _scan_chunk_work(2, proj, num_seqs, longest, heads, dk, dv)
     _call("recurrence", "spy_gla_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), oq, ok, ov, _ptr(decay_pre), _ptr(decay_bias), ctypes.c_float(1.0 / tau),
           _ptr(state), state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk, dv,
-          ctypes.c_float(q_scale), _ptr(status), _stream())
+          ctypes.c_float(q_scale), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
     return out
 
 

@@ -1,0 +1,156 @@
+"""Runs of tokens walked in chunks (csrc/recurrence.cu) against the token-by-token walk and against 64-bit arithmetic."""
+import math
+
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+HEADS = 2
+SHAPES = {"memory": [(64, 32), (128, 48)], "linear": [(64, 16), (128, 48)], "delta": [(64, 64)]}
+CASES = [(kind, dk, dv) for kind, sizes in SHAPES.items() for dk, dv in sizes]
+
+
+def inputs(kind, dk, dv, T, seed, hard=False):
+    """Columns [q | k | v | x1 | x2] and the decay's pre-activation; ``hard``: decays near nothing as well as near one."""
+    g = torch.Generator().manual_seed(seed)
+    n, nv = HEADS * dk, HEADS * dv
+    x1 = n if kind == "delta" else 4
+    x = torch.randn(T, 2 * n + nv + 2 * x1, generator=g)
+    if kind == "memory":
+        x[:, -2 * x1:] *= 4.0
+    pre = torch.randn(T, n, generator=g) * (20.0 if hard else 2.0)
+    return x, pre, torch.randn(n, generator=g) + 1.0, torch.randn(n, generator=g)
+
+
+def exact(kind, dk, dv, x, pre, b1, b2):
+    """Outputs of one request's tokens in 64-bit."""
+    H, n, nv = HEADS, HEADS * dk, HEADS * dv
+    x = x.double()
+    q, k, v = x[:, :n].view(-1, H, dk), x[:, n:2 * n].view(-1, H, dk), x[:, 2 * n:2 * n + nv].view(-1, H, dv)
+    S = torch.zeros(H, dk, dv, dtype=torch.float64)
+    out = []
+    if kind == "memory":
+        ig = 6.0 * torch.tanh((x[:, 2 * n + nv:2 * n + nv + H] + b1[:H].double()) / 6.0)
+        fg = torch.nn.functional.logsigmoid(6.0 * torch.tanh((x[:, 2 * n + nv + 4:2 * n + nv + 4 + H] + b2[:H].double()) / 6.0))
+        N, m = torch.zeros(H, dk, dtype=torch.float64), torch.zeros(H, dtype=torch.float64)
+        for t in range(x.shape[0]):
+            new = torch.maximum(fg[t] + m, ig[t])
+            a, b = torch.exp(fg[t] + m - new), torch.exp(ig[t] - new)
+            S = a[:, None, None] * S + b[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+            N = a[:, None] * N + b[:, None] * k[t]
+            m = new
+            qs = q[t] * dk ** -0.5
+            out.append(torch.einsum("hij,hi->hj", S, qs) / (torch.maximum((N * qs).sum(1).abs(), torch.exp(-m)) + 1e-6)[:, None])
+    elif kind == "linear":
+        a = torch.sigmoid(pre.double() + b2.double()).pow(1 / 16.0).view(-1, H, dk)
+        for t in range(x.shape[0]):
+            S = a[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            out.append(torch.einsum("hij,hi->hj", S, q[t] * dk ** -0.5))
+    else:
+        rate = torch.sigmoid(x[:, 2 * n + nv:3 * n + nv] + b1.double()).view(-1, H, dk)
+        w = torch.exp(-math.exp(-0.5) * torch.sigmoid(pre.double() + b2.double())).view(-1, H, dk)
+        for t in range(x.shape[0]):
+            u = k[t] / torch.sqrt((k[t] ** 2).sum(1, keepdim=True) + 1e-6)
+            S = w[t][:, :, None] * S - (rate[t] * u)[:, :, None] * torch.einsum("hij,hi->hj", S, u)[:, None, :] + k[t][:, :, None] * v[t][:, None, :]
+            out.append(torch.einsum("hij,hi->hj", S, q[t]))
+    return torch.stack(out).reshape(-1, nv)
+
+
+def run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad):
+    """One step of several requests; ``pad`` columns ahead of q: with one, no row starts on a 16-byte border and every request is walked
+    token by token."""
+    from spyinfer_b200 import kernels
+
+    n, nv = HEADS * dk, HEADS * dv
+    x = torch.cat(xs)
+    x = torch.cat([torch.zeros(len(x), pad), x, torch.zeros(len(x), -(x.shape[1] + pad) % 4)], 1).contiguous().cuda()
+    pre = torch.cat(pres).cuda()
+    starts = torch.tensor([0] + [len(p) for p in xs]).cumsum(0).to(torch.int32).cuda()
+    where = torch.tensor(slots, dtype=torch.int32, device="cuda")
+    out = torch.full((len(x), nv), 9.0, device="cuda")
+    offs = [pad, pad + n, pad + 2 * n, pad + 2 * n + nv, pad + 2 * n + nv + 4]
+    if kind == "memory":
+        kernels.mlstm_scan(x, offs, b1[:HEADS].cuda(), b2[:HEADS].cuda(), state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5, 6.0)
+    elif kind == "linear":
+        kernels.gla_scan(x, offs[:3], pre, b2.cuda(), 16.0, state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5)
+    else:
+        kernels.delta_scan(x, offs[:4], pre, b1.cuda(), b2.cuda(), state, starts, where, len(xs), out, HEADS, dk)
+    return out.cpu()
+
+
+def new_state(kind, dk, dv, slots):
+    from spyinfer_b200 import kernels
+
+    return torch.zeros((slots, HEADS * (kernels.mlstm_record(dk, dv) if kind == "memory" else dk * dv)), device="cuda")
+
+
+@gpu
+@pytest.mark.parametrize("hard", [False, True])
+@pytest.mark.parametrize("kind,dk,dv", CASES)
+def test_chunks_carry_the_state_through_portions_as_the_walk_by_tokens_does(kind, dk, dv, hard):
+    """Portions around the chunk's length and the least length, short ones beside them, slots out of order, and a state that the one
+    form leaves and the other goes on from."""
+    portions = [[48, 64, 3, 131], [65, 1, 63, 47], [32, 96, 200, 64]]          # [step][request]
+    slots = [4, 0, 3, 2]
+    total = [sum(step[r] for step in portions) for r in range(4)]
+    data = [inputs(kind, dk, dv, total[r], 10 * r + dk, hard) for r in range(4)]
+    b1, b2 = data[0][2], data[0][3]
+    want = [exact(kind, dk, dv, data[r][0], data[r][1], b1, b2) for r in range(4)]
+    errors = {}
+    for name, pads in {"chunks": [0, 0, 0], "tokens": [1, 1, 1], "in turns": [0, 1, 0]}.items():
+        state, at, got = new_state(kind, dk, dv, 5), [0] * 4, [[] for _ in range(4)]
+        state[1] = 7.0
+        for step, pad in zip(portions, pads):
+            out = run(kind, dk, dv, [data[r][0][at[r]:at[r] + step[r]] for r in range(4)], [data[r][1][at[r]:at[r] + step[r]] for r in range(4)], b1, b2,
+                      state, slots, pad)
+            for r, part in enumerate(out.split(step)):
+                got[r].append(part)
+                at[r] += step[r]
+        assert bool((state[1] == 7.0).all())
+        errors[name] = max(float((torch.cat(got[r]).double() - want[r]).norm() / want[r].norm()) for r in range(4))
+    print(f"\n  {kind} {dk} x {dv}{' hard' if hard else ''}: error against 64 bits {errors}")
+    # 32-bit sums of up to 128 terms over some hundred tokens: a few roundings of 6e-8 each
+    assert max(errors.values()) < 3e-6, errors
+
+
+@gpu
+@pytest.mark.parametrize("where", ["q", "k", "v", "decay"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3e20])
+@pytest.mark.parametrize("kind,dk,dv", [("memory", 64, 32), ("linear", 64, 16), ("delta", 64, 64)])
+def test_requests_with_numbers_out_of_range_are_walked_by_tokens(kind, dk, dv, value, where):
+    """A number that is none, or a huge one: the head's outputs are those of the walk by tokens bit for bit (nothing of it reaches an
+    earlier token), its neighbour's are finite."""
+    xs, pres = [], []
+    for r in range(2):
+        x, pre, b1, b2 = inputs(kind, dk, dv, 100, r)
+        xs.append(x)
+        pres.append(pre)
+    n = HEADS * dk
+    if where == "decay":
+        if kind == "memory":
+            xs[1][70, -8] = value
+        else:
+            pres[1][70, 5] = value
+    else:
+        xs[1][70, {"q": 5, "k": n + 5, "v": 2 * n + 5}[where]] = value
+    outs = [run(kind, dk, dv, xs, pres, b1, b2, new_state(kind, dk, dv, 2), [1, 0], pad) for pad in (0, 1)]
+    assert bool(outs[0][:100].isfinite().all()) and torch.allclose(outs[0][:100], outs[1][:100], rtol=1e-4, atol=1e-4)
+    assert bool(outs[0][100:170].isfinite().all())
+    h = slice(0, dv)                                                         # the head that holds the number
+    if math.isnan(value) or where != "decay":
+        assert torch.equal(outs[0][100:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5), outs[1][100:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5))
+    else:
+        assert torch.allclose(outs[0][100:, h], outs[1][100:, h], rtol=1e-4, atol=1e-4)     # a saturated gate is an ordinary one
+
+
+def test_which_sizes_take_chunks():
+    """The rule of the entry point: scratch for the sizes that are served, none for others (the library answers without a device)."""
+    import ctypes
+
+    from spyinfer_b200.csrc import build
+
+    f = build.load("recurrence").spy_scan_chunk_floats
+    f.restype = ctypes.c_longlong
+    assert f(0, 48, 1, 8, 128, 256) > 0 and f(2, 2000, 8, 16, 128, 256) > 0 and f(1, 2047, 1, 32, 64, 64) > 0
+    assert f(0, 47, 1, 8, 128, 256) == 0 and f(0, 48, 1, 8, 96, 256) == 0 and f(0, 48, 1, 8, 128, 250) == 0 and f(1, 48, 1, 8, 128, 128) == 0
+    assert f(1, 65536, 64, 64, 64, 64) == 0                                  # more scratch than the limit
