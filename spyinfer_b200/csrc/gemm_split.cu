@@ -48,27 +48,27 @@ constexpr int MAX_STAGES = 8;
 constexpr int MAX_SLICES = 8;     // blocks of a cluster
 constexpr float PIECE_SCALE = 256.f;   // of the second piece; of the third its square (split3)
 
-template <int BN> struct Shape {
-    static constexpr int FIRST_SUM_WARP = 3;               // warp 0: TMA and tensor memory; 1 and 2: the leading pieces' products, the others'; then four warps that sum
-    static constexpr int FIRST_SPLIT_WARP = 7;             // and four that make the pieces
-    static constexpr int THREADS = 32 * 11;
-    static constexpr int ROWS = 128;                       // weight rows of a tile, at most
+template <int BN, int HALVES> struct Shape {
+    static constexpr int ISSUERS = 2 * HALVES;             // warps that issue products: a half's leading pieces, a half's two others
+    static constexpr int FIRST_SUM_WARP = 1 + ISSUERS;     // warp 0: TMA and tensor memory; then the issuers; then four warps a half that sum
+    static constexpr int THREADS = 32 * FIRST_SUM_WARP + 128 * HALVES;
+    static constexpr int ROWS = 128 * HALVES;              // weight rows of a tile, at most
     static constexpr int Y_BYTES = BN * BK * 2;            // one piece of the tokens
-    static constexpr int COLS = 8 * BN;                    // tensor-memory columns: buffers of the leading pieces' sums, then the two other pieces'
+    static constexpr int COLS = (HALVES == 1 ? 8 : 4) * BN;   // tensor-memory columns of a half: buffers of the leading pieces' sums, then the two other pieces'
     static constexpr int BUFFERS = COLS / BN - 2;          // blocks of K whose sums may wait to be taken out
-    static constexpr int PER_SM = BN <= 32 ? 2 : 1;
+    static constexpr int PER_SM = HALVES == 1 && BN <= 32 ? 2 : 1;
     static constexpr int AREA = (PER_SM == 2 ? 110 : 224) * 1024;
     static constexpr size_t SMEM = (size_t)AREA + 1024 /* alignment */ + 512 /* barriers */;
     static constexpr int LD = ROWS + 4;                    // floats between the tokens of the staged result
     __host__ __device__ static constexpr int x_bytes(int rows) { return (rows * BK * 2 + 1023) & ~1023; }
-    // The tensor core reads 128 rows: spare ones come from what lies behind and feed sums that are never stored; the area ends with room for that
+    // The tensor core reads 128 rows a half: spare ones come from what lies behind and feed sums that are never stored; the area ends with room for that
     __host__ __device__ static constexpr int stages(int rows)
     {
         const int n = (AREA - (ROWS * BK * 2 - x_bytes(rows))) / (x_bytes(rows) + 3 * Y_BYTES);
         return n < MAX_STAGES ? n : MAX_STAGES;
     }
     static_assert(BN * LD * 4 <= AREA, "the staged result fits the stages' place");
-    static_assert(COLS * PER_SM <= 512, "tensor memory");
+    static_assert(COLS * HALVES * PER_SM <= 512, "tensor memory");
 };
 
 __device__ __forceinline__ float4 ld_cluster4(uint32_t addr)
@@ -105,62 +105,29 @@ __device__ __noinline__ float plain_sum(const float* a, const bf16* w, int K)
     return s;
 }
 
-// The three pieces of a 32-bit number.  One that is not finite goes into the first piece alone.
-// The second piece is stored PIECE_SCALE times as large, the third its square: as they are, their last bits would lie below the smallest
-// bfloat16 number (2^-133) for numbers under 2^-110.
-__device__ __forceinline__ void split3(float a, uint32_t& p0, uint32_t& p1, uint32_t& p2)
-{
-    const uint32_t u = __float_as_uint(a);
-    if ((u & 0x7f800000u) == 0x7f800000u) {
-        p0 = (u >> 16) | ((u & 0x7fffffu) != 0 ? 0x40u : 0u);      // a NaN stays one
-        p1 = p2 = 0;
-        return;
-    }
-    p0 = u >> 16;
-    const float r = (a - __uint_as_float(u & 0xffff0000u)) * PIECE_SCALE;        // exact: the low 16 bits of the mantissa, below 2^-7 of the number
-    const uint32_t ur = __float_as_uint(r);
-    p1 = ur >> 16;
-    p2 = __float_as_uint((r - __uint_as_float(ur & 0xffff0000u)) * PIECE_SCALE) >> 16;   // what is left has at most eight bits
-}
-
-// Eight numbers' pieces, two a word.
-__device__ __forceinline__ void split8(const float (&v)[8], uint32_t (&p)[3][4])
-{
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        uint32_t a[3], b[3];
-        split3(v[2 * e], a[0], a[1], a[2]);
-        split3(v[2 * e + 1], b[0], b[1], b[2]);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) p[j][e] = a[j] | (b[j] << 16);
-    }
-}
-
-// W [n_rows, K] through map_w (boxes of tile_rows rows).  The tokens' pieces are made here: four warps, a K block each in turns, read the
-// numbers of their next block while the others' are at work and write its three pieces where the products read them (a kernel of its own
-// for them took 1.9 us a product of few tokens, and their way to memory and back).
-template <int BN>
-__global__ void __launch_bounds__(Shape<BN>::THREADS, Shape<BN>::PER_SM)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__ out, long long ldc,
+// W [n_rows, K] through map_w (boxes of tile_rows rows), the pieces [3][m_rows][K] through map_a (boxes of BN rows).
+template <int BN, int HALVES>
+__global__ void __launch_bounds__(Shape<BN, HALVES>::THREADS, Shape<BN, HALVES>::PER_SM)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ out, long long ldc,
                   const float* __restrict__ A, long long lda, const bf16* __restrict__ W, long long ldw, int n_rows, int m_rows, int K,
-                  int k_blocks_per_slice, int tile_rows, int vec, int* status)
+                  int k_blocks_per_slice, int tile_rows, int* status)
 {
-    using S = Shape<BN>;
+    using S = Shape<BN, HALVES>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + S::AREA);
     uint64_t* empty_bar = full_bar + MAX_STAGES;
     constexpr int NB = S::BUFFERS;
-    uint64_t* sum_full = empty_bar + MAX_STAGES;           // [NB] a K block's sums of the leading pieces are complete
-    uint64_t* sum_empty = sum_full + NB;                   // [NB] they have been taken out
-    uint64_t* done_bar = sum_empty + NB;
+    uint64_t* sum_full = empty_bar + MAX_STAGES;           // [HALVES][NB] a K block's sums of the leading pieces are complete
+    uint64_t* sum_empty = sum_full + NB * HALVES;          // [HALVES][NB] they have been taken out
+    uint64_t* done_bar = sum_empty + NB * HALVES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x0 = blockIdx.y * tile_rows, y0 = blockIdx.x * BN;
     const int x_bytes = S::x_bytes(tile_rows), stage_bytes = x_bytes + 3 * S::Y_BYTES, stages = S::stages(tile_rows);
-    const uint32_t stage_tx = (uint32_t)tile_rows * BK * 2;
+    const uint32_t stage_tx = (uint32_t)tile_rows * BK * 2 + 3 * S::Y_BYTES;
     const int k_blocks = (K + BK - 1) / BK;
     const int kb0 = blockIdx.z * k_blocks_per_slice;
     const int num_kb = min(k_blocks - kb0, k_blocks_per_slice);      // at least one (plan_slices)
@@ -168,18 +135,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
-            mbar_init(full_bar + s, 2);                    // the weights and the pieces
-            mbar_init(empty_bar + s, 2);
+            mbar_init(full_bar + s, 1);
+            mbar_init(empty_bar + s, S::ISSUERS);
         }
-        for (int i = 0; i < NB; ++i) {
+        for (int i = 0; i < NB * HALVES; ++i) {
             mbar_init(sum_full + i, 1);
             mbar_init(sum_empty + i, 4);
         }
-        mbar_init(done_bar, 2);
+        mbar_init(done_bar, S::ISSUERS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)S::COLS);
+    if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)(S::COLS * HALVES));
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -188,13 +155,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
     pdl_launch_dependents();
     if (warp == 0) {
         if (lane == 0) {
-            // the weights depend on no earlier kernel: nothing here waits for the kernels ahead
+            // the weights depend on no earlier kernel: the first stages' are requested before the wait for the kernels ahead
+            const int pre = min(num_kb, stages);
+            for (int i = 0; i < pre; ++i) {
+                mbar_expect_tx(full_bar + i, stage_tx);
+                tma_load_2d(smem_u32(tiles + (size_t)i * stage_bytes), &map_w, (kb0 + i) * BK, x0, full_bar + i);
+            }
+            pdl_wait();
+            for (int i = 0; i < pre; ++i) {
+                uint8_t* ys = tiles + (size_t)i * stage_bytes + x_bytes;
+                for (int p = 0; p < 3; ++p) tma_load_2d(smem_u32(ys + p * S::Y_BYTES), &map_a, (kb0 + i) * BK, y0 + p * m_rows, full_bar + i);
+            }
             int s = 0;
-            uint32_t phase = 1;                            // the first round's waits end at once
-            for (int i = 0; i < num_kb; ++i) {
+            uint32_t phase = 0;
+            for (int i = pre; i < num_kb; ++i) {
                 if (!mbar_wait(empty_bar + s, phase, abort_flag)) break;
+                uint8_t* xs = tiles + (size_t)s * stage_bytes;
                 mbar_expect_tx(full_bar + s, stage_tx);
-                tma_load_2d(smem_u32(tiles + (size_t)s * stage_bytes), &map_w, (kb0 + i) * BK, x0, full_bar + s);
+                tma_load_2d(smem_u32(xs), &map_w, (kb0 + i) * BK, x0, full_bar + s);
+                for (int p = 0; p < 3; ++p) tma_load_2d(smem_u32(xs + x_bytes + p * S::Y_BYTES), &map_a, (kb0 + i) * BK, y0 + p * m_rows, full_bar + s);
                 if (++s == stages) {
                     s = 0;
                     phase ^= 1;
@@ -203,24 +182,27 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
         }
     } else if (warp < S::FIRST_SUM_WARP) {
         if (lane == 0) {
-            const bool lead = warp == 1;
-            const uint32_t acc = tmem;
+            const int half = (warp - 1) >> 1;
+            const bool lead = ((warp - 1) & 1) == 0;
+            const uint32_t acc = tmem + (uint32_t)(half * S::COLS), x_off = (uint32_t)(half * 128 * BK * 2);
             int s = 0;
             uint32_t phase = 0;
             if (lead) {
                 const uint32_t idesc = instr_desc_bf16(128, BN, false, false);
+                uint64_t* full = sum_full + NB * half;
+                uint64_t* empty = sum_empty + NB * half;
                 int b = 0;
                 uint32_t taken = 1;                        // the parity of a buffer's release that its next use waits for
                 for (int i = 0; i < num_kb; ++i) {
                     if (!mbar_wait(full_bar + s, phase, abort_flag)) break;
                     const uint32_t xs = smem_u32(tiles + (size_t)s * stage_bytes);
-                    const uint64_t dx = desc_k_major(xs), dy = desc_k_major(xs + x_bytes);
-                    if (i >= NB && !mbar_wait(sum_empty + b, taken, abort_flag)) break;
+                    const uint64_t dx = desc_k_major(xs + x_off), dy = desc_k_major(xs + x_bytes);
+                    if (i >= NB && !mbar_wait(empty + b, taken, abort_flag)) break;
                     fence_after_sync();
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         umma(acc + (uint32_t)(b * BN), dx + (uint64_t)(k * UMMA_K * 2 >> 4), dy + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, k > 0 ? 1u : 0u);
-                    umma_commit(sum_full + b);
+                    umma_commit(full + b);
                     if (++b == NB) {
                         b = 0;
                         taken ^= 1;
@@ -237,7 +219,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
                     if (!mbar_wait(full_bar + s, phase, abort_flag)) break;
                     fence_after_sync();
                     const uint32_t xs = smem_u32(tiles + (size_t)s * stage_bytes);
-                    const uint64_t dx = desc_k_major(xs), dy = desc_k_major(xs + x_bytes + S::Y_BYTES);
+                    const uint64_t dx = desc_k_major(xs + x_off), dy = desc_k_major(xs + x_bytes + S::Y_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         umma(acc + NB * BN, dx + (uint64_t)(k * UMMA_K * 2 >> 4), dy + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (i > 0 || k > 0) ? 1u : 0u);
@@ -250,52 +232,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
             }
             umma_commit(done_bar);
         }
-    } else if (warp >= S::FIRST_SPLIT_WARP) {
-        // A lane's places: eight numbers of one token each, 128 places a piece of 16 tokens, four at a time.
-        pdl_wait();
-        constexpr int GROUPS = BN / 16;
-        for (int i = warp - S::FIRST_SPLIT_WARP; i < num_kb; i += 4) {
-            const int s = i % stages, round = i / stages;
-            uint8_t* ys = tiles + (size_t)s * stage_bytes + x_bytes;
-#pragma unroll 1
-            for (int grp = 0; grp < GROUPS; ++grp) {
-                float v[4][8];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int t = grp * 16 + u * 4 + (lane >> 3), k = (kb0 + i) * BK + 8 * (lane & 7);
-                    const float* src = A + (size_t)(y0 + t) * lda + k;
-                    if (y0 + t < m_rows && k < K) {        // K is a multiple of 8
-                        if (vec) {
-                            *reinterpret_cast<float4*>(v[u]) = *reinterpret_cast<const float4*>(src);
-                            *reinterpret_cast<float4*>(v[u] + 4) = *reinterpret_cast<const float4*>(src + 4);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) v[u][e] = src[e];
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[u][e] = 0.f;
-                    }
-                }
-                if (grp == 0 && round > 0 && !mbar_wait_warp(empty_bar + s, (uint32_t)(round - 1) & 1, abort_flag)) break;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int t = grp * 16 + u * 4 + (lane >> 3);
-                    uint8_t* at = ys + t * 128 + (((lane & 7) ^ (t & 7)) << 4);        // the 128-byte swizzle that the products read
-                    uint32_t p[3][4];
-                    split8(v[u], p);
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(at + j * S::Y_BYTES) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
-                }
-            }
-            if (__shfl_sync(0xffffffffu, *abort_flag, 0) != 0) break;
-            fence_async_proxy();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full_bar + s);
-        }
     } else {
-        const int quarter = warp & 3;
-        const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        const int half = (warp - S::FIRST_SUM_WARP) >> 2, quarter = warp & 3;
+        const uint32_t acc = tmem + (uint32_t)(half * S::COLS) + ((uint32_t)(quarter * 32) << 16);
         constexpr int C = BN < 32 ? BN : 32;
         float sum[BN];
 #pragma unroll
@@ -303,7 +242,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
         int b = 0;
         uint32_t phase = 0;
         for (int n = 0; n < num_kb; ++n) {
-            if (!mbar_wait_warp(sum_full + b, phase, abort_flag)) break;
+            if (!mbar_wait_warp(sum_full + NB * half + b, phase, abort_flag)) break;
             fence_after_sync();
 #pragma unroll
             for (int c = 0; c < BN; c += C) {
@@ -315,7 +254,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
             }
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(sum_empty + b);
+            if (lane == 0) mbar_arrive(sum_empty + NB * half + b);
             if (++b == NB) {
                 b = 0;
                 phase ^= 1;
@@ -323,15 +262,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
         }
         mbar_wait_warp(done_bar, 0, abort_flag);           // every product is complete: the stages are free as well
         fence_after_sync();
-        float* staged = reinterpret_cast<float*>(tiles) + quarter * 32 + lane;
+        float* staged = reinterpret_cast<float*>(tiles) + half * 128 + quarter * 32 + lane;
 #pragma unroll
-        for (int c = 0; c < BN; c += 16) {
-            uint32_t r1[16], r2[16];
-            tmem_load<16>(acc + (uint32_t)(NB * BN + c), r1);
-            tmem_load<16>(acc + (uint32_t)((NB + 1) * BN + c), r2);
+        for (int c = 0; c < BN; c += C) {
+            uint32_t r1[C], r2[C];
+            tmem_load<C>(acc + (uint32_t)(NB * BN + c), r1);
+            tmem_load<C>(acc + (uint32_t)((NB + 1) * BN + c), r2);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) staged[(size_t)(c + e) * S::LD] =
+            for (int e = 0; e < C; ++e) staged[(size_t)(c + e) * S::LD] =
                 fmaf(fmaf(__uint_as_float(r2[e]), 1.f / PIECE_SCALE, __uint_as_float(r1[e])), 1.f / PIECE_SCALE, sum[c + e]);   // the scales are powers of two: two rounded additions
         }
         fence_before_sync();
@@ -394,7 +333,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__
     else __syncthreads();
     if (warp == 0) {
         fence_after_sync();
-        tmem_dealloc(tmem, (uint32_t)S::COLS);
+        tmem_dealloc(tmem, (uint32_t)(S::COLS * HALVES));
     }
 }
 
@@ -684,7 +623,24 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const float* __restri
     }
 }
 
-// The three pieces of 32-bit rows, for products of more than 64: pieces[p][m][k], eight numbers a thread.
+// The three pieces of 32-bit rows: pieces[p][m][k], eight numbers a thread.  Numbers that are not finite go into the first piece alone.
+// The second piece is stored 2^PIECE_SHIFT times as large, the third 2^(2 PIECE_SHIFT): as they are, their last bits would lie below the smallest
+// bfloat16 number (2^-133) for numbers under 2^-110.
+__device__ __forceinline__ void split3(float a, uint32_t& p0, uint32_t& p1, uint32_t& p2)
+{
+    const uint32_t u = __float_as_uint(a);
+    if ((u & 0x7f800000u) == 0x7f800000u) {
+        p0 = (u >> 16) | ((u & 0x7fffffu) != 0 ? 0x40u : 0u);      // a NaN stays one
+        p1 = p2 = 0;
+        return;
+    }
+    p0 = u >> 16;
+    const float r = (a - __uint_as_float(u & 0xffff0000u)) * PIECE_SCALE;        // exact: the low 16 bits of the mantissa, below 2^-7 of the number
+    const uint32_t ur = __float_as_uint(r);
+    p1 = ur >> 16;
+    p2 = __float_as_uint((r - __uint_as_float(ur & 0xffff0000u)) * PIECE_SCALE) >> 16;   // what is left has at most eight bits
+}
+
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, long long lda, bf16* __restrict__ pieces, int m_rows, int K, int vec)
 {
     pdl_enter();
@@ -701,7 +657,14 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
             for (int e = 0; e < 8; ++e) v[e] = src[e];
         }
         uint32_t p[3][4];
-        split8(v, p);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            uint32_t a[3], b[3];
+            split3(v[2 * e], a[0], a[1], a[2]);
+            split3(v[2 * e + 1], b[0], b[1], b[2]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) p[j][e] = a[j] | (b[j] << 16);
+        }
 #pragma unroll
         for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(pieces + j * plane + m * K + k) = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
     }
@@ -721,21 +684,21 @@ int make_map(CUtensorMap* map, const void* base, long long rows, int K, long lon
     return 0;
 }
 
-template <int BN> int set_up()
+template <int BN, int HALVES> int set_up()
 {
     SPY_ONCE_PER_DEVICE
     {
-        SPY_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<BN>::SMEM));
-        SPY_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+        SPY_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<BN, HALVES>::SMEM));
+        SPY_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN, HALVES>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
     }
     return 0;
 }
 
-template <int BN> void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], dim3 grid, int slices, cudaStream_t stream)
+template <int BN, int HALVES> void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], dim3 grid, int slices, cudaStream_t stream)
 {
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(Shape<BN>::THREADS);
-    cfg.dynamicSmemBytes = Shape<BN>::SMEM;
+    cfg.blockDim = dim3(Shape<BN, HALVES>::THREADS);
+    cfg.dynamicSmemBytes = Shape<BN, HALVES>::SMEM;
     cfg.stream = stream;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
@@ -757,13 +720,13 @@ int resident_clusters(int slices, int per_sm, int* count)
     const int ask = halve ? slices / 2 : slices;
     int& c = known[spy_device()][ask];
     if (c == 0) {
-        if (int rc = set_up<16>()) return rc;
+        if (int rc = set_up<16, 1>()) return rc;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
-        configure<16>(cfg, attr, dim3(1, 1, ask), ask, nullptr);
+        configure<16, 1>(cfg, attr, dim3(1, 1, ask), ask, nullptr);
         cfg.numAttrs = 1;
         int n = 0;
-        SPY_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<16>, &cfg));
+        SPY_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<16, 1>, &cfg));
         if (n <= 0) SPY_FAIL("gemm_split: no cluster of %d blocks fits the device", ask);
         c = n;
     }
@@ -813,17 +776,17 @@ int plan_slices(int n_rows, int k_blocks, int* slices_out)
     return 0;
 }
 
-template <int BN>
-int launch(const CUtensorMap& mw, float* C, long long ldc, const float* A, long long lda, const bf16* W, long long ldw, int N, int M, int K,
-           int slices, int per, int tile_rows, int vec, int* status, cudaStream_t stream)
+template <int BN, int HALVES>
+int launch(const CUtensorMap& mw, const CUtensorMap& ma, float* C, long long ldc, const float* A, long long lda, const bf16* W, long long ldw, int N, int M, int K,
+           int slices, int per, int tile_rows, int* status, cudaStream_t stream)
 {
-    if (int rc = set_up<BN>()) return rc;
+    if (int rc = set_up<BN, HALVES>()) return rc;
     const int tiles = (N + tile_rows - 1) / tile_rows;
     if (tiles > 65535) SPY_FAIL("gemm_split: %d weight rows exceed the grid", N);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    configure<BN>(cfg, attr, dim3((M + BN - 1) / BN, tiles, slices), slices, stream);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<BN>, mw, C, ldc, A, lda, W, ldw, N, M, K, per, tile_rows, vec, status);
+    configure<BN, HALVES>(cfg, attr, dim3((M + BN - 1) / BN, tiles, slices), slices, stream);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<BN, HALVES>, mw, ma, C, ldc, A, lda, W, ldw, N, M, K, per, tile_rows, status);
     if (e != cudaSuccess) SPY_FAIL("gemm_split: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }
@@ -893,7 +856,7 @@ PairPlan plan_pairs(int M, int N, int slices, int per, int clusters)
 extern "C" long long spy_gemm_split_scratch(int M, int N, int K)
 {
     const long long pieces = (3LL * M * K * 2 + 15) / 16 * 16;
-    if (M <= 64 || N <= 0 || K <= 0) return 16;                // few rows' pieces are made where they are used
+    if (M <= 64 || N <= 0 || K <= 0) return pieces;
     int slices = 1, clusters = 0;
     const int k_blocks = (K + BK - 1) / BK;
     if (plan_slices(N, k_blocks, &slices) || resident_pairs(&clusters)) return 0;
@@ -905,27 +868,27 @@ extern "C" long long spy_gemm_split_scratch(int M, int N, int K)
 extern "C" int spy_gemm_split_slices(int N, int K, int* slices) { return plan_slices(N, (K + BK - 1) / BK, slices); }
 
 // A [M, K] and C [M, N] float32, W [N, K] bfloat16, rows lda/ldc/ldw elements apart (W's on 16-byte borders; K a multiple of 8).
-// pieces: scratch of spy_gemm_split_scratch bytes, 16-byte aligned (up to 64 rows: not used, may be null).
+// pieces: scratch of spy_gemm_split_scratch bytes, 16-byte aligned (up to 64 rows: 3 * M * K bfloat16).
 extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long long ldw, float* C, long long ldc, int M, int N, int K, void* pieces,
                               int* status, cudaStream_t stream)
 {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 != 0) SPY_FAIL("gemm_split: K %d must be a positive multiple of 8 (16-byte rows for TMA)", K);
     if (lda < K || ldw < K || ldc < N) SPY_FAIL("gemm_split: row strides %lld/%lld/%lld are shorter than the rows", lda, ldw, ldc);
-    if (ldw % 8 != 0 || (reinterpret_cast<uintptr_t>(W) & 15) || (M > 64 && ((reinterpret_cast<uintptr_t>(pieces) & 15) || pieces == nullptr)))
+    if (ldw % 8 != 0 || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(pieces) & 15) || pieces == nullptr)
         SPY_FAIL("gemm_split: weight rows and pieces must start on 16-byte borders");
     if (M > (0x7fffffff - 64) / 3) SPY_FAIL("gemm_split: %d rows", M);
     const int vec = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    long long blocks = ((long long)M * (K / 8) + 255) / 256;
+    if (blocks > 8LL * spy_sm_count()) blocks = 8LL * spy_sm_count();
+    spy_launch(split_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, A, lda, (bf16*)pieces, M, K, vec);
+    SPY_CHECK_LAUNCH("gemm_split (pieces)");
 
     const int k_blocks = (K + BK - 1) / BK;
     int slices = 1;
     if (int rc = plan_slices(N, k_blocks, &slices)) return rc;
     const int per = (k_blocks + slices - 1) / slices;
     if (M > 64) {
-        long long blocks = ((long long)M * (K / 8) + 255) / 256;
-        if (blocks > 8LL * spy_sm_count()) blocks = 8LL * spy_sm_count();
-        spy_launch(split_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, A, lda, (bf16*)pieces, M, K, vec);
-        SPY_CHECK_LAUNCH("gemm_split (pieces)");
         int clusters = 0;
         if (int rc = resident_pairs(&clusters)) return rc;
         const PairPlan plan = plan_pairs(M, N, slices, per, clusters);
@@ -952,9 +915,11 @@ extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long
     int tile_rows = 128, clusters = 0;
     if (int rc = resident_clusters(slices, bn == 64 ? 1 : 2, &clusters)) return rc;
     plan_rows(N, slices, clusters, per, &tile_rows);
-    CUtensorMap mw;
-    if (make_map(&mw, W, N, K, ldw, tile_rows)) return 1;
-    if (bn == 16) return launch<16>(mw, C, ldc, A, lda, (const bf16*)W, ldw, N, M, K, slices, per, tile_rows, vec, status, stream);
-    if (bn == 32) return launch<32>(mw, C, ldc, A, lda, (const bf16*)W, ldw, N, M, K, slices, per, tile_rows, vec, status, stream);
-    return launch<64>(mw, C, ldc, A, lda, (const bf16*)W, ldw, N, M, K, slices, per, tile_rows, vec, status, stream);
+    CUtensorMap mw, ma;
+    if (make_map(&mw, W, N, K, ldw, tile_rows) || make_map(&ma, pieces, 3LL * M, K, K, bn)) return 1;
+#define SPY_SPLIT_LAUNCH(BN_, H_) launch<BN_, H_>(mw, ma, C, ldc, A, lda, (const bf16*)W, ldw, N, M, K, slices, per, tile_rows, status, stream)
+    if (bn == 16) return SPY_SPLIT_LAUNCH(16, 1);
+    if (bn == 32) return SPY_SPLIT_LAUNCH(32, 1);
+    return SPY_SPLIT_LAUNCH(64, 1);
+#undef SPY_SPLIT_LAUNCH
 }
