@@ -337,292 +337,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
 }
 
-// ---- many tokens: pairs of blocks --------------------------------------------------------------------------------------------------
-//
-// A cluster of two blocks (cta_group::2) takes 256 weight rows x up to 128 tokens: each block brings its 128 weight rows and its half of
-// the tokens' three pieces, the leader issues products of 256 x n (the leading pieces) and 256 x 2 n (the other two side by side), each block
-// sums its own 128 rows.  Against 256 rows x 64 tokens on one block this reads a third less of the shared memory for the same products (an
-// instruction of 128 x 64 reads more than it can be fed while it multiplies) and brings a weight tile from L2 half as often.  A block's eight
-// summing warps hold 64 tokens' sums each; the slices of K (the same as with few tokens, so that a row's result stays the same) follow one
-// another and are added in order.  With too few tiles for the pairs, the slices of a tile are shared out in runs (`parts`): the first run
-// leaves its sum, every later slice its own, and split_reduce_kernel adds them in order.
-// PAIR_MEASURED_PLACEHOLDER
-constexpr int PAIR_MAX_TOKENS = 128;
-constexpr int PAIR_STAGES = 4;
-constexpr int PAIR_SUM_WARPS = 8;
-constexpr int PAIR_THREADS = 32 * (3 + PAIR_SUM_WARPS);   // warp 0: TMA and tensor memory; 1 and 2: the leading pieces' products, the others'; then the summing warps
-constexpr int PAIR_W_BYTES = 128 * BK * 2;
-constexpr int PAIR_STAGE_BYTES = PAIR_W_BYTES + 3 * (PAIR_MAX_TOKENS / 2) * BK * 2;
-constexpr int PAIR_TOTAL_BYTES = PAIR_MAX_TOKENS * 128 * 4;   // the slices' sums so far, [token][weight row]
-constexpr size_t PAIR_SMEM = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_TOTAL_BYTES + 1024 /* alignment */ + 256 /* barriers */;
-constexpr int PAIR_OTHERS = 2 * PAIR_MAX_TOKENS;          // first tensor-memory column of the two other pieces' sums, behind two buffers of the leading ones'
-
-// Tokens in `count` tiles whose heights are multiples of 32 and differ by 32 at most: the first `tall` have `rows`, the others 32 fewer.
-struct TokenTiles {
-    int count, rows, tall;
-    __host__ __device__ int first(int t) const { return t * rows - (t > tall ? (t - tall) * 32 : 0); }
-    __host__ __device__ int height(int t) const { return t < tall ? rows : rows - 32; }
-};
-
-struct PairArgs {
-    float* out;             // parts == 1: C; else [planes][M][N] sums
-    long long ldc;
-    const float* A;
-    long long lda;
-    const bf16* W;
-    long long ldw;
-    int n_rows, m_rows, K, per, slices, parts, part_slices;   // per: K blocks a slice; part_slices: slices a part (the last may have fewer)
-    TokenTiles tokens;
-    int units;              // tiles x parts
-    int* status;
-};
-
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-gemm_split_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_low, PairArgs P)
-{
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    float* totals = reinterpret_cast<float*>(tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(totals) + PAIR_TOTAL_BYTES);   // the leader's are used
-    uint64_t* empty_bar = full_bar + PAIR_STAGES;      // every block's own
-    uint64_t* sum_full = empty_bar + PAIR_STAGES;      // [2] every block's own: a K block's sums of the leading pieces are complete
-    uint64_t* sum_empty = sum_full + 2;                // [2] the leader's are used: they have been taken out by both blocks
-    uint64_t* other_full = sum_empty + 2;              // every block's own: the slice's sums of the other pieces are complete
-    uint64_t* other_empty = other_full + 1;            // the leader's is used
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(other_empty + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();
-    const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
-    const int k_blocks = (P.K + BK - 1) / BK;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < PAIR_STAGES; ++s) {
-            mbar_init(full_bar + s, 1);
-            mbar_init(empty_bar + s, 2);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(sum_full + b, 1);
-            mbar_init(sum_empty + b, 2 * PAIR_SUM_WARPS);
-        }
-        mbar_init(other_full, 1);
-        mbar_init(other_empty, 2 * PAIR_SUM_WARPS);
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) tmem_alloc_pair(tmem_slot, 512);
-    fence_before_sync();
-    __syncthreads();
-    cluster_sync();   // both blocks' barriers are initialised and their tensor memory is allocated before either is used from the other side
-    fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-
-    // Unit u: part u % parts of tile u / parts, token tiles fastest.  Every role walks the units the same way.
-    pdl_launch_dependents();
-    if (warp == 0) {
-        if (lane == 0) {
-            bool ok = true, waited = false;
-            int s = 0;
-            uint32_t phase = 0;
-            for (int u = cluster; ok && u < P.units; u += clusters) {
-                const int tile = u / P.parts, part = u - tile * P.parts, ty = tile % P.tokens.count, h2 = P.tokens.height(ty) / 2;
-                const int x0 = (tile / P.tokens.count) * 256 + (int)rank * 128, y0 = P.tokens.first(ty) + (int)rank * h2;
-                const int kb0 = part * P.part_slices * P.per, kb1 = min(k_blocks, kb0 + P.part_slices * P.per);
-                const CUtensorMap* ma = ty < P.tokens.tall ? &map_a : &map_low;
-                const uint32_t bytes = PAIR_W_BYTES + 3u * h2 * BK * 2;
-                int pre = 0;
-                if (!waited) {
-                    // the weights of the first stages are requested before the wait for the pieces' kernel
-                    pre = min(kb1 - kb0, PAIR_STAGES);
-                    for (int i = 0; i < pre; ++i) {
-                        if (rank == 0) mbar_expect_tx(full_bar + i, 2 * bytes);   // both blocks'
-                        tma_load_2d_pair(smem_u32(tiles + (size_t)i * PAIR_STAGE_BYTES), &map_w, (kb0 + i) * BK, x0, map_to_rank(smem_u32(full_bar + i), 0));
-                    }
-                    pdl_wait();
-                    waited = true;
-                }
-                for (int kb = kb0; kb < kb1; ++kb) {
-                    const bool ahead = kb - kb0 < pre;
-                    if (!ahead && !mbar_wait(empty_bar + s, phase ^ 1, abort_flag)) { ok = false; break; }
-                    const uint32_t xs = smem_u32(tiles + (size_t)s * PAIR_STAGE_BYTES), bar = map_to_rank(smem_u32(full_bar + s), 0);
-                    if (!ahead) {
-                        if (rank == 0) mbar_expect_tx(full_bar + s, 2 * bytes);
-                        tma_load_2d_pair(xs, &map_w, kb * BK, x0, bar);
-                    }
-                    for (int p = 0; p < 3; ++p) tma_load_2d_pair(xs + PAIR_W_BYTES + p * h2 * BK * 2, ma, kb * BK, y0 + p * P.m_rows, bar);
-                    if (++s == PAIR_STAGES) {
-                        s = 0;
-                        phase ^= 1;
-                    }
-                }
-            }
-            if (!waited) pdl_wait();
-        }
-    } else if (warp < 3) {
-        if (lane == 0 && rank == 0) {
-            const bool lead = warp == 1;
-            int s = 0, b = 0;
-            uint32_t phase = 0, taken = 1, other = 1;      // parities of the releases that a buffer's next use waits for
-            bool ok = true;
-            for (int u = cluster; ok && u < P.units; u += clusters) {
-                const int tile = u / P.parts, part = u - tile * P.parts, n = P.tokens.height(tile % P.tokens.count);
-                const uint32_t idesc = instr_desc_bf16(256, lead ? n : 2 * n, false, false), off = PAIR_W_BYTES + (lead ? 0 : n / 2 * BK * 2);
-                const int z0 = part * P.part_slices, z1 = min(P.slices, z0 + P.part_slices);
-                for (int z = z0; ok && z < z1; ++z) {
-                    const int kb0 = z * P.per, kb1 = min(k_blocks, kb0 + P.per);
-                    if (!lead) {
-                        if (!mbar_wait(other_empty, other, abort_flag)) { ok = false; break; }
-                        other ^= 1;
-                    }
-                    for (int kb = kb0; kb < kb1; ++kb) {
-                        if (!mbar_wait(full_bar + s, phase, abort_flag)) { ok = false; break; }
-                        if (lead && !mbar_wait(sum_empty + b, taken, abort_flag)) { ok = false; break; }
-                        fence_after_sync();
-                        const uint32_t xs = smem_u32(tiles + (size_t)s * PAIR_STAGE_BYTES);
-                        const uint64_t dx = desc_k_major(xs), dy = desc_k_major(xs + off);
-                        const uint32_t acc = tmem + (lead ? (uint32_t)(b * PAIR_MAX_TOKENS) : (uint32_t)PAIR_OTHERS);
-#pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_pair(acc, dx + (uint64_t)(k * UMMA_K * 2 >> 4), dy + (uint64_t)(k * UMMA_K * 2 >> 4), idesc, (lead ? k > 0 : kb > kb0 || k > 0) ? 1u : 0u);
-                        if (lead) {
-                            umma_commit_pair(sum_full + b);
-                            if (++b == 2) {
-                                b = 0;
-                                taken ^= 1;
-                            }
-                        }
-                        umma_commit_pair(empty_bar + s);
-                        if (++s == PAIR_STAGES) {
-                            s = 0;
-                            phase ^= 1;
-                        }
-                    }
-                    if (ok && !lead) umma_commit_pair(other_full);
-                }
-            }
-        }
-    } else {
-        const int quarter = warp & 3, half = (warp - 3) >> 2;     // this warp's 32 weight rows of the block's and its half of the tile's tokens
-        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16);
-        const uint32_t my_sum_empty = map_to_rank(smem_u32(sum_empty), 0), my_other_empty = map_to_rank(smem_u32(other_empty), 0);
-        int b = 0;
-        uint32_t phase = 0, other = 0;
-        bool ok = true;
-        pdl_wait();   // the output may still be in use by a kernel ahead in the stream
-        for (int u = cluster; ok && u < P.units; u += clusters) {
-            const int tile = u / P.parts, part = u - tile * P.parts, ty = tile % P.tokens.count, h2 = P.tokens.height(ty) / 2;
-            const int x0 = (tile / P.tokens.count) * 256 + (int)rank * 128 + quarter * 32, y0 = P.tokens.first(ty) + half * h2;
-            const int z0 = part * P.part_slices, z1 = min(P.slices, z0 + P.part_slices);
-            float* total = totals + (size_t)half * h2 * 128 + quarter * 32;      // this warp's 32 weight rows of its first token
-            for (int z = z0; ok && z < z1; ++z) {
-                const int num_kb = min(k_blocks, (z + 1) * P.per) - z * P.per;
-                float sum[64];
-#pragma unroll
-                for (int c = 0; c < 64; ++c) sum[c] = 0.f;
-                for (int i = 0; i < num_kb; ++i) {
-                    if (!mbar_wait_warp(sum_full + b, phase, abort_flag)) { ok = false; break; }
-                    fence_after_sync();
-#pragma unroll
-                    for (int c = 0; c < 64; c += 16)
-                        if (c < h2) {
-                            uint32_t r[16];
-                            tmem_load<16>(base + (uint32_t)(b * PAIR_MAX_TOKENS + half * h2 + c), r);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) sum[c + e] += __uint_as_float(r[e]);
-                        }
-                    fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(my_sum_empty + 8 * b);
-                    if (++b == 2) {
-                        b = 0;
-                        phase ^= 1;
-                    }
-                }
-                if (!ok || !mbar_wait_warp(other_full, other, abort_flag)) { ok = false; break; }
-                other ^= 1;
-                fence_after_sync();
-                // the columns of 2 n tokens: block 0's half of the second pieces, of the third ones, block 1's of both
-#pragma unroll
-                for (int c = 0; c < 64; c += 16)
-                    if (c < h2) {
-                        uint32_t r1[16], r2[16];
-                        tmem_load<16>(base + (uint32_t)(PAIR_OTHERS + half * 2 * h2 + c), r1);
-                        tmem_load<16>(base + (uint32_t)(PAIR_OTHERS + half * 2 * h2 + h2 + c), r2);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            float* to = total + (c + e) * 128 + lane;
-                            const float v = fmaf(fmaf(__uint_as_float(r2[e]), 1.f / PIECE_SCALE, __uint_as_float(r1[e])), 1.f / PIECE_SCALE, sum[c + e]);
-                            *to = z == z0 || part > 0 ? v : *to + v;
-                        }
-                    }
-                fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(my_other_empty);
-                if ((P.parts == 1 || part == 0) && z != z1 - 1) continue;        // more of this sum follows
-                const int count = min(h2, P.m_rows - y0), outs = min(32, P.n_rows - x0);   // tokens and outputs of this warp
-                if (count > 0 && outs > 0) {
-                    const float* arow = P.A + (size_t)y0 * P.lda;
-                    const bf16* wrow = P.W + (size_t)x0 * P.ldw;
-                    float* dst = P.out + (P.parts > 1 && part > 0 ? (size_t)(z - P.part_slices + 1) * P.m_rows * P.n_rows : 0) + (size_t)y0 * P.ldc + x0;
-                    if (outs == 32 && (P.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll 1
-                        for (int t = lane >> 3; t < count; t += 4) {
-                            const int q = 4 * (lane & 7);
-                            float v[4];
-                            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(total + t * 128 + q);
-                            if (P.parts == 1)
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    if (!isfinite(v[e])) v[e] = plain_sum(arow + (size_t)t * P.lda, wrow + (size_t)(q + e) * P.ldw, P.K);
-                            *reinterpret_cast<float4*>(dst + (size_t)t * P.ldc + q) = make_float4(v[0], v[1], v[2], v[3]);
-                        }
-                    } else if (lane < outs) {
-                        for (int t = 0; t < count; ++t) {
-                            float v = total[t * 128 + lane];
-                            if (P.parts == 1 && !isfinite(v)) v = plain_sum(arow + (size_t)t * P.lda, wrow + (size_t)lane * P.ldw, P.K);
-                            dst[(size_t)t * P.ldc + lane] = v;
-                        }
-                    }
-                }
-                __syncwarp();   // the next slice's sums may come
-            }
-        }
-    }
-    fence_before_sync();
-    __syncthreads();
-    if (*abort_flag) {
-        if (threadIdx.x == 0) {
-            // a wait ran out: copies that may still be in flight get time to land before the shared memory is released
-            const unsigned long long t0 = global_timer();
-            while (global_timer() - t0 < 2000000ull) { }
-            report_status(P.status, SPY_STATUS_WAIT_TIMEOUT, (int)blockIdx.x);
-        }
-        __syncthreads();
-    }
-    cluster_sync();   // neither block leaves (and frees tensor memory the pair shares) while the other may still use it
-    if (warp == 0) {
-        fence_after_sync();
-        tmem_dealloc_pair(tmem, 512);
-    }
-}
-
-// The planes of a product whose slices were shared out, added in order.
-__global__ void __launch_bounds__(256) split_reduce_kernel(const float* __restrict__ sums, int planes, float* __restrict__ C, long long ldc, const float* __restrict__ A,
-                                                           long long lda, const bf16* __restrict__ W, long long ldw, int M, int N, int K)
-{
-    pdl_enter();
-    const long long total = (long long)M * N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int t = (int)(i / N), x = (int)(i - (long long)t * N);
-        float v = sums[i];
-        for (int p = 1; p < planes; ++p) v += sums[p * total + i];
-        if (!isfinite(v)) v = plain_sum(A + (size_t)t * lda, W + (size_t)x * ldw, K);
-        C[(size_t)t * ldc + x] = v;
-    }
-}
-
 // The three pieces of 32-bit rows: pieces[p][m][k], eight numbers a thread.  Numbers that are not finite go into the first piece alone.
 // The second piece is stored 2^PIECE_SHIFT times as large, the third 2^(2 PIECE_SHIFT): as they are, their last bits would lie below the smallest
 // bfloat16 number (2^-133) for numbers under 2^-110.
@@ -791,84 +505,13 @@ int launch(const CUtensorMap& mw, const CUtensorMap& ma, float* C, long long ldc
     return 0;
 }
 
-// How many clusters of two blocks of the pair kernel the device holds, asked once per device.
-int resident_pairs(int* count)
-{
-    static int known[SPY_MAX_DEVICES] = {};
-    int& c = known[spy_device()];
-    if (c == 0) {
-        SPY_CUDA(cudaFuncSetAttribute(gemm_split_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(spy_sm_count() / 2 * 2);
-        cfg.blockDim = dim3(PAIR_THREADS);
-        cfg.dynamicSmemBytes = PAIR_SMEM;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        SPY_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_split_pair_kernel, &cfg));
-        if (n <= 0) SPY_FAIL("gemm_split: no cluster of two blocks fits the device");
-        c = n < spy_sm_count() / 2 ? n : spy_sm_count() / 2;
-    }
-    *count = c;
-    return 0;
-}
-
-// The way of a product of more than 64 rows: into how many token tiles, and into how many parts a tile's slices.  Cycles of a K block:
-// what its 12 products take (6 n) and no less than its bytes' way from L2 (45 a cycle and block); of a slice's end and a unit's start about
-// 600 and 3,000; the planes of shared-out slices are written and read once more (4 bytes each, 4,000 a cycle) by a kernel more.
-struct PairPlan {
-    TokenTiles tokens;
-    int parts, part_slices, planes;
-};
-PairPlan plan_pairs(int M, int N, int slices, int per, int clusters)
-{
-    PairPlan best = {};
-    double least = 0;
-    const int runs = (M + 31) / 32, columns = (N + 255) / 256, fewest = (M + PAIR_MAX_TOKENS - 1) / PAIR_MAX_TOKENS, most = runs < 256 ? runs : fewest + 2;
-    for (int count = fewest; count <= most; ++count) {
-        const int each = runs / count, more = runs % count;
-        if (each == 0 || 32 * (each + (more > 0)) > PAIR_MAX_TOKENS) continue;
-        const TokenTiles t = {count, 32 * (more > 0 ? each + 1 : each), more > 0 ? more : count};
-        const double products = 6.0 * t.rows, bytes = (PAIR_W_BYTES + 192.0 * t.rows) / 45.0, block = products > bytes ? products : bytes;
-        for (int parts = 1; parts <= slices; ++parts) {
-            const int ps = (slices + parts - 1) / parts;
-            if ((slices + ps - 1) / ps != parts) continue;
-            const long long units = (long long)columns * count * parts, rounds = (units + clusters - 1) / clusters;
-            const int planes = parts > 1 ? 1 + slices - ps : 1;
-            const double cost = rounds * (ps * (per * block + 600.0) + 3000.0) + (parts > 1 ? 4000.0 + 8.0 * planes * M * N / 4000.0 : 0.0);
-            if (least == 0 || cost < least) {
-                least = cost;
-                best = {t, parts, ps, planes};
-            }
-        }
-    }
-    return best;
-}
-
 }  // namespace
-
-// Bytes of scratch that spy_gemm_split needs for M rows: the pieces, and for more than 64 rows what shared-out slices leave.  0: an error.
-extern "C" long long spy_gemm_split_scratch(int M, int N, int K)
-{
-    const long long pieces = (3LL * M * K * 2 + 15) / 16 * 16;
-    if (M <= 64 || N <= 0 || K <= 0) return pieces;
-    int slices = 1, clusters = 0;
-    const int k_blocks = (K + BK - 1) / BK;
-    if (plan_slices(N, k_blocks, &slices) || resident_pairs(&clusters)) return 0;
-    const PairPlan plan = plan_pairs(M, N, slices, (k_blocks + slices - 1) / slices, clusters);
-    return pieces + (plan.parts > 1 ? 4LL * plan.planes * M * N : 0);
-}
 
 // Slices of K that a weight of this shape is cut into (for the tests).
 extern "C" int spy_gemm_split_slices(int N, int K, int* slices) { return plan_slices(N, (K + BK - 1) / BK, slices); }
 
 // A [M, K] and C [M, N] float32, W [N, K] bfloat16, rows lda/ldc/ldw elements apart (W's on 16-byte borders; K a multiple of 8).
-// pieces: scratch of spy_gemm_split_scratch bytes, 16-byte aligned (up to 64 rows: 3 * M * K bfloat16).
+// pieces: scratch of 3 * M * K bfloat16, 16-byte aligned.
 extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long long ldw, float* C, long long ldc, int M, int N, int K, void* pieces,
                               int* status, cudaStream_t stream)
 {
@@ -888,36 +531,18 @@ extern "C" int spy_gemm_split(const float* A, long long lda, const void* W, long
     int slices = 1;
     if (int rc = plan_slices(N, k_blocks, &slices)) return rc;
     const int per = (k_blocks + slices - 1) / slices;
-    if (M > 64) {
-        int clusters = 0;
-        if (int rc = resident_pairs(&clusters)) return rc;
-        const PairPlan plan = plan_pairs(M, N, slices, per, clusters);
-        float* sums = reinterpret_cast<float*>((char*)pieces + (3LL * M * K * 2 + 15) / 16 * 16);
-        CUtensorMap mw, ma, mlow;
-        const int low = plan.tokens.rows > 32 ? plan.tokens.rows - 32 : 32;
-        if (make_map(&mw, W, N, K, ldw, 128) || make_map(&ma, pieces, 3LL * M, K, K, plan.tokens.rows / 2) || make_map(&mlow, pieces, 3LL * M, K, K, low / 2)) return 1;
-        const bool shared = plan.parts > 1;
-        const PairArgs P = {shared ? sums : C, shared ? (long long)N : ldc, A, lda, (const bf16*)W, ldw, N, M, K, per, slices, plan.parts, plan.part_slices, plan.tokens,
-                            (N + 255) / 256 * plan.tokens.count * plan.parts, status};
-        const int pairs = P.units < clusters ? P.units : clusters;
-        spy_launch_cluster(gemm_split_pair_kernel, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, stream, 2u, mw, ma, mlow, P);
-        SPY_CHECK_LAUNCH("gemm_split (pairs)");
-        if (shared) {
-            long long reduce_blocks = ((long long)M * N + 255) / 256;
-            if (reduce_blocks > 8LL * spy_sm_count()) reduce_blocks = 8LL * spy_sm_count();
-            spy_launch(split_reduce_kernel, dim3((unsigned)reduce_blocks), dim3(256), 0, stream, (const float*)sums, plan.planes, C, ldc, A, lda, (const bf16*)W, ldw, M, N, K);
-            SPY_CHECK_LAUNCH("gemm_split (sum of slices)");
-        }
-        return 0;
-    }
-    // 64 tokens and fewer: one token tile, as narrow as it may be.
+    // 64 tokens and fewer: one token tile, as narrow as it may be.  More: 256 weight rows under every 64 tokens.
     const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
-    int tile_rows = 128, clusters = 0;
-    if (int rc = resident_clusters(slices, bn == 64 ? 1 : 2, &clusters)) return rc;
-    plan_rows(N, slices, clusters, per, &tile_rows);
+    int tile_rows = 256;
+    if (M <= 64) {
+        int clusters = 0;
+        if (int rc = resident_clusters(slices, bn == 64 ? 1 : 2, &clusters)) return rc;
+        plan_rows(N, slices, clusters, per, &tile_rows);
+    }
     CUtensorMap mw, ma;
     if (make_map(&mw, W, N, K, ldw, tile_rows) || make_map(&ma, pieces, 3LL * M, K, K, bn)) return 1;
 #define SPY_SPLIT_LAUNCH(BN_, H_) launch<BN_, H_>(mw, ma, C, ldc, A, lda, (const bf16*)W, ldw, N, M, K, slices, per, tile_rows, status, stream)
+    if (M > 64) return SPY_SPLIT_LAUNCH(64, 2);
     if (bn == 16) return SPY_SPLIT_LAUNCH(16, 1);
     if (bn == 32) return SPY_SPLIT_LAUNCH(32, 1);
     return SPY_SPLIT_LAUNCH(64, 1);

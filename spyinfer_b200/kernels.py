@@ -920,15 +920,7 @@ def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Opti
         raise KernelError(f"gemm: shapes do not fit: input {tuple(a.shape)}, weight {tuple(w.shape)}, output {tuple(out.shape)}")
     if status is None:
         status = status_word(a.device)
-    nbytes = 6 * min(M, GEMM_SPLIT_ROWS) * K
-    if M > 64:                                                # a pass's last rows may take another plan than a whole pass
-        f = build.load("gemm_split").spy_gemm_split_scratch
-        f.restype = ctypes.c_longlong
-        needs = [int(f(m, N, K)) for m in {min(M, GEMM_SPLIT_ROWS), M % GEMM_SPLIT_ROWS} if m > 0]
-        if 0 in needs:
-            raise KernelError(build.last_error("gemm_split"))
-        nbytes = max(needs)
-    pieces = torch.empty(nbytes, dtype=torch.uint8, device=a.device)
+    pieces = torch.empty((3, min(M, GEMM_SPLIT_ROWS), K), dtype=torch.bfloat16, device=a.device)
     for first in range(0, M, GEMM_SPLIT_ROWS):
         rows = min(GEMM_SPLIT_ROWS, M - first)
         _call("gemm_split", "spy_gemm_split", _ptr(a[first:]), ctypes.c_longlong(K), _ptr(w), ctypes.c_longlong(ldw), _ptr(out[first:]), ctypes.c_longlong(N),
