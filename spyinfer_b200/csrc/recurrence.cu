@@ -14,7 +14,8 @@
 // kept and updated by each tile for itself (dk + 1 numbers for every 8 columns in the state record: no tile ever reads
 // what another writes, whenever their blocks happen to run).  Two kernels: one for steps with prompt portions (scan_kernel),
 // whose arithmetic for a token does not depend on where a portion starts or ends, and one for steps in which every request
-// brings one token (scan_decode_kernel: `longest` = 1), whose sums over a column's rows run in another order.
+// brings one token (scan_decode_kernel: `longest` = 1), whose sums over a column's rows run in another order.  Long portions are taken in
+// chunks of tokens instead (see "runs of tokens as products"), whose results depend on where a portion starts to a few roundings of 32 bits.
 //
 // Inputs are columns of one 32-bit activation matrix `proj` [T, ld] (the fused projection of the mixer's input).
 #include "common.cuh"
@@ -56,7 +57,9 @@ struct ScanArgs {
 };
 
 // Which form a request takes where both run: see "runs of tokens as products" below.
-constexpr int CHUNK_MIN = 48;
+// The least tokens: where the forms meet for one request (us, tokens / chunks: matrix memory of 4 heads, 80 tokens 22 / 27, 100 27 / 27, 128 32 / 27; delta rule
+// of 32 heads, 100 tokens 34 / 38, 128 41 / 36; linear attention of 8 heads, 128 tokens 39 / 46, 256 72 / 54).
+__host__ __device__ constexpr int chunk_min(int mode) { return mode == 0 ? 96 : (mode == 1 ? 128 : 160); }
 template <int MODE> struct ChunkOf { static constexpr int C = MODE == 1 ? 32 : 64; };   // tokens of a chunk
 // A chunk's place in the scratch: chunk j of sequence s at q_start[s] / C + s + j, which no two chunks share.
 __device__ __forceinline__ int chunk_slot(int t_begin, int seq, int C) { return t_begin / C + seq; }
@@ -65,7 +68,7 @@ template <int MODE>
 __device__ __forceinline__ bool takes_chunks(const ScanArgs& A, int seq, int h, int t_begin, int t_end)
 {
     constexpr int C = ChunkOf<MODE>::C;
-    if (A.flags == nullptr || t_end - t_begin < CHUNK_MIN) return false;
+    if (A.flags == nullptr || t_end - t_begin < chunk_min(MODE)) return false;
     const int first = chunk_slot(t_begin, seq, C), n = (t_end - t_begin + C - 1) / C;
     int bad = 0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) bad |= A.flags[(size_t)(first + j) * A.H + h];
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 
 // ---- runs of tokens as products --------------------------------------------------------------------------------------------
 //
-// A request that brings CHUNK_MIN tokens or more is walked in chunks of C tokens instead of token by token.  Written out over a
+// A request that brings many tokens (chunk_min and more) is walked in chunks of C tokens instead of token by token.  Written out over a
 // chunk, each recurrence gives the chunk's outputs and the state behind it as products with the state S ahead of it and the
 // chunk's values V, whose other factors do not depend on S:
 //   matrix memory:  o_t = (alpha_t (P V)_t + beta_t S^T q_t) / ...,   S' = g S + K^T diag(kappa) V,   P_ts = exp(F_t - F_s + i_s - l_t) q_t . k_s
@@ -566,12 +569,16 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 // decays of linear attention are taken relative to sub-blocks of 16 tokens, so that no factor exceeds 1.)
 //
 // Two kernels: chunk_*_kernel makes these factors, a block a (chunk, head), all chunks side by side; walk_*_kernel carries S through a
-// request's chunks, a block 16 value columns of a (request, head).  What bounds the walk is the CUDA cores' additions (a chunk of 64
-// tokens at 128 x 16 needs 330 K of them) and the shared-memory reads beside them; the token-by-token kernel above spends 270
-// to 300 ns a token, nearly all of it waiting.
-// MEASURED_PLACEHOLDER
+// request's chunks, a block 16 value columns of a (request, head).  What bounds the walk is the way through a chunk on eight warps (a chunk of
+// 64 tokens at 128 x 16 takes 4.5 us, its 330 K additions 1.4, its shared-memory reads about 2); the token-by-token kernel above
+// spends 270 to 300 ns a token on one request, nearly all of it waiting.  Measured, chunks' kernels and walk together (us, by tokens before / in chunks):
+//   matrix memory, 8 heads of 128 x 256: one request of 256 tokens 76 / 38, of 2,047 567 / 176; 8 of 100 to 400 460 / 233; 16 of 1,024 2,581 / 1,495;
+//   delta rule, 32 heads of 64: one request of 256 79 / 49, of 2,047 607 / 297; two of 1,024 385 / 300;
+//   linear attention, 16 heads of 128 x 256: one of 256 101 / 70, of 2,047 774 / 372; 8 of 100 to 400 704 / 475; 16 of 1,024 4,094 / 2,967.
+// Error against 64 bits over some hundred tokens (2-norm): matrix memory half of the walk's by tokens (2.0e-5 and 9.7e-6, its divisions), linear attention
+// 1.75e-7 and 1.9e-7, delta rule 1.1e-7 and 1.8e-7: all sums stay in 32-bit, products of decays are taken in 64-bit and rounded once.
 //
-// Which form a request takes is decided on the device by one rule (takes_chunks) in both kernels: runs of fewer than CHUNK_MIN tokens and
+// Which form a request takes is decided on the device by one rule (takes_chunks) in both kernels: runs of fewer than chunk_min tokens and
 // requests with a number among their q, k, v, decays or gates that is not below HUGE_INPUT in magnitude (or is no number) are walked token
 // by token as before: in the products an infinity of a later token would meet the zeros of an earlier one.
 constexpr float HUGE_INPUT = 1e10f;
@@ -592,9 +599,10 @@ __host__ __device__ constexpr int chunk_floats(int mode, int dk)
 }
 
 // The (sequence, chunk) of a place in the scratch; false where there is none.
-template <int C>
+template <int MODE>
 __device__ __forceinline__ bool chunk_of_slot(const ChunkArgs& A, int slot, int& seq, int& t0, int& n_tok)
 {
+    constexpr int C = ChunkOf<MODE>::C;
     int lo = 0, hi = A.num_seqs;           // the last sequence whose first place is at most `slot`
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -605,7 +613,7 @@ __device__ __forceinline__ bool chunk_of_slot(const ChunkArgs& A, int slot, int&
     const int t_begin = A.s.q_start[lo], t_end = A.s.q_start[lo + 1];
     t0 = t_begin + (slot - chunk_slot(t_begin, lo, C)) * C;
     n_tok = min(C, t_end - t0);
-    return slot >= chunk_slot(t_begin, lo, C) && t0 < t_end && t_end - t_begin >= CHUNK_MIN;
+    return slot >= chunk_slot(t_begin, lo, C) && t0 < t_end && t_end - t_begin >= chunk_min(MODE);
 }
 
 __device__ __forceinline__ bool huge(float x) { return !(fabsf(x) < HUGE_INPUT); }
@@ -649,7 +657,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
     pdl_enter();
     int seq, t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<0>(A, blockIdx.x, seq, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(0, DK);
     float *P = mine, *F = mine + C * C, *loc = F + C, *kap = loc + C, *psum = kap + C, *ksum = psum + C;
@@ -751,7 +759,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     pdl_enter();
     int seq, t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<2>(A, blockIdx.x, seq, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(2, DK);
     float *P = mine, *Q = mine + C * C, *K = Q + C * DK, *dec = K + C * DK;
@@ -773,41 +781,57 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
     // inside a sub-block: k_s carried from its token on, a decay at a time; a warp takes every eighth token, a lane DK / 32 channels
     for (int s = warp; s < C; s += THREADS / 32) {
-        const int end = (s / B + 1) * B;
+        const int b0 = s & ~(B - 1), first = s - b0;
         constexpr int E = DK / 32;
-        float w[E];
+        float w[E], d[B];
 #pragma unroll
         for (int e = 0; e < E; ++e) w[e] = k_s[s * LD + lane + 32 * e];
-        float keep = 0.f;                          // lane t - s keeps P_ts
-        for (int t = s; t < end; ++t) {
-            float d = 0.f;
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                if (t > s) w[e] *= a_s[t * LD + lane + 32 * e];
-                d = fmaf(w[e], q_s[t * LD + lane + 32 * e], d);
+        for (int i = 0; i < B; ++i) {
+            d[i] = 0.f;
+            if (i >= first) {                      // the same for the whole warp
+                const float* at = a_s + (b0 + i) * LD + lane;
+                const float* qt = q_s + (b0 + i) * LD + lane;
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    if (i > first) w[e] *= at[32 * e];
+                    d[i] = fmaf(w[e], qt[32 * e], d[i]);
+                }
             }
-            d = warp_sum(d);
-            if (lane == t - s) keep = d;
         }
-        if (s + lane < end) P[(s + lane) * C + s] = keep * a.q_scale;
+        // the sixteen sums over the warp together: with every step a lane keeps half of its sums
+        int mine = 0;
+#pragma unroll
+        for (int o = 16, n = B / 2; n > 0; o >>= 1, n >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                const float own = up ? d[i + n] : d[i], give = up ? d[i] : d[i + n];
+                d[i] = own + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            mine += up ? n : 0;
+        }
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+        if ((lane & 1) == 0) P[(b0 + mine) * C + s] = d[0] * a.q_scale;       // zero above the diagonal
     }
     for (int idx = tid; idx < C * C; idx += THREADS)
-        if ((idx & (C - 1)) > idx / C) P[idx] = 0.f;
+        if ((idx & (C - 1)) / B > idx / C / B) P[idx] = 0.f;
     __syncthreads();
     // q from its sub-block's start, k to its sub-block's end; a_s's last row of a sub-block then holds the sub-block's product
     for (int idx = tid; idx < DK * (C / B); idx += THREADS) {
         const int c = idx % DK, b0 = idx / DK * B;
-        float run = 1.f;
-        for (int t = b0; t < b0 + B; ++t) {
-            run *= a_s[t * LD + c];
-            q_s[t * LD + c] *= run * a.q_scale;
+        double run = 1.0, back = 1.0;              // products of up to sixteen decays, rounded once
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            run *= a_s[(b0 + i) * LD + c];
+            q_s[(b0 + i) * LD + c] *= (float)run * a.q_scale;
         }
-        float back = 1.f;
-        for (int t = b0 + B - 1; t >= b0; --t) {
-            k_s[t * LD + c] *= back;
-            back *= a_s[t * LD + c];
+#pragma unroll
+        for (int i = B - 1; i >= 0; --i) {
+            k_s[(b0 + i) * LD + c] *= (float)back;
+            back *= a_s[(b0 + i) * LD + c];
         }
-        a_s[(b0 + B - 1) * LD + c] = run;
+        a_s[(b0 + B - 1) * LD + c] = (float)run;
     }
     __syncthreads();
     // across sub-blocks, one after the other: the keys so far reach the end of the sub-block ahead.  A thread has row t = b B + tid / 16
@@ -846,7 +870,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     }
 }
 
-__global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
+__global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
 {
     constexpr int C = 32, D = 64, LD = D + 4, R = D + C, LDM = R + 4;
     extern __shared__ __align__(16) float sm[];
@@ -860,7 +884,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
     pdl_enter();
     int seq, t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<C>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<1>(A, blockIdx.x, seq, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* W = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(1, D);
     const float* rows = a.proj + (size_t)t0 * a.ld;
@@ -889,16 +913,18 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
     }
     __syncthreads();
     if (tid < D) {
+        double product = 1.0;                      // of the decays so far, rounded where it is used
         float run = 1.f;
+#pragma unroll 8
         for (int t = 0; t < C; ++t) {
             const float k = bc[(C + t) * LD + tid], u = k * inv_s[t], rate = bc[t * LD + tid];
             pg[t * LD + tid] = u * run;
-            run *= PM[t * LDM + tid];
-            const float back = 1.0f / run;
+            product *= PM[t * LDM + tid];
+            run = (float)product;
             pg[(C + t) * LD + tid] *= run;
-            const float b = rate * u * back;
+            const float b = rate * u / run;
             bc[t * LD + tid] = b;
-            bc[(C + t) * LD + tid] = k * back;
+            bc[(C + t) * LD + tid] = k / run;
             XB[t * LDM + C + tid] = b;
         }
         last_s[tid] = run;
@@ -949,16 +975,16 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
     }
     __syncthreads();
     {
-        // [X; b^T] [P' | M'], 96 x 96: rows ty + 16 i (outputs, then the state's rows), columns tx + 16 j
+        // [X; b^T] [P' | M'], 96 x 96: rows 6 ty + i (outputs, then the state's rows), columns 6 tx + j
         const int tx = tid & 15, ty = tid >> 4;
         float acc[6][6] = {};
 #pragma unroll 4
         for (int s = 0; s < C; ++s) {
             float x[6], m[6];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                x[i] = XB[s * LDM + ty + 16 * i];
-                m[i] = PM[s * LDM + tx + 16 * i];
+            for (int i = 0; i < 6; i += 2) {
+                *reinterpret_cast<float2*>(x + i) = *reinterpret_cast<const float2*>(XB + s * LDM + 6 * ty + i);
+                *reinterpret_cast<float2*>(m + i) = *reinterpret_cast<const float2*>(PM + s * LDM + 6 * tx + i);
             }
 #pragma unroll
             for (int i = 0; i < 6; ++i)
@@ -966,15 +992,18 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
                 for (int j = 0; j < 6; ++j) acc[i][j] = fmaf(x[i], m[j], acc[i][j]);
         }
 #pragma unroll
-        for (int i = 0; i < 6; ++i)
+        for (int i = 0; i < 6; ++i) {
+            const int row = 6 * ty + i;
+            float v[6];
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
-                const int row = ty + 16 * i, col = tx + 16 * j;
-                float v;
-                if (i < 2) v = (j < 4 ? pg[(C + row) * LD + col] : Y[row * (C + 1) + col - D]) - acc[i][j];
-                else v = last_s[row - C] * ((j < 4 ? (row - C == col ? 1.f : 0.f) : bc[(C + col - D) * LD + row - C]) - acc[i][j]);
-                W[row * R + col] = v;
+                const int col = 6 * tx + j;
+                if (row < C) v[j] = (col < D ? pg[(C + row) * LD + col] : Y[row * (C + 1) + col - D]) - acc[i][j];
+                else v[j] = last_s[row - C] * ((col < D ? (row - C == col ? 1.f : 0.f) : bc[(C + col - D) * LD + row - C]) - acc[i][j]);
             }
+#pragma unroll
+            for (int j = 0; j < 6; j += 2) *reinterpret_cast<float2*>(W + row * R + 6 * tx + j) = make_float2(v[j], v[j + 1]);
+        }
     }
 }
 
@@ -1022,9 +1051,9 @@ template <int MODE, int DK> struct WalkSmem {
     static constexpr int C = 64, LDK = DK + 4, LDP = C + 4;
     static constexpr int Q = 0, P = Q + C * LDK, K = P + C * LDP, V = K + C * LDK, X = V + C * WALK_LD;     // floats; X: F, l, kappa, psum, ksum | the decays
     static constexpr int STAGE = X + (MODE == 0 ? 4 * C + DK : DK);
-    static constexpr int S = 2 * STAGE, N = S + DK * WALK_LD, TOTAL = N + DK + 3 * C;      // N: n; then alpha, beta, n . q
+    static constexpr int S = 2 * STAGE, N = S + DK * WALK_LD, RED = N + DK, TOTAL = RED + 8 * C * WALK_COLS;      // N: n; RED: the warps' parts of the outputs
     static constexpr size_t BYTES = TOTAL * sizeof(float);
-    static_assert(8 * C * WALK_COLS <= K, "the parts of the outputs fit the place of q and P");
+    static_assert(BYTES <= 227 * 1024, "a block's shared memory");
 };
 
 template <int MODE, int DK>
@@ -1033,7 +1062,7 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
     using L = WalkSmem<MODE, DK>;
     constexpr int C = L::C, LDK = L::LDK, LDP = L::LDP, KW = DK / 8;       // KW: rows of S a warp owns
     extern __shared__ __align__(16) float sm[];
-    float *S_s = sm + L::S, *n_s = sm + L::N, *alpha_s = n_s + DK, *beta_s = alpha_s + C, *nq_s = beta_s + C;
+    float *S_s = sm + L::S, *n_s = sm + L::N, *red = sm + L::RED;
     pdl_enter();
     const ScanArgs& a = A.s;
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS, dv = a.dv;
@@ -1090,70 +1119,44 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
         cp_async_wait_all();
         __syncthreads();                           // this chunk has landed, the chunk before is done with
         if (t0 + C < t_end) request(t0 + C, stage ^ 1);
-        float keep = 1.f, add = 1.f;               // of the old state and of the chunk's sum
+        float keep = 1.f, add = 1.f, nq = 0.f;     // of the old state and of the chunk's sum; n . q of token tid / 4
+        const auto taken = [&](int t, float& alpha, float& beta) {     // what a token's output takes of the chunk and of the state ahead
+            const float l = X[C + t], f = X[t] + m, top = fmaxf(f, l);
+            alpha = expf(l - top);
+            beta = expf(f - top);
+        };
         if (MODE == 0) {
-            if (tid < C) {
-                const float l = X[C + tid], f = X[tid] + m, top = fmaxf(f, l);
-                alpha_s[tid] = expf(l - top);
-                beta_s[tid] = expf(f - top);
-            }
-            const float l = X[C + C - 1], f = X[C - 1] + m, top = fmaxf(f, l);     // behind the chunk (padding tokens change nothing)
-            keep = expf(f - top);
-            add = expf(l - top);
-            // n . q: four threads a token
+            taken(C - 1, add, keep);               // behind the chunk (padding tokens change nothing)
             const int t = tid >> 2, part = tid & 3;
-            float s = 0.f;
 #pragma unroll
-            for (int c = 0; c < DK / 4; c += 4) s = dot4(ld4(Q + t * LDK + 4 * c + 4 * part), ld4(n_s + 4 * c + 4 * part), s);
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if (part == 0) nq_s[t] = s;
+            for (int c = 0; c < DK / 4; c += 4) nq = dot4(ld4(Q + t * LDK + 4 * c + 4 * part), ld4(n_s + 4 * c + 4 * part), nq);
+            nq += __shfl_xor_sync(0xffffffffu, nq, 1);
+            nq += __shfl_xor_sync(0xffffffffu, nq, 2);
         }
-        // what the state ahead of the chunk gives: this warp's rows of it
+        // what the state ahead of the chunk gives: this warp's rows of it; then this warp's share of the chunk's own tokens
         float acc[8][4] = {};
 #pragma unroll
         for (int k = 0; k < KW; k += 4) tile_fma<8, LDK>(acc, Q + g * LDK + warp * KW + k, S_s + (warp * KW + k) * WALK_LD + 4 * cg);
         if (MODE == 0) {
-            __syncthreads();                       // alpha, beta and n . q are there; n has been read
             float own[8][4] = {};
 #pragma unroll
             for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(own, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float al = alpha_s[g + 8 * j], be = beta_s[g + 8 * j] * a.q_scale;
+                float alpha, beta;
+                taken(g + 8 * j, alpha, beta);
+                beta *= a.q_scale;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(be, acc[j][c], al * own[j][c]);
+                for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(beta, acc[j][c], alpha * own[j][c]);
             }
         } else {
 #pragma unroll
             for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(acc, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
         }
-        __syncthreads();                           // q, P and the values as they came have been read
-        float* red = Q;
         put_parts<8>(red, warp, g, cg, acc);
-        if (MODE == 0) {
-            if (tid < C * 4) {                     // the values as the state takes them
-                float* v = V + (tid >> 2) * WALK_LD + 4 * (tid & 3);
-                const float s = X[2 * C + (tid >> 2)] * add;
-                float4 x = ld4(v);
-                st4(v, make_float4(x.x * s, x.y * s, x.z * s, x.w * s));
-            }
-            for (int r = tid; r < DK; r += THREADS) n_s[r] = fmaf(keep, n_s[r], add * X[4 * C + r]);
-        }
-        __syncthreads();
-        {
-            const int t = tid >> 2, part = tid & 3;
-            float4 o = sum_parts<C>(red, t, part);
-            if (MODE == 0) {
-                const float l = X[C + t], f = X[t] + m;
-                const float nq = fmaf(beta_s[t] * a.q_scale, nq_s[t], alpha_s[t] * X[3 * C + t]);
-                const float d = fmaxf(fabsf(nq), expf(-fmaxf(f, l))) + 1e-6f;
-                o = make_float4(o.x / d, o.y / d, o.z / d, o.w / d);
-            }
-            if (t < n_tok) st4(a.out + (size_t)(t0 + t) * a.H * dv + h * dv + c0 + 4 * part, o);
-        }
-        // The state behind the chunk.  A warp's rows: a lane has half of them and four columns, over every fourth token; the four sums meet
-        // by shuffles, each lane keeping a quarter.
+        // The state behind the chunk.  A warp's rows (no other warp reads them): a lane has half of them and four columns, over every fourth
+        // token; the four sums meet by shuffles, each lane keeping a quarter.
+        __syncwarp();
         {
             constexpr int RL = KW / 2;             // rows of a lane
             const int rg = lane >> 4, sg = lane >> 2 & 3, r0 = warp * KW + rg * RL;
@@ -1164,6 +1167,11 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
 #pragma unroll
                 for (int r = 0; r < RL; r += 4) *reinterpret_cast<float4*>(kk + r) = ld4(K + s * LDK + r0 + r);
                 *reinterpret_cast<float4*>(vv) = ld4(V + s * WALK_LD + 4 * cg);
+                if (MODE == 0) {
+                    const float f = X[2 * C + s] * add;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) vv[c] *= f;
+                }
 #pragma unroll
                 for (int r = 0; r < RL; ++r)
 #pragma unroll
@@ -1196,7 +1204,23 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
                 st4(s, make_float4(fmaf(d, o.x, mine[r][0]), fmaf(d, o.y, mine[r][1]), fmaf(d, o.z, mine[r][2]), fmaf(d, o.w, mine[r][3])));
             }
         }
-        if (MODE == 0) m = fmaxf(X[C - 1] + m, X[C + C - 1]);
+        __syncthreads();                           // the outputs' parts are there; n has been read
+        {
+            const int t = tid >> 2, part = tid & 3;
+            float4 o = sum_parts<C>(red, t, part);
+            if (MODE == 0) {
+                float alpha, beta;
+                taken(t, alpha, beta);
+                nq = fmaf(beta * a.q_scale, nq, alpha * X[3 * C + t]);
+                const float d = fmaxf(fabsf(nq), expf(-fmaxf(X[t] + m, X[C + t]))) + 1e-6f;
+                o = make_float4(o.x / d, o.y / d, o.z / d, o.w / d);
+            }
+            if (t < n_tok) st4(a.out + (size_t)(t0 + t) * a.H * dv + h * dv + c0 + 4 * part, o);
+        }
+        if (MODE == 0) {
+            for (int r = tid; r < DK; r += THREADS) n_s[r] = fmaf(keep, n_s[r], add * X[4 * C + r]);
+            m = fmaxf(X[C - 1] + m, X[C + C - 1]);
+        }
     }
     __syncthreads();
     for (int idx = tid; idx < DK * 4; idx += THREADS) st4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3), ld4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3)));
@@ -1281,11 +1305,14 @@ template <typename Args> static int launch_chunk_kernel(void (*kernel)(Args), di
     return 0;
 }
 
-// Which sizes take chunks: keys of 64 or 128 channels (the delta rule's states of 64 x 64), value columns in sixteens, steps of
-// CHUNK_MIN tokens or more whose factors fit 512 MB (200 K tokens of 8 heads of the matrix memory, 14 K of 32 heads of the delta rule).
+// Which steps take chunks: keys of 64 or 128 channels (the delta rule's states of 64 x 64), value columns in sixteens, requests that bring half
+// of chunk_min or more on average (with fewer the kernels that find nothing to do are what is left), factors that fit 512 MB (200 K tokens of
+// 8 heads of the matrix memory).  The delta rule with up to 64 (request, head) pairs: with more, the walk by tokens has work for every SM and does
+// fewer additions (32 heads, requests of 1,024 tokens, us by tokens / in chunks: two 385 / 300, four 477 / 583).
 static long long chunk_work_floats(int mode, int tokens, int num_seqs, int H, int dk, int dv)
 {
-    if (tokens < CHUNK_MIN || dv % WALK_COLS != 0 || !(mode == 1 ? dk == 64 && dv == 64 : dk == 64 || dk == 128)) return 0;
+    if (tokens < chunk_min(mode) || 2LL * tokens < (long long)num_seqs * chunk_min(mode) || dv % WALK_COLS != 0) return 0;
+    if (mode == 1 ? dk != 64 || dv != 64 || (long long)num_seqs * H > 64 : dk != 64 && dk != 128) return 0;
     const long long slots = tokens / (mode == 1 ? 32 : 64) + (long long)num_seqs + 1;
     const long long floats = slots * H * (chunk_floats(mode, dk) + 4LL);
     return floats <= (128LL << 20) && slots <= 0x7fffffff ? floats : 0;
@@ -1398,7 +1425,7 @@ static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, int tok
     const bool aligned = ((A.ld | A.off_q | A.off_k | A.off_v | (mode == 1 ? A.off_x1 : 0)) & 3) == 0 && A.record % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(A.proj) | reinterpret_cast<uintptr_t>(A.state) | reinterpret_cast<uintptr_t>(A.out) |
                            reinterpret_cast<uintptr_t>(work)) & 15) == 0;
-    if (work != nullptr && longest >= CHUNK_MIN && aligned) {
+    if (work != nullptr && longest >= chunk_min(mode) && aligned) {
         const long long need = chunk_work_floats(mode, tokens, num_seqs, A.H, A.dk, A.dv);
         if (need > work_floats) SPY_FAIL("recurrence: %lld floats of scratch for %d tokens, %lld are needed", work_floats, tokens, need);
         if (need > 0) {

@@ -88,9 +88,9 @@ def new_state(kind, dk, dv, slots):
 @pytest.mark.parametrize("hard", [False, True])
 @pytest.mark.parametrize("kind,dk,dv", CASES)
 def test_chunks_carry_the_state_through_portions_as_the_walk_by_tokens_does(kind, dk, dv, hard):
-    """Portions around the chunk's length and the least length, short ones beside them, slots out of order, and a state that the one
+    """Portions around the chunks' lengths and the least ones, short ones beside them, slots out of order, and a state that the one
     form leaves and the other goes on from."""
-    portions = [[48, 64, 3, 131], [65, 1, 63, 47], [32, 96, 200, 64]]          # [step][request]
+    portions = [[96, 64, 3, 231], [165, 1, 163, 128], [160, 95, 200, 159]]      # [step][request]
     slots = [4, 0, 3, 2]
     total = [sum(step[r] for step in portions) for r in range(4)]
     data = [inputs(kind, dk, dv, total[r], 10 * r + dk, hard) for r in range(4)]
@@ -109,8 +109,10 @@ def test_chunks_carry_the_state_through_portions_as_the_walk_by_tokens_does(kind
         assert bool((state[1] == 7.0).all())
         errors[name] = max(float((torch.cat(got[r]).double() - want[r]).norm() / want[r].norm()) for r in range(4))
     print(f"\n  {kind} {dk} x {dv}{' hard' if hard else ''}: error against 64 bits {errors}")
-    # 32-bit sums of up to 128 terms over some hundred tokens: a few roundings of 6e-8 each
-    assert max(errors.values()) < 3e-6, errors
+    # 32-bit sums of up to 128 terms over some hundred tokens: a few roundings of 6e-8 each; the matrix memory's outputs are also divided by a sum
+    # that may nearly cancel, which hurts both forms alike
+    assert errors["tokens"] < (3e-5 if kind == "memory" else 1e-6), errors
+    assert max(errors.values()) < 1.5 * errors["tokens"] + 1e-7, errors
 
 
 @gpu
@@ -122,25 +124,25 @@ def test_requests_with_numbers_out_of_range_are_walked_by_tokens(kind, dk, dv, v
     earlier token), its neighbour's are finite."""
     xs, pres = [], []
     for r in range(2):
-        x, pre, b1, b2 = inputs(kind, dk, dv, 100, r)
+        x, pre, b1, b2 = inputs(kind, dk, dv, 200, r)
         xs.append(x)
         pres.append(pre)
     n = HEADS * dk
     if where == "decay":
         if kind == "memory":
-            xs[1][70, -8] = value
+            xs[1][170, -8] = value
         else:
-            pres[1][70, 5] = value
+            pres[1][170, 5] = value
     else:
-        xs[1][70, {"q": 5, "k": n + 5, "v": 2 * n + 5}[where]] = value
+        xs[1][170, {"q": 5, "k": n + 5, "v": 2 * n + 5}[where]] = value
     outs = [run(kind, dk, dv, xs, pres, b1, b2, new_state(kind, dk, dv, 2), [1, 0], pad) for pad in (0, 1)]
-    assert bool(outs[0][:100].isfinite().all()) and torch.allclose(outs[0][:100], outs[1][:100], rtol=1e-4, atol=1e-4)
-    assert bool(outs[0][100:170].isfinite().all())
+    assert bool(outs[0][:200].isfinite().all()) and torch.allclose(outs[0][:200], outs[1][:200], rtol=1e-4, atol=1e-4)
+    assert bool(outs[0][200:370].isfinite().all())
     h = slice(0, dv)                                                         # the head that holds the number
     if math.isnan(value) or where != "decay":
-        assert torch.equal(outs[0][100:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5), outs[1][100:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5))
+        assert torch.equal(outs[0][200:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5), outs[1][200:, h].nan_to_num(nan=1.25, posinf=2.5, neginf=-2.5))
     else:
-        assert torch.allclose(outs[0][100:, h], outs[1][100:, h], rtol=1e-4, atol=1e-4)     # a saturated gate is an ordinary one
+        assert torch.allclose(outs[0][200:, h], outs[1][200:, h], rtol=1e-4, atol=1e-4)     # a saturated gate is an ordinary one
 
 
 def test_which_sizes_take_chunks():
@@ -151,6 +153,8 @@ def test_which_sizes_take_chunks():
 
     f = build.load("recurrence").spy_scan_chunk_floats
     f.restype = ctypes.c_longlong
-    assert f(0, 48, 1, 8, 128, 256) > 0 and f(2, 2000, 8, 16, 128, 256) > 0 and f(1, 2047, 1, 32, 64, 64) > 0
-    assert f(0, 47, 1, 8, 128, 256) == 0 and f(0, 48, 1, 8, 96, 256) == 0 and f(0, 48, 1, 8, 128, 250) == 0 and f(1, 48, 1, 8, 128, 128) == 0
-    assert f(1, 65536, 64, 64, 64, 64) == 0                                  # more scratch than the limit
+    assert f(0, 96, 1, 8, 128, 256) > 0 and f(2, 2000, 8, 16, 128, 256) > 0 and f(1, 2047, 1, 32, 64, 64) > 0
+    assert f(0, 95, 1, 8, 128, 256) == 0 and f(0, 96, 1, 8, 96, 256) == 0 and f(0, 96, 1, 8, 128, 250) == 0 and f(1, 128, 1, 8, 128, 128) == 0
+    assert f(0, 480, 10, 8, 128, 256) > 0 and f(0, 479, 10, 8, 128, 256) == 0                     # short requests on average
+    assert f(1, 3000, 2, 32, 64, 64) > 0 and f(1, 3000, 3, 32, 64, 64) == 0                       # enough pairs for the walk by tokens
+    assert f(0, 1 << 19, 1, 8, 128, 256) == 0                                                     # more scratch than the limit
