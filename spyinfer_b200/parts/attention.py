@@ -155,7 +155,9 @@ class Attention(Mixer):
             self._split_plans[num_seqs] = plan
         return plan
 
-    def forward(self, x, batch, cache):
+    takes_stream = True
+
+    def forward(self, x, batch, cache, stream=None):
         if self.rope_table is None and self.position is not None:
             self.rope_table = self.position.rotation_table()   # built by the first step (an eager one)
         qkv = self.qkv(x, defer=True)
@@ -168,7 +170,7 @@ class Attention(Mixer):
                                   pairing=self.position.pairing if self.position is not None else "half")
         out = torch.empty((x.shape[0], self.nh * self.hd), dtype=x.dtype, device=x.device)
         self.attend(q, out, batch, cache)
-        return self.o(out, defer=self.defer_output)
+        return self.o.add_to(stream, out, defer=self.defer_output) if stream is not None else self.o(out, defer=self.defer_output)
 
     def attend(self, q, out, batch, cache, out_scale=None):
         """The attention itself, ``q [T, >= nh hd]`` over the cache into ``out [T, nh hd]``, on the kernel that the sizes, the
@@ -228,6 +230,8 @@ class PooledWindowAttention(Attention):
     ``max(window, pool)`` positions."""
 
     graph_safe = True
+
+    takes_stream = False
 
     def __init__(self, params, ctx):
         base = dict(params)
@@ -336,6 +340,8 @@ class LatentAttention(Attention):
 
     graph_safe = True
     any_head_dim = True
+
+    takes_stream = False
 
     def __init__(self, params, ctx):
         self.d, self.rd, self.vd = int(params["head_dim"]), int(params["rot_dim"]), int(params["v_head_dim"])
@@ -459,6 +465,8 @@ class DifferentialAttention(Attention):
     graph_safe = True
     any_head_dim = True
 
+    takes_stream = False
+
     def __init__(self, params, ctx):
         self.heads, self.groups = int(params["heads"]), int(params["kv_heads"])
         self.d, self.vd, self.diff, self.eps = int(params["dim"]), int(params["vdim"]), float(params["diff"]), float(params["eps"])
@@ -540,6 +548,8 @@ class KeptWindowAttention(Attention):
     ``position`` and what ``attention`` takes beside them."""
 
     any_head_dim = True
+
+    takes_stream = False
 
     def __init__(self, params, ctx):
         self.heads, self.groups = int(params["heads"]), int(params["kv_heads"])
