@@ -63,7 +63,14 @@ class StepBatch:
     #: not laid out that way): an attention part may run those through its kernel for decoding and the rest through the
     #: one for prompt portions
     one_token_head: int = 0
+    #: no request of the batch holds more than ``SHORT_CONTEXT`` keys after this step (a captured step is replayed only for batches that agree in this)
+    short_context: bool = False
     extras: Dict[str, object] = field(default_factory=dict)
+
+
+#: Keys up to which a step counts as one of short contexts: up to here the attention kernel whose blocks take a few rows each, and read keys as they come,
+#: ends ahead of the one that first brings tiles of 128 keys together (see ``Attention.attend``).
+SHORT_CONTEXT = 64
 
 
 class BatchStager:
@@ -115,4 +122,5 @@ class BatchStager:
             state_slot=v[6], block_tables=[v[7 + i].view(S, widths[i]) for i in range(len(tables))], status=self.status,
             host_positions=positions, host_q_start=q_start, host_ctx_len=ctx_len, host_state_slot=state_slot,
             max_q_len=int(np.max(q_start[1:] - q_start[:-1])) if S else 0, max_ctx_len=int(ctx_len.max()) if S else 0,
+            short_context=bool(S > 0 and int(ctx_len.max()) <= SHORT_CONTEXT),
             one_token_each=bool(S > 0 and T == S and int(np.min(q_start[1:] - q_start[:-1])) == 1))
