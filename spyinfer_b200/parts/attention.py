@@ -172,6 +172,9 @@ class Attention(Mixer):
         self.attend(q, out, batch, cache)
         return self.o.add_to(stream, out, defer=self.defer_output) if stream is not None else self.o(out, defer=self.defer_output)
 
+    #: query rows (tokens x heads) up to which prompts of short contexts go to the kernel of small tiles
+    SHORT_ROWS = 10240
+
     def attend(self, q, out, batch, cache, out_scale=None):
         """The attention itself, ``q [T, >= nh hd]`` over the cache into ``out [T, nh hd]``, on the kernel that the sizes, the
         page size and the kind of batch call for."""
@@ -191,6 +194,12 @@ class Attention(Mixer):
             kernels.attention_mma(q, self.nh, self.hd, out, cache.pages, cache.block_table, batch.positions, batch.q_start,
                                   batch.num_seqs, self.scale, window=self.key_mask, split_keys=split_keys, max_splits=max_splits,
                                   status=batch.status)
+        elif boxes and mma and batch.short_context and batch.one_token_head == 0 and batch.num_tokens * self.nh <= self.SHORT_ROWS:
+            # a question's prompt: a block of 256 rows spends its time on the way to its first tile of 128 keys (one prompt of 16, 37, 64 and
+            # 100 tokens, 32 heads over 8, us: 7.8, 10.0, 11.4 and 11.3 there, 4.6, 6.0, 7.9 and 10.9 here; five of 64, 320 tokens: 12.0 and 8.3, of
+            # 40 heads 12.8 and 12.9)
+            kernels.attention_mma(q, self.nh, self.hd, out, cache.pages, cache.block_table, batch.positions, batch.q_start,
+                                  batch.num_seqs, self.scale, window=self.key_mask, status=batch.status)
         elif boxes:
             # prompt portions on blocks of 256 query rows; requests that decode beside them (laid out first in the batch)
             # go through the decode kernel, which reads a cache two to three times faster for one token than a 256-row block does

@@ -339,6 +339,51 @@ def test_small_steps_with_decode_kernel_requests_replayed_from_graphs(tiny_model
         np.testing.assert_allclose(outs[0][k][1], ref_new[-1], rtol=3e-2, atol=5e-2 * scale)
 
 
+@pytest.mark.parametrize("heads", [4, 16])
+def test_prompts_of_short_contexts_and_of_longer_ones_in_the_same_padded_sizes(heads):
+    """Portions around the context up to which another attention kernel is taken, in steps that are padded to the same sizes: first short
+    contexts (launched, captured, replayed), then the same sizes behind cached keys and back; several requests at once.  Each as the plain
+    implementation has it, and the steps from graphs as the eager ones."""
+    from spyinfer_b200 import config_from_json
+    from spyinfer_b200.config import EngineConfig
+    from spyinfer_b200.engine import StepEntry
+    from spyinfer_b200.engine.model import Model
+    from spyinfer_b200.engine.runner import ModelRunner
+
+    cfg = {"architectures": ["Qwen3ForCausalLM"], "model_type": "qwen3", "hidden_act": "silu", "num_hidden_layers": 2, "hidden_size": 128,
+           "num_attention_heads": heads, "num_key_value_heads": 2, "head_dim": 64, "intermediate_size": 256, "vocab_size": 500, "rope_theta": 10000.0,
+           "rms_norm_eps": 1e-6, "tie_word_embeddings": False, "max_position_embeddings": 512, "eos_token_id": -1}
+    weights = plain_model.random_weights(cfg, seed=5, std=0.08, norm_std=0.1)
+    rng = np.random.default_rng(heads)
+    tokens = {r: rng.integers(0, 500, 200).tolist() for r in "abcdefgh"}
+    ref = {r: plain_model.forward_logits(weights, cfg, t).numpy() for r, t in tokens.items()}
+    # (request, tokens) of every step; steps of 40 tokens are padded to 64, whatever is cached
+    steps = [[("a", 40)], [("b", 64)], [("c", 40)], [("a", 40)], [("c", 24)], [("c", 1), ("d", 39)], [("b", 1), ("e", 39)], [("d", 40)], [("f", 20), ("g", 20)], [("h", 65)], [("f", 44), ("g", 44)],
+             [("e", 26)]]
+    outs = []
+    for graphs in (True, False):
+        config = EngineConfig(dtype="bfloat16", kvcache_block_size=16, num_kvcache_blocks=128, max_num_seqs=8, max_model_len=256, max_num_batched_tokens=256,
+                              use_cuda_graphs=graphs)
+        model = Model(config_from_json(cfg).to_spec(), torch.bfloat16, config.device, config.max_model_len)
+        model.bind({k: v.cuda() for k, v in weights.items()})
+        runner, at, got = ModelRunner(model, config), dict.fromkeys(tokens, 0), []
+        for step in steps:
+            entries = [StepEntry(r, tokens[r][at[r]:at[r] + n], [n - 1]) for r, n in step]
+            got.append(runner.step(entries).float().cpu().numpy().copy())
+            for r, n in step:
+                at[r] += n
+            for (r, n), row in zip(step, got[-1]):
+                want = ref[r][at[r] - 1]
+                np.testing.assert_allclose(row, want, rtol=3e-2, atol=5e-2 * np.abs(want).max(), err_msg=f"{step} {r} graphs {graphs}")
+        runner.check_status()
+        if graphs:
+            kinds = {k[0] for k, held in runner._graphs.items() if isinstance(k, tuple) and held != "warm"}
+            assert kinds == {"short step", "step"}, kinds
+        outs.append(got)
+    for a, b in zip(*outs):
+        np.testing.assert_allclose(a, b, rtol=3e-2, atol=3e-2)
+
+
 def test_one_long_request_decoding_beside_a_portion(tiny_models):
     """A single decoded token whose request holds more than a thousand keys, beside a prompt portion of another request: the
     decode kernel takes it (one 256-row block would walk its cache alone); logits as the plain implementation has them."""
