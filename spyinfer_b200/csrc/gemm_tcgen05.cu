@@ -907,31 +907,24 @@ __device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int l
             }
         }
     } else {
-        const int outs = min(32, x_rows - x0);
-        TC* dst = base + (size_t)y * ld + x0;
-        const bool pieces = outs == 32 && (ld & (16 / (int)sizeof(TC) - 1)) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
-        float4 had[8];                         // what is added to (EPI == 5): requested together, ahead of the turn
-        if constexpr (EPI == 5) {
-            if (pieces) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int t = i * 4 + (lane >> 3);
-                    if (t < count) had[i] = *reinterpret_cast<const float4*>(dst + (size_t)t * ld + (lane & 7) * 4);
-                }
-            }
-        }
 #pragma unroll
         for (int j = 0; j < 32; ++j) staged[j * PAIR_STAGED_LD + lane] = EPI == 2 ? relu_squared(__uint_as_float(r[j])) : __uint_as_float(r[j]);
         __syncwarp();
-        if (pieces) {
+        const int outs = min(32, x_rows - x0);
+        TC* dst = base + (size_t)y * ld + x0;
+        if (outs == 32 && (ld & (16 / (int)sizeof(TC) - 1)) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
             if constexpr (sizeof(TC) == 4) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int t = i * 4 + (lane >> 3), part = lane & 7;
                     if (t >= count) continue;
                     float4 v = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
-                    if constexpr (EPI == 5) v = make_float4(had[i].x + v.x, had[i].y + v.y, had[i].z + v.z, had[i].w + v.w);
-                    *reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4) = v;
+                    float4* to = reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4);
+                    if constexpr (EPI == 5) {
+                        const float4 had = *to;
+                        v = make_float4(had.x + v.x, had.y + v.y, had.z + v.z, had.w + v.w);
+                    }
+                    *to = v;
                 }
             } else {
 #pragma unroll
