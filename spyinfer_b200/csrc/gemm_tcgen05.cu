@@ -917,14 +917,7 @@ __device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int l
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int t = i * 4 + (lane >> 3), part = lane & 7;
-                    if (t >= count) continue;
-                    float4 v = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
-                    float4* to = reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4);
-                    if constexpr (EPI == 5) {
-                        const float4 had = *to;
-                        v = make_float4(had.x + v.x, had.y + v.y, had.z + v.z, had.w + v.w);
-                    }
-                    *to = v;
+                    if (t < count) *reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4) = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
                 }
             } else {
 #pragma unroll
@@ -938,7 +931,7 @@ __device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int l
                 }
             }
         } else if (lane < outs) {
-            for (int t = 0; t < count; ++t) store_elem(dst + (size_t)t * ld + lane, (EPI == 5 ? to_f32(dst[(size_t)t * ld + lane]) : 0.f) + staged[t * PAIR_STAGED_LD + lane]);
+            for (int t = 0; t < count; ++t) store_elem(dst + (size_t)t * ld + lane, staged[t * PAIR_STAGED_LD + lane]);
         }
     }
     __syncwarp();   // the next chunk's numbers may come
@@ -1403,13 +1396,6 @@ Plan make_plan(int M, int N, int K, bool may_split)
 
 }  // namespace
 
-// Whether a product of this shape can add its result to the output (epilogue 5): one that runs on pairs of blocks with whole sums over K.
-static bool adds_in_place(int M, int N, int K)
-{
-    return make_plan(M, N, K, true).splits == 1 && make_plan(M, N, K, false).kind == PAIRS;
-}
-extern "C" int spy_gemm_tcgen05_adds(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && adds_in_place(M, N, K) ? 1 : 0; }
-
 // How many splits of K a product of this shape uses, and the floats of scratch it needs.
 // A plan that would need more than scratch_limit floats falls back to one pass over K.
 extern "C" int spy_gemm_tcgen05_plan(int M, int N, int K, long long scratch_limit, int* splits_out, long long* scratch_floats_out)
@@ -1430,7 +1416,6 @@ extern "C" int spy_gemm_tcgen05_plan(int M, int N, int K, long long scratch_limi
 // epilogue 1 (SwiGLU): W's rows alternate gate and up rows, C is [M, N / 2], K is not split.
 // epilogue 2: C = relu(A W^T)^2 element by element, K is not split.
 // epilogue 3: as 1 with gelu_tanh(gate) * up.
-// epilogue 5: C += A W^T, C float32, for the shapes that spy_gemm_tcgen05_adds names.
 // defer_reduce: when the plan splits K, the partial products stay in scratch as
 // [splits][M][N] floats for the consumer to sum (C is not written); *splits_used tells.
 // next_weights / next_bytes (may be null / 0; used by products of up to 256 tokens only): memory that a
@@ -1451,10 +1436,9 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
     if (lda % 8 != 0 || ldw % 8 != 0) SPY_FAIL("gemm_tcgen05: row strides %lld/%lld must be multiples of 8 elements", lda, ldw);
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) SPY_FAIL("gemm_tcgen05: operands must be 16-byte aligned");
     if (c_dtype != SPY_F32 && c_dtype != SPY_BF16) SPY_FAIL("gemm_tcgen05: unknown output dtype code %d", c_dtype);
-    if (epilogue < 0 || epilogue > 5) SPY_FAIL("gemm_tcgen05: unknown epilogue %d", epilogue);
+    if (epilogue < 0 || epilogue > 4) SPY_FAIL("gemm_tcgen05: unknown epilogue %d", epilogue);
     if (epilogue == 4 && !(glu.limit > 0.f)) SPY_FAIL("gemm_tcgen05: the clamped epilogue needs a positive limit");
     if (epilogue == 2 && c_dtype != SPY_BF16) SPY_FAIL("gemm_tcgen05: the relu-squared epilogue needs bfloat16 output");
-    if (epilogue == 5 && (c_dtype != SPY_F32 || !adds_in_place(M, N, K))) SPY_FAIL("gemm_tcgen05: the adding epilogue needs a float32 output and many tokens (M %d, N %d, K %d)", M, N, K);
     if ((epilogue == 1 || epilogue == 3 || epilogue == 4) && (N % 2 != 0 || c_dtype != SPY_BF16)) SPY_FAIL("gemm_tcgen05: a gated epilogue needs an even N and bfloat16 output");
     Plan plan = make_plan(M, N, K, epilogue == 0);
     if (plan.splits > 1 && (scratch == nullptr || (long long)plan.splits * M * N > scratch_floats)) plan = make_plan(M, N, K, false);
@@ -1491,7 +1475,6 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
             SPY_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<bf16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
             SPY_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<bf16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
             SPY_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<bf16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
-            SPY_CUDA(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<float, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM));
             const int sms = spy_sm_count();
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(sms / 2 * 2);
@@ -1549,9 +1532,6 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
                                N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (epilogue == 4)
             spy_launch_cluster(gemm_tcgen05_pair_kernel<bf16, 4>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (bf16*)C, ldc,
-                               N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
-        else if (epilogue == 5)
-            spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 5>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (float*)C, ldc,
                                N, M, k_blocks, tokens, (int)num_tiles, 1, k_blocks, 0LL, tail_tiles, tail_p, tail_x, scratch, status, glu);
         else if (c_dtype == SPY_F32)
             spy_launch_cluster(gemm_tcgen05_pair_kernel<float, 0>, dim3(2 * clusters), dim3(NUM_THREADS), PAIR_SMEM, stream, 2u, mx, my, (float*)C, ldc,

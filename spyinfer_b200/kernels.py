@@ -1182,12 +1182,6 @@ def _scratch(device) -> torch.Tensor:
     return _gemm_scratch[key]
 
 
-def gemm_tcgen05_adds(rows: int, w: torch.Tensor) -> bool:
-    """Whether a product of ``rows`` tokens with this weight can add its result to a float32 output in its epilogue: one of many tokens, on pairs
-    of blocks with whole sums over K."""
-    return rows > 128 and build.load("gemm_tcgen05").spy_gemm_tcgen05_adds(int(rows), int(w.shape[0]), int(w.shape[1])) != 0
-
-
 def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, epilogue: Optional[str] = None, defer: bool = False,
                  prefetch: Optional[torch.Tensor] = None, prefetch_bytes: int = 0, glu: Optional[tuple] = None) -> torch.Tensor:
@@ -1195,8 +1189,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
     bfloat16 or float32 output.  K must be a multiple of 8.
 
     ``epilogue="swiglu"``: ``w``'s rows alternate gate and up rows and the result is
-    ``silu(gate) * up``, ``[M, N / 2]``; ``epilogue="geglu_tanh"``: the same with the tanh form of gelu on the gate.  ``epilogue="relu2"``: the result is ``relu(a @ w^T)^2`` (bfloat16 output).  ``epilogue="add"``
-    (sizes that ``gemm_tcgen05_adds`` names): the result is added to the float32 ``out``.  ``defer=True``: when the kernel splits K, the float32
+    ``silu(gate) * up``, ``[M, N / 2]``; ``epilogue="geglu_tanh"``: the same with the tanh form of gelu on the gate.  ``epilogue="relu2"``: the result is ``relu(a @ w^T)^2`` (bfloat16 output).  ``defer=True``: when the kernel splits K, the float32
     partial products are returned unsummed as ``[splits, M, N]`` for a consumer that adds them
     (``rmsnorm``'s delta, ``qk_rope_store``'s input); otherwise the result is ``[M, N]``.
     ``prefetch``: a tensor that a later kernel will read (the next product's weights); with up to 256
@@ -1210,7 +1203,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
         raise KernelError(f"gemm: the weight's rows must start on 16-byte borders (row distance {ldw}, address {w.data_ptr():#x})")
     if w.shape[1] != K:
         raise KernelError(f"gemm: shapes do not fit: input {tuple(a.shape)}, weight {tuple(w.shape)}")
-    if epilogue not in (None, "swiglu", "relu2", "geglu_tanh", "clamped_swish", "add"):
+    if epilogue not in (None, "swiglu", "relu2", "geglu_tanh", "clamped_swish"):
         raise KernelError(f"gemm: unknown epilogue {epilogue!r}")
     if epilogue == "clamped_swish":
         # glu = (bias or None, limit, slope): the bias [N] float32 lies in the order of the weight's rows (gate and up in turns)
@@ -1220,8 +1213,6 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
             _check(glu[0], "gate|up bias", torch.float32, 1)
             if glu[0].shape[0] != N:
                 raise KernelError("gemm: the clamped epilogue's bias has one entry per weight row")
-    if epilogue == "add" and (out is None or out.dtype != torch.float32):
-        raise KernelError("gemm: the adding epilogue needs a float32 output to add to")
     if epilogue == "relu2" and (out_dtype or torch.bfloat16) != torch.bfloat16:
         raise KernelError("gemm: the relu2 epilogue writes bfloat16")
     n_out = N // 2 if epilogue in ("swiglu", "geglu_tanh", "clamped_swish") else N
@@ -1258,7 +1249,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
         return out
     _call("gemm_tcgen05", "spy_gemm_tcgen05_ex", _ptr(a), ctypes.c_longlong(K), _ptr(w), ctypes.c_longlong(ldw), _ptr(out),
           _code(out, "gemm output"), ctypes.c_longlong(n_out), M, N, K, _ptr(scratch), ctypes.c_longlong(scratch.numel()),
-          {None: 0, "swiglu": 1, "relu2": 2, "geglu_tanh": 3, "add": 5}[epilogue], 0, None, _ptr(status), _stream(), pf_ptr, ctypes.c_longlong(pf_bytes))
+          {None: 0, "swiglu": 1, "relu2": 2, "geglu_tanh": 3}[epilogue], 0, None, _ptr(status), _stream(), pf_ptr, ctypes.c_longlong(pf_bytes))
     return out
 
 

@@ -155,9 +155,7 @@ class Attention(Mixer):
             self._split_plans[num_seqs] = plan
         return plan
 
-    takes_stream = True
-
-    def forward(self, x, batch, cache, stream=None):
+    def forward(self, x, batch, cache):
         if self.rope_table is None and self.position is not None:
             self.rope_table = self.position.rotation_table()   # built by the first step (an eager one)
         qkv = self.qkv(x, defer=True)
@@ -170,7 +168,7 @@ class Attention(Mixer):
                                   pairing=self.position.pairing if self.position is not None else "half")
         out = torch.empty((x.shape[0], self.nh * self.hd), dtype=x.dtype, device=x.device)
         self.attend(q, out, batch, cache)
-        return self.o.add_to(stream, out, defer=self.defer_output) if stream is not None else self.o(out, defer=self.defer_output)
+        return self.o(out, defer=self.defer_output)
 
     #: query rows (tokens x heads) up to which prompts of short contexts go to the kernel of small tiles
     SHORT_ROWS = 10240
@@ -239,8 +237,6 @@ class PooledWindowAttention(Attention):
     ``max(window, pool)`` positions."""
 
     graph_safe = True
-
-    takes_stream = False
 
     def __init__(self, params, ctx):
         base = dict(params)
@@ -349,8 +345,6 @@ class LatentAttention(Attention):
 
     graph_safe = True
     any_head_dim = True
-
-    takes_stream = False
 
     def __init__(self, params, ctx):
         self.d, self.rd, self.vd = int(params["head_dim"]), int(params["rot_dim"]), int(params["v_head_dim"])
@@ -474,8 +468,6 @@ class DifferentialAttention(Attention):
     graph_safe = True
     any_head_dim = True
 
-    takes_stream = False
-
     def __init__(self, params, ctx):
         self.heads, self.groups = int(params["heads"]), int(params["kv_heads"])
         self.d, self.vd, self.diff, self.eps = int(params["dim"]), int(params["vdim"]), float(params["diff"]), float(params["eps"])
@@ -557,8 +549,6 @@ class KeptWindowAttention(Attention):
     ``position`` and what ``attention`` takes beside them."""
 
     any_head_dim = True
-
-    takes_stream = False
 
     def __init__(self, params, ctx):
         self.heads, self.groups = int(params["heads"]), int(params["kv_heads"])

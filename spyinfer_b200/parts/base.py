@@ -160,9 +160,6 @@ class Mixer(Part):
     #: None: the result has the activations' dtype; a mixer that is one of several side by side is asked for float32
     #: here, so that the norm which adds the weighted results reads them all in one format (parts that cannot do not)
     output_dtype: Optional[torch.dtype] = None
-    #: True: ``forward`` takes ``stream``, the float32 residual stream, to which its last product may add the result itself; it then
-    #: returns None
-    takes_stream: bool = False
 
     def cache_need(self):
         """A ``PagedCacheNeed``, a ``StateCacheNeed``, a ``CompositeCacheNeed`` of them, or None."""
@@ -174,7 +171,6 @@ class Mixer(Part):
 
 class FeedForward(Part):
     defer_output: bool = True     # as ``Mixer.defer_output``
-    takes_stream: bool = False    # as ``Mixer.takes_stream``
     #: set by a block arrangement whose next norm adds a projection's bias itself: a feed-forward whose last projection has a
     #: bias then leaves it out and offers it as ``output_bias`` (float32 ``[size]``, None when there is none)
     leave_output_bias: bool = False

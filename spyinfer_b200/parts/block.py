@@ -39,10 +39,8 @@ class PreNormBlock(Block):
 
     def forward(self, hidden, delta, batch, cache):
         x = self.mixer_norm.forward_add(hidden, delta)
-        a = self.mixer.forward(x, batch, cache, stream=hidden) if self.mixer.takes_stream else self.mixer.forward(x, batch, cache)
+        a = self.mixer.forward(x, batch, cache)
         x = self.ffn_norm.forward_add(hidden, a)
-        if self.feed_forward.takes_stream:
-            return hidden, self.feed_forward.forward(x, stream=hidden)
         return hidden, self.run_feed_forward(x, batch)
 
 

@@ -128,11 +128,7 @@ class GatedMLP(FeedForward):
     def modules(self):
         return ([] if self.fused else ["swiglu"]) + self.gate_up.modules() + self.down.modules()
 
-    takes_stream = True
-
-    def forward(self, x, stream=None):
-        if self.fused and stream is not None and self.activation != "clamped_swish":
-            return self.down.add_to(stream, self.gate_up(x, epilogue="swiglu" if self.activation == "silu" else "geglu_tanh"), defer=self.defer_output)
+    def forward(self, x):
         if self.fused and self.activation == "clamped_swish":
             return self.down(self.gate_up(x, epilogue="clamped_swish", glu=(self.gate_up_bias, self.limit, self.slope)), defer=self.defer_output)
         if self.fused:

@@ -66,15 +66,6 @@ class Linear:
         y = self._product(x, out_dtype, epilogue, defer, glu)
         return kernels.add_bias(y, self.bias) if self.bias is not None else y
 
-    def add_to(self, stream: torch.Tensor, x: torch.Tensor, defer: bool = False) -> Optional[torch.Tensor]:
-        """Adds the product to the float32 ``stream`` and returns None where the tensor-core kernel can do that in its epilogue (products of many
-        tokens, whose result then makes no way to memory and back in 16 bits); elsewhere the result as ``__call__`` gives it, for the
-        stream's next norm to add."""
-        if self.fast and self.bias is None and kernels.gemm_tcgen05_adds(x.shape[0], self.weight):
-            kernels.gemm_tcgen05(x, self.weight, out=stream, epilogue="add")
-            return None
-        return self(x, defer=defer)
-
     def _product(self, x, out_dtype, epilogue, defer, glu=None):
         if self.fast:
             hint = self.next_weight if self.hint_next and x.shape[0] <= 256 and self.prefetch_bytes > 0 else None

@@ -885,28 +885,6 @@ def test_gemm_tcgen05_cuts_many_tokens_into_tiles_of_several_heights(M, epilogue
         torch.testing.assert_close(out[:M].float(), ref.to(torch.bfloat16).float(), rtol=1.6e-2, atol=4e-3)
 
 
-@pytest.mark.parametrize("M,N,K", [(513, 4096, 264), (700, 9612, 136), (1100, 5000, 1032), (2048, 4096, 4096), (448, 24576, 72), (160, 9610, 72)])
-def test_gemm_tcgen05_adds_to_a_float32_output(M, N, K, monkeypatch):
-    """The adding epilogue at sizes with and without shared-out tail tiles, an N that ends inside a warp's outputs and rows that are no multiple of
-    16 bytes: the output is what it was plus the plain product, the row behind it stays; sizes that cannot add are refused."""
-    from spyinfer_b200 import kernels
-    monkeypatch.setenv("SPYINFER_GEMM_TAIL_MIN", "0")
-    torch.manual_seed(M)
-    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
-    w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
-    assert kernels.gemm_tcgen05_adds(M, w)
-    before = torch.randn(M + 1, N, device=DEV)
-    out = before.clone()
-    kernels.gemm_tcgen05(a, w, out[:M], epilogue="add")
-    product = kernels.gemm_tcgen05(a, w, out_dtype=torch.float32)
-    torch.cuda.synchronize()
-    assert torch.equal(out[M], before[M]) and torch.equal(out[:M], before[:M] + product)
-    few = a[:64].contiguous()
-    assert not kernels.gemm_tcgen05_adds(64, w)
-    with pytest.raises(kernels.KernelError, match="adding epilogue"):
-        kernels.gemm_tcgen05(few, w, out[:64].clone(), epilogue="add")
-
-
 @pytest.mark.parametrize("M,I,K", [(3, 100, 64), (16, 328, 200), (40, 1000, 136), (64, 6144, 512), (70, 520, 264), (128, 12288, 1024), (130, 520, 264), (300, 12288, 1024),
                                    (520, 1000, 136), (1100, 2304, 512)])   # 512 rows and more: pairs of blocks on 256 x 256 tiles
 def test_gemm_tcgen05_swiglu_epilogue(M, I, K):
