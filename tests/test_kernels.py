@@ -202,6 +202,25 @@ def test_swiglu(dtype, T, I):
     torch.testing.assert_close(out.float(), ((g / (1 + torch.exp(-g))) * u).to(dtype).float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,I,shift", [(1, 4, 0), (3, 1001, 0), (5, 1002, 0), (9, 1004, 0), (9, 1004, 1), (700, 12288, 0)])
+def test_swiglu_of_whole_quads_and_of_other_rows_is_the_same_arithmetic(dtype, T, I, shift):
+    """Rows of a multiple of four elements on 16-byte borders take quads, others and shifted views single elements: a
+    row's numbers do not depend on which, and an infinity or a NaN stays where it is."""
+    from spyinfer_b200 import kernels
+    gu = (torch.randn(T, 2 * I, device=DEV) * 4).to(dtype)
+    gu[0, 0], gu[0, 1], gu[-1, I - 1] = float("inf"), float("nan"), float("-inf")
+    store = torch.empty(2 * T * I + 8, device=DEV, dtype=dtype)
+    x = store[shift:shift + 2 * T * I].view(T, 2 * I)
+    x.copy_(gu)
+    out = kernels.swiglu(x, torch.empty(T, I, device=DEV, dtype=dtype))
+    single = store[1:1 + 2 * T * I].view(T, 2 * I)         # never on a 16-byte border
+    single.copy_(gu)
+    assert torch.equal(out.nan_to_num(nan=12345.0), kernels.swiglu(single, torch.empty_like(out)).nan_to_num(nan=12345.0))
+    g, u = gu.float()[:, :I], gu.float()[:, I:]
+    torch.testing.assert_close(out.float(), ((g / (1 + torch.exp(-g))) * u).to(dtype).float(), equal_nan=True, **tol(dtype))
+
+
 def paged_setup(S, lens, nkv, hd, page_size, dtype, shuffle=True):
     """Random keys and values of S sequences scattered over shuffled pages."""
     width = max((l + page_size - 1) // page_size for l in lens)
