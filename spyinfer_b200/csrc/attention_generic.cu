@@ -586,6 +586,346 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
     }
 }
 
+// ---- prompts with head sizes above 64: 32 rows a block, four rows by four keys (or dimensions) a thread -------------------------
+// The kernel above reads shared memory more than it multiplies: a key's quad and 16 queries' for 64 multiply-adds.  Here a thread reads four
+// keys' quads and four queries' for as many, and in the value sums a quad of probabilities and one of values for 16, so that the multiply-adds
+// are what is left, and a block's keys and values serve twice the rows.  Every sum runs in the same order as above: the bits are the same.
+// WIDE_MEASURED
+constexpr int WIDE_ROWS = 32, WIDE_THREADS = 256, WIDE_PLD = WIDE_ROWS + 4;
+
+// v[0..4) over the eight lanes whose numbers differ in their lowest three bits; the result is row `*row`'s in lanes whose `*row` is not negative.
+template <typename OP>
+__device__ __forceinline__ float reduce_four(float (&v)[4], int* row)
+{
+    const int lane = threadIdx.x & 31;
+    const bool up2 = (lane & 4) != 0, up1 = (lane & 2) != 0;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const float keep = up2 ? v[r + 2] : v[r], give = up2 ? v[r] : v[r + 2];
+        v[r] = OP::of(keep, __shfl_xor_sync(0xffffffffu, give, 4));
+    }
+    const float keep = up1 ? v[1] : v[0], give = up1 ? v[0] : v[1];
+    float x = OP::of(keep, __shfl_xor_sync(0xffffffffu, give, 2));
+    x = OP::of(x, __shfl_xor_sync(0xffffffffu, x, 1));
+    *row = (lane & 1) == 0 ? (up2 ? 2 : 0) + (up1 ? 1 : 0) : -1;
+    return x;
+}
+
+template <typename TA, typename TC>
+__global__ void __launch_bounds__(WIDE_THREADS, 2)
+attention_wide_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* __restrict__ pages, AttnArgs A)
+{
+    constexpr int R = WIDE_ROWS, PLD = WIDE_PLD;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ __align__(16) float p_s[CHUNK][PLD];
+    __shared__ __align__(16) float red[2][R][4];           // by row and quarter of the chunk: maxima, sums
+    __shared__ long long row_s[CHUNK];
+    __shared__ int pos_s[R], lo_s[R], kept_s[R];
+    __shared__ float slope_s[R];
+    __shared__ long long at_s[R];                          // token * nh + head
+    __shared__ float2 take_s[R], end_s[R];
+    pdl_wait();
+    pdl_launch_dependents();                               // behind the wait, as above
+    const int hd = A.hd, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kld = A.kld, qld = hd + 4;
+    // Scores: a warp takes 16 rows and a quarter of the chunk; a lane's rows are four apart, its keys eight (lanes side by side then read rows of
+    // shared memory that meet no bank twice).  Value sums: four rows side by side and four dimensions.
+    const int half = warp >> 2, quarter = warp & 3, row_lane = lane >> 3, key_lane = lane & 7;
+    const int quad = 4 * ((warp & 3) * 8 + (lane & 7)), v_row = 4 * ((warp >> 2) * 4 + (lane >> 3));
+    const bool has_quad = quad < hd;
+    float* q_s = sm;                    // [R][qld]
+    TC* const area0 = reinterpret_cast<TC*>(sm + R * qld);          // the keys' halves, then the values of the chunk's halves in their place
+    TC* const area1 = area0 + A.area;
+    const int kvh = blockIdx.y / A.head_groups, G = A.nh / A.nkv;
+    const int h0 = kvh * G + (blockIdx.y % A.head_groups) * A.heads, nheads = min(A.heads, (kvh + 1) * G - h0);
+    const int t_first = blockIdx.x * A.per_tile;
+    const long long v_offset = A.planes == 2 ? (long long)A.nkv * A.page_size * hd : 0;
+    const auto copy_rows = [&](TC* dst, int ld, int j0, int j1, long long offset, int d0, int dims) {
+        const int lanes = dims > KD ? 32 : 16, d = 4 * (tid & (lanes - 1));
+        if (d < dims) {
+#pragma unroll 4
+            for (int j = j0 + tid / lanes; j < j1; j += WIDE_THREADS / lanes) {
+                const long long at = row_s[j];
+                if (at >= 0) copy_quad((uint32_t)__cvta_generic_to_shared(dst + (j - j0) * ld + d), pages + at + offset + d0 + d);
+            }
+        }
+        copy_commit();
+    };
+    const TileTokens T = load_tile(A, t_first);
+
+    for (int i = 0; i < T.n;) {                                                  // runs of tokens of one sequence
+        const Run run = run_from(A, T, i);
+        i += run.len;
+        if (warp == 0 && blockIdx.z == 0 && lane >= run.first && lane < i && T.pos / CHUNK >= A.max_chunks)
+            report_status(A.status, SPY_STATUS_BAD_PAGE, t_first + lane);        // as above: a position beyond the table
+        const bool parts = in_parts(A, run);
+        if (blockIdx.z > 0 && (!parts || (int)blockIdx.z > run.last_chunk)) continue;
+        const int kept_chunks = (run.kept_max + CHUNK - 1) / CHUNK, lo_chunk = run.lo_min / CHUNK, step = parts ? gridDim.z : 1;
+        const auto seen_from = [&](int c) { return c >= kept_chunks && c < lo_chunk ? c + (lo_chunk - c + step - 1) / step * step : c; };
+        const int* bt = A.block_table + (size_t)run.seq * A.table_width;
+        const auto page_index = [&](int key) { return A.page_shift >= 0 ? key >> A.page_shift : key / A.page_size; };
+        const auto page_of = [&](int c) {
+            const int lp = tid < CHUNK && c <= run.last_chunk ? page_index(c * CHUNK + tid) : A.table_width;
+            return lp < A.table_width ? bt[lp] : -1;
+        };
+        int c = seen_from(parts ? blockIdx.z : 0);
+        if (parts && c > run.last_chunk) continue;
+
+        const int rows = run.len * nheads;
+        int page = page_of(c);
+        {
+            constexpr int WARPS = WIDE_THREADS / 32;
+            float x[R / WARPS][4];                                               // a warp a row, everything requested at once
+#pragma unroll
+            for (int k = 0; k < R / WARPS; ++k) {
+                const int r = warp + WARPS * k, t = r / nheads;
+                const TA* src = q + (size_t)(t_first + run.first + t) * A.q_row_stride + (size_t)(h0 + r - t * nheads) * hd;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[k][e] = r < rows && lane + 32 * e < hd ? to_f32(src[lane + 32 * e]) : 0.f;
+            }
+            __syncthreads();                                                     // the run before is done with the shared arrays
+#pragma unroll
+            for (int k = 0; k < R / WARPS; ++k)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (lane + 32 * e < hd) q_s[(warp + WARPS * k) * qld + lane + 32 * e] = x[k][e];
+        }
+        int my_head = 0;                                                         // of warp 0's lanes, a row each
+        float m = -INFINITY, l = 0.f;                                            // the row's maximum and sum
+        if (warp == 0) {
+            const int t = run.first + lane / nheads;
+            my_head = h0 + lane % nheads;
+            const int pos = __shfl_sync(0xffffffffu, T.pos, t & 31), lo = __shfl_sync(0xffffffffu, T.lo, t & 31), kept = __shfl_sync(0xffffffffu, T.kept, t & 31);
+            pos_s[lane] = lane < rows ? pos : -1;
+            lo_s[lane] = lane < rows ? lo : 0;
+            kept_s[lane] = lane < rows ? kept : 0;
+            slope_s[lane] = A.sc.slopes != nullptr && lane < rows ? A.sc.slopes[my_head] : 0.f;
+            at_s[lane] = (long long)(t_first + t) * A.nh + my_head;
+        }
+        __syncthreads();
+        float acc[4][4];                                                         // of rows v_row + r, dimensions quad + e
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+        while (c <= run.last_chunk) {
+            const int c0 = c * CHUNK, c_next = seen_from(c + step);
+            const int first = c < kept_chunks ? 0 : max(run.lo_min - c0, 0), last = min(run.pos_max - c0, CHUNK - 1);   // of the keys that any row sees
+            bool any = false;
+            long long key_row = -1;
+            if (tid < CHUNK) {
+                const int j = c0 + tid;
+                any = j >= run.lo_max && j <= run.pos_min;                       // every row sees it
+                int first_seer = 0;                                              // the first row whose token sees the key
+                if (!any)
+                    for (int r = rows - nheads; r >= 0; r -= nheads)
+                        if ((j >= lo_s[r] || j < kept_s[r]) && j <= pos_s[r]) {
+                            any = true;
+                            first_seer = r;
+                        }
+                if (any) {
+                    if (page < 0 || page >= A.num_pages) report_status(A.status, SPY_STATUS_BAD_PAGE, t_first + run.first + first_seer / nheads);
+                    else key_row = ((((long long)page * A.planes) * A.nkv + kvh) * A.page_size + (j - page_index(j) * A.page_size)) * hd;
+                }
+                row_s[tid] = key_row;
+            }
+            page = page_of(c_next);
+            const bool bad = __syncthreads_or(any && key_row < 0) != 0;          // a page that is none: its key is left out by every row
+            const bool all_see = !bad && rows == R && c0 >= run.lo_max && c0 + CHUNK - 1 <= run.pos_min;
+            const bool warp_sees = quarter * 32 <= last && quarter * 32 + 31 >= first && half * 16 < rows;
+            float s[4][4];                                                       // of rows 16 half + 4 r + row_lane, keys 32 quarter + 8 e + key_lane
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[r][e] = 0.f;
+            copy_rows(area0, kld, 0, last + 1, 0, 0, KD);
+            copy_rows(area1, kld, 0, last + 1, 0, KD, hd - KD);
+#pragma unroll 1
+            for (int d0 = 0; d0 < hd; d0 += KD) {
+                copy_wait<1>();
+                __syncthreads();
+                if (warp_sees) {
+                    const TC* key = (d0 == 0 ? area0 : area1) + (quarter * 32 + key_lane) * kld;
+                    const float* query = q_s + (half * 16 + row_lane) * qld + d0;
+                    const int dims = min(KD, hd - d0);
+#pragma unroll 2
+                    for (int d = 0; d < dims; d += 4) {
+                        float kq[4][4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) Vec4<TC>::load(key + 8 * e * kld + d, kq[e]);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const float4 qv = *reinterpret_cast<const float4*>(query + 4 * r * qld + d);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                s[r][e] = fmaf(qv.x, kq[e][0], s[r][e]);
+                                s[r][e] = fmaf(qv.y, kq[e][1], s[r][e]);
+                                s[r][e] = fmaf(qv.z, kq[e][2], s[r][e]);
+                                s[r][e] = fmaf(qv.w, kq[e][3], s[r][e]);
+                            }
+                        }
+                    }
+                }
+                __syncthreads();                                                 // this half of the keys has been read
+                if (d0 == 0) copy_rows(area0, hd, 0, min(last + 1, CHUNK / 2), v_offset, 0, hd);
+                else copy_rows(area1, hd, CHUNK / 2, last + 1, v_offset, 0, hd);
+            }
+            unsigned seen = 0xffffu;                                             // bit 4 r + e
+            if (!all_see) {
+                seen = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int at = quarter * 32 + 8 * e + key_lane, j = c0 + at;
+                    const bool there = row_s[at] >= 0;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int row = half * 16 + 4 * r + row_lane;            // beyond the run's: pos_s = -1
+                        seen |= (there && (j >= lo_s[row] || j < kept_s[row]) && j <= pos_s[row] ? 1u : 0u) << (4 * r + e);
+                    }
+                }
+            }
+            int mine;
+            {
+                float tops[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int row = half * 16 + 4 * r + row_lane;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float x = s[r][e] * A.scale;
+                        if (A.sc.softcap > 0.f) x = A.sc.softcap * tanhf(x / A.sc.softcap);
+                        if (A.sc.slopes != nullptr) x -= slope_s[row] * (float)(pos_s[row] - (c0 + quarter * 32 + 8 * e + key_lane));
+                        s[r][e] = (seen >> (4 * r + e) & 1) != 0 ? x : -INFINITY;
+                    }
+                    tops[r] = fmaxf(fmaxf(s[r][0], s[r][2]), fmaxf(s[r][1], s[r][3]));
+                }
+                const float top = reduce_four<TakeMax>(tops, &mine);
+                if (mine >= 0) red[0][half * 16 + 4 * mine + row_lane][quarter] = top;
+            }
+            __syncthreads();
+            {
+                float sums[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int row = half * 16 + 4 * r + row_lane;
+                    const float4 x = *reinterpret_cast<const float4*>(red[0][row]);
+                    const float mc = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w));
+                    float w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const bool sees = (seen >> (4 * r + e) & 1) != 0;
+                        const float p = mc != -INFINITY ? expf(s[r][e] - mc) : isnan(s[r][e]) ? s[r][e] : 0.f;
+                        w[e] = sees ? p : 0.f;
+                        p_s[quarter * 32 + 8 * e + key_lane][row] = sees || row >= rows ? w[e] * (1.f / CHUNK) : -1.f;
+                    }
+                    sums[r] = (w[0] + w[2]) + (w[1] + w[3]);                     // keys 16 apart, then 8: the order of a warp's sum
+                }
+                const float sum = reduce_four<TakeSum>(sums, &mine);
+                if (mine >= 0) red[1][half * 16 + 4 * mine + row_lane][quarter] = sum;
+            }
+            copy_wait<1>();
+            __syncthreads();
+            if (warp == 0) {
+                const float4 x = *reinterpret_cast<const float4*>(red[0][lane]), y = *reinterpret_cast<const float4*>(red[1][lane]);
+                const float mc = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)), lc = ((y.x + y.y) + y.z) + y.w;
+                if (parts) {
+                    if (lane < rows) {
+                        float* part = A.partial + ((size_t)at_s[lane] * A.slots + c) * (hd + 2) + hd;
+                        part[0] = mc;
+                        part[1] = lc;
+                    }
+                } else {
+                    float alpha = -1.f, beta = 0.f;                              // alpha below zero: there is nothing to take
+                    if (!take_chunk(m, l, mc, lc, alpha, beta)) alpha = -1.f;
+                    take_s[lane] = make_float2(alpha, CHUNK * beta);
+                }
+            }
+            float vs[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) vs[r][e] = 0.f;
+            {
+                // [fa, fb): keys that every row of the block sees; elsewhere a row leaves out the keys whose p is below zero
+                const int fa = max(first, run.lo_max - c0), fb = bad ? 0 : min(run.pos_min - c0, last) + 1;
+                const float* p_g = &p_s[0][v_row];
+                const TC* v_s = area0 + (has_quad ? quad : 0);
+                int j = first, end = min(CHUNK / 2, last + 1);
+#pragma unroll 1
+                while (true) {
+#pragma unroll 1
+                    while (j < end) {
+                        float v[4];
+                        if (j >= fa && j < fb) {
+                            const int whole = min(fb, end);
+#pragma unroll 4
+                            for (; j < whole; ++j) {
+                                Vec4<TC>::load(v_s + j * hd, v);
+                                const float4 p = *reinterpret_cast<const float4*>(p_g + j * PLD);
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    vs[0][e] = fmaf(p.x, v[e], vs[0][e]);
+                                    vs[1][e] = fmaf(p.y, v[e], vs[1][e]);
+                                    vs[2][e] = fmaf(p.z, v[e], vs[2][e]);
+                                    vs[3][e] = fmaf(p.w, v[e], vs[3][e]);
+                                }
+                            }
+                        } else {
+                            Vec4<TC>::load(v_s + j * hd, v);
+                            float p[4];
+                            load_probabilities<4>(p_g + j * PLD, p);
+#pragma unroll
+                            for (int r = 0; r < 4; ++r)
+                                if (!(p[r] < 0.f)) {
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) vs[r][e] = fmaf(p[r], v[e], vs[r][e]);
+                                }
+                            ++j;
+                        }
+                    }
+                    if (end > last) break;
+                    copy_wait<0>();
+                    __syncthreads();
+                    v_s = area1 + (has_quad ? quad : 0) - (CHUNK / 2) * hd;
+                    end = last + 1;
+                }
+            }
+            __syncthreads();                                                     // take_s is there; the next chunk rewrites the shared arrays
+#pragma unroll
+            for (int rr = 0; rr < 4; ++rr) {
+                const int r = v_row + rr;
+                if (parts) {
+                    if (r < rows && has_quad) {
+                        float* part = A.partial + ((size_t)at_s[r] * A.slots + c) * (hd + 2) + quad;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) part[e] = vs[rr][e];
+                    }
+                } else {
+                    const float2 f = take_s[r];
+                    if (!(f.x < 0.f)) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[rr][e] = fmaf(acc[rr][e], f.x, vs[rr][e] * f.y);
+                    }
+                }
+            }
+            c = c_next;
+        }
+        if (parts) continue;
+        if (warp == 0) end_s[lane] = make_float2(with_sinks(A, my_head, m, l), A.sc.out_scale != nullptr && lane < rows ? A.sc.out_scale[at_s[lane]] : 1.f);
+        __syncthreads();
+        if (has_quad) {
+#pragma unroll
+            for (int rr = 0; rr < 4; ++rr) {
+                const int r = v_row + rr;
+                const float2 f = end_s[r];
+                if (r < rows) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) out[at_s[r] * hd + quad + e] = from_f32<TA>(f.x > 0.f ? acc[rr][e] / f.x * f.y : 0.f);
+                }
+            }
+        }
+    }
+}
+
 // The rows whose chunks went to blocks of their own: the chunks added in order.
 template <typename TA>
 __global__ void __launch_bounds__(CHUNK) attention_merge_kernel(TA* __restrict__ out, AttnArgs A)
@@ -634,9 +974,23 @@ static int launch_rows(const void* q, void* out, const void* pages, const AttnAr
     return 0;
 }
 
+template <typename TA, typename TC>
+static int launch_wide(const void* q, void* out, const void* pages, const AttnArgs& A, dim3 grid, cudaStream_t stream)
+{
+    const size_t smem = WIDE_ROWS * (A.hd + 4) * sizeof(float) + (size_t)2 * A.area * sizeof(TC);
+    SPY_ONCE_PER_DEVICE
+    {
+        const int most = (int)(WIDE_ROWS * (CHUNK + 4) * sizeof(float) + 2 * CHUNK * (KD + 4) * sizeof(TC));
+        SPY_CUDA(cudaFuncSetAttribute(attention_wide_kernel<TA, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    }
+    spy_launch(attention_wide_kernel<TA, TC>, grid, dim3(WIDE_THREADS), smem, stream, (const TA*)q, (TA*)out, (const TC*)pages, A);
+    if (A.slots > 0) spy_launch(attention_merge_kernel<TA>, dim3(A.tokens, A.nh), dim3(CHUNK), 0, stream, (TA*)out, A);
+    return 0;
+}
+
 // How the rows are shared out; the results are the same to the last bit whatever is chosen here.
 struct RowsPlan {
-    int rows, heads, per_tile, head_groups;   // of a block: rows at most (4, 8, 16), heads, tokens; blocks a kv head
+    int rows, heads, per_tile, head_groups;   // of a block: rows at most (4, 8, 16, 32), heads, tokens; blocks a kv head
     long long blocks;                         // without the split
     int chunks, slots, split;                 // of the table; chunks a row that the scratch holds (0: no scratch); blocks a row group's chunks are dealt to
 };
@@ -653,13 +1007,13 @@ static RowsPlan plan_rows(int tokens, int num_seqs, int nh, int nkv, int hd, int
     // by the wider choice.  A table of more than 64 chunks tells little about the contexts in it: 16 are assumed, for prompts their own length.
     const bool prompts = tokens > 2 * (long long)num_seqs;
     const long long work = all_rows * (P.chunks <= 64 ? P.chunks : prompts ? tokens / (num_seqs > 0 ? num_seqs : 1) / CHUNK + 1 : 16);
-    const int most = work < 16LL * sms ? 4 : work < 32LL * sms ? 8 : 16;
+    const int most = work < 16LL * sms ? 4 : work < 32LL * sms ? 8 : hd > KD && prompts && work >= 32LL * sms ? WIDE_ROWS : 16;
     P.head_groups = (group + most - 1) / most;
     P.heads = (group + P.head_groups - 1) / P.head_groups;
     // several tokens a block where they outnumber the sequences by far (prompts), one where most tokens are their sequence's only one
     P.per_tile = prompts ? most / P.heads : 1;
     const int rows = P.heads * P.per_tile;
-    P.rows = rows <= 4 ? 4 : rows <= 8 ? 8 : 16;
+    P.rows = rows <= 4 ? 4 : rows <= 8 ? 8 : rows <= 16 ? 16 : WIDE_ROWS;
     P.blocks = ((long long)tokens + P.per_tile - 1) / P.per_tile * nkv * P.head_groups;
     // Chunks on blocks of their own: worth it while the device holds the blocks about twice at most and a row may have more than two
     // chunks (a launch more costs what a second chunk does).  The table says how many chunks there may be, not how many there are: the
@@ -711,7 +1065,7 @@ extern "C" int spy_attention_generic(const void* q, long long q_row_stride, void
                              : hd <= 64 ? launch_rows<TA, TC, R_, 2>(q, out, pages, A, grid, stream) : launch_rows<TA, TC, R_, 1>(q, out, pages, A, grid, stream))
         SPY_DISPATCH_DTYPE(act_dtype, TA, {
             SPY_DISPATCH_DTYPE(cache_dtype, TC, {
-                const int rc = P.rows == 4 ? SPY_ROWS_LAUNCH(4) : P.rows == 8 ? SPY_ROWS_LAUNCH(8) : SPY_ROWS_LAUNCH(16);
+                const int rc = P.rows == WIDE_ROWS ? launch_wide<TA, TC>(q, out, pages, A, grid, stream) : P.rows == 4 ? SPY_ROWS_LAUNCH(4) : P.rows == 8 ? SPY_ROWS_LAUNCH(8) : SPY_ROWS_LAUNCH(16);
                 if (rc) return rc;
             })
         })
