@@ -318,6 +318,38 @@ def test_attention_generic_rows_do_not_depend_on_their_company(nh, nkv, hd, page
     assert torch.equal(out[:129], whole[:129]) and out[129:131].isinf().any()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd,page_size,planes", [(32, 8, 128, 16, 2), (6, 2, 72, 8, 1), (5, 5, 100, 6, 2), (34, 2, 128, 16, 2)])
+@pytest.mark.parametrize("window,keep,scores", [(0, 0, False), (0, 0, True), (100, 0, True), (150, 130, False)])
+def test_attention_generic_of_prompts_in_wide_blocks_is_bit_by_bit_that_of_single_tokens(dtype, nh, nkv, hd, page_size, planes, window, keep, scores):
+    """Many rows of prompts (32 a block, heads of one and of several kv groups, whole and ragged tiles, several requests a tile) against the
+    same tokens given as requests of their own, which take the other kernel: the same bits, with the options on the scores, with values
+    and keys that are no finite numbers and with a page that is none."""
+    from spyinfer_b200 import kernels
+    torch.manual_seed(hd)
+    runs = [(0, 405), (300, 37), (127, 3), (255, 1), (700, 203)]             # (position of the first token, tokens)
+    width = -(-920 // page_size)
+    pages = torch.randn(len(runs) * width, planes, nkv, page_size, hd, device=DEV).to(dtype)
+    table = torch.randperm(len(runs) * width, device=DEV).view(len(runs), width).to(torch.int32)
+    pages[table[0, 300 // page_size], -1, :, 300 % page_size, 3] = float("inf")
+    pages[table[1, 310 // page_size], 0, 0, 310 % page_size, 1] = float("nan")
+    table[4, 800 // page_size] = -1
+    pos = torch.tensor([p + i for p, n in runs for i in range(n)], dtype=torch.int32, device=DEV)
+    seq = torch.tensor([s for s, (_, n) in enumerate(runs) for _ in range(n)], dtype=torch.int32, device=DEV)
+    T = len(pos)
+    q = torch.randn(T, nh * hd, device=DEV).to(dtype)
+    more = dict(softcap=20.0, slopes=torch.rand(nh, device=DEV) * 0.01, sinks=torch.randn(nh, device=DEV), out_scale=torch.rand(T, nh, device=DEV)) if scores else {}
+
+    def attend(table, seq):
+        out, status = torch.full((T, nh * hd), 7.0, device=DEV, dtype=dtype), torch.zeros(2, dtype=torch.int32, device=DEV)
+        kernels.attention_generic(q, nh, hd, out, pages, table, pos, seq, hd ** -0.5, window=window, keep_first=keep, status=status, **more)
+        return out.nan_to_num(nan=1234.0), status[0].item()
+
+    wide, status = attend(table, seq)
+    single, same = attend(table[seq.long()].contiguous(), torch.arange(T, dtype=torch.int32, device=DEV))
+    assert status == same != 0 and torch.equal(wide, single)
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(8, 2, 32), (6, 6, 128), (16, 1, 20)])
 @pytest.mark.parametrize("window,keep", [(0, 0), (100, 0), (150, 130)])
 def test_attention_generic_of_positions_outside_the_table(nh, nkv, hd, window, keep):
