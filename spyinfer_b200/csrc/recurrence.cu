@@ -583,7 +583,6 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 // by token as before: in the products an infinity of a later token would meet the zeros of an earlier one.
 constexpr float HUGE_INPUT = 1e10f;
 constexpr int WALK_COLS = 16;          // value columns a block of the walk owns
-constexpr int WALK_THREADS = 512;      // sixteen warps: an eighth of a product's terms and half of its rows each
 constexpr int WALK_LD = WALK_COLS + 4; // floats between the rows of a tile of them in shared memory
 
 struct ChunkArgs {
@@ -1008,6 +1007,27 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
     }
 }
 
+// Sums the eight warps' parts of a tile of ROWS x 16 that a thread's accumulators hold (rows g + 8 j, columns 4 cg ..): through shared memory.
+template <int NJ>
+__device__ __forceinline__ void put_parts(float* red, int warp, int g, int cg, const float (&acc)[NJ][4])
+{
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) st4(red + ((size_t)warp * 8 * NJ + g + 8 * j) * WALK_COLS + 4 * cg, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+}
+template <int ROWS>
+__device__ __forceinline__ float4 sum_parts(const float* red, int row, int cg)
+{
+    float4 v = ld4(red + (size_t)row * WALK_COLS + 4 * cg);
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+        const float4 p = ld4(red + ((size_t)w * ROWS + row) * WALK_COLS + 4 * cg);
+        v.x += p.x;
+        v.y += p.y;
+        v.z += p.z;
+        v.w += p.w;
+    }
+    return v;
+}
 // acc[j][c] += sum over four k of x[row g + 8 j][k ..] * y[k ..][4 cg + c]; x rows LDX floats apart, y rows WALK_LD
 template <int NJ, int LDX>
 __device__ __forceinline__ void tile_fma(float (&acc)[NJ][4], const float* x, const float* y)
@@ -1026,7 +1046,7 @@ __device__ __forceinline__ void tile_fma(float (&acc)[NJ][4], const float* x, co
     }
 }
 
-// Matrix memory and linear attention: two warps share DK / 8 rows of the block's 16 columns of S, for half of a chunk's tokens each.
+// Matrix memory and linear attention: a warp owns DK / 8 rows of the block's 16 columns of S.
 template <int MODE, int DK> struct WalkSmem {
     static constexpr int C = 64, LDK = DK + 4, LDP = C + 4;
     static constexpr int Q = 0, P = Q + C * LDK, K = P + C * LDP, V = K + C * LDK, X = V + C * WALK_LD;     // floats; X: F, l, kappa, psum, ksum | the decays
@@ -1037,16 +1057,16 @@ template <int MODE, int DK> struct WalkSmem {
 };
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
+__global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
 {
     using L = WalkSmem<MODE, DK>;
-    constexpr int C = L::C, LDK = L::LDK, LDP = L::LDP, KW = DK / 8;       // KW: rows of S that a pair of warps owns
+    constexpr int C = L::C, LDK = L::LDK, LDP = L::LDP, KW = DK / 8;       // KW: rows of S a warp owns
     extern __shared__ __align__(16) float sm[];
     float *S_s = sm + L::S, *n_s = sm + L::N, *red = sm + L::RED;
     pdl_enter();
     const ScanArgs& a = A.s;
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS, dv = a.dv;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5 & 7, half = tid >> 8, g = lane >> 2, cg = lane & 3;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
     const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
     if (t_begin >= t_end || !takes_chunks<MODE>(a, seq, h, t_begin, t_end)) return;
     const int slot = a.state_slot[seq];
@@ -1056,10 +1076,10 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
     }
     float* st = a.state + ((size_t)slot * a.H + h) * a.record;
     float* st_nm = st + (size_t)DK * dv + (size_t)(c0 / 8) * (DK + 1);      // two copies of n and m: one for every 8 columns
-    for (int idx = tid; idx < DK * 4; idx += WALK_THREADS) st4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3), ld4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3)));
+    for (int idx = tid; idx < DK * 4; idx += THREADS) st4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3), ld4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3)));
     float m = 0.f;
     if (MODE == 0) {
-        for (int r = tid; r < DK; r += WALK_THREADS) n_s[r] = st_nm[r];
+        for (int r = tid; r < DK; r += THREADS) n_s[r] = st_nm[r];
         m = st_nm[DK];
     }
     const int first_slot = chunk_slot(t_begin, seq, C);
@@ -1068,7 +1088,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
         float* base = sm + stage * L::STAGE;
         const float* mine = A.work + ((size_t)(first_slot + (t0 - t_begin) / C) * a.H + h) * chunk_floats(MODE, DK);
         const float* rows = a.proj + (size_t)t0 * a.ld;
-        for (int idx = tid; idx < C * (DK / 4); idx += WALK_THREADS) {
+        for (int idx = tid; idx < C * (DK / 4); idx += THREADS) {
             const int t = idx / (DK / 4), c = 4 * (idx - t * (DK / 4));
             if (MODE == 2) {
                 cp_async16(base + L::Q + t * LDK + c, mine + C * C + t * DK + c);
@@ -1081,14 +1101,14 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
                 st4(base + L::K + t * LDK + c, make_float4(0.f, 0.f, 0.f, 0.f));
             }
         }
-        for (int idx = tid; idx < C * C / 4; idx += WALK_THREADS) cp_async16(base + L::P + (idx >> 4) * LDP + 4 * (idx & 15), mine + 4 * idx);
-        for (int idx = tid; idx < C * 4; idx += WALK_THREADS) {
+        for (int idx = tid; idx < C * C / 4; idx += THREADS) cp_async16(base + L::P + (idx >> 4) * LDP + 4 * (idx & 15), mine + 4 * idx);
+        for (int idx = tid; idx < C * 4; idx += THREADS) {
             const int t = idx >> 2, c = 4 * (idx & 3);
             if (t < n_tok) cp_async16(base + L::V + t * WALK_LD + c, rows + (size_t)t * a.ld + a.off_v + h * dv + c0 + c);
             else st4(base + L::V + t * WALK_LD + c, make_float4(0.f, 0.f, 0.f, 0.f));
         }
         const float* extra = mine + C * C + (MODE == 2 ? 2 * C * DK : 0);
-        for (int idx = tid; idx < (MODE == 0 ? 4 * C + DK : DK) / 4; idx += WALK_THREADS) cp_async16(base + L::X + 4 * idx, extra + 4 * idx);
+        for (int idx = tid; idx < (MODE == 0 ? 4 * C + DK : DK) / 4; idx += THREADS) cp_async16(base + L::X + 4 * idx, extra + 4 * idx);
     };
     request(t_begin, 0);
     int stage = 0;
@@ -1099,7 +1119,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
         cp_async_wait_all();
         __syncthreads();                           // this chunk has landed, the chunk before is done with
         if (t0 + C < t_end) request(t0 + C, stage ^ 1);
-        float keep = 1.f, add = 1.f, nq = 0.f;     // of the old state and of the chunk's sum; n . q of token tid / 8
+        float keep = 1.f, add = 1.f, nq = 0.f;     // of the old state and of the chunk's sum; n . q of token tid / 4
         const auto taken = [&](int t, float& alpha, float& beta) {     // what a token's output takes of the chunk and of the state ahead
             const float l = X[C + t], f = X[t] + m, top = fmaxf(f, l);
             alpha = expf(l - top);
@@ -1107,47 +1127,45 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
         };
         if (MODE == 0) {
             taken(C - 1, add, keep);               // behind the chunk (padding tokens change nothing)
-            const int t = tid >> 3, part = tid & 7;
+            const int t = tid >> 2, part = tid & 3;
 #pragma unroll
-            for (int c = 0; c < DK; c += 32) nq = dot4(ld4(Q + t * LDK + c + 4 * part), ld4(n_s + c + 4 * part), nq);
+            for (int c = 0; c < DK / 4; c += 4) nq = dot4(ld4(Q + t * LDK + 4 * c + 4 * part), ld4(n_s + 4 * c + 4 * part), nq);
             nq += __shfl_xor_sync(0xffffffffu, nq, 1);
             nq += __shfl_xor_sync(0xffffffffu, nq, 2);
-            nq += __shfl_xor_sync(0xffffffffu, nq, 4);
         }
-        // what the state ahead of the chunk gives: this pair's rows of it; then this pair's share of the chunk's own tokens
-        const int t_row = half * (C / 2) + g;      // this lane's first token
-        float acc[4][4] = {};
+        // what the state ahead of the chunk gives: this warp's rows of it; then this warp's share of the chunk's own tokens
+        float acc[8][4] = {};
 #pragma unroll
-        for (int k = 0; k < KW; k += 4) tile_fma<4, LDK>(acc, Q + t_row * LDK + warp * KW + k, S_s + (warp * KW + k) * WALK_LD + 4 * cg);
+        for (int k = 0; k < KW; k += 4) tile_fma<8, LDK>(acc, Q + g * LDK + warp * KW + k, S_s + (warp * KW + k) * WALK_LD + 4 * cg);
         if (MODE == 0) {
-            float own[4][4] = {};
+            float own[8][4] = {};
 #pragma unroll
-            for (int k = 0; k < C / 8; k += 4) tile_fma<4, LDP>(own, P + t_row * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
+            for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(own, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 8; ++j) {
                 float alpha, beta;
-                taken(t_row + 8 * j, alpha, beta);
+                taken(g + 8 * j, alpha, beta);
                 beta *= a.q_scale;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(beta, acc[j][c], alpha * own[j][c]);
             }
         } else {
 #pragma unroll
-            for (int k = 0; k < C / 8; k += 4) tile_fma<4, LDP>(acc, P + t_row * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
+            for (int k = 0; k < C / 8; k += 4) tile_fma<8, LDP>(acc, P + g * LDP + warp * (C / 8) + k, V + (warp * (C / 8) + k) * WALK_LD + 4 * cg);
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) st4(red + (warp * C + t_row + 8 * j) * WALK_COLS + 4 * cg, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
-        // The state behind the chunk.  A pair's rows (no other warp reads them), half of them a warp: a lane has four and four columns, over every
-        // SG-th token; the sums meet by shuffles, each lane keeping its share.
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory");     // both warps of the pair have read the state
+        put_parts<8>(red, warp, g, cg, acc);
+        // The state behind the chunk.  A warp's rows (no other warp reads them): a lane has half of them and four columns, over every fourth
+        // token; the four sums meet by shuffles, each lane keeping a quarter.
+        __syncwarp();
         {
-            constexpr int SG = DK == 128 ? 4 : 8;
-            const int sg = g % SG, r0 = warp * KW + half * (KW / 2) + 4 * (g / SG);
-            float u[4][4] = {};
+            constexpr int RL = KW / 2;             // rows of a lane
+            const int rg = lane >> 4, sg = lane >> 2 & 3, r0 = warp * KW + rg * RL;
+            float u[RL][4] = {};
 #pragma unroll 4
-            for (int s = sg; s < C; s += SG) {
-                float kk[4], vv[4];
-                *reinterpret_cast<float4*>(kk) = ld4(K + s * LDK + r0);
+            for (int s = sg; s < C; s += 4) {
+                float kk[RL], vv[4];
+#pragma unroll
+                for (int r = 0; r < RL; r += 4) *reinterpret_cast<float4*>(kk + r) = ld4(K + s * LDK + r0 + r);
                 *reinterpret_cast<float4*>(vv) = ld4(V + s * WALK_LD + 4 * cg);
                 if (MODE == 0) {
                     const float f = X[2 * C + s] * add;
@@ -1155,79 +1173,66 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(ChunkArgs A)
                     for (int c = 0; c < 4; ++c) vv[c] *= f;
                 }
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < RL; ++r)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) u[r][c] = fmaf(kk[r], vv[c], u[r][c]);
             }
-            // lanes SG / 2 apart halve the rows, then SG / 4 apart; with eight groups neighbours halve the columns
-            const bool up2 = (sg & SG / 2) != 0, up1 = (sg & SG / 4) != 0;
-            float two[2][4], one[4];
+            // lanes sg and sg ^ 2 halve the rows, then sg and sg ^ 1: a lane ends with RL / 4 rows
+            constexpr int H2 = RL / 2, H4 = RL / 4;
+            const bool up2 = (sg & 2) != 0, up1 = (sg & 1) != 0;
+            float half[H2][4], mine[H4][4];
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+            for (int r = 0; r < H2; ++r)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float give = up2 ? u[r][c] : u[r + 2][c], own = up2 ? u[r + 2][c] : u[r][c];
-                    two[r][c] = own + __shfl_xor_sync(0xffffffffu, give, 2 * SG);
+                    const float give = up2 ? u[r][c] : u[r + H2][c], own = up2 ? u[r + H2][c] : u[r][c];
+                    half[r][c] = own + __shfl_xor_sync(0xffffffffu, give, 8);
                 }
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float give = up1 ? two[0][c] : two[1][c], own = up1 ? two[1][c] : two[0][c];
-                one[c] = own + __shfl_xor_sync(0xffffffffu, give, SG);
-            }
-            const int row = r0 + (up2 ? 2 : 0) + (up1 ? 1 : 0);
-            const float d = MODE == 0 ? keep : X[row];
-            float* to = S_s + row * WALK_LD + 4 * cg;
-            if constexpr (SG == 4) {
-                const float4 o = ld4(to);
-                st4(to, make_float4(fmaf(d, o.x, one[0]), fmaf(d, o.y, one[1]), fmaf(d, o.z, one[2]), fmaf(d, o.w, one[3])));
-            } else {
-                const bool up0 = (sg & 1) != 0;
-                float2* pair = reinterpret_cast<float2*>(to + (up0 ? 2 : 0));
-                float v[2];
+            for (int r = 0; r < H4; ++r)
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const float give = up0 ? one[c] : one[c + 2], own = up0 ? one[c + 2] : one[c];
-                    v[c] = own + __shfl_xor_sync(0xffffffffu, give, 4);
+                for (int c = 0; c < 4; ++c) {
+                    const float give = up1 ? half[r][c] : half[r + H4][c], own = up1 ? half[r + H4][c] : half[r][c];
+                    mine[r][c] = own + __shfl_xor_sync(0xffffffffu, give, 4);
                 }
-                const float2 o = *pair;
-                *pair = make_float2(fmaf(d, o.x, v[0]), fmaf(d, o.y, v[1]));
+#pragma unroll
+            for (int r = 0; r < H4; ++r) {
+                const int row = r0 + (up2 ? H2 : 0) + (up1 ? H4 : 0) + r;
+                float* s = S_s + row * WALK_LD + 4 * cg;
+                const float d = MODE == 0 ? keep : X[row];
+                float4 o = ld4(s);
+                st4(s, make_float4(fmaf(d, o.x, mine[r][0]), fmaf(d, o.y, mine[r][1]), fmaf(d, o.z, mine[r][2]), fmaf(d, o.w, mine[r][3])));
             }
         }
         __syncthreads();                           // the outputs' parts are there; n has been read
         {
-            const int t = tid >> 3, part = tid & 7;
-            float2 o = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 v = *reinterpret_cast<const float2*>(red + (i * C + t) * WALK_COLS + 2 * part);
-                o.x += v.x;
-                o.y += v.y;
-            }
+            const int t = tid >> 2, part = tid & 3;
+            float4 o = sum_parts<C>(red, t, part);
             if (MODE == 0) {
                 float alpha, beta;
                 taken(t, alpha, beta);
                 nq = fmaf(beta * a.q_scale, nq, alpha * X[3 * C + t]);
                 const float d = fmaxf(fabsf(nq), expf(-fmaxf(X[t] + m, X[C + t]))) + 1e-6f;
-                o = make_float2(o.x / d, o.y / d);
+                o = make_float4(o.x / d, o.y / d, o.z / d, o.w / d);
             }
-            if (t < n_tok) *reinterpret_cast<float2*>(a.out + (size_t)(t0 + t) * a.H * dv + h * dv + c0 + 2 * part) = o;
+            if (t < n_tok) st4(a.out + (size_t)(t0 + t) * a.H * dv + h * dv + c0 + 4 * part, o);
         }
         if (MODE == 0) {
-            for (int r = tid; r < DK; r += WALK_THREADS) n_s[r] = fmaf(keep, n_s[r], add * X[4 * C + r]);
+            for (int r = tid; r < DK; r += THREADS) n_s[r] = fmaf(keep, n_s[r], add * X[4 * C + r]);
             m = fmaxf(X[C - 1] + m, X[C + C - 1]);
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < DK * 4; idx += WALK_THREADS) st4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3), ld4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3)));
+    for (int idx = tid; idx < DK * 4; idx += THREADS) st4(st + (size_t)(idx >> 2) * dv + c0 + 4 * (idx & 3), ld4(S_s + (idx >> 2) * WALK_LD + 4 * (idx & 3)));
     if (MODE == 0) {
         for (int cp = 0; cp < 2; ++cp) {
-            for (int r = tid; r < DK; r += WALK_THREADS) st_nm[(size_t)cp * (DK + 1) + r] = n_s[r];
+            for (int r = tid; r < DK; r += THREADS) st_nm[(size_t)cp * (DK + 1) + r] = n_s[r];
             if (tid == 0) st_nm[(size_t)cp * (DK + 1) + DK] = m;
         }
     }
 }
 
-// Delta rule: [outputs of 32 tokens; the state's 64 rows] = W [the state; the values], a warp 12 of the 96 columns of W and half of its rows.
+// Delta rule: [outputs of 32 tokens; the state's 64 rows] = W [the state; the values], a warp 12 of the 96 columns of W.
 struct DeltaSmem {
     static constexpr int C = 32, D = 64, R = C + D, LDW = R + 4;
     static constexpr int W = 0, V = W + R * LDW, STAGE = V + C * WALK_LD;
@@ -1235,7 +1240,7 @@ struct DeltaSmem {
     static constexpr size_t BYTES = TOTAL * sizeof(float);
 };
 
-__global__ void __launch_bounds__(WALK_THREADS, 1) walk_delta_kernel(ChunkArgs A)
+__global__ void __launch_bounds__(THREADS, 1) walk_delta_kernel(ChunkArgs A)
 {
     using L = DeltaSmem;
     constexpr int C = L::C, D = L::D, R = L::R, LDW = L::LDW, KW = R / 8;
@@ -1244,7 +1249,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_delta_kernel(ChunkArgs A
     pdl_enter();
     const ScanArgs& a = A.s;
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5 & 7, half = tid >> 8, g = lane >> 2, cg = lane & 3;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
     const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
     if (t_begin >= t_end || !takes_chunks<1>(a, seq, h, t_begin, t_end)) return;
     const int slot = a.state_slot[seq];
@@ -1253,13 +1258,13 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_delta_kernel(ChunkArgs A
         return;
     }
     float* st = a.state + ((size_t)slot * a.H + h) * a.record;
-    if (tid < D * 4) st4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3), ld4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3)));
+    st4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3), ld4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3)));      // 64 rows of four quads: one a thread
     const int first_slot = chunk_slot(t_begin, seq, C);
     auto request = [&](int t0, int stage) {
         const int n_tok = min(C, t_end - t0);
         float* base = sm + stage * L::STAGE;
         const float* W = A.work + ((size_t)(first_slot + (t0 - t_begin) / C) * a.H + h) * chunk_floats(1, D);
-        for (int idx = tid; idx < R * R / 4; idx += WALK_THREADS) cp_async16(base + L::W + idx / (R / 4) * LDW + 4 * (idx % (R / 4)), W + 4 * idx);
+        for (int idx = tid; idx < R * R / 4; idx += THREADS) cp_async16(base + L::W + idx / (R / 4) * LDW + 4 * (idx % (R / 4)), W + 4 * idx);
         if (tid < C * 4) {
             const int t = tid >> 2, c = 4 * (tid & 3);
             if (t < n_tok) cp_async16(base + L::V + t * WALK_LD + c, a.proj + (size_t)(t0 + t) * a.ld + a.off_v + h * D + c0 + c);
@@ -1274,36 +1279,29 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) walk_delta_kernel(ChunkArgs A
         cp_async_wait_all();
         __syncthreads();                           // this chunk has landed, the state of the chunk before is written
         if (t0 + C < t_end) request(t0 + C, stage ^ 1);
-        const int row0 = half * (R / 2) + g;       // this lane's first row of W
-        float acc[R / 16][4] = {};
+        float acc[R / 8][4] = {};
 #pragma unroll
         for (int i = 0; i < KW; i += 4) {
             const int k = warp * KW + i;           // 4 consecutive columns of W: all of the state or all of the values
-            tile_fma<R / 16, LDW>(acc, W + row0 * LDW + k, (k < D ? S_s + k * WALK_LD : V + (k - D) * WALK_LD) + 4 * cg);
+            tile_fma<R / 8, LDW>(acc, W + g * LDW + k, (k < D ? S_s + k * WALK_LD : V + (k - D) * WALK_LD) + 4 * cg);
         }
-#pragma unroll
-        for (int j = 0; j < R / 16; ++j) st4(red + (warp * R + row0 + 8 * j) * WALK_COLS + 4 * cg, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+        put_parts<R / 8>(red, warp, g, cg, acc);
         __syncthreads();
-        if (tid < R * 4) {
-            const int row = tid >> 2, part = tid & 3;
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 v = ld4(red + (i * R + row) * WALK_COLS + 4 * part);
-                o = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
-            }
+        for (int idx = tid; idx < R * 4; idx += THREADS) {
+            const int row = idx >> 2, part = idx & 3;
+            const float4 o = sum_parts<R>(red, row, part);
             if (row >= C) st4(S_s + (row - C) * WALK_LD + 4 * part, o);
             else if (row < n_tok) st4(a.out + (size_t)(t0 + row) * a.H * D + h * D + c0 + 4 * part, o);
         }
     }
     __syncthreads();
-    if (tid < D * 4) st4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3), ld4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3)));
+    st4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3), ld4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3)));
 }
 
-template <typename Args> static int launch_chunk_kernel(void (*kernel)(Args), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args& A)
+template <typename Args> static int launch_chunk_kernel(void (*kernel)(Args), dim3 grid, size_t smem, cudaStream_t stream, const Args& A)
 {
     SPY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    spy_launch(kernel, grid, dim3(threads), smem, stream, A);
+    spy_launch(kernel, grid, dim3(THREADS), smem, stream, A);
     return 0;
 }
 
@@ -1330,14 +1328,14 @@ template <int MODE> static int launch_chunks(ScanArgs& S, int tokens, int num_se
     int rc;
     if constexpr (MODE == 1) {
         constexpr int C = 32, D = 64, R = C + D;
-        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, THREADS, (4 * C * (D + 4) + 2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
-        if (!rc) rc = launch_chunk_kernel(walk_delta_kernel, walk, WALK_THREADS, DeltaSmem::BYTES, stream, A);
+        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, (4 * C * (D + 4) + 2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
+        if (!rc) rc = launch_chunk_kernel(walk_delta_kernel, walk, DeltaSmem::BYTES, stream, A);
     } else {
         const size_t rows = (MODE == 0 ? 2 : 3) * 64 * (size_t)(S.dk + 4) * sizeof(float);
         auto chunk = MODE == 0 ? (S.dk == 64 ? chunk_memory_kernel<64> : chunk_memory_kernel<128>) : (S.dk == 64 ? chunk_linear_kernel<64> : chunk_linear_kernel<128>);
-        rc = launch_chunk_kernel(chunk, chunks, THREADS, rows, stream, A);
-        if (!rc) rc = S.dk == 64 ? launch_chunk_kernel(walk_kernel<MODE, 64>, walk, WALK_THREADS, WalkSmem<MODE, 64>::BYTES, stream, A)
-                                 : launch_chunk_kernel(walk_kernel<MODE, 128>, walk, WALK_THREADS, WalkSmem<MODE, 128>::BYTES, stream, A);
+        rc = launch_chunk_kernel(chunk, chunks, rows, stream, A);
+        if (!rc) rc = S.dk == 64 ? launch_chunk_kernel(walk_kernel<MODE, 64>, walk, WalkSmem<MODE, 64>::BYTES, stream, A)
+                                 : launch_chunk_kernel(walk_kernel<MODE, 128>, walk, WalkSmem<MODE, 128>::BYTES, stream, A);
     }
     if (rc) return rc;
     SPY_CHECK_LAUNCH("recurrence (chunks)");
