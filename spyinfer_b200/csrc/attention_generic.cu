@@ -791,9 +791,9 @@ attention_wide_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
                     const int row = half * 16 + 4 * r + row_lane;
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        float x = s[r][e] * A.scale;
-                        if (A.sc.softcap > 0.f) x = A.sc.softcap * tanhf(x / A.sc.softcap);
-                        if (A.sc.slopes != nullptr) x -= slope_s[row] * (float)(pos_s[row] - (c0 + quarter * 32 + 8 * e + key_lane));
+                        float x = __fmul_rn(s[r][e], A.scale);                   // rounded before the bias comes off, as above
+                        if (A.sc.softcap > 0.f) x = __fmul_rn(A.sc.softcap, tanhf(x / A.sc.softcap));
+                        if (A.sc.slopes != nullptr) x = fmaf(-slope_s[row], (float)(pos_s[row] - (c0 + quarter * 32 + 8 * e + key_lane)), x);
                         s[r][e] = (seen >> (4 * r + e) & 1) != 0 ? x : -INFINITY;
                     }
                     tops[r] = fmaxf(fmaxf(s[r][0], s[r][2]), fmaxf(s[r][1], s[r][3]));
