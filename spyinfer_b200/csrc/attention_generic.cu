@@ -1,6 +1,6 @@
 // Attention over the paged cache for any mix of queries, every head size, every page size, 32-bit
-// or bfloat16 storage, everything computed in 32-bit with expf.  Two kernels: head sizes up to 128 in
-// quads take the one for several query rows a block (attention_rows_kernel), the others one block per
+// or bfloat16 storage, everything computed in 32-bit with expf.  Three kernels: head sizes up to 128 in
+// quads take one of two for several query rows a block (attention_rows_kernel; attention_wide_kernel for prompts), the others one block per
 // (query token, head).  It is the
 // engine's float32 path and the fallback of the bfloat16 path for sizes its fast kernels
 // refuse.  A cache of one plane (`planes` = 1) holds keys only and the values are the keys
@@ -590,7 +590,9 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
 // The kernel above reads shared memory more than it multiplies: a key's quad and 16 queries' for 64 multiply-adds.  Here a thread reads four
 // keys' quads and four queries' for as many, and in the value sums a quad of probabilities and one of values for 16, so that the multiply-adds
 // are what is left, and a block's keys and values serve twice the rows.  Every sum runs in the same order as above: the bits are the same.
-// WIDE_MEASURED
+// Measured with the merge, 32 heads over 8 of 128, 32-bit, kernel above with 16 rows / this one (us): prompts of 150 tokens 52 / 40, of 300 95 / 66, of 600
+// 286 / 178, of 2,000 2,266 / 1,405; 64 tokens behind 2,000 183 / 113; 8 of 100 115 / 76.  What is left beside the multiply-adds (18 us of the 300
+// tokens' 66): a block's copies, maxima and sums wait for one another, and two blocks an SM are what shared memory holds.
 constexpr int WIDE_ROWS = 32, WIDE_THREADS = 256, WIDE_PLD = WIDE_ROWS + 4;
 
 // v[0..4) over the eight lanes whose numbers differ in their lowest three bits; the result is row `*row`'s in lanes whose `*row` is not negative.
@@ -1004,7 +1006,8 @@ static RowsPlan plan_rows(int tokens, int num_seqs, int nh, int nkv, int hd, int
     // Rows a block: few where a block's way through one chunk is what counts, more where blocks share the reading of many chunks.  Measured
     // with 4 / 8 / 16 (us): 16 heads a kv head, 100 keys, 1 to 16 requests 11.5 / 14 / 20; 16 requests of 4,096 keys 83 / 78 / 62; 4 of 4,096 40 / 32 / 37;
     // prompts of 32 heads over 8: 37 tokens 9.3 / 12 / 17, 300 tokens 116 / 112 / 92, 20 tokens behind 8,000 326 / 304 / 233: two blocks an SM are kept busy
-    // by the wider choice.  A table of more than 64 chunks tells little about the contexts in it: 16 are assumed, for prompts their own length.
+    // by the wider choice.  Prompts with head sizes above 64 take 32 rows in place of 16 (attention_wide_kernel) wherever 16 would be chosen: at the least work
+    // there (300 tokens of 5 heads over 1) 38.4 with 16 and 37.7, from there on 0.59 to 0.86 of the time.  A table of more than 64 chunks tells little about the contexts in it: 16 are assumed, for prompts their own length.
     const bool prompts = tokens > 2 * (long long)num_seqs;
     const long long work = all_rows * (P.chunks <= 64 ? P.chunks : prompts ? tokens / (num_seqs > 0 ? num_seqs : 1) / CHUNK + 1 : 16);
     const int most = work < 16LL * sms ? 4 : work < 32LL * sms ? 8 : hd > KD && prompts && work >= 32LL * sms ? WIDE_ROWS : 16;
