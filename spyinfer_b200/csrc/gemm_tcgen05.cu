@@ -844,7 +844,7 @@ __device__ int g_pair_tail_count[2 * PAIR_TAIL_MAX_TILES];   // [tail tile][bloc
 constexpr int PAIR_MAX_STAGES = 10;
 constexpr int PAIR_X_BYTES = BM * BK * 2;                    // 128 rows of weights
 constexpr int PAIR_AREA = 6 * 2 * PAIR_X_BYTES;              // the ring: six stages at 256 tokens a tile, more at fewer
-constexpr int PAIR_STAGED_LD = 36;                           // floats between the tokens of a warp's staged chunk (32 outputs and a pad, rows 16 bytes aligned)
+constexpr int PAIR_STAGED_LD = 36;                           // words between the tokens (bfloat16: pairs of them) of a warp's staged chunk (32 outputs and a pad, rows 16 bytes aligned)
 constexpr int PAIR_STAGED_BYTES = 32 * PAIR_STAGED_LD * 4;   // a warp's 32 tokens
 constexpr size_t PAIR_SMEM = (size_t)PAIR_AREA + 4 * PAIR_STAGED_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 __host__ __device__ constexpr int pair_stage_bytes(int token_rows) { return PAIR_X_BYTES + token_rows / 2 * BK * 2; }
@@ -871,10 +871,26 @@ static inline TokenTiles token_tiles(int M)
     return t;
 }
 
+// Eight outputs of two tokens, an output of both in a word (the first token's below): a row of 16 bytes for each of the `count` tokens that there are.
+__device__ __forceinline__ void store_token_pair(bf16* dst, long long ld, int count, uint4 v, uint4 w)
+{
+    if (count > 0)
+        *reinterpret_cast<uint4*>(dst) = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410), __byte_perm(w.x, w.y, 0x5410),
+                                                    __byte_perm(w.z, w.w, 0x5410));
+    if (count > 1)
+        *reinterpret_cast<uint4*>(dst + ld) = make_uint4(__byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632), __byte_perm(w.x, w.y, 0x7632),
+                                                         __byte_perm(w.z, w.w, 0x7632));
+}
+
 // Stores one chunk of a tile that has the weights in its rows: this lane holds output x0 + lane of the 32 tokens from y on, `staged`
 // is the warp's own place in shared memory, where the chunk is turned so that it leaves in rows of 16 bytes a lane.  For the gated
-// epilogues lanes 2i and 2i + 1 hold gate row and up row of output x0 / 2 + i: of two tokens at a time the even lane sends the
-// second's gate and finishes the first, the odd lane sends the first's up and finishes the second.
+// epilogues lanes 2i and 2i + 1 hold gate row and up row of output x0 / 2 + i: of four tokens at a time the even lane sends the
+// last two's gates and finishes the first two, the odd lane sends the first two's ups and finishes the others.
+// bfloat16 results are staged as pairs of tokens, an output of both in a word: half of the words.  The read-out of a product's last tiles
+// hides behind nothing, and with a 32-bit word for every number tiles of full height were slower than rows of 16 bytes straight from a lane that holds a
+// token (tokens in the M slot / a word a number / pairs, us): 2,048 x 2,048, 1,025 tokens 15.3 / 15.9 / 15.2; 10,240 x 5,120, 512 tokens 58.9 / 60.8 / 59.5;
+// 8,192 x 2,048, 512 tokens 18.6 / 19.0 / 18.2; SwiGLU of 16,384 x 2,048, 256 tokens 19.3 / 20.5 / 20.0, 480 tokens 29.9 / 30.4 / 29.9.  What is left are gated products
+// whose tiles are of nearly full height (24,576 x 4,096, 256 tokens 52.2 / 55.0 / 54.8, 192 tokens 49.7 / 46.0 / 45.9): the exchange between lanes.
 template <typename TC, int EPI>
 __device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int lane, int x0, int y, int x_rows, int y_rows, const uint32_t (&r)[32],
                                                    float* staged, float row_bias, const GluArgs& glu)
@@ -882,56 +898,71 @@ __device__ __forceinline__ void store_chunk_turned(TC* base, long long ld, int l
     const int count = min(32, y_rows - y);
     if (x0 >= x_rows || count <= 0) return;    // the same for the whole warp
     if constexpr (gated_epilogue(EPI)) {
-        constexpr int LD = 24;                 // bfloat16 elements between the tokens: 16 outputs and a pad, rows 16 bytes aligned
-        bf16* turned = reinterpret_cast<bf16*>(staged);
+        // [16 pairs of tokens][16]: an output of both tokens in a word; the quads of every other two rows change places in turns, so that
+        // neither the stores nor the loads of 16 bytes meet in a bank
+        uint32_t* pairs = reinterpret_cast<uint32_t*>(staged);
         const bool odd = (lane & 1) != 0;
-        const int outs = min(16, (x_rows - x0) / 2);
+        const int outs = min(16, (x_rows - x0) / 2), o = lane >> 1;
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            const float a = __uint_as_float(r[j]) + row_bias, b = __uint_as_float(r[j + 1]) + row_bias;
-            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-            turned[(j + (odd ? 1 : 0)) * LD + (lane >> 1)] = __float2bfloat16_rn(gated_mul<EPI>(odd ? got : a, odd ? b : got, glu));
+        for (int k = 0; k < 8; ++k) {          // of four tokens the even lane finishes the first two, the odd lane the others
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float a = __uint_as_float(r[4 * k + e]) + row_bias, b = __uint_as_float(r[4 * k + 2 + e]) + row_bias;
+                const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+                v[e] = gated_mul<EPI>(odd ? got : a, odd ? b : got, glu);
+            }
+            pairs[(2 * k + (odd ? 1 : 0)) * 16 + (o ^ (k & 1) * 4)] = pack_bf16(v[0], v[1]);
         }
         __syncwarp();
         TC* dst = base + (size_t)y * ld + x0 / 2;
         if (outs == 16 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int t = i * 16 + (lane >> 1), part = lane & 1;
-                if (t < count) *reinterpret_cast<uint4*>(dst + (size_t)t * ld + part * 8) = *reinterpret_cast<const uint4*>(turned + t * LD + part * 8);
-            }
+            const int row = lane >> 1, part = lane & 1, turn = (row >> 1 & 1) * 4;
+            const uint4 v = *reinterpret_cast<const uint4*>(pairs + row * 16 + (part * 8 ^ turn));
+            const uint4 w = *reinterpret_cast<const uint4*>(pairs + row * 16 + ((part * 8 + 4) ^ turn));
+            store_token_pair(dst + (size_t)(2 * row) * ld + part * 8, ld, count - 2 * row, v, w);
         } else {
             for (int i = lane; i < 32 * 16; i += 32) {
-                const int t = i >> 4, o = i & 15;
-                if (t < count && o < outs) dst[(size_t)t * ld + o] = from_f32<TC>(__bfloat162float(turned[t * LD + o]));
+                const int t = i >> 4, c = i & 15;
+                if (t < count && c < outs) dst[(size_t)t * ld + c] = reinterpret_cast<const TC*>(pairs + (t >> 1) * 16 + (c ^ (t >> 2 & 1) * 4))[t & 1];
             }
         }
-    } else {
+    } else if constexpr (sizeof(TC) == 2) {
+        uint32_t* pairs = reinterpret_cast<uint32_t*>(staged);     // [16 pairs of tokens][PAIR_STAGED_LD]: an output of both in a word
 #pragma unroll
-        for (int j = 0; j < 32; ++j) staged[j * PAIR_STAGED_LD + lane] = EPI == 2 ? relu_squared(__uint_as_float(r[j])) : __uint_as_float(r[j]);
+        for (int j = 0; j < 32; j += 2) {
+            const float a = __uint_as_float(r[j]), b = __uint_as_float(r[j + 1]);
+            pairs[j / 2 * PAIR_STAGED_LD + lane] = EPI == 2 ? pack_bf16(relu_squared(a), relu_squared(b)) : pack_bf16(a, b);
+        }
         __syncwarp();
         const int outs = min(32, x_rows - x0);
         TC* dst = base + (size_t)y * ld + x0;
-        if (outs == 32 && (ld & (16 / (int)sizeof(TC) - 1)) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            if constexpr (sizeof(TC) == 4) {
+        if (outs == 32 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int t = i * 4 + (lane >> 3), part = lane & 7;
-                    if (t < count) *reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4) = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int t = i * 8 + (lane >> 2), part = lane & 3;
-                    const float4 v = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 8);
-                    const float4 w = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 8 + 4);
-                    if (t < count)
-                        *reinterpret_cast<uint4*>(dst + (size_t)t * ld + part * 8) =
-                            make_uint4(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w), pack_bf16(w.x, w.y), pack_bf16(w.z, w.w));
-                }
+            for (int i = 0; i < 2; ++i) {
+                const int t = 2 * (i * 8 + (lane >> 2)), part = lane & 3;
+                const uint4 v = *reinterpret_cast<const uint4*>(pairs + t / 2 * PAIR_STAGED_LD + part * 8);
+                const uint4 w = *reinterpret_cast<const uint4*>(pairs + t / 2 * PAIR_STAGED_LD + part * 8 + 4);
+                store_token_pair(dst + (size_t)t * ld + part * 8, ld, count - t, v, w);
             }
         } else if (lane < outs) {
-            for (int t = 0; t < count; ++t) store_elem(dst + (size_t)t * ld + lane, staged[t * PAIR_STAGED_LD + lane]);
+            for (int t = 0; t < count; ++t)
+                dst[(size_t)t * ld + lane] = reinterpret_cast<const TC*>(pairs + (t >> 1) * PAIR_STAGED_LD + lane)[t & 1];
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) staged[j * PAIR_STAGED_LD + lane] = __uint_as_float(r[j]);
+        __syncwarp();
+        const int outs = min(32, x_rows - x0);
+        TC* dst = base + (size_t)y * ld + x0;
+        if (outs == 32 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int t = i * 4 + (lane >> 3), part = lane & 7;
+                if (t < count) *reinterpret_cast<float4*>(dst + (size_t)t * ld + part * 4) = *reinterpret_cast<const float4*>(staged + t * PAIR_STAGED_LD + part * 4);
+            }
+        } else if (lane < outs) {
+            for (int t = 0; t < count; ++t) dst[(size_t)t * ld + lane] = staged[t * PAIR_STAGED_LD + lane];
         }
     }
     __syncwarp();   // the next chunk's numbers may come
