@@ -1276,7 +1276,7 @@ static int launch(const CUtensorMap& mx, const CUtensorMap& my, void* out, long 
 namespace {
 
 // The plan of a product: the kernel it runs on (choose_kind), how many ways K is split and how many weight rows a block takes.
-// Pairs and single blocks (many tokens): 256 x 256 or 128 x 256 tiles; K is cut into ranges by plan only for pairs with
+// Pairs and single blocks (many tokens): tiles of 256 weight rows x up to 256 tokens or 128 tokens x 256 weight rows; K is cut into ranges by plan only for pairs with
 // few tiles (the single-block kernel shares K blocks out itself when there are fewer tiles than SMs).
 // The swapped kernel (few tokens: decoding; the weights sit in the instruction's M slot, two blocks share an
 // SM; the token tile is 16, 32, 64 or 128 tokens (65 to 128 tokens in ONE tile of 128: against two tiles of
@@ -1348,34 +1348,33 @@ struct Plan {
     Kind kind;
 };
 
-static inline int pair_min_tiles() { return (spy_sm_count() / 2 + 1) / 2; }   // whole 256 x 256 tiles occupy at least half of the clusters (SMs / 2) from here on
+static inline int pair_min_tiles() { return (spy_sm_count() / 2 + 1) / 2; }   // the pairs' tiles occupy at least half of the clusters (SMs / 2) from here on
 
 // Which kernel a product runs on.  Up to 128 tokens: the swapped kernel (weights in the instruction's M slot, one or
-// two token tiles of 64).  Beyond: pairs of blocks on 256 x 256 tiles where they find enough work (whole tiles for
+// two token tiles of 64).  Beyond: pairs of blocks (256 weight rows x up to 256 tokens, see TokenTiles) where they find enough work (whole tiles for
 // at least half of the clusters, or, where K may be cut into ranges, at least 8 tiles), else the swapped kernel up
-// to 256 tokens and single blocks on 128 x 256 tiles above.  129 to 256 tokens (one row of 256-token tiles; a third and
-// fourth token tile of the swapped kernel would read every weight tile from L2 again: measured at 256 tokens, 8B
-// sizes q‖k‖v 26 -> 21 us, gate‖up 75 -> 51, down 37 -> 29; 14B sizes gate‖up 127 -> 79, down 88 -> 48; at 128 tokens
-// the swapped kernel is still ahead).  257 to 511 tokens (a third or fourth 128-token tile that pairs round up to 512):
-// pairs when the single blocks would have fewer tiles than SMs (their shared K blocks cost more than the pairs' K
-// ranges: at 320 to 448 tokens q‖k‖v 33-40 -> 28-29 us, o 33-36 -> 20, down 54-78 -> 42-44), and otherwise when the
-// pairs' rounds of tiles, the last one counted by what sharing it out leaves of it, are no more than the single
-// blocks' (gate‖up at 320 and 384 tokens: 288 tiles are two rounds of single blocks = 67-69 us, 192 tiles 2.6 rounds
-// of pairs = 79-81 us; at 448 tokens three rounds either way, 88 against 83 us).  From 512 tokens on: pairs.
+// to 256 tokens and single blocks on 128 x 256 tiles above.  129 to 256 tokens (one token tile of the pairs; a third and
+// fourth token tile of the swapped kernel would read every weight tile from L2 again: when the pairs' tiles still held 256 tokens always,
+// q‖k‖v of the 8B sizes took 26 us on the swapped kernel and 21 on pairs at 256 tokens, gate‖up 75 and 51, down 37 and 29; since then 129 tokens 14, 43 and
+// 28 on pairs, 256 tokens 16, 53 and 33; at 128 tokens the swapped kernel is still ahead).  257 to 384 tokens are three tiles of 128 rows on single blocks and two
+// of 129 to 192 on pairs, so that a round of pairs costs less than one of single blocks, and their last round is shared out: pairs take it up to
+// 1.15 of the single blocks' rounds.  Measured, rounds of pairs (tiles over clusters) over rounds of single blocks, then single blocks / pairs at 257, 320 and
+// 384 tokens in us: 28,672 x 4,096 SwiGLU 1.01, 106 / 97, 96 / 86, 97 / 88; 51,200 x 5,120 SwiGLU 1.08, 194 / 190, 201 / 193, 204 / 194; 40,960 x 2,048 SwiGLU 1.08, 75 / 76,
+// 60 / 58, 69 / 69; 32,000 x 4,096 1.13, 122 / 121, 100 / 93, 109 / 102; 34,816 x 5,120 SwiGLU 1.23, 113 / 113, 122 / 134, 127 / 137; 151,936 x 4,096 1.23, 384 tokens 490 / 512;
+// 24,576 x 4,096 SwiGLU 1.30, 68 / 78, 71 / 82, 66 / 73.  385 to 511 tokens have four rows of single blocks' tiles and as few of the pairs': 16,384 to 51,200
+// rows 0.71 to 0.96 of the time on pairs.  From 512 tokens on: pairs.
 Kind choose_kind(int M, int N, bool may_split)
 {
     if (M <= 2 * 64) return SWAPPED;
     const Kind other = M <= 256 ? SWAPPED : SINGLE;
     if (!pair_kernel_enabled()) return other;
-    const int sms = spy_sm_count();
+    const long long sms = spy_sm_count(), clusters = sms / 2;
     const long long y_tiles = (N + 255) / 256;
     const long long tiles1 = (long long)((M + BM - 1) / BM) * y_tiles, tiles2 = (long long)((M + 2 * BM - 1) / (2 * BM)) * y_tiles;
     if (!(tiles2 >= pair_min_tiles() || (may_split && tiles2 >= 8))) return other;
-    if (M <= 256 || M >= 512 || tiles1 < sms) return PAIRS;
-    const long long clusters = sms / 2;
-    const long long r1 = (tiles1 + sms - 1) / sms;
-    const long long r2 = (tiles2 * 10 - 3 * clusters + 10 * clusters - 1) / (10 * clusters);   // ceil(tiles2 / clusters - 0.3)
-    return r2 <= r1 ? PAIRS : SINGLE;
+    if (M <= 256 || M >= 512) return PAIRS;
+    const long long rounds1 = (tiles1 + sms - 1) / sms;
+    return 20 * tiles2 <= 23 * clusters * rounds1 ? PAIRS : SINGLE;
 }
 
 Plan make_plan(int M, int N, int K, bool may_split)
@@ -1383,7 +1382,7 @@ Plan make_plan(int M, int N, int K, bool may_split)
     const int k_blocks = (K + BK - 1) / BK;
     Plan best = {1, BM, choose_kind(M, N, may_split)};
     if (best.kind == PAIRS && may_split) {
-        // a few hundred tokens on pairs of blocks: with too few 256 x 256 tiles for the clusters (o and down at the 8B
+        // a few hundred tokens on pairs of blocks: with too few tiles for the clusters (o and down at the 8B
         // shape: 32), K is cut into two to four ranges, so that tiles x ranges occupy most of the clusters (SMs / 2); the
         // partial tiles are summed by the caller or by the reduce kernel.  At least 16 K blocks a range.
         const long long tiles = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
@@ -1489,10 +1488,10 @@ static int run_gemm_tcgen05(const void* A, long long lda, const void* W, long lo
     const long long ld = splits > 1 ? N : ldc;
     const long long split_stride = splits > 1 ? (long long)M * N : 0;
     const bool f32_out = splits > 1 || c_dtype == SPY_F32;
-    // pairs need enough 256 x 256 tiles to occupy at least half of the clusters; smaller products go to single
+    // pairs need enough tiles to occupy at least half of the clusters; smaller products go to single
     // blocks, which share the K blocks of their 128 x 256 tiles out over all SMs
     if (plan.kind == PAIRS) {
-        // many tokens, one pass over K, at least two 256-row tiles: pairs of blocks on 256 x 256 tiles
+        // many tokens: pairs of blocks on tiles of 256 weight rows and even heights of tokens
         const TokenTiles tokens = token_tiles(M);
         if (make_map(&mx, W, N, K, ldw, BM) || make_map(&my, A, M, K, lda, tokens.rows / 2)) return 1;
         const long long num_tiles = (long long)((N + 2 * BM - 1) / (2 * BM)) * tokens.count;

@@ -700,7 +700,7 @@ def test_sampling_top_k_draws_only_among_the_largest():
                                    (2048, 4096, 512), (1500, 3000, 264), (4100, 2600, 72)])
 def test_gemm_tcgen05(out_dtype, M, N, K):
     """Tensor-core product at sizes that exercise every tile class (16/32/64/128 tokens swapped, one and two
-    token tiles; pairs with one row of 256 x 256 tiles, with and without K ranges; 128 x 256 tiles), tails in M, N and K, split-K, and the persistent kernel with one, two and
+    token tiles; pairs with one row of tiles, with and without K ranges; 128 x 256 tiles), tails in M, N and K, split-K, and the persistent kernel with one, two and
     several tiles per block."""
     from spyinfer_b200 import kernels
     torch.manual_seed(M * 7 + N)
@@ -869,7 +869,7 @@ def test_attention_mma_finds_one_far_key(split_keys):
 
 
 @pytest.mark.parametrize("M,N,K,epilogue,out_dtype", [
-    (2048, 4096, 4096, None, torch.bfloat16),        # 128 tiles of 256 x 256 on 74 clusters: 54 tail tiles (the o projection at 2,048 tokens)
+    (2048, 4096, 4096, None, torch.bfloat16),        # 128 tiles on 74 clusters: 54 tail tiles (the o projection at 2,048 tokens)
     (2048, 6144, 4096, None, torch.float32),         # 192 tiles: 44 tail tiles
     (1500, 5000, 1032, None, torch.bfloat16),        # tails in M, N and K as well: 6 x 20 tiles, 17 K blocks with 8 columns in the last
     (2048, 5120, 8192, None, torch.bfloat16),        # 160 tiles: 12 tail tiles of 128 K blocks, shared by default (the o projection of the 32B shape)
@@ -877,7 +877,7 @@ def test_attention_mma_finds_one_far_key(split_keys):
     (2048, 3328, 2048, None, torch.float32),         # 104 tiles: 30 tail tiles, two main clusters a tile and 14 helpers with three turns each
 ])
 def test_gemm_tcgen05_shares_the_last_round_of_tiles(M, N, K, epilogue, out_dtype, monkeypatch):
-    """Many tokens on pairs of blocks: when the last round of 256 x 256 tiles would leave clusters idle,
+    """Many tokens on pairs of blocks: when the last round of tiles would leave clusters idle,
     the K blocks of its tiles are shared out over all clusters and the partial tiles are summed by the
     block that arrives last.  The result is the one of whole tiles (same products, sums in K order),
     against a 32-bit reference, twice in a row (the arrival counters return to zero by themselves).
@@ -911,6 +911,27 @@ def test_gemm_tcgen05_shares_the_last_round_of_tiles(M, N, K, epilogue, out_dtyp
         assert (outs[0].float() - outs[2].float()).abs().max().item() <= 2.0 ** -6 * max(1.0, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("epilogue", [None, "swiglu"])
+@pytest.mark.parametrize("M,N", [(257, 32000), (384, 51200), (320, 34816), (384, 24576)])
+def test_gemm_tcgen05_of_some_hundred_tokens_on_both_sides_of_the_kernels_line(M, N, epilogue, monkeypatch):
+    """257 to 384 tokens by many weight rows: the pairs of blocks up to 1.15 of the single blocks' rounds (the first two), single blocks
+    beyond; the kernel that is taken and the single blocks against a 32-bit reference and one another."""
+    from spyinfer_b200 import kernels
+    torch.manual_seed(M + N)
+    K = 136
+    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV) / math.sqrt(K)).to(torch.bfloat16)
+    ref = a.float() @ w.float().t()
+    if epilogue:
+        ref = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
+    outs = []
+    for pairs in ("1", "0"):
+        monkeypatch.setenv("SPYINFER_GEMM_PAIRS", pairs)
+        outs.append(kernels.gemm_tcgen05(a, w, epilogue=epilogue))
+        torch.testing.assert_close(outs[-1].float(), ref.to(torch.bfloat16).float(), rtol=1.6e-2, atol=2e-3)
+    assert torch.equal(outs[0], outs[1])                     # one pass over K on both: the same sums
+
+
 @pytest.mark.parametrize("epilogue,out_dtype", [(None, torch.bfloat16), (None, torch.float32), ("swiglu", torch.bfloat16), ("relu2", torch.bfloat16)])
 @pytest.mark.parametrize("M", [129, 160, 161, 257, 320, 513, 545, 800, 1025])
 def test_gemm_tcgen05_cuts_many_tokens_into_tiles_of_several_heights(M, epilogue, out_dtype):
@@ -937,7 +958,7 @@ def test_gemm_tcgen05_cuts_many_tokens_into_tiles_of_several_heights(M, epilogue
 
 
 @pytest.mark.parametrize("M,I,K", [(3, 100, 64), (16, 328, 200), (40, 1000, 136), (64, 6144, 512), (70, 520, 264), (128, 12288, 1024), (130, 520, 264), (300, 12288, 1024),
-                                   (520, 1000, 136), (1100, 2304, 512)])   # 512 rows and more: pairs of blocks on 256 x 256 tiles
+                                   (520, 1000, 136), (1100, 2304, 512)])   # 512 rows and more: pairs of blocks on tiles of 256 weight rows and up to 256 tokens
 def test_gemm_tcgen05_swiglu_epilogue(M, I, K):
     """Gate and up rows interleaved in the weight; the product's epilogue applies SwiGLU."""
     from spyinfer_b200 import kernels
@@ -982,7 +1003,7 @@ def test_gemm_tcgen05_shares_k_blocks_evenly(M, N, K, epilogue, monkeypatch):
                                    (512, 4096, 4096), (600, 3000, 4096), (700, 1500, 12288)])
 def test_gemm_tcgen05_deferred_reduction(M, N, K):
     """With defer=True a split-K product hands back its partial products; their sum is the product.  The last three
-    are 512 tokens and more with too few 256 x 256 tiles for the pairs of blocks: K is cut into two to four ranges
+    are 512 tokens and more with too few tiles for the pairs of blocks: K is cut into two to four ranges
     (32 tiles x 2, 36 x 2 with tails in both directions, 18 x 4)."""
     from spyinfer_b200 import kernels
     a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
