@@ -573,10 +573,13 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 // 64 tokens at 128 x 16 takes 4.5 us, its 330 K additions 1.4, its shared-memory reads about 2); the token-by-token kernel above
 // spends 270 to 300 ns a token on one request, nearly all of it waiting.  Measured, chunks' kernels and walk together (us, by tokens before / in chunks):
 //   matrix memory, 8 heads of 128 x 256: one request of 256 tokens 76 / 38, of 2,047 567 / 176; 8 of 100 to 400 460 / 233; 16 of 1,024 2,581 / 1,495;
-//   delta rule, 32 heads of 64: one request of 256 79 / 49, of 2,047 607 / 297; two of 1,024 385 / 300;
-//   linear attention, 16 heads of 128 x 256: one of 256 101 / 70, of 2,047 774 / 372; 8 of 100 to 400 704 / 475; 16 of 1,024 4,094 / 2,967.
-// Error against 64 bits over some hundred tokens (2-norm): matrix memory half of the walk's by tokens (2.0e-5 and 9.7e-6, its divisions), linear attention
-// 1.75e-7 and 1.9e-7, delta rule 1.1e-7 and 1.8e-7: all sums stay in 32-bit, products of decays are taken in 64-bit and rounded once.
+//   delta rule, 32 heads of 64: one request of 256 79 / 50, of 2,047 610 / 351; two of 1,024 385 / 353;
+//   linear attention, 16 heads of 128 x 256: one of 256 103 / 71, of 2,047 777 / 378; 8 of 100 to 400 632 / 445; 16 of 1,024 4,109 / 2,988.
+// Error against 64 bits, tokens / chunks, 2,047 tokens (2-norm; matrix memory: the median token's): matrix memory of 128 x 48 1.85e-7 / 1.12e-7, linear attention 1.73e-7 /
+// 1.70e-7 (decays near nothing 1.03e-7 / 0.94e-7), delta rule 1.04e-7 / 0.99e-7 (1.13e-7 / 1.08e-7).  What is summed into a chunk's factors is what counts:
+// with the delta rule's 64-term sums and the linear attention's sums inside sub-blocks in 32-bit, and chains of 128 terms between sub-blocks, the chunks'
+// errors were 1.74e-7 and 2.02e-7.  So those sums are taken in 64-bit (delta rule of 2,047 tokens 298 us with 32-bit ones, 351 now; linear attention 373
+// and 378) or in short chains; products of decays are taken in 64-bit and rounded once; all else is in 32-bit.
 //
 // Which form a request takes is decided on the device by one rule (takes_chunks) in both kernels: runs of fewer than chunk_min tokens and
 // requests with a number among their q, k, v, decays or gates that is not below HUGE_INPUT in magnitude (or is no number) are walked token
@@ -713,9 +716,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
     }
     const int any = __syncthreads_or(bad);
     if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
-    // P: a thread has 4 x 4 of the 64 x 64, rows 4 ty + i, columns tx + 16 j
+    // P: a thread has 4 x 4 of the 64 x 64, rows 4 ty + i, columns tx + 16 j, each in two chains of sums
     const int tx = tid & 15, ty = tid >> 4;
-    float acc[4][4] = {};
+    float acc[4][4] = {}, acc2[4][4] = {};
     for (int c = 0; c < DK; c += 4) {
         float4 kk[4];
 #pragma unroll
@@ -724,7 +727,10 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
         for (int i = 0; i < 4; ++i) {
             const float4 qq = ld4(q_s + (4 * ty + i) * LD + c);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = dot4(qq, kk[j], acc[i][j]);
+            for (int j = 0; j < 4; ++j) {
+                acc[i][j] = fmaf(qq.x, kk[j].x, fmaf(qq.y, kk[j].y, acc[i][j]));
+                acc2[i][j] = fmaf(qq.z, kk[j].z, fmaf(qq.w, kk[j].w, acc2[i][j]));
+            }
         }
     }
 #pragma unroll
@@ -734,7 +740,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int s = tx + 16 * j;
-            const float p = s <= t ? expf((float)(to_s[t] + from_s[s])) * (acc[i][j] * a.q_scale) : 0.f;
+            const float p = s <= t ? expf((float)(to_s[t] + from_s[s])) * ((acc[i][j] + acc2[i][j]) * a.q_scale) : 0.f;
             P[t * C + s] = p;
             row += p;
         }
@@ -799,20 +805,23 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
                 }
             }
         }
-        // the sixteen sums over the warp together: with every step a lane keeps half of its sums
+        // the sixteen sums over the warp together, in 64-bit: with every step a lane keeps half of its sums
         int mine = 0;
+        double wide[B];
+#pragma unroll
+        for (int i = 0; i < B; ++i) wide[i] = d[i];
 #pragma unroll
         for (int o = 16, n = B / 2; n > 0; o >>= 1, n >>= 1) {
             const bool up = (lane & o) != 0;
 #pragma unroll
             for (int i = 0; i < n; ++i) {
-                const float own = up ? d[i + n] : d[i], give = up ? d[i] : d[i + n];
-                d[i] = own + __shfl_xor_sync(0xffffffffu, give, o);
+                const double own = up ? wide[i + n] : wide[i], give = up ? wide[i] : wide[i + n];
+                wide[i] = own + __shfl_xor_sync(0xffffffffu, give, o);
             }
             mine += up ? n : 0;
         }
-        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
-        if ((lane & 1) == 0) P[(b0 + mine) * C + s] = d[0] * a.q_scale;       // zero above the diagonal
+        wide[0] += __shfl_xor_sync(0xffffffffu, wide[0], 1);
+        if ((lane & 1) == 0) P[(b0 + mine) * C + s] = (float)(wide[0] * a.q_scale);       // zero above the diagonal
     }
     for (int idx = tid; idx < C * C; idx += THREADS)
         if ((idx & (C - 1)) / B > idx / C / B) P[idx] = 0.f;
@@ -838,16 +847,22 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     // and the columns tid % 16 + 16 j.
     for (int b = 1; b < C / B; ++b) {
         const int t = b * B + (tid >> 4), s0 = tid & 15;
-        float acc[C / B - 1] = {};
+        float acc[C / B - 1][4] = {};              // four short chains of sums instead of one of DK terms
         for (int c = 0; c < DK; c += 4) {
             const float4 qq = ld4(q_s + t * LD + c);
 #pragma unroll
             for (int j = 0; j < C / B - 1; ++j)
-                if (j < b) acc[j] = dot4(qq, ld4(k_s + (s0 + 16 * j) * LD + c), acc[j]);
+                if (j < b) {
+                    const float4 kk = ld4(k_s + (s0 + 16 * j) * LD + c);
+                    acc[j][0] = fmaf(qq.x, kk.x, acc[j][0]);
+                    acc[j][1] = fmaf(qq.y, kk.y, acc[j][1]);
+                    acc[j][2] = fmaf(qq.z, kk.z, acc[j][2]);
+                    acc[j][3] = fmaf(qq.w, kk.w, acc[j][3]);
+                }
         }
 #pragma unroll
         for (int j = 0; j < C / B - 1; ++j)
-            if (j < b) P[t * C + s0 + 16 * j] = acc[j];
+            if (j < b) P[t * C + s0 + 16 * j] = (acc[j][0] + acc[j][1]) + (acc[j][2] + acc[j][3]);
         __syncthreads();
         for (int idx = tid; idx < b * B * DK; idx += THREADS) {
             const int s = idx / DK, c = idx - s * DK;
@@ -870,13 +885,13 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     }
 }
 
-__global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
+__global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
 {
-    constexpr int C = 32, D = 64, LD = D + 4, R = D + C, LDM = R + 4;
+    constexpr int C = 32, D = 64, LD = D + 2, R = D + C, LDM = R + 4;
     extern __shared__ __align__(16) float sm[];
-    float* pg = sm;                    // [2 C][LD]: p, then g (first: q)
-    float* bc = pg + 2 * C * LD;       // [2 C][LD]: b, then c (first: the rates, k)
-    float* PM = bc + 2 * C * LD;       // [C][LDM]: P' | M' (first: the decays)
+    double* pg = reinterpret_cast<double*>(sm);   // [2 C][LD]: p, then g (first: q)
+    double* bc = pg + 2 * C * LD;      // [2 C][LD]: b, then c (first: the rates, k)
+    float* PM = reinterpret_cast<float*>(bc + 2 * C * LD);   // [C][LDM]: P' | M' (first: the decays)
     float* XB = PM + C * LDM;          // [C][LDM]: token s: X_ts of the outputs t, then b_s of the state's rows
     float* L = XB + C * LDM;           // [C][C + 1]
     float* Y = L + C * (C + 1);        // [C][C + 1]
@@ -888,26 +903,30 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
     const ScanArgs& a = A.s;
     float* W = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(1, D);
     const float* rows = a.proj + (size_t)t0 * a.ld;
-    bool bad = load_rows<C, D, LD>(pg + C * LD, rows + a.off_q + h * D, a.ld, n_tok);
-    bad |= load_rows<C, D, LD>(bc + C * LD, rows + a.off_k + h * D, a.ld, n_tok);
-    bad |= huge_values(a, h, t0, n_tok);
+    bool bad = huge_values(a, h, t0, n_tok);
+#pragma unroll 4
     for (int idx = tid; idx < C * D; idx += THREADS) {
         const int t = idx / D, c = idx - t * D;
-        float rate = 0.f, w = 1.f;
+        float q = 0.f, k = 0.f, rate = 0.f, w = 1.f;
         if (t < n_tok) {
-            const float x1 = rows[(size_t)t * a.ld + a.off_x1 + h * D + c] + a.bias1[h * D + c];
+            const float* row = rows + (size_t)t * a.ld + h * D + c;
+            q = row[a.off_q];
+            k = row[a.off_k];
+            const float x1 = row[a.off_x1] + a.bias1[h * D + c];
             const float x2 = a.extra[(size_t)(t0 + t) * a.H * D + h * D + c] + a.bias2[h * D + c];
-            bad |= isnan(x1) || isnan(x2);
+            bad |= huge(q) | huge(k) | isnan(x1) | isnan(x2);
             rate = sigmoidf_(x1);
             w = expf(-0.60653065971263342f * sigmoidf_(x2));     // exp(-1/2) = 0.6065...
         }
+        pg[(C + t) * LD + c] = q;
+        bc[(C + t) * LD + c] = k;
         bc[t * LD + c] = rate;
         PM[t * LDM + c] = w;
     }
     const int any = __syncthreads_or(bad);
     if (tid == 0) A.flags[(size_t)blockIdx.x * a.H + h] = any;
     for (int t = warp; t < C; t += THREADS / 32) {
-        const float k0 = bc[(C + t) * LD + lane], k1 = bc[(C + t) * LD + lane + 32];
+        const float k0 = (float)bc[(C + t) * LD + lane], k1 = (float)bc[(C + t) * LD + lane + 32];
         const float sq = warp_sum(k0 * k0 + k1 * k1);
         if (lane == 0) inv_s[t] = 1.0f / sqrtf(sq + 1e-6f);
     }
@@ -917,11 +936,11 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
         float run = 1.f;
 #pragma unroll 8
         for (int t = 0; t < C; ++t) {
-            const float k = bc[(C + t) * LD + tid], u = k * inv_s[t], rate = bc[t * LD + tid];
+            const float k = (float)bc[(C + t) * LD + tid], u = k * inv_s[t], rate = (float)bc[t * LD + tid];
             pg[t * LD + tid] = u * run;
             product *= PM[t * LDM + tid];
             run = (float)product;
-            pg[(C + t) * LD + tid] *= run;
+            pg[(C + t) * LD + tid] = (float)pg[(C + t) * LD + tid] * run;
             const float b = rate * u / run;
             bc[t * LD + tid] = b;
             bc[(C + t) * LD + tid] = k / run;
@@ -931,18 +950,24 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
     }
     __syncthreads();
     {
-        // [p; g] [b; c]^T, 64 x 64: rows 4 ty + i, columns tx + 16 j
+        // [p; g] [b; c]^T, 64 x 64, summed in 64-bit (what these sums round off, every output and the state carry on: with 32-bit sums the outputs' error
+        // was half as large again as the walk's by tokens): rows 4 ty + i, columns tx + 16 j; a warp whose rows are tokens below 16
+        // leaves out the columns of the later tokens
         const int tx = tid & 15, ty = tid >> 4;
-        float acc[4][4] = {};
-        for (int c = 0; c < D; c += 4) {
-            float4 kk[4];
+        const bool early = (ty & 7) < 4;
+        double acc[4][4] = {};
+#pragma unroll 2
+        for (int c = 0; c < D; c += 2) {
+            double2 kk[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) kk[j] = ld4(bc + (tx + 16 * j) * LD + c);
+            for (int j = 0; j < 4; ++j)
+                if (!early || (j & 1) == 0) kk[j] = *reinterpret_cast<const double2*>(bc + (tx + 16 * j) * LD + c);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 qq = ld4(pg + (4 * ty + i) * LD + c);
+                const double2 qq = *reinterpret_cast<const double2*>(pg + (4 * ty + i) * LD + c);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = dot4(qq, kk[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j)
+                    if (!early || (j & 1) == 0) acc[i][j] = fma(qq.x, kk[j].x, fma(qq.y, kk[j].y, acc[i][j]));
             }
         }
 #pragma unroll
@@ -950,7 +975,7 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int row = 4 * ty + i, s = (tx + 16 * j) & (C - 1), t = row & (C - 1);
-                const float v = acc[i][j];
+                const float v = (float)acc[i][j];
                 if (row < C) {
                     if (j < 2) L[t * (C + 1) + s] = s < t ? v : 0.f;
                     else PM[t * LDM + D + s] = s < t ? v : 0.f;
@@ -960,7 +985,7 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
                 }
             }
     }
-    for (int idx = tid; idx < C * D; idx += THREADS) PM[idx / D * LDM + idx % D] = pg[idx / D * LD + idx % D];     // the decays have been used
+    for (int idx = tid; idx < C * D; idx += THREADS) PM[idx / D * LDM + idx % D] = (float)pg[idx / D * LD + idx % D];     // the decays have been used
     __syncthreads();
     if (tid < R) {
         float x[C];
@@ -998,8 +1023,8 @@ __global__ void __launch_bounds__(THREADS, 3) chunk_delta_kernel(ChunkArgs A)
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
                 const int col = 6 * tx + j;
-                if (row < C) v[j] = (col < D ? pg[(C + row) * LD + col] : Y[row * (C + 1) + col - D]) - acc[i][j];
-                else v[j] = last_s[row - C] * ((col < D ? (row - C == col ? 1.f : 0.f) : bc[(C + col - D) * LD + row - C]) - acc[i][j]);
+                if (row < C) v[j] = (col < D ? (float)pg[(C + row) * LD + col] : Y[row * (C + 1) + col - D]) - acc[i][j];
+                else v[j] = last_s[row - C] * ((col < D ? (row - C == col ? 1.f : 0.f) : (float)bc[(C + col - D) * LD + row - C]) - acc[i][j]);
             }
 #pragma unroll
             for (int j = 0; j < 6; j += 2) *reinterpret_cast<float2*>(W + row * R + 6 * tx + j) = make_float2(v[j], v[j + 1]);
@@ -1017,16 +1042,14 @@ __device__ __forceinline__ void put_parts(float* red, int warp, int g, int cg, c
 template <int ROWS>
 __device__ __forceinline__ float4 sum_parts(const float* red, int row, int cg)
 {
-    float4 v = ld4(red + (size_t)row * WALK_COLS + 4 * cg);
+    float4 v[8];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) {
-        const float4 p = ld4(red + ((size_t)w * ROWS + row) * WALK_COLS + 4 * cg);
-        v.x += p.x;
-        v.y += p.y;
-        v.z += p.z;
-        v.w += p.w;
-    }
-    return v;
+    for (int w = 0; w < 8; ++w) v[w] = ld4(red + ((size_t)w * ROWS + row) * WALK_COLS + 4 * cg);
+#pragma unroll
+    for (int n = 4; n > 0; n >>= 1)              // as a tree: three roundings a number instead of seven
+#pragma unroll
+        for (int w = 0; w < n; ++w) v[w] = make_float4(v[w].x + v[w + n].x, v[w].y + v[w + n].y, v[w].z + v[w + n].z, v[w].w + v[w + n].w);
+    return v[0];
 }
 // acc[j][c] += sum over four k of x[row g + 8 j][k ..] * y[k ..][4 cg + c]; x rows LDX floats apart, y rows WALK_LD
 template <int NJ, int LDX>
@@ -1328,7 +1351,7 @@ template <int MODE> static int launch_chunks(ScanArgs& S, int tokens, int num_se
     int rc;
     if constexpr (MODE == 1) {
         constexpr int C = 32, D = 64, R = C + D;
-        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, (4 * C * (D + 4) + 2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
+        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, 4 * C * (D + 2) * sizeof(double) + (2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
         if (!rc) rc = launch_chunk_kernel(walk_delta_kernel, walk, DeltaSmem::BYTES, stream, A);
     } else {
         const size_t rows = (MODE == 0 ? 2 : 3) * 64 * (size_t)(S.dk + 4) * sizeof(float);

@@ -56,6 +56,15 @@ def exact(kind, dk, dv, x, pre, b1, b2):
     return torch.stack(out).reshape(-1, nv)
 
 
+def distance(kind, got, want, dv):
+    """Relative 2-norm.  The matrix memory's outputs are divided by a sum that nearly cancels at some tokens, whose errors would be all that the norm
+    shows: there the median of the tokens' own distances, each head's alone."""
+    if kind != "memory":
+        return float((got.double() - want).norm() / want.norm())
+    d, w = (got.double() - want).view(-1, dv), want.view(-1, dv)
+    return float((d.norm(dim=1) / w.norm(dim=1)).median())
+
+
 def run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad):
     """One step of several requests; ``pad`` columns ahead of q: with one, no row starts on a 16-byte border and every request is walked
     token by token."""
@@ -107,12 +116,23 @@ def test_chunks_carry_the_state_through_portions_as_the_walk_by_tokens_does(kind
                 got[r].append(part)
                 at[r] += step[r]
         assert bool((state[1] == 7.0).all())
-        errors[name] = max(float((torch.cat(got[r]).double() - want[r]).norm() / want[r].norm()) for r in range(4))
+        errors[name] = max(distance(kind, torch.cat(got[r]), want[r], dv) for r in range(4))
     print(f"\n  {kind} {dk} x {dv}{' hard' if hard else ''}: error against 64 bits {errors}")
-    # 32-bit sums of up to 128 terms over some hundred tokens: a few roundings of 6e-8 each; the matrix memory's outputs are also divided by a sum
-    # that may nearly cancel, which hurts both forms alike
-    assert errors["tokens"] < (3e-5 if kind == "memory" else 1e-6), errors
-    assert max(errors.values()) < 1.5 * errors["tokens"] + 1e-7, errors
+    # 32-bit sums of up to 128 terms over some hundred tokens: a few roundings of 6e-8 each.  The chunks may not be the less exact form: 1.03 is what
+    # the largest of four requests' errors, each over thousands of outputs, may scatter by
+    assert errors["tokens"] < 1e-6, errors
+    assert max(errors.values()) < 1.03 * errors["tokens"], errors
+
+
+@gpu
+@pytest.mark.parametrize("kind,dk,dv", CASES)
+def test_chunks_of_a_long_prompt_are_as_exact_as_the_walk_by_tokens(kind, dk, dv):
+    """2,047 tokens, 32 or 64 chunks of them: what one chunk rounds off does not grow through the others."""
+    x, pre, b1, b2 = inputs(kind, dk, dv, 2047, 3)
+    want = exact(kind, dk, dv, x, pre, b1, b2)
+    errors = [distance(kind, run(kind, dk, dv, [x], [pre], b1, b2, new_state(kind, dk, dv, 1), [0], pad), want, dv) for pad in (0, 1)]
+    print(f"\n  {kind} {dk} x {dv}, 2,047 tokens: error against 64 bits in chunks {errors[0]:.3g}, by tokens {errors[1]:.3g}")
+    assert errors[0] < 1.03 * errors[1], errors
 
 
 @gpu
