@@ -63,7 +63,7 @@ class StepBatch:
     #: not laid out that way): an attention part may run those through its kernel for decoding and the rest through the
     #: one for prompt portions
     one_token_head: int = 0
-    #: no request of the batch holds more than ``SHORT_CONTEXT`` keys after this step (a captured step is replayed only for batches that agree in this)
+    #: no request of the batch holds more than ``SHORT_CONTEXT`` keys after this step
     short_context: bool = False
     extras: Dict[str, object] = field(default_factory=dict)
 

@@ -55,6 +55,7 @@ class Model:
                 if self.stream_rows.setdefault(e.before.tensor, e.before.rows) != e.before.rows or not 0 <= e.before.row < e.before.rows:
                     raise ValueError(f"run order: the rows of the stream offset {e.before.tensor!r} do not agree")
         self.stream_tensors: Dict[str, torch.Tensor] = {}
+        self._choosing = None
         # projections of [stream; embedding output] that take the stream's place between layers
         self.stream_products: Dict[str, Optional[Linear]] = {e.before.tensor: None for e in spec.run_order if isinstance(e.before, StreamProject)}
         if self.stream_products and getattr(self.embedding, "pairs", None) is not None:
@@ -155,6 +156,12 @@ class Model:
         parts = self.parts()
         nested = [p.position for p in parts if getattr(p, "position", None) is not None]
         return all(p.graph_safe for p in parts + nested) and all(l.block.graph_safe for l in self.layers)
+
+    def choices(self, batch, page_size: int) -> tuple:
+        """What a batch's content, beside its padded sizes, decides about the launches (``Part.choice``)."""
+        if self._choosing is None:
+            self._choosing = list({(type(p), p.choice_sizes()): p for part in self.parts() for p in part.choosing()}.values())
+        return tuple(p.choice(batch, page_size) for p in self._choosing)
 
     # ---- cache needs -------------------------------------------------------------------------
     def cache_needs(self):

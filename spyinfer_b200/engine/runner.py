@@ -18,7 +18,7 @@ import torch
 from .. import kernels
 from ..cache import CacheManager
 from ..config.engine_config import EngineConfig
-from .batch import SHORT_CONTEXT, BatchStager, StepBatch, StepEntry
+from .batch import BatchStager, StepBatch, StepEntry
 from .model import Model
 
 
@@ -338,9 +338,11 @@ class ModelRunner:
                 sizes = padded_step_sizes(len(filled[1]), len(entries), wanted, self.config.max_num_seqs, self.stager.max_tokens,
                                           self.config.graph_step_tokens, head)
             if sizes is not None:
-                # what a part may choose its kernels by is in the key: the padded sizes and whether all contexts are short
-                kind = "short step" if int(filled[5].max()) <= SHORT_CONTEXT else "step"
-                logits = self._run_through_graph((kind,) + sizes, self._padded_batch(filled, head, *sizes))[:wanted]
+                batch = self._padded_batch(filled, head, *sizes)
+                # what the parts choose their launches by beside the padded sizes is in the key
+                choices = self.model.choices(batch, self.cache.page_size)
+                kind = " ".join(list(dict.fromkeys(c for c in choices if c)) + ["step"])
+                logits = self._run_through_graph((kind,) + sizes + choices, batch)[:wanted]
                 mixed = [k for k in self._graphs if isinstance(k, tuple)]
                 if len(mixed) > self.GRAPH_STEP_LIMIT:
                     del self._graphs[mixed[0]]

@@ -170,8 +170,25 @@ class Attention(Mixer):
         self.attend(q, out, batch, cache)
         return self.o(out, defer=self.defer_output)
 
-    #: query rows (tokens x heads) up to which prompts of short contexts go to the kernel of small tiles
-    SHORT_ROWS = 10240
+    #: query rows (tokens x heads) an SM up to which prompts of short contexts go to the kernel of small tiles (16 rows a block: about four blocks an SM;
+    #: us there / on blocks of 256 rows: five prompts of 64 tokens, 32 heads, 69 rows an SM 8.3 / 12.0; of 40 heads, 86 rows an SM, 12.9 / 12.8)
+    SHORT_ROWS = 70
+
+    def choosing(self):
+        return [self] if self.tc and self.mma else []
+
+    def choice_sizes(self):
+        return (self.nh, self.nkv, self.hd, bool(self.softcap or self.distance_bias or self.learned_sink))
+
+    def choice(self, batch, page_size):
+        return "short" if self.small_tiles(batch, page_size) else ""
+
+    def small_tiles(self, batch, page_size) -> bool:
+        """Whether a batch's prompts go to the kernel of small tiles (``attend``)."""
+        if not (batch.short_context and self.mma and self.tc and page_size in kernels.ATTENTION_TMA_PAGE_SIZES) or batch.one_token_head or batch.one_token_each \
+                or self.softcap or self.distance_bias or self.learned_sink:
+            return False
+        return batch.num_tokens * self.nh <= self.SHORT_ROWS * torch.cuda.get_device_properties(self.ctx.device).multi_processor_count
 
     def attend(self, q, out, batch, cache, out_scale=None):
         """The attention itself, ``q [T, >= nh hd]`` over the cache into ``out [T, nh hd]``, on the kernel that the sizes, the
@@ -192,10 +209,9 @@ class Attention(Mixer):
             kernels.attention_mma(q, self.nh, self.hd, out, cache.pages, cache.block_table, batch.positions, batch.q_start,
                                   batch.num_seqs, self.scale, window=self.key_mask, split_keys=split_keys, max_splits=max_splits,
                                   status=batch.status)
-        elif boxes and mma and batch.short_context and batch.one_token_head == 0 and batch.num_tokens * self.nh <= self.SHORT_ROWS:
+        elif boxes and mma and self.small_tiles(batch, cache.page_size):
             # a question's prompt: a block of 256 rows spends its time on the way to its first tile of 128 keys (one prompt of 16, 37, 64 and
-            # 100 tokens, 32 heads over 8, us: 7.8, 10.0, 11.4 and 11.3 there, 4.6, 6.0, 7.9 and 10.9 here; five of 64, 320 tokens: 12.0 and 8.3, of
-            # 40 heads 12.8 and 12.9)
+            # 100 tokens, 32 heads over 8, us: 7.8, 10.0, 11.4 and 11.3 there, 4.6, 6.0, 7.9 and 10.9 here)
             kernels.attention_mma(q, self.nh, self.hd, out, cache.pages, cache.block_table, batch.positions, batch.q_start,
                                   batch.num_seqs, self.scale, window=self.key_mask, status=batch.status)
         elif boxes:
@@ -252,6 +268,9 @@ class PooledWindowAttention(Attention):
         names = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight"}
         names.update(params.get("names") or {})
         self.names = names
+
+    def choosing(self):
+        return []                    # it has kernels of its own
 
     def weight_decls(self):
         p, nh, nkv, hd, H, n = self.prefix, self.nh, self.nkv, self.hd, self.hidden, self.names

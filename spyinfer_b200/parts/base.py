@@ -84,8 +84,8 @@ class Part:
     #: kernel modules (``csrc/<name>.cu``) this part launches; built before the first step
     kernel_modules: Sequence[str] = ()
     #: True when ``forward`` launches the same kernels with the same arguments for every batch of the same sizes
-    #: (tokens, requests, wanted rows): no look at the batch's content on the host, no wait for the device, no
-    #: allocation that outlives the call.  A model whose parts all say so has its small steps captured in CUDA
+    #: (tokens, requests, wanted rows) and the same ``choice``: no other look at the batch's content on the host, no wait for the
+    #: device, no allocation that outlives the call.  A model whose parts all say so has its small steps captured in CUDA
     #: graphs and replayed; one part that does not keeps the whole model on launches one by one.
     graph_safe: bool = False
 
@@ -110,6 +110,18 @@ class Part:
 
     def modules(self) -> List[str]:
         return list(self.kernel_modules)
+
+    def choosing(self) -> List["Part"]:
+        """The parts (this one, or those it is made of) that launch other kernels, or with other arguments, for batches of the same padded
+        sizes: a graph of such a step is captured for every answer of their ``choice``.  Parts of equal ``choice_sizes`` answer alike."""
+        return []
+
+    def choice_sizes(self):
+        raise NotImplementedError
+
+    def choice(self, batch, page_size: int) -> str:
+        """What the batch's content decides: a word for it, empty for what is usual."""
+        raise NotImplementedError
 
     def linears(self) -> List:
         """The part's ``Linear`` products in the order ``forward`` runs them (the model tells each

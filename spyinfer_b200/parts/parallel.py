@@ -56,6 +56,9 @@ class ParallelMixers(Mixer):
     def modules(self):
         return ["residual_norm" if self.out_norm is not None else "layernorm"] + self.left.modules() + self.right.modules()
 
+    def choosing(self):
+        return self.left.choosing() + self.right.choosing()
+
     def linears(self):
         return self.left.linears() + self.right.linears()
 

@@ -339,6 +339,39 @@ def test_small_steps_with_decode_kernel_requests_replayed_from_graphs(tiny_model
         np.testing.assert_allclose(outs[0][k][1], ref_new[-1], rtol=3e-2, atol=5e-2 * scale)
 
 
+@pytest.mark.parametrize("dtype,heads,page_size,beside,graphs", [("bfloat16", 4, 16, 0, 2), ("bfloat16", 4, 16, 4, 1), ("bfloat16", 4, 4, 0, 1), ("bfloat16", 400, 16, 0, 1),
+                                                                   ("float32", 4, 16, 0, 1)])
+def test_steps_of_short_contexts_have_graphs_of_their_own_only_where_another_kernel_takes_them(dtype, heads, page_size, beside, graphs):
+    """The same padded sizes with contexts below and above the length up to which another attention kernel is taken: two graphs where it is, one
+    where the kernels are the same (32-bit, pages that are no box of a copy, too many rows, requests that decode beside the portion)."""
+    from spyinfer_b200 import config_from_json
+    from spyinfer_b200.config import EngineConfig
+    from spyinfer_b200.engine import StepEntry
+    from spyinfer_b200.engine.model import Model
+    from spyinfer_b200.engine.runner import ModelRunner
+
+    cfg = {"architectures": ["Qwen3ForCausalLM"], "num_hidden_layers": 1, "hidden_size": 128, "num_attention_heads": heads, "num_key_value_heads": heads // 2,
+           "head_dim": 64, "intermediate_size": 256, "vocab_size": 200, "rope_theta": 10000.0, "rms_norm_eps": 1e-6, "tie_word_embeddings": False,
+           "max_position_embeddings": 512, "eos_token_id": -1}
+    spec = config_from_json(cfg).to_spec()
+    config = EngineConfig(dtype=dtype, max_num_seqs=8, max_model_len=256, kvcache_block_size=page_size, num_kvcache_blocks=200, max_num_batched_tokens=256)
+    config.clamp_to_model(spec.max_position)
+    model = Model(spec, torch.float32 if dtype == "float32" else torch.bfloat16, config.device, config.max_model_len)
+    model.init_random(1)
+    runner = ModelRunner(model, config)
+    others = [f"o{i}" for i in range(beside)]
+    if others:
+        runner.step([StepEntry(r, [3], []) for r in others])
+    before = len(runner._graphs)
+    for cached in (0, 100):
+        if cached:
+            runner.step([StepEntry("long", [5] * cached, [])])       # nothing wanted: not through a graph
+        for _ in range(2):
+            runner.step([StepEntry(r, [7], [0]) for r in others] + [StepEntry("long" if cached else "short", [9] * 20, [19])])
+        runner.finish("short")
+    assert len(runner._graphs) - before == graphs, list(runner._graphs)
+
+
 @pytest.mark.parametrize("heads", [4, 16])
 def test_prompts_of_short_contexts_and_of_longer_ones_in_the_same_padded_sizes(heads):
     """Portions around the context up to which another attention kernel is taken, in steps that are padded to the same sizes: first short
