@@ -15,7 +15,8 @@
 // what another writes, whenever their blocks happen to run).  Two kernels: one for steps with prompt portions (scan_kernel),
 // whose arithmetic for a token does not depend on where a portion starts or ends, and one for steps in which every request
 // brings one token (scan_decode_kernel: `longest` = 1), whose sums over a column's rows run in another order.  Long portions are taken in
-// chunks of tokens instead (see "runs of tokens as products"), whose results depend on where a portion starts to a few roundings of 32 bits.
+// chunks of tokens instead (see "runs of tokens as products"), whose results depend on where a portion starts, and on whether the other long requests of
+// its step let it take chunks, to a few roundings of 32 bits.
 //
 // Inputs are columns of one 32-bit activation matrix `proj` [T, ld] (the fused projection of the mixer's input).
 #include "common.cuh"
@@ -57,19 +58,26 @@ struct ScanArgs {
 };
 
 // Which form a request takes where both run: see "runs of tokens as products" below.
-// The least tokens: where the forms meet for one request (us, tokens / chunks: matrix memory of 4 heads, 80 tokens 22 / 27, 100 27 / 27, 128 32 / 27; delta rule
-// of 32 heads, 100 tokens 34 / 38, 128 41 / 36; linear attention of 8 heads, 128 tokens 39 / 46, 256 72 / 54).
+// In a step that takes chunks every request of chunk_min tokens and more does.  A step takes them for two such requests, or for one of chunk_alone tokens: a
+// little above where the forms meet for one request (us, tokens / chunks: matrix memory of 4 heads, 96 tokens 26 / 28, 112 30 / 28, 128 33 / 28; delta rule of 32
+// heads, 100 tokens 34 / 43, 128 42 / 42, 160 51 / 44; linear attention of 8 heads, 160 tokens 48 / 52, 192 56 / 52, 256 73 / 56).
 __host__ __device__ constexpr int chunk_min(int mode) { return mode == 0 ? 96 : (mode == 1 ? 128 : 160); }
+__host__ __device__ constexpr int chunk_alone(int mode) { return mode == 0 ? 112 : (mode == 1 ? 128 : 192); }
 template <int MODE> struct ChunkOf { static constexpr int C = MODE == 1 ? 32 : 64; };   // tokens of a chunk
-// A chunk's place in the scratch: chunk j of sequence s at q_start[s] / C + s + j, which no two chunks share.
-__device__ __forceinline__ int chunk_slot(int t_begin, int seq, int C) { return t_begin / C + seq; }
+// The place in the scratch of the first chunk of a request that starts at token t: its chunks take the places from there on.  The places run ahead of
+// the chunks by a factor with which requests of chunk_min tokens and more never meet, however many shorter ones lie between them:
+// floor(n f) is at least the n / C chunks, rounded up, of n tokens (f C = 3/2, 5/4 and 4/3).
+__host__ __device__ constexpr int chunk_slot(int mode, int t)
+{
+    return (int)(mode == 0 ? 3LL * t / (2 * 64) : (mode == 1 ? 5LL * t / (4 * 32) : 4LL * t / (3 * 64)));
+}
 // Whether head h of a request takes the products: every block that asks gets the same answer.
 template <int MODE>
-__device__ __forceinline__ bool takes_chunks(const ScanArgs& A, int seq, int h, int t_begin, int t_end)
+__device__ __forceinline__ bool takes_chunks(const ScanArgs& A, int h, int t_begin, int t_end)
 {
     constexpr int C = ChunkOf<MODE>::C;
     if (A.flags == nullptr || t_end - t_begin < chunk_min(MODE)) return false;
-    const int first = chunk_slot(t_begin, seq, C), n = (t_end - t_begin + C - 1) / C;
+    const int first = chunk_slot(MODE, t_begin), n = (t_end - t_begin + C - 1) / C;
     int bad = 0;
     for (int j = threadIdx.x; j < n; j += blockDim.x) bad |= A.flags[(size_t)(first + j) * A.H + h];
     return __syncthreads_or(bad) == 0;
@@ -114,7 +122,7 @@ __global__ void __launch_bounds__(THREADS, NR <= 8 ? 2 : 1) scan_kernel(ScanArgs
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col = warp * CW + lane % CW, rg = lane / CW, r0 = rg * NR;
     const int t_begin = A.q_start[seq], t_end = A.q_start[seq + 1];
-    if (t_begin >= t_end || takes_chunks<MODE>(A, seq, h, t_begin, t_end)) return;
+    if (t_begin >= t_end || takes_chunks<MODE>(A, h, t_begin, t_end)) return;
     const int slot = A.state_slot[seq];
     if (slot < 0 || slot >= A.num_slots) {
         if (tid == 0) report_status(A.status, SPY_STATUS_BAD_PAGE, t_begin);
@@ -573,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 // 64 tokens at 128 x 16 takes 4.5 us, its 330 K additions 1.4, its shared-memory reads about 2); the token-by-token kernel above
 // spends 270 to 300 ns a token on one request, nearly all of it waiting.  Measured, chunks' kernels and walk together (us, by tokens before / in chunks):
 //   matrix memory, 8 heads of 128 x 256: one request of 256 tokens 76 / 38, of 2,047 567 / 176; 8 of 100 to 400 460 / 233; 16 of 1,024 2,581 / 1,495;
-//   delta rule, 32 heads of 64: one request of 256 79 / 50, of 2,047 610 / 351; two of 1,024 385 / 353;
+//   delta rule, 32 heads of 64: one request of 256 79 / 50, of 2,047 610 / 351; 16 heads 80 / 49 and 614 / 250;
 //   linear attention, 16 heads of 128 x 256: one of 256 103 / 71, of 2,047 777 / 378; 8 of 100 to 400 632 / 445; 16 of 1,024 4,109 / 2,988.
 // Error against 64 bits, tokens / chunks, 2,047 tokens (2-norm; matrix memory: the median token's): matrix memory of 128 x 48 1.85e-7 / 1.12e-7, linear attention 1.73e-7 /
 // 1.70e-7 (decays near nothing 1.03e-7 / 0.94e-7), delta rule 1.04e-7 / 0.99e-7 (1.13e-7 / 1.08e-7).  What is summed into a chunk's factors is what counts:
@@ -581,9 +589,10 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 // errors were 1.74e-7 and 2.02e-7.  So those sums are taken in 64-bit (delta rule of 2,047 tokens 298 us with 32-bit ones, 351 now; linear attention 373
 // and 378) or in short chains; products of decays are taken in 64-bit and rounded once; all else is in 32-bit.
 //
-// Which form a request takes is decided on the device by one rule (takes_chunks) in both kernels: runs of fewer than chunk_min tokens and
-// requests with a number among their q, k, v, decays or gates that is not below HUGE_INPUT in magnitude (or is no number) are walked token
-// by token as before: in the products an infinity of a later token would meet the zeros of an earlier one.
+// Which form a request takes in a step that takes chunks (chunk_work_floats) is decided on the device, head by head, by one rule (takes_chunks) in both
+// kernels: runs of fewer than chunk_min tokens, and heads of a request with a number among their q, k and v that is not below HUGE_INPUT in magnitude
+// or with a NaN among these or their gates and decays (whose infinities saturate), are walked token by token: in the products an infinity of a
+// later token would meet the zeros of an earlier one.
 constexpr float HUGE_INPUT = 1e10f;
 constexpr int WALK_COLS = 16;          // value columns a block of the walk owns
 constexpr int WALK_LD = WALK_COLS + 4; // floats between the rows of a tile of them in shared memory
@@ -601,22 +610,39 @@ __host__ __device__ constexpr int chunk_floats(int mode, int dk)
     return mode == 0 ? 64 * 64 + 4 * 64 + dk : (mode == 2 ? 64 * 64 + 2 * 64 * dk + dk : (dk + 32) * (dk + 32));
 }
 
-// The (sequence, chunk) of a place in the scratch; false where there is none.
+// The chunk at a place in the scratch (its first token and its tokens); false where there is none.
 template <int MODE>
-__device__ __forceinline__ bool chunk_of_slot(const ChunkArgs& A, int slot, int& seq, int& t0, int& n_tok)
+__device__ __forceinline__ bool chunk_of_slot(const ChunkArgs& A, int slot, int& t0, int& n_tok)
 {
     constexpr int C = ChunkOf<MODE>::C;
-    int lo = 0, hi = A.num_seqs;           // the last sequence whose first place is at most `slot`
+    int lo = 0, hi = A.num_seqs;           // the last request whose first place is at most `slot`: none behind a place's request starts before its end
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (chunk_slot(A.s.q_start[mid], mid, C) <= slot) lo = mid;
+        if (chunk_slot(MODE, A.s.q_start[mid]) <= slot) lo = mid;
         else hi = mid;
     }
-    seq = lo;
     const int t_begin = A.s.q_start[lo], t_end = A.s.q_start[lo + 1];
-    t0 = t_begin + (slot - chunk_slot(t_begin, lo, C)) * C;
+    t0 = t_begin + (slot - chunk_slot(MODE, t_begin)) * C;
     n_tok = min(C, t_end - t0);
-    return slot >= chunk_slot(t_begin, lo, C) && t0 < t_end && t_end - t_begin >= chunk_min(MODE);
+    return t0 < t_end && t_end - t_begin >= chunk_min(MODE);
+}
+
+// The request of a block of the walk: the x-th of those with chunk_min tokens and more; -1 where there are fewer.  Every warp finds it for itself.
+template <int MODE>
+__device__ __forceinline__ int long_request(const ChunkArgs& A, int x)
+{
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < A.num_seqs; s0 += 32) {
+        const int s = s0 + lane;
+        unsigned found = __ballot_sync(0xffffffffu, s < A.num_seqs && A.s.q_start[s + 1] - A.s.q_start[s] >= chunk_min(MODE));
+        const int n = __popc(found);
+        if (x < n) {
+            for (; x > 0; --x) found &= found - 1;
+            return s0 + __ffs(found) - 1;
+        }
+        x -= n;
+    }
+    return -1;
 }
 
 __device__ __forceinline__ bool huge(float x) { return !(fabsf(x) < HUGE_INPUT); }
@@ -658,9 +684,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_kernel(ChunkArgs A)
     __shared__ double from_s[C], to_s[C];          // i_s - F_s and F_t - l_t
     __shared__ float kappa_s[C];
     pdl_enter();
-    int seq, t0, n_tok;
+    int t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<0>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<0>(A, blockIdx.x, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(0, DK);
     float *P = mine, *F = mine + C * C, *loc = F + C, *kap = loc + C, *psum = kap + C, *ksum = psum + C;
@@ -763,9 +789,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_linear_kernel(ChunkArgs A)
     extern __shared__ __align__(16) float sm[];
     float *q_s = sm, *k_s = q_s + C * LD, *a_s = k_s + C * LD;
     pdl_enter();
-    int seq, t0, n_tok;
+    int t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<2>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<2>(A, blockIdx.x, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* mine = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(2, DK);
     float *P = mine, *Q = mine + C * C, *K = Q + C * DK, *dec = K + C * DK;
@@ -897,9 +923,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_delta_kernel(ChunkArgs A)
     float* Y = L + C * (C + 1);        // [C][C + 1]
     __shared__ float inv_s[C], last_s[D];
     pdl_enter();
-    int seq, t0, n_tok;
+    int t0, n_tok;
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (!chunk_of_slot<1>(A, blockIdx.x, seq, t0, n_tok)) return;
+    if (!chunk_of_slot<1>(A, blockIdx.x, t0, n_tok)) return;
     const ScanArgs& a = A.s;
     float* W = A.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats(1, D);
     const float* rows = a.proj + (size_t)t0 * a.ld;
@@ -1088,10 +1114,11 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
     float *S_s = sm + L::S, *n_s = sm + L::N, *red = sm + L::RED;
     pdl_enter();
     const ScanArgs& a = A.s;
-    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS, dv = a.dv;
+    const int seq = long_request<MODE>(A, blockIdx.x), h = blockIdx.y, c0 = blockIdx.z * WALK_COLS, dv = a.dv;
+    if (seq < 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
     const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
-    if (t_begin >= t_end || !takes_chunks<MODE>(a, seq, h, t_begin, t_end)) return;
+    if (!takes_chunks<MODE>(a, h, t_begin, t_end)) return;
     const int slot = a.state_slot[seq];
     if (slot < 0 || slot >= a.num_slots) {
         if (tid == 0) report_status(a.status, SPY_STATUS_BAD_PAGE, t_begin);
@@ -1105,7 +1132,7 @@ __global__ void __launch_bounds__(THREADS, 1) walk_kernel(ChunkArgs A)
         for (int r = tid; r < DK; r += THREADS) n_s[r] = st_nm[r];
         m = st_nm[DK];
     }
-    const int first_slot = chunk_slot(t_begin, seq, C);
+    const int first_slot = chunk_slot(MODE, t_begin);
     auto request = [&](int t0, int stage) {
         const int n_tok = min(C, t_end - t0);
         float* base = sm + stage * L::STAGE;
@@ -1271,10 +1298,11 @@ __global__ void __launch_bounds__(THREADS, 1) walk_delta_kernel(ChunkArgs A)
     float *S_s = sm + L::S, *red = sm + L::RED;
     pdl_enter();
     const ScanArgs& a = A.s;
-    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS;
+    const int seq = long_request<1>(A, blockIdx.x), h = blockIdx.y, c0 = blockIdx.z * WALK_COLS;
+    if (seq < 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, cg = lane & 3;
     const int t_begin = a.q_start[seq], t_end = a.q_start[seq + 1];
-    if (t_begin >= t_end || !takes_chunks<1>(a, seq, h, t_begin, t_end)) return;
+    if (!takes_chunks<1>(a, h, t_begin, t_end)) return;
     const int slot = a.state_slot[seq];
     if (slot < 0 || slot >= a.num_slots) {
         if (tid == 0) report_status(a.status, SPY_STATUS_BAD_PAGE, t_begin);
@@ -1282,7 +1310,7 @@ __global__ void __launch_bounds__(THREADS, 1) walk_delta_kernel(ChunkArgs A)
     }
     float* st = a.state + ((size_t)slot * a.H + h) * a.record;
     st4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3), ld4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3)));      // 64 rows of four quads: one a thread
-    const int first_slot = chunk_slot(t_begin, seq, C);
+    const int first_slot = chunk_slot(1, t_begin);
     auto request = [&](int t0, int stage) {
         const int n_tok = min(C, t_end - t0);
         float* base = sm + stage * L::STAGE;
@@ -1321,46 +1349,52 @@ __global__ void __launch_bounds__(THREADS, 1) walk_delta_kernel(ChunkArgs A)
     st4(st + (size_t)(tid >> 2) * D + c0 + 4 * (tid & 3), ld4(S_s + (tid >> 2) * WALK_LD + 4 * (tid & 3)));
 }
 
-template <typename Args> static int launch_chunk_kernel(void (*kernel)(Args), dim3 grid, size_t smem, cudaStream_t stream, const Args& A)
+// Which steps take chunks: keys of 64 or 128 channels (the delta rule's states of 64 x 64), value columns in sixteens, requests long enough (chunk_alone),
+// factors that fit 512 MB (130 K tokens of 8 heads of the matrix memory).  Only the long requests count: those of a token or a few beside
+// them take no place in the scratch and no blocks of these kernels, and are walked by tokens behind them.  Measured, the step's kernels together (us, by tokens / in chunks): one prompt
+// portion of 1,501 tokens beside 47 replies, matrix memory of 8 heads 705 / 290, delta rule of 32 heads 739 / 341, linear attention of 16 heads 1,023 / 454; of 200 beside 8
+// 98 / 59, 101 / 61, 142 / 95; of 200 beside 250 866 / 811, 389 / 363, 945 / 926; 60 tokens each of 16 beside one of 200 276 / 221, 182 / 169, 392 / 375.
+// The delta rule with up to 32 (long request, head) pairs: with more, the walk by tokens has work for most SMs and does fewer additions (32 heads, by tokens / in
+// chunks: one request of 160 tokens 51 / 44, two 64 / 73; one of 1,024 313 / 190, two 385 / 354).
+static long long chunk_work_floats(int mode, int tokens, int long_requests, int longest, int H, int dk, int dv)
 {
-    SPY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    spy_launch(kernel, grid, dim3(THREADS), smem, stream, A);
-    return 0;
+    if (long_requests <= 0 || longest < (long_requests > 1 ? chunk_min(mode) : chunk_alone(mode)) || dv % WALK_COLS != 0 || dv / WALK_COLS > 65535) return 0;
+    if (mode == 1 ? dk != 64 || dv != 64 || (long long)long_requests * H > 32 : dk != 64 && dk != 128) return 0;
+    const long long floats = (long long)chunk_slot(mode, tokens) * H * (chunk_floats(mode, dk) + 4LL);
+    return floats <= (128LL << 20) ? floats : 0;
 }
 
-// Which steps take chunks: keys of 64 or 128 channels (the delta rule's states of 64 x 64), value columns in sixteens, requests that bring half
-// of chunk_min or more on average (with fewer the kernels that find nothing to do are what is left), factors that fit 512 MB (200 K tokens of
-// 8 heads of the matrix memory).  The delta rule with up to 64 (request, head) pairs: with more, the walk by tokens has work for every SM and does
-// fewer additions (32 heads, requests of 1,024 tokens, us by tokens / in chunks: two 385 / 300, four 477 / 583).
-static long long chunk_work_floats(int mode, int tokens, int num_seqs, int H, int dk, int dv)
+// walks: the most requests of chunk_min tokens that there can be.
+template <int MODE> static int launch_chunks(ScanArgs& S, int tokens, int num_seqs, int walks, float* work, cudaStream_t stream)
 {
-    if (tokens < chunk_min(mode) || 2LL * tokens < (long long)num_seqs * chunk_min(mode) || dv % WALK_COLS != 0) return 0;
-    if (mode == 1 ? dk != 64 || dv != 64 || (long long)num_seqs * H > 64 : dk != 64 && dk != 128) return 0;
-    const long long slots = tokens / (mode == 1 ? 32 : 64) + (long long)num_seqs + 1;
-    const long long floats = slots * H * (chunk_floats(mode, dk) + 4LL);
-    return floats <= (128LL << 20) && slots <= 0x7fffffff ? floats : 0;
-}
-
-template <int MODE> static int launch_chunks(ScanArgs& S, int tokens, int num_seqs, float* work, cudaStream_t stream)
-{
-    const int slots = tokens / ChunkOf<MODE>::C + num_seqs + 1;
+    const int slots = chunk_slot(MODE, tokens);
     ChunkArgs A = {S, work, nullptr, num_seqs};
     A.flags = reinterpret_cast<int*>(work + (size_t)slots * S.H * chunk_floats(MODE, S.dk));
     A.s.flags = S.flags = A.flags;
-    const dim3 chunks(slots, S.H), walk(num_seqs, S.H, S.dv / WALK_COLS);
-    int rc;
+    const dim3 chunks(slots, S.H), walk(walks, S.H, S.dv / WALK_COLS), threads(THREADS);
     if constexpr (MODE == 1) {
         constexpr int C = 32, D = 64, R = C + D;
-        rc = launch_chunk_kernel(chunk_delta_kernel, chunks, 4 * C * (D + 2) * sizeof(double) + (2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float), stream, A);
-        if (!rc) rc = launch_chunk_kernel(walk_delta_kernel, walk, DeltaSmem::BYTES, stream, A);
+        constexpr size_t factors = 4 * C * (D + 2) * sizeof(double) + (2 * C * (R + 4) + 2 * C * (C + 1)) * sizeof(float);
+        SPY_ONCE_PER_DEVICE {
+            SPY_CUDA(cudaFuncSetAttribute(chunk_delta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)factors));
+            SPY_CUDA(cudaFuncSetAttribute(walk_delta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem::BYTES));
+        }
+        spy_launch(chunk_delta_kernel, chunks, threads, factors, stream, A);
+        spy_launch(walk_delta_kernel, walk, threads, DeltaSmem::BYTES, stream, A);
     } else {
-        const size_t rows = (MODE == 0 ? 2 : 3) * 64 * (size_t)(S.dk + 4) * sizeof(float);
-        auto chunk = MODE == 0 ? (S.dk == 64 ? chunk_memory_kernel<64> : chunk_memory_kernel<128>) : (S.dk == 64 ? chunk_linear_kernel<64> : chunk_linear_kernel<128>);
-        rc = launch_chunk_kernel(chunk, chunks, rows, stream, A);
-        if (!rc) rc = S.dk == 64 ? launch_chunk_kernel(walk_kernel<MODE, 64>, walk, WalkSmem<MODE, 64>::BYTES, stream, A)
-                                 : launch_chunk_kernel(walk_kernel<MODE, 128>, walk, WalkSmem<MODE, 128>::BYTES, stream, A);
+        void (*const chunk64)(ChunkArgs) = MODE == 0 ? chunk_memory_kernel<64> : chunk_linear_kernel<64>;
+        void (*const chunk128)(ChunkArgs) = MODE == 0 ? chunk_memory_kernel<128> : chunk_linear_kernel<128>;
+        const auto factors = [](int dk) { return (MODE == 0 ? 2 : 3) * 64 * (size_t)(dk + 4) * sizeof(float); };
+        SPY_ONCE_PER_DEVICE {
+            SPY_CUDA(cudaFuncSetAttribute(chunk64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)factors(64)));
+            SPY_CUDA(cudaFuncSetAttribute(chunk128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)factors(128)));
+            SPY_CUDA(cudaFuncSetAttribute(walk_kernel<MODE, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WalkSmem<MODE, 64>::BYTES));
+            SPY_CUDA(cudaFuncSetAttribute(walk_kernel<MODE, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WalkSmem<MODE, 128>::BYTES));
+        }
+        spy_launch(S.dk == 64 ? chunk64 : chunk128, chunks, threads, factors(S.dk), stream, A);
+        if (S.dk == 64) spy_launch(walk_kernel<MODE, 64>, walk, threads, WalkSmem<MODE, 64>::BYTES, stream, A);
+        else spy_launch(walk_kernel<MODE, 128>, walk, threads, WalkSmem<MODE, 128>::BYTES, stream, A);
     }
-    if (rc) return rc;
     SPY_CHECK_LAUNCH("recurrence (chunks)");
     return 0;
 }
@@ -1437,8 +1471,9 @@ template <int MODE> static int launch_scan_mode(ScanArgs& A, int num_seqs, int l
     return launch_scan_rg<MODE, 32>(A, num_seqs, longest, stream);
 }
 
-// work: null, or scratch of spy_scan_chunk_floats floats for `tokens` tokens, 16-byte aligned.
-static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, int tokens, float* work, long long work_floats, cudaStream_t stream)
+// work: null (every request is walked by tokens), or scratch of spy_scan_chunk_floats floats for `tokens` tokens, 16-byte aligned;
+// walks: the most requests that can bring chunk_min tokens in any step that this launch serves.
+static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, int tokens, float* work, long long work_floats, int walks, cudaStream_t stream)
 {
     if (num_seqs <= 0) return 0;
     if (A.H <= 0 || A.dk <= 0 || A.dv <= 0) SPY_FAIL("recurrence: heads %d, key size %d and value size %d must be positive", A.H, A.dk, A.dv);
@@ -1448,54 +1483,62 @@ static int launch_scan(int mode, ScanArgs& A, int num_seqs, int longest, int tok
     const bool aligned = ((A.ld | A.off_q | A.off_k | A.off_v | (mode == 1 ? A.off_x1 : 0)) & 3) == 0 && A.record % 4 == 0 &&
                          ((reinterpret_cast<uintptr_t>(A.proj) | reinterpret_cast<uintptr_t>(A.state) | reinterpret_cast<uintptr_t>(A.out) |
                            reinterpret_cast<uintptr_t>(work)) & 15) == 0;
-    if (work != nullptr && longest >= chunk_min(mode) && aligned) {
-        const long long need = chunk_work_floats(mode, tokens, num_seqs, A.H, A.dk, A.dv);
-        if (need > work_floats) SPY_FAIL("recurrence: %lld floats of scratch for %d tokens, %lld are needed", work_floats, tokens, need);
-        if (need > 0) {
-            const int rc = mode == 0 ? launch_chunks<0>(A, tokens, num_seqs, work, stream)
-                           : mode == 1 ? launch_chunks<1>(A, tokens, num_seqs, work, stream) : launch_chunks<2>(A, tokens, num_seqs, work, stream);
-            if (rc) return rc;
-        }
+    if (work != nullptr && walks > 0 && aligned) {
+        const long long need = chunk_work_floats(mode, tokens, 1, tokens, A.H, A.dk, A.dv);
+        if (need <= 0 || need > work_floats) SPY_FAIL("recurrence: %lld floats of scratch for %d tokens, %lld are needed", work_floats, tokens, need);
+        const int rc = mode == 0 ? launch_chunks<0>(A, tokens, num_seqs, walks, work, stream)
+                       : mode == 1 ? launch_chunks<1>(A, tokens, num_seqs, walks, work, stream) : launch_chunks<2>(A, tokens, num_seqs, walks, work, stream);
+        if (rc) return rc;
     }
     if (mode == 2) return launch_scan_mode<2>(A, num_seqs, longest, stream);
     return mode == 0 ? launch_scan_mode<0>(A, num_seqs, longest, stream) : launch_scan_mode<1>(A, num_seqs, longest, stream);
 }
 
-// Floats of scratch with which a step's longer requests are walked in chunks; 0: these sizes are walked token by token.
-extern "C" long long spy_scan_chunk_floats(int mode, int tokens, int num_seqs, int H, int dk, int dv) { return chunk_work_floats(mode, tokens, num_seqs, H, dk, dv); }
+// The tokens from which on a request is walked in chunks where its step takes them.
+extern "C" int spy_scan_chunk_min(int mode) { return chunk_min(mode); }
+
+// Floats of scratch with which a step of `tokens` tokens takes chunks, `long_requests` of its requests bringing chunk_min tokens or more and the longest
+// `longest`; 0: it does not take them.
+extern "C" long long spy_scan_chunk_floats(int mode, int tokens, int long_requests, int longest, int H, int dk, int dv)
+{
+    return chunk_work_floats(mode, tokens, long_requests, longest, H, dk, dv);
+}
 
 // State record of one head, in floats.
 extern "C" long long spy_mlstm_record(int dk, int dv) { return ((long long)dk * dv + (long long)((dv + 7) / 8) * (dk + 1) + 3) / 4 * 4; }
 
 extern "C" int spy_mlstm_scan(const float* proj, long long ld, int off_q, int off_k, int off_v, int off_i, int off_f, const float* bias_i, const float* bias_f,
                               float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest, float* out, int H, int dk,
-                              int dv, float q_scale, float cap, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
+                              int dv, float q_scale, float cap, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats,
+                              int walks)
 {
     if (!(cap > 0.f)) SPY_FAIL("mlstm: the gates' cap must be positive");
     ScanArgs A = {proj, ld, off_q, off_k, off_v, off_i, off_f, nullptr, bias_i, bias_f, state, spy_mlstm_record(dk, dv), num_slots, q_start, state_slot, out,
                   H, dk, dv, q_scale, cap, status, nullptr};
-    return launch_scan(0, A, num_seqs, longest, tokens, work, work_floats, stream);
+    return launch_scan(0, A, num_seqs, longest, tokens, work, work_floats, walks, stream);
 }
 
 extern "C" int spy_delta_scan(const float* proj, long long ld, int off_r, int off_k, int off_v, int off_a, const float* decay_pre, const float* bias_a,
                               const float* decay_offset, float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest,
-                              float* out, int H, int dk, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
+                              float* out, int H, int dk, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats,
+                              int walks)
 {
     ScanArgs A = {proj, ld, off_r, off_k, off_v, off_a, 0, decay_pre, bias_a, decay_offset, state, (long long)dk * dk, num_slots, q_start, state_slot, out,
                   H, dk, dk, 1.0f, 1.0f, status, nullptr};
-    return launch_scan(1, A, num_seqs, longest, tokens, work, work_floats, stream);
+    return launch_scan(1, A, num_seqs, longest, tokens, work, work_floats, walks, stream);
 }
 
 // Gated linear attention with a decay per key channel: proj holds q, k, v at `off_*`; decay_pre [T, H * dk] the decay's
 // pre-activation z, to which decay_bias [H * dk] is added: a = exp(logsigmoid(z + bias) / tau).  q is scaled by q_scale.
 extern "C" int spy_gla_scan(const float* proj, long long ld, int off_q, int off_k, int off_v, const float* decay_pre, const float* decay_bias, float inv_tau,
                             float* state, int num_slots, const int* q_start, const int* state_slot, int num_seqs, int longest, float* out, int H, int dk, int dv,
-                            float q_scale, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats)
+                            float q_scale, int* status, cudaStream_t stream, int tokens, float* work, long long work_floats,
+                              int walks)
 {
     if (!(inv_tau > 0.f)) SPY_FAIL("gated linear attention: tau must be positive");
     ScanArgs A = {proj, ld, off_q, off_k, off_v, 0, 0, decay_pre, nullptr, decay_bias, state, (long long)dk * dv, num_slots, q_start, state_slot, out,
                   H, dk, dv, q_scale, inv_tau, status, nullptr};
-    return launch_scan(2, A, num_seqs, longest, tokens, work, work_floats, stream);
+    return launch_scan(2, A, num_seqs, longest, tokens, work, work_floats, walks, stream);
 }
 
 // out[t, j] = act(proj[t, off + j]) for j < n: the inner activation of a two-step (low-rank) projection; act 0: tanh, 1: none.

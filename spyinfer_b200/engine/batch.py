@@ -65,7 +65,13 @@ class StepBatch:
     one_token_head: int = 0
     #: no request of the batch holds more than ``SHORT_CONTEXT`` keys after this step
     short_context: bool = False
+    #: the launches are captured and replayed for other batches of the same padded sizes (and the same ``Part.choice``)
+    replayed: bool = False
     extras: Dict[str, object] = field(default_factory=dict)
+
+    def runs(self, least: int):
+        """(how many requests bring ``least`` tokens or more, the most tokens that one brings)."""
+        return (int(np.count_nonzero(self.host_q_start[1:] - self.host_q_start[:-1] >= least)), self.max_q_len) if self.max_q_len >= least else (0, self.max_q_len)
 
 
 #: Keys up to which a step counts as one of short contexts: up to here the attention kernel whose blocks take a few rows each, and read keys as they come,

@@ -292,7 +292,7 @@ class ModelRunner:
             t[S + extra:, 0] = cache.spare_page(g)
             tables.append(t)
         batch = self.stager.stage(token_ids, positions, seq_of_token, starts, ctx_len, slots, logit_rows, tables, Tb, Sb)
-        batch.one_token_head = Hb
+        batch.one_token_head, batch.replayed = Hb, True
         return batch
 
     def step(self, entries: Sequence[StepEntry], tokens_from: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:

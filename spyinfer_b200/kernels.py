@@ -7,6 +7,7 @@ if the C side refuses the sizes.  Nothing here falls back to a library or to the
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -495,23 +496,48 @@ def _scan_common(proj, state, q_start, state_slot, out, heads, dv):
         raise KernelError(f"recurrence output: expected {(proj.shape[0], heads * dv)}, found {tuple(out.shape)}")
 
 
-def _scan_chunk_work(mode: int, proj: torch.Tensor, num_seqs: int, longest: Optional[int], heads: int, dk: int, dv: int):
-    """Scratch for a step whose longer requests are walked in chunks (csrc/recurrence.cu), and its floats; None and 0 where none are."""
-    if longest is not None and longest <= 1:
-        return None, 0
+SCAN_MODES = {"matrix memory": 0, "delta rule": 1, "linear attention": 2}
+
+
+@functools.lru_cache(maxsize=None)
+def scan_chunk_min(kind: str) -> int:
+    """The tokens from which on a request is walked in chunks, where its step takes them (csrc/recurrence.cu)."""
+    return int(build.load("recurrence").spy_scan_chunk_min(SCAN_MODES[kind]))
+
+
+@functools.lru_cache(maxsize=4096)
+def scan_chunk_floats(kind: str, tokens: int, long_requests: int, longest: int, heads: int, dk: int, dv: int) -> int:
+    """Floats of scratch with which a step of ``tokens`` tokens takes chunks, ``long_requests`` of its requests bringing ``scan_chunk_min(kind)``
+    tokens or more and the longest ``longest``; 0 where all its requests are walked token by token."""
     f = build.load("recurrence").spy_scan_chunk_floats
     f.restype = ctypes.c_longlong
-    floats = int(f(mode, proj.shape[0], int(num_seqs), heads, dk, dv))
-    return (torch.empty(floats, dtype=torch.float32, device=proj.device), floats) if floats else (None, 0)
+    return int(f(SCAN_MODES[kind], int(tokens), int(long_requests), int(longest), int(heads), int(dk), int(dv)))
+
+
+def _scan_chunk_work(kind: str, proj: torch.Tensor, num_seqs: int, longest: Optional[int], runs, replayed: bool, heads: int, dk: int, dv: int):
+    """What ``spy_*_scan`` is told of the chunks: scratch or None, its floats, and the most requests that are walked in chunks."""
+    T = proj.shape[0]
+    if longest is not None and longest <= 1:
+        return None, 0, 0
+    most = min(int(num_seqs), T // scan_chunk_min(kind))
+    count, length = (most, longest or T) if runs is None else runs
+    floats = scan_chunk_floats(kind, T, count, min(length, T), heads, dk, dv)
+    if floats == 0:
+        return None, 0, 0
+    return torch.empty(floats, dtype=torch.float32, device=proj.device), floats, most if replayed else int(count)
 
 
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i: torch.Tensor, bias_f: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
                state_slot: torch.Tensor, num_seqs: int, out: torch.Tensor, heads: int, dk: int, dv: int, q_scale: float, cap: float,
-               status: Optional[torch.Tensor] = None, longest: Optional[int] = None) -> torch.Tensor:
+               status: Optional[torch.Tensor] = None, longest: Optional[int] = None,
+               runs: Optional[tuple] = None, replayed: bool = False) -> torch.Tensor:
     """The gated matrix memory over every request's tokens of this step, in order, from and into ``state [slots, heads * record]``.
     ``proj [T, ld]`` float32 holds q, k, v and the two gates' pre-activations at the columns ``offsets = (q, k, v, i, f)``.
     ``longest``: the most tokens a request brings, or more (default: all the batch's tokens): it sizes the kernel's staging, and 1
-    says that every request brings exactly one token (the kernel made for decoding then runs; ``delta_scan`` likewise)."""
+    says that every request brings exactly one token (the kernel made for decoding then runs; ``delta_scan`` likewise).
+    ``runs = (how many requests bring scan_chunk_min("matrix memory") tokens or more, the longest request's tokens)``: whether such requests are
+    walked in chunks goes by them (None: by what the batch's sizes allow; the count may not be too small).  ``replayed``: the launch is captured and replayed for
+    other batches of these sizes, for which the same holds, but with other counts (``delta_scan`` and ``gla_scan`` likewise)."""
     _scan_common(proj, state, q_start, state_slot, out, heads, dv)
     if state.dim() != 2 or state.shape[1] != heads * mlstm_record(dk, dv):
         raise KernelError(f"mlstm: state {tuple(state.shape)} does not fit {heads} heads of {dk} x {dv}")
@@ -520,16 +546,17 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i: torch.Tensor, bias_f: torch.
     oq, ok, ov, oi, of = (int(o) for o in offsets)
     if max(oq + heads * dk, ok + heads * dk, ov + heads * dv, oi + heads, of + heads) > proj.shape[1] or bias_i.shape[0] != heads or bias_f.shape[0] != heads:
         raise KernelError("mlstm: the column offsets or the biases do not fit the projection")
-    work, floats = _scan_chunk_work(0, proj, num_seqs, longest, heads, dk, dv)
+    work, floats, walks = _scan_chunk_work("matrix memory", proj, num_seqs, longest, runs, replayed, heads, dk, dv)
     _call("recurrence", "spy_mlstm_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), oq, ok, ov, oi, of, _ptr(bias_i), _ptr(bias_f), _ptr(state),
           state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk, dv,
-          ctypes.c_float(q_scale), ctypes.c_float(cap), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
+          ctypes.c_float(q_scale), ctypes.c_float(cap), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats), walks)
     return out
 
 
 def delta_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, bias_a: torch.Tensor, decay_offset: torch.Tensor, state: torch.Tensor,
                q_start: torch.Tensor, state_slot: torch.Tensor, num_seqs: int, out: torch.Tensor, heads: int, dk: int,
-               status: Optional[torch.Tensor] = None, longest: Optional[int] = None) -> torch.Tensor:
+               status: Optional[torch.Tensor] = None, longest: Optional[int] = None,
+               runs: Optional[tuple] = None, replayed: bool = False) -> torch.Tensor:
     """The generalised delta rule over every request's tokens of this step, from and into ``state [slots, heads * dk * dk]``.
     ``proj [T, ld]`` float32 holds r, k, v and the removal rate's pre-activation at ``offsets = (r, k, v, a)``;
     ``decay_pre [T, heads * dk]`` the decay's pre-activation."""
@@ -543,16 +570,17 @@ def delta_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, bias_a: tor
     n = heads * dk
     if max(o_r, ok, ov, oa) + n > proj.shape[1] or tuple(decay_pre.shape) != (proj.shape[0], n) or bias_a.shape[0] != n or decay_offset.shape[0] != n:
         raise KernelError("delta rule: the column offsets, the decay or the biases do not fit the projection")
-    work, floats = _scan_chunk_work(1, proj, num_seqs, longest, heads, dk, dk)
+    work, floats, walks = _scan_chunk_work("delta rule", proj, num_seqs, longest, runs, replayed, heads, dk, dk)
     _call("recurrence", "spy_delta_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), o_r, ok, ov, oa, _ptr(decay_pre), _ptr(bias_a), _ptr(decay_offset),
           _ptr(state), state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk,
-          _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
+          _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats), walks)
     return out
 
 
 def gla_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, decay_bias: torch.Tensor, tau: float, state: torch.Tensor, q_start: torch.Tensor,
              state_slot: torch.Tensor, num_seqs: int, out: torch.Tensor, heads: int, dk: int, dv: int, q_scale: float,
-             status: Optional[torch.Tensor] = None, longest: Optional[int] = None) -> torch.Tensor:
+             status: Optional[torch.Tensor] = None, longest: Optional[int] = None,
+             runs: Optional[tuple] = None, replayed: bool = False) -> torch.Tensor:
     """Gated linear attention with a decay per key channel over every request's tokens of this step, from and into
     ``state [slots, heads * dk * dv]``: ``S = diag(a) S + k v^T``, ``o = S^T (q_scale q)``, ``a = sigmoid(z + bias)^(1 / tau)``.
     ``proj [T, ld]`` float32 holds q, k, v at ``offsets = (q, k, v)``; ``decay_pre [T, heads * dk]`` is ``z``."""
@@ -565,10 +593,10 @@ def gla_scan(proj: torch.Tensor, offsets, decay_pre: torch.Tensor, decay_bias: t
     n = heads * dk
     if max(oq + n, ok + n, ov + heads * dv) > proj.shape[1] or tuple(decay_pre.shape) != (proj.shape[0], n) or decay_bias.shape[0] != n or not tau > 0:
         raise KernelError("gated linear attention: the column offsets, the decay or its bias do not fit the projection, or tau is not positive")
-    work, floats = _scan_chunk_work(2, proj, num_seqs, longest, heads, dk, dv)
+    work, floats, walks = _scan_chunk_work("linear attention", proj, num_seqs, longest, runs, replayed, heads, dk, dv)
     _call("recurrence", "spy_gla_scan", _ptr(proj), ctypes.c_longlong(proj.shape[1]), oq, ok, ov, _ptr(decay_pre), _ptr(decay_bias), ctypes.c_float(1.0 / tau),
           _ptr(state), state.shape[0], _ptr(q_start), _ptr(state_slot), int(num_seqs), int(longest or proj.shape[0]), _ptr(out), heads, dk, dv,
-          ctypes.c_float(q_scale), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats))
+          ctypes.c_float(q_scale), _ptr(status), _stream(), proj.shape[0], _ptr(work), ctypes.c_longlong(floats), walks)
     return out
 
 

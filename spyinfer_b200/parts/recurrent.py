@@ -43,6 +43,25 @@ _TILE = 8     # value columns of the narrowest tile of the scan kernel, each of 
 class _Recurrent(Mixer):
     graph_safe = True
     gate = "sigmoid"       # the output gate's activation
+    #: what the kernels call the recurrence if they walk long runs of tokens in chunks, and its (heads, dk, dv)
+    chunks, sizes = None, None
+
+    def choosing(self):
+        return [self] if self.chunks is not None else []
+
+    def choice_sizes(self):
+        return (self.chunks,) + self.sizes
+
+    def choice(self, batch, page_size):
+        """Whether the batch's long requests are walked in chunks."""
+        count, longest = batch.runs(kernels.scan_chunk_min(self.chunks))
+        return self.chunks + " in chunks" if count > 0 and kernels.scan_chunk_floats(self.chunks, batch.num_tokens, count, longest, *self.sizes) > 0 else ""
+
+    def _runs(self, batch):
+        """What the scan kernels are told of a batch's requests."""
+        if batch.one_token_each:
+            return {"longest": 1}
+        return {"longest": batch.num_tokens, "runs": batch.runs(kernels.scan_chunk_min(self.chunks)), "replayed": batch.replayed}
 
     #: (relative tensor name, rows as a function of the sizes) of the projections that are fused, in column order
     def _fused_names(self):
@@ -78,6 +97,7 @@ class MatrixMemory(_Recurrent):
             raise ValueError("matrix_memory: sizes and the gates' cap must be positive")
         self.prefix = params.get("prefix", "")
         H, dk, dv = self.heads, self.dk, self.dv
+        self.chunks, self.sizes = "matrix memory", (H, dk, dv)
         self.offsets = (0, H * dk, 2 * H * dk, 2 * H * dk + 2 * H * dv, 2 * H * dk + 2 * H * dv + H)      # q, k, v, i, f
         self.gate_offset = 2 * H * dk + H * dv
         self.record = (dk * dv + -(-dv // _TILE) * (dk + 1) + 3) // 4 * 4
@@ -107,8 +127,7 @@ class MatrixMemory(_Recurrent):
         proj = self.fused(x, out_dtype=torch.float32)
         o = torch.empty((x.shape[0], self.heads * self.dv), dtype=torch.float32, device=x.device)
         kernels.mlstm_scan(proj, self.offsets, self.bias_i, self.bias_f, cache.state, batch.q_start, batch.state_slot, batch.num_seqs, o,
-                           self.heads, self.dk, self.dv, self.dk ** -0.5, self.cap, status=batch.status,
-                           longest=1 if batch.one_token_each else batch.num_tokens)
+                           self.heads, self.dk, self.dv, self.dk ** -0.5, self.cap, status=batch.status, **self._runs(batch))
         return self._finish(o, proj, self.gate_offset, self.heads, self.dv)
 
 
@@ -126,6 +145,7 @@ class DeltaRule(_Recurrent):
             raise ValueError("delta_rule: sizes must be positive")
         self.prefix = params.get("prefix", "")
         n = self.heads * self.d
+        self.chunks, self.sizes = "delta rule", (self.heads, self.d, self.d)
         self.offsets = (0, n, 2 * n, 4 * n)       # r, k, v, a
         self.gate_offset, self.rank_offset = 3 * n, 5 * n
         self.fused = self.w2 = self.o = self.norm_weight = self.bias_a = self.decay_offset = None
@@ -158,7 +178,7 @@ class DeltaRule(_Recurrent):
         decay_pre = self.w2(inner, out_dtype=torch.float32)
         o = torch.empty((x.shape[0], self.heads * self.d), dtype=torch.float32, device=x.device)
         kernels.delta_scan(proj, self.offsets, decay_pre, self.bias_a, self.decay_offset, cache.state, batch.q_start, batch.state_slot,
-                           batch.num_seqs, o, self.heads, self.d, status=batch.status, longest=1 if batch.one_token_each else batch.num_tokens)
+                           batch.num_seqs, o, self.heads, self.d, status=batch.status, **self._runs(batch))
         return self._finish(o, proj, self.gate_offset, self.heads, self.d)
 
 
@@ -180,6 +200,7 @@ class GatedLinearAttention(_Recurrent):
             raise ValueError("gated_linear_attention: sizes and tau must be positive")
         self.prefix = params.get("prefix", "")
         H, dk, dv = self.heads, self.dk, self.dv
+        self.chunks, self.sizes = "linear attention", (H, dk, dv)
         self.offsets = (0, H * dk, 2 * H * dk)                       # q, k, v
         self.gate_offset, self.rank_offset = 2 * H * dk + H * dv, 2 * H * dk + 2 * H * dv
         self.fused = self.a2 = self.o = self.norm_weight = self.decay_bias = None
@@ -212,7 +233,7 @@ class GatedLinearAttention(_Recurrent):
         decay_pre = self.a2(inner, out_dtype=torch.float32)
         o = torch.empty((x.shape[0], self.heads * self.dv), dtype=torch.float32, device=x.device)
         kernels.gla_scan(proj, self.offsets, decay_pre, self.decay_bias, self.tau, cache.state, batch.q_start, batch.state_slot, batch.num_seqs, o,
-                         self.heads, self.dk, self.dv, self.dk ** -0.5, status=batch.status, longest=1 if batch.one_token_each else batch.num_tokens)
+                         self.heads, self.dk, self.dv, self.dk ** -0.5, status=batch.status, **self._runs(batch))
         return self._finish(o, proj, self.gate_offset, self.heads, self.dv)
 
 

@@ -65,7 +65,7 @@ def distance(kind, got, want, dv):
     return float((d.norm(dim=1) / w.norm(dim=1)).median())
 
 
-def run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad):
+def run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad, **kw):
     """One step of several requests; ``pad`` columns ahead of q: with one, no row starts on a 16-byte border and every request is walked
     token by token."""
     from spyinfer_b200 import kernels
@@ -79,11 +79,11 @@ def run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad):
     out = torch.full((len(x), nv), 9.0, device="cuda")
     offs = [pad, pad + n, pad + 2 * n, pad + 2 * n + nv, pad + 2 * n + nv + 4]
     if kind == "memory":
-        kernels.mlstm_scan(x, offs, b1[:HEADS].cuda(), b2[:HEADS].cuda(), state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5, 6.0)
+        kernels.mlstm_scan(x, offs, b1[:HEADS].cuda(), b2[:HEADS].cuda(), state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5, 6.0, **kw)
     elif kind == "linear":
-        kernels.gla_scan(x, offs[:3], pre, b2.cuda(), 16.0, state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5)
+        kernels.gla_scan(x, offs[:3], pre, b2.cuda(), 16.0, state, starts, where, len(xs), out, HEADS, dk, dv, dk ** -0.5, **kw)
     else:
-        kernels.delta_scan(x, offs[:4], pre, b1.cuda(), b2.cuda(), state, starts, where, len(xs), out, HEADS, dk)
+        kernels.delta_scan(x, offs[:4], pre, b1.cuda(), b2.cuda(), state, starts, where, len(xs), out, HEADS, dk, **kw)
     return out.cpu()
 
 
@@ -165,6 +165,122 @@ def test_requests_with_numbers_out_of_range_are_walked_by_tokens(kind, dk, dv, v
         assert torch.allclose(outs[0][200:, h], outs[1][200:, h], rtol=1e-4, atol=1e-4)     # a saturated gate is an ordinary one
 
 
+@gpu
+@pytest.mark.parametrize("kind,dk,dv", [("memory", 64, 32), ("linear", 64, 16), ("delta", 64, 64)])
+def test_long_requests_anywhere_among_short_ones_take_the_same_chunks(kind, dk, dv):
+    """Long requests between requests of one token, of a few and of none: every token once, as the walk by tokens has it; and the same bits whatever
+    is said of the batch (the long requests counted, an upper bound as in a replayed step, nothing), and alone without the others."""
+    from spyinfer_b200 import kernels
+
+    name = {"memory": "matrix memory", "linear": "linear attention", "delta": "delta rule"}[kind]
+    least = kernels.scan_chunk_min(name)
+    for order in ([1, 1, least, 2, least + 1, 0, 300, 1], [1] * 70 + [0, 257, 1, least + 64, 0], [257] + [1] * 40 + [5, 200, least], [0, 300, 0, 1]):
+        data = [inputs(kind, dk, dv, n, r)[:2] for r, n in enumerate(order)]
+        _, _, b1, b2 = inputs(kind, dk, dv, 1, 99)
+        xs, pres, slots = [d[0] for d in data], [d[1] for d in data], list(range(len(order)))[::-1]
+        runs = (sum(n >= least for n in order), max(order))
+        outs, states = [], []
+        for pad, kw in ((0, dict(runs=runs)), (0, dict(runs=runs, replayed=True)), (0, {}), (1, {})):
+            state = new_state(kind, dk, dv, len(order))
+            outs.append(run(kind, dk, dv, xs, pres, b1, b2, state, slots, pad, **kw))
+            states.append(state.cpu())
+        for k in (1, 2):
+            assert torch.equal(outs[0], outs[k]) and torch.equal(states[0], states[k])
+        assert torch.allclose(outs[0], outs[3], rtol=2e-3, atol=2e-4) and torch.allclose(states[0], states[3], rtol=2e-4, atol=2e-5)
+        assert not torch.equal(outs[0], outs[3])                                # chunks were taken
+        at = 0
+        for r, n in enumerate(order):
+            if n >= 257:                                                        # long enough to take chunks alone
+                alone = run(kind, dk, dv, [xs[r]], [pres[r]], b1, b2, new_state(kind, dk, dv, 1), [0], 0, runs=(1, n))
+                assert torch.equal(alone, outs[0][at:at + n])
+            at += n
+
+
+@gpu
+@pytest.mark.parametrize("kind", ["memory", "linear", "delta"])
+def test_a_step_without_long_requests_asks_for_no_scratch(kind):
+    from spyinfer_b200 import kernels
+
+    name = {"memory": "matrix memory", "linear": "linear attention", "delta": "delta rule"}[kind]
+    least, sizes = kernels.scan_chunk_min(name), (2, 64, 64)
+    proj = torch.empty((8 * (least - 1), 4), device="cuda")
+
+    def asks(tokens, runs, **kw):
+        return kernels._scan_chunk_work(name, proj[:tokens], 8, tokens, runs, kw.get("replayed", False), *sizes)
+
+    assert asks(8 * (least - 1), (0, least - 1)) == (None, 0, 0)                 # many tokens, no request long enough
+    work, floats, walks = asks(7 + 300, (1, 300))                                # one portion beside seven replies
+    assert work.numel() == floats > 0 and walks == 1
+    assert asks(7 + 300, (1, 300), replayed=True)[2] == (7 + 300) // least       # a replayed step: as many as there can be
+
+
+@gpu
+@pytest.mark.parametrize("design", ["nezolorn", "daronex"])
+def test_models_take_chunks_whole_in_portions_and_replayed_beside_replies(design):
+    """A matrix memory, a delta rule and a linear attention of sizes that take chunks, in whole models: prompts of some 200 tokens at once and in portions
+    around the least length, then portions beside replies at one padded size, launched, captured and replayed for batches of other shapes
+    and for one whose requests are all too short (which has a graph of its own)."""
+    import importlib
+
+    import numpy as np
+    from spyinfer_b200 import config_from_json
+    from spyinfer_b200.config import EngineConfig
+    from spyinfer_b200.engine.batch import StepEntry
+    from spyinfer_b200.engine.model import Model
+    from spyinfer_b200.engine.runner import ModelRunner
+
+    plain = importlib.import_module("plain_" + design)
+    if design == "nezolorn":
+        cfg = {"architecture": "Nezolorn", "vocab": 211, "width": 128, "residual_mult": 0.5, "norm": {"eps": 1e-6}, "embedding": {"scale": 1.0}, "layers": [
+            {"type": "parallel", "mlp": {"kind": "dense", "ff": 96}, "mixer": {"left_scale": 1.0, "right_scale": 1.0,
+             "left": {"heads": 2, "kv_heads": 1, "dim": 32, "vdim": 32, "scale": 0.2, "mask": {"size": 40, "pool": 8}, "rot": {"base": 1000.0, "dims": 32}},
+             "right": {"heads": 2, "dim": 64, "vdim": 32, "gate_cap": 10.0}}},
+            {"type": "general_delta", "mlp": {"kind": "dense", "ff": 80}, "mixer": {"heads": 2, "dim": 64, "decay_rank": 8}}]}
+    else:
+        cfg = {"architecture": "Daronex", "vocab": 211, "width": 128, "norm": {"eps": 1e-6}, "logit_scale": 1.0, "layers": [
+            {"type": "latent_attention", "mlp": {"kind": "dense", "ff": 96}, "mixer": {"heads": 2, "dim": 16, "rot_dim": 8, "vdim": 24, "q_rank": 24, "kv_rank": 24,
+                                                                                      "scale": 0.3, "rot": {"base": 500.0, "dims": 8}}},
+            {"type": "gla", "mlp": {"kind": "dense", "ff": 80}, "mixer": {"heads": 2, "dim": 64, "vdim": 32, "tau": 16.0, "decay_rank": 8}}]}
+    weights = plain.random_weights(cfg, 3)
+    config = EngineConfig(dtype="float32", kvcache_block_size=16, num_kvcache_blocks=200, max_num_seqs=8, max_model_len=400, max_num_batched_tokens=512)
+    model = Model(config_from_json(cfg).to_spec(), torch.float32, config.device, config.max_model_len)
+    model.bind({k: v.cuda() for k, v in weights.items()})
+    runner = ModelRunner(model, config)
+    rng = np.random.default_rng(5)
+    tokens = {r: rng.integers(0, 211, 240).tolist() for r in "abcdefgh"}
+    want = {r: plain.forward(weights, cfg, t).numpy() for r, t in tokens.items()}
+
+    def close(got, ref):
+        return float(np.abs(got - ref).max() / np.abs(ref).max())
+
+    cuts = {}
+    for name, sizes in {"whole": [240], "two": [200, 40], "least": [95, 145], "mixed": [1, 163, 5, 71]}.items():
+        rows, at = [], 0
+        for n in sizes:
+            rows.append(runner.step([StepEntry("a", tokens["a"][at:at + n], list(range(n)))]).float().cpu().numpy().copy())
+            at += n
+        runner.finish("a")
+        cuts[name] = np.concatenate(rows)
+        assert close(cuts[name], want["a"]) < 2e-4 and close(cuts[name], cuts["whole"]) < 2e-6, name
+    done = {r: 0 for r in tokens}
+
+    def step(shares):
+        entries = [StepEntry(r, tokens[r][done[r]:done[r] + n], [n - 1]) for r, n in shares]
+        got = runner.step(entries).float().cpu().numpy()
+        for (r, n), row in zip(shares, got):
+            done[r] += n
+            assert close(row, want[r][done[r] - 1]) < 2e-4, (shares, r)
+
+    step([("a", 60), ("b", 60)])
+    before = len(runner._graphs)
+    for shares in ([("c", 200), ("a", 1), ("b", 1)], [("a", 1), ("d", 196), ("b", 1)], [("e", 12), ("f", 222), ("b", 5)], [("g", 195), ("h", 3), ("a", 40)]):
+        step(shares)
+    assert len(runner._graphs) - before == 1 and runner.graph_steps > 0
+    step([("h", 90), ("a", 70), ("b", 50)])                                      # the same padded sizes, no request long enough
+    assert len(runner._graphs) - before == 2
+    runner.check_status()
+
+
 def test_which_sizes_take_chunks():
     """The rule of the entry point: scratch for the sizes that are served, none for others (the library answers without a device)."""
     import ctypes
@@ -173,8 +289,19 @@ def test_which_sizes_take_chunks():
 
     f = build.load("recurrence").spy_scan_chunk_floats
     f.restype = ctypes.c_longlong
-    assert f(0, 96, 1, 8, 128, 256) > 0 and f(2, 2000, 8, 16, 128, 256) > 0 and f(1, 2047, 1, 32, 64, 64) > 0
-    assert f(0, 95, 1, 8, 128, 256) == 0 and f(0, 96, 1, 8, 96, 256) == 0 and f(0, 96, 1, 8, 128, 250) == 0 and f(1, 128, 1, 8, 128, 128) == 0
-    assert f(0, 480, 10, 8, 128, 256) > 0 and f(0, 479, 10, 8, 128, 256) == 0                     # short requests on average
-    assert f(1, 3000, 2, 32, 64, 64) > 0 and f(1, 3000, 3, 32, 64, 64) == 0                       # enough pairs for the walk by tokens
-    assert f(0, 1 << 19, 1, 8, 128, 256) == 0                                                     # more scratch than the limit
+    # (mode, tokens, long requests, the longest, heads, dk, dv); one long request from 112, 128 and 192 tokens on, two from 96, 128 and 160
+    assert f(0, 112, 1, 112, 8, 128, 256) > 0 and f(2, 2000, 8, 400, 16, 128, 256) > 0 and f(1, 2047, 1, 2047, 32, 64, 64) > 0
+    assert f(0, 111, 1, 111, 8, 128, 256) == 0 and f(0, 192, 2, 96, 8, 128, 256) > 0 and f(2, 191, 1, 191, 16, 128, 256) == 0 and f(2, 320, 2, 160, 16, 128, 256) > 0
+    assert f(0, 112, 1, 112, 8, 96, 256) == 0 and f(0, 112, 1, 112, 8, 128, 250) == 0 and f(1, 128, 1, 128, 8, 128, 128) == 0
+    assert f(0, 8000, 0, 95, 8, 128, 256) == 0 and f(0, 8000, 1, 1000, 8, 128, 256) > 0           # short requests, many or beside a long one
+    assert f(1, 3000, 2, 1000, 16, 64, 64) > 0 and f(1, 3000, 2, 1000, 32, 64, 64) == 0           # enough pairs for the walk by tokens
+    assert f(0, 1 << 19, 1, 1 << 19, 8, 128, 256) == 0                                            # more scratch than the limit
+    assert f(0, 4096, 1, 4096, 1, 64, 16 * 65536) == 0                                            # more columns than a grid takes
+    # places run with a request's first token: those of long requests never meet, whatever lies ahead of them
+    for mode, least, C, place in ((0, 96, 64, lambda t: 3 * t // 128), (1, 128, 32, lambda t: 5 * t // 128), (2, 160, 64, lambda t: 4 * t // 192)):
+        assert build.load("recurrence").spy_scan_chunk_min(mode) == least
+        for n in range(least, least + 4 * C + 1):
+            assert all(place(t + n) - place(t) >= -(-n // C) for t in range(384))
+        for T in (256, 1000, 4097):
+            per_place = 2 * (f(mode, T, 1, T, 2, 64, 64) // (2 * place(T)))
+            assert f(mode, T, 1, T, 2, 64, 64) == per_place * place(T)
