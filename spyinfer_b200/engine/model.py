@@ -163,6 +163,10 @@ class Model:
             self._choosing = list({(type(p), p.choice_sizes()): p for part in self.parts() for p in part.choosing()}.values())
         return tuple(p.choice(batch, page_size) for p in self._choosing)
 
+    def scratch_bytes(self, step_tokens: int) -> int:
+        """The most that any part takes for a while in a step of this many tokens (``Part.scratch_bytes``)."""
+        return max(p.scratch_bytes(step_tokens) for p in self.parts())
+
     # ---- cache needs -------------------------------------------------------------------------
     def cache_needs(self):
         """Per run-order entry: its mixer's need, and the entry whose cache it reads instead."""

@@ -111,7 +111,8 @@ class ModelRunner:
                     size *= int(d)
                 states += (cfg.max_num_seqs + 1) * size
         free, total = torch.cuda.mem_get_info(self.device)
-        budget = free - int(total * (1.0 - cfg.gpu_memory_utilization)) - (2 << 30) - fixed - states  # room for activations
+        scratch = self.model.scratch_bytes(step)                                                     # of one part at a time, in a step of prompts
+        budget = free - int(total * (1.0 - cfg.gpu_memory_utilization)) - (2 << 30) - scratch - fixed - states  # room for activations
         pages = budget // per_page
         most = cfg.max_num_seqs * ((cfg.max_model_len + page - 1) // page)
         if pages <= 0:

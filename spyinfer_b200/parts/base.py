@@ -123,6 +123,10 @@ class Part:
         """What the batch's content decides: a word for it, empty for what is usual."""
         raise NotImplementedError
 
+    def scratch_bytes(self, step_tokens: int) -> int:
+        """Device memory that a step of this many tokens takes for a while beside its activations."""
+        return 0
+
     def linears(self) -> List:
         """The part's ``Linear`` products in the order ``forward`` runs them (the model tells each
         which weight is read next, so that it can ask for it ahead of time)."""

@@ -59,6 +59,9 @@ class ParallelMixers(Mixer):
     def choosing(self):
         return self.left.choosing() + self.right.choosing()
 
+    def scratch_bytes(self, step_tokens):
+        return max(self.left.scratch_bytes(step_tokens), self.right.scratch_bytes(step_tokens))
+
     def linears(self):
         return self.left.linears() + self.right.linears()
 

@@ -57,6 +57,9 @@ class _Recurrent(Mixer):
         count, longest = batch.runs(kernels.scan_chunk_min(self.chunks))
         return self.chunks + " in chunks" if count > 0 and kernels.scan_chunk_floats(self.chunks, batch.num_tokens, count, longest, *self.sizes) > 0 else ""
 
+    def scratch_bytes(self, step_tokens):
+        return 4 * kernels.scan_chunk_floats(self.chunks, step_tokens, 1, step_tokens, *self.sizes) if self.chunks is not None else 0
+
     def _runs(self, batch):
         """What the scan kernels are told of a batch's requests."""
         if batch.one_token_each:

@@ -305,3 +305,29 @@ def test_which_sizes_take_chunks():
         for T in (256, 1000, 4097):
             per_place = 2 * (f(mode, T, 1, T, 2, 64, 64) // (2 * place(T)))
             assert f(mode, T, 1, T, 2, 64, 64) == per_place * place(T)
+
+
+def test_the_page_pool_leaves_room_for_the_chunks_scratch(monkeypatch):
+    """A pool sized from the free memory (told by a stand-in): with steps of so many tokens that the linear attention's chunks need some hundred MB, the
+    pool is smaller by as much."""
+    from spyinfer_b200 import config_from_json, kernels
+    from spyinfer_b200.config import EngineConfig
+    from spyinfer_b200.engine.model import Model
+    from spyinfer_b200.engine.runner import ModelRunner
+
+    cfg = {"architecture": "Daronex", "vocab": 211, "width": 128, "norm": {"eps": 1e-6}, "logit_scale": 1.0, "layers": [
+        {"type": "latent_attention", "mlp": None, "mixer": {"heads": 2, "dim": 16, "rot_dim": 8, "vdim": 24, "q_rank": 24, "kv_rank": 24, "scale": 0.3,
+                                                            "rot": {"base": 500.0, "dims": 8}}},
+        {"type": "gla", "mlp": None, "mixer": {"heads": 8, "dim": 128, "vdim": 256, "tau": 16.0, "decay_rank": 8}}]}
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (60 << 30, 180 << 30))
+    pages = {}
+    for tokens in (100, 16384):
+        config = EngineConfig(dtype="float32", kvcache_block_size=16, max_num_seqs=64, max_model_len=1 << 24, max_num_batched_tokens=tokens)
+        runner = object.__new__(ModelRunner)
+        runner.model, runner.config, runner.device = Model(config_from_json(cfg).to_spec(), torch.float32, None, 1 << 24), config, None
+        needs, _ = runner.model.cache_needs()
+        pages[tokens] = runner._pages_from_free_memory(needs)
+    per_page = 16 * 32 * 4
+    scratch = 4 * kernels.scan_chunk_floats("linear attention", 16384, 1, 16384, 8, 128, 256)
+    assert scratch > 50 << 20 and pages[100] < 64 * (1 << 20)                    # the free memory, not the requests, sets the pool
+    assert pages[100] - pages[16384] in (scratch // per_page, scratch // per_page + 1)
