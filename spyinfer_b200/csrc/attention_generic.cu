@@ -591,8 +591,8 @@ attention_rows_kernel(const TA* __restrict__ q, TA* __restrict__ out, const TC* 
 // keys' quads and four queries' for as many, and in the value sums a quad of probabilities and one of values for 16, so that the multiply-adds
 // are what is left, and a block's keys and values serve twice the rows.  Every sum runs in the same order as above: the bits are the same.
 // Measured with the merge, 32 heads over 8 of 128, 32-bit, kernel above with 16 rows / this one (us): prompts of 150 tokens 52 / 40, of 300 95 / 66, of 600
-// 286 / 178, of 2,000 2,266 / 1,405; 64 tokens behind 2,000 183 / 113; 8 of 100 115 / 76.  What is left beside the multiply-adds (18 us of the 300
-// tokens' 66): a block's copies, maxima and sums wait for one another, and two blocks an SM are what shared memory holds.
+// 286 / 178, of 2,000 2,266 / 1,405; 64 tokens behind 2,000 183 / 113; 8 of 100 115 / 76.  What is left beside the multiply-adds (the FMA pipes are busy for 14 us
+// of the 300 tokens' 66, 20 on the busiest SM): a block's copies, maxima and sums wait for one another, and two blocks an SM are what shared memory holds.
 constexpr int WIDE_ROWS = 32, WIDE_THREADS = 256, WIDE_PLD = WIDE_ROWS + 4;
 
 // v[0..4) over the eight lanes whose numbers differ in their lowest three bits; the result is row `*row`'s in lanes whose `*row` is not negative.

@@ -760,8 +760,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
 // nearly equal height (TokenTiles), where whole tiles of 256 tokens in the M slot multiplied up to 255 rows
 // of nothing and fetched the weights once more for them.  What bounds the loop is the tiles' way from L2 to the
 // SMs (11 to 11.7 TB/s whatever the height), so the gain is what the lower tiles need not fetch.  Four products of a layer (us; 256-token
-// tiles in the M slot, then these): 8B sizes, 129 tokens 111 -> 93, 192 113 -> 98, 257 151 -> 142, 513 227 -> 213, 576 229 -> 217, 769 276 ->
-// 260, 1,025 343 -> 326, 2,048 538 -> 539; 14B sizes, 576 366 -> 331, 800 475 -> 436, 1,300 672 -> 638, 1,548 776 -> 742.
+// tiles in the M slot, then these): 8B sizes, 129 tokens 127 -> 105, 192 128 -> 110, 257 173 -> 157, 513 266 -> 247, 576 253 -> 235, 769 285 ->
+// 267, 1,025 367 -> 344, 2,048 569 -> 549; 14B sizes, 576 409 -> 362, 800 491 -> 448, 1,300 703 -> 659, 1,548 852 -> 802.
 // Barriers: the TMA loads of
 // both blocks complete on the LEADER's full barrier (no multicast of data; the barrier operand is
 // the leader's, which cta_group::2 loads allow); a commit with cluster multicast frees a stage,

@@ -578,9 +578,9 @@ __global__ void __launch_bounds__(THREADS, NR <= 16 ? 4 : 1) scan_decode_kernel(
 //
 // Two kernels: chunk_*_kernel makes these factors, a block a (chunk, head), all chunks side by side; walk_*_kernel carries S through a
 // request's chunks, a block 16 value columns of a (request, head).  What bounds the walk is the way through a chunk on eight warps (a chunk of
-// 64 tokens at 128 x 16 takes 4.5 us, its 330 K additions 1.4, its shared-memory reads about 2); the token-by-token kernel above
-// spends 270 to 300 ns a token on one request, nearly all of it waiting.  Measured, chunks' kernels and walk together (us, by tokens before / in chunks):
-//   matrix memory, 8 heads of 128 x 256: one request of 256 tokens 76 / 38, of 2,047 567 / 176; 8 of 100 to 400 460 / 233; 16 of 1,024 2,581 / 1,495;
+// 64 tokens at 128 x 16 takes 4.7 us; the counters show shared memory busy for 64 % of the time and the FMA pipes for 33); the token-by-token kernel above
+// spends 270 to 300 ns a token on one request, nearly all of it waiting.  Measured, chunks' kernels and walk together (us, by tokens / in chunks):
+//   matrix memory, 8 heads of 128 x 256: one request of 256 tokens 76 / 38, of 2,047 570 / 179; 8 of 100 to 400 417 / 212; 16 of 1,024 2,585 / 1,523;
 //   delta rule, 32 heads of 64: one request of 256 79 / 50, of 2,047 610 / 351; 16 heads 80 / 49 and 614 / 250;
 //   linear attention, 16 heads of 128 x 256: one of 256 103 / 71, of 2,047 777 / 378; 8 of 100 to 400 632 / 445; 16 of 1,024 4,109 / 2,988.
 // Error against 64 bits, tokens / chunks, 2,047 tokens (2-norm; matrix memory: the median token's): matrix memory of 128 x 48 1.85e-7 / 1.12e-7, linear attention 1.73e-7 /

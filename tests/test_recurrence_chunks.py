@@ -197,6 +197,22 @@ def test_long_requests_anywhere_among_short_ones_take_the_same_chunks(kind, dk, 
 
 
 @gpu
+@pytest.mark.parametrize("kind,dk,dv,heads", [("linear", 128, 256, 16), ("delta", 64, 64, 32)])
+def test_chunks_of_many_heads_are_the_walks_by_tokens(kind, dk, dv, heads, monkeypatch):
+    """The heads of the large layers: every head and column tile, against the walk by tokens (whose distance from 64 bits is the same)."""
+    monkeypatch.setitem(globals(), "HEADS", heads)
+    x, pre, b1, b2 = inputs(kind, dk, dv, 300, 7)
+    states, outs = [], []
+    for pad in (0, 1):
+        state = new_state(kind, dk, dv, 1)
+        outs.append(run(kind, dk, dv, [x], [pre], b1, b2, state, [0], pad))
+        states.append(state.cpu())
+    assert not torch.equal(outs[0], outs[1])
+    for a, b in (outs, states):
+        assert float((a - b).norm() / b.norm()) < 4e-7                        # the two forms' distances from 64 bits, 1.7e-7 each at most
+
+
+@gpu
 @pytest.mark.parametrize("kind", ["memory", "linear", "delta"])
 def test_a_step_without_long_requests_asks_for_no_scratch(kind):
     from spyinfer_b200 import kernels
