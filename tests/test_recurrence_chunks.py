@@ -263,7 +263,7 @@ def test_models_take_chunks_whole_in_portions_and_replayed_beside_replies(design
     model.bind({k: v.cuda() for k, v in weights.items()})
     runner = ModelRunner(model, config)
     rng = np.random.default_rng(5)
-    tokens = {r: rng.integers(0, 211, 240).tolist() for r in "abcdefgh"}
+    tokens = {r: rng.integers(0, 211, 340 if r in "ij" else 240).tolist() for r in "abcdefghij"}
     want = {r: plain.forward(weights, cfg, t).numpy() for r, t in tokens.items()}
 
     def close(got, ref):
@@ -294,6 +294,15 @@ def test_models_take_chunks_whole_in_portions_and_replayed_beside_replies(design
     assert len(runner._graphs) - before == 1 and runner.graph_steps > 0
     step([("h", 90), ("a", 70), ("b", 50)])                                      # the same padded sizes, no request long enough
     assert len(runner._graphs) - before == 2
+    for r in "abcdefgh":
+        runner.finish(r)
+    # one portion alone, too short to take chunks by itself, the next as long beside another that is: the other form goes on from the state
+    n = 100 if design == "nezolorn" else 165
+    assert not any(model.choices(runner.build_batch([StepEntry("i", tokens["i"][:n], [])]), 16))
+    step([("i", n)])
+    assert any(model.choices(runner.build_batch([StepEntry("i", tokens["i"][n:2 * n], []), StepEntry("j", tokens["j"][:n], [])]), 16))
+    step([("i", n), ("j", n)])
+    step([("i", 10), ("j", 1)])
     runner.check_status()
 
 
